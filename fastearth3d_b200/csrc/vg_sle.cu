@@ -915,7 +915,9 @@ void update_dev(vg_handle* h, const double* d_ice1, double dt_yr) {
       }
       double fac = errsc <= 0.0 ? p.grow_max : p.safety * std::pow(errsc, -expo);
       fac = std::min(p.grow_max, std::max(p.shrink_min, fac));
-      h->dt_try = std::min(p.dt_max, std::max(p.dt_min, dts * fac));
+      // carried as a value that survives seconds -> years -> seconds (one round trip reaches it), so that a run
+      // restarted from vg_get_step_state continues with the same step
+      h->dt_try = std::min(p.dt_max, std::max(p.dt_min, dts * fac)) / SEC_PER_YEAR * SEC_PER_YEAR;
       if (h->dt_try <= 1.0e-12 * span)
         throw Error("vilma_timestep: implicit adaptive step collapsed (tolerance unreachable)");
     }
@@ -973,6 +975,7 @@ void update_dev(vg_handle* h, const double* d_ice1, double dt_yr) {
   k_zbed<<<eg, eb, 0, s>>>(ng, h->d_z_bed_eq.p, h->d_rsl.p, h->d_zbed.p); ++h->n_launch;
   VG_CUDA(cudaGetLastError());
   h->time_yr += dt_yr;
+  h->time_s = h->time_yr * SEC_PER_YEAR;  // not the sub-steps' sum: a restart's clock (seconds) gives time_yr back
   update_bsl(h);
 }
 
