@@ -146,7 +146,6 @@ int vg_create(const vg_params* p, vg_handle** out) {
     VG_CUDA(cudaStreamCreateWithFlags(&h->aux, cudaStreamNonBlocking));
     VG_CUDA(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
     VG_CUDA(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
-    VG_CUDA(cudaStreamCreateWithFlags(&h->aux2, cudaStreamNonBlocking));
     VG_CUDA(cudaEventCreateWithFlags(&h->ev_dfork, cudaEventDisableTiming));
     VG_CUDA(cudaEventCreateWithFlags(&h->ev_djoin, cudaEventDisableTiming));
     vg::setup_handle(h);
@@ -167,14 +166,12 @@ int vg_destroy(vg_handle* h) {
   if (!h) return 0;
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->aux) cudaStreamSynchronize(h->aux);
-  if (h->aux2) cudaStreamSynchronize(h->aux2);
   if (h->h_sc) cudaFreeHost(h->h_sc);
-  cudaStream_t s = h->stream, a = h->aux, a2 = h->aux2;
+  cudaStream_t s = h->stream, a = h->aux;
   cudaEvent_t ev[4] = {h->ev_fork, h->ev_join, h->ev_dfork, h->ev_djoin};
   delete h;
   for (cudaEvent_t e : ev)
     if (e) cudaEventDestroy(e);
-  if (a2) cudaStreamDestroy(a2);
   if (a) cudaStreamDestroy(a);
   if (s) cudaStreamDestroy(s);
   return 0;

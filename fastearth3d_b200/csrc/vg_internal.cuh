@@ -129,14 +129,10 @@ struct vg_handle {
   // into an error (vg_set_wait_limit)
   unsigned long long wait_ns = 2000000000ull;
   cudaStream_t stream = nullptr;
-  // second stream: the degree-1 drift (one CTA) runs there beside the band
-  // sweeps of degrees >= 2, forked after the forcing and joined before the
-  // drift is read
+  // second stream: the spectral memory advance beside the 3-D pass, and the
+  // drift beside the sea-level pass setup, joined before the fused loop reads it
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  // the whole drift on the second stream (its degree 1 on a third) beside the
-  // sea-level pass setup, joined before the fused loop reads it
-  cudaStream_t aux2 = nullptr;
   cudaEvent_t ev_dfork = nullptr, ev_djoin = nullptr;
   // sizes
   int nr = 0, ne = 0, ndof = 0, nk = 0, ne3d = 0;
@@ -154,6 +150,7 @@ struct vg_handle {
   vg::DArr<double> d_ab, d_dr, d_dc, d_rdiag;  // degrees 2..lmax (band, column-major, ldab 19)
   vg::DArr<int> d_ipiv;
   vg::DArr<double> d_ab1, d_dr1, d_dc1, d_null1, d_G1;  // degree 1 (bordered, dense band)
+  vg::DArr<double> d_lrec, d_urec;              // the band factors as the drift sweeps read them (vg_sweep.cuh)
   vg::DArr<double> d_bh;                        // equilibrated drift RHS (2, 2*nr, nk)
   vg::DArr<double> d_Krhs;                      // dissipative-forcing coefficients (lmax+1, ne, 48)
   vg::DArr<int4> d_tasks;                       // drift sweep tasks: (degree, first slot, slots)
@@ -237,7 +234,8 @@ struct vg_handle {
   vg::DArr<double> d_rot_mem;   // memory [ch][A re, A im, B re, B im, C re, C im][ne][4]
   vg::DArr<double> d_rot_dn;    // nodal drift [ch][dUn re, dUn im, dVn re, dVn im][nr]
   vg::DArr<double> d_rot_sc;    // scalars (see vg_rotation.cu)
-  vg::DArr<double> d_rot_f;     // channel solve work (4 x ndof)
+  vg::DArr<double> d_rot_f;     // channel forcing at the U and V dofs [2 nr][4] (setup: 3 x ndof of work)
+  vg::DArr<double> d_rot_y;     // channel solve scratch (vg_sweep.cuh)
   vg::DArr<double> d_rot_fl;    // channel element contributions (4 x ne x 4)
   vg::DArr<double> d_rot_rows;  // per-row partial inertia sums (2 x nlat)
   vg::DArr<double> d_rot_geo;   // sin(theta)cos(theta) [nlat], cos(lon), sin(lon) [nphi each]
@@ -263,8 +261,8 @@ void build_grid(Grid& G, int lmax, int nlat, int nphi, cudaStream_t s);
 // drift of memory buffer buf (-1: the current one) into the nodal targets
 // (nullptr: the handle's dUn, dVn) and the surface drift
 void launch_drift(vg_handle* h, int buf = -1, double* dUn = nullptr, double* dVn = nullptr, double* dWn = nullptr);
-// the same without the toroidal drift, the band sweeps on s0 and degree 1 on s1
-void launch_drift_on(vg_handle* h, int buf, double* dUn, double* dVn, cudaStream_t s0, cudaStream_t s1);
+// the same without the toroidal drift, on stream s
+void launch_drift_on(vg_handle* h, int buf, double* dUn, double* dVn, cudaStream_t s);
 // memory advance of one step (3-D elements pseudo-spectrally, the others per
 // slot), current buffer -> the other one, with the strain of (sigma, dUn,
 // dVn) (nullptr: the handle's drift), and the next buffer's per-slot norms and

@@ -25,6 +25,7 @@
 
 #include "vg_device.cuh"
 #include "vg_internal.cuh"
+#include "vg_sweep.cuh"
 
 namespace vg {
 
@@ -35,9 +36,9 @@ struct RotArgs {
   int ne, nr, nd, nlat, nphi;
   const double *r, *mu, *mkdt, *x;    // x: unit responses [ch][U, V][nr]
   const double *sa, *sb, *sc, *nrm;  // degree-2 strain constants (16, 16, 16, 4)
-  const double *ab, *dr, *dc;        // degree-2 band factor (equilibrated)
-  const int* ipiv;
+  const double *lrec, *urec, *dr;    // degree-2 band factor's sweep records, row scales
   double *mem, *dn, *scal, *f, *fl;  // fl: element contributions [4][ne][4]
+  double* y;                         // sweep scratch
 };
 
 // channel_begin of both channels (src/vilma_rotation.f90:442-463): the
@@ -50,12 +51,12 @@ struct RotArgs {
 //   k_rot_begin  one block: the nodal forcing of the four right-hand sides
 //                (node n: element n-1's second test dof, then element n's
 //                first, as the serial loop adds them) times the row scales,
-//                the degree-2 band factor and its pivots staged in shared
-//                memory when they fit (rot_smem below), one thread per
-//                right-hand side for the sequential sweeps with their active
-//                window in registers (band_solve_window), then the column
-//                scales and the outputs.
-// The arithmetic and its order are the reference's throughout.
+//                then one warp, a lane per right-hand side, runs the band
+//                sweeps of vg_sweep.cuh on the degree-2 records and writes the
+//                scaled outputs. Two sequential recurrences over the dofs of
+//                four right-hand sides bound it: a thread each with operands
+//                loaded one step ahead and a division per column took 120 us
+//                at 100 elements (403 dofs).
 constexpr int ROT_THREADS = 256;
 constexpr int ROT_ELEM_THREADS = 64;
 
@@ -89,58 +90,34 @@ __global__ void __launch_bounds__(ROT_ELEM_THREADS) k_rot_elem(RotArgs A) {
   for (int tt = 0; tt < 4; ++tt) A.fl[((size_t)q * ne + e) * 4 + tt] = floc[tt];
 }
 
-__global__ void __launch_bounds__(ROT_THREADS) k_rot_begin(RotArgs A, int staged) {
-  extern __shared__ double rsm[];
+__global__ void __launch_bounds__(ROT_THREADS) k_rot_begin(RotArgs A) {
+  __shared__ __align__(16) double rsm[sw::SMEM];
   const int t = threadIdx.x;
-  const int ne = A.ne, nr = A.nr, nd = A.nd;
-  const double* sfl = A.fl;  // [4][ne][4] element contributions
-  const double* ab = A.ab;
-  const int* ipiv = A.ipiv;
-  double* fbase = A.f;
-  if (staged) {
-    double* sab = rsm;                                       // [nd][VG_LDAB]
-    double* sf = sab + (size_t)nd * VG_LDAB;                 // [4][nd]
-    int* sip = reinterpret_cast<int*>(sf + (size_t)4 * nd);  // [nd]
-    for (int i = t; i < nd * VG_LDAB; i += blockDim.x) sab[i] = A.ab[i];
-    for (int i = t; i < nd; i += blockDim.x) sip[i] = A.ipiv[i];
-    ab = sab;
-    ipiv = sip;
-    fbase = sf;
-  }
-  __syncthreads();
+  const int ne = A.ne, nr = A.nr;
   // the nodal forcing of the four right-hand sides times the row scales
-  for (int w = t; w < 4 * nd; w += blockDim.x) {
-    const int q = w / nd, i = w % nd, n = i >> 2, c = i & 3;
-    const double* fl = sfl + (size_t)q * ne * 4;
+  for (int w = t; w < 8 * nr; w += blockDim.x) {
+    const int q = w & 3, i = w >> 2, n = i >> 1, c = i & 1;
+    const double* fl = A.fl + (size_t)q * ne * 4;
     double u = 0.0;
-    if (c < 2 && n < nr) {
-      if (n >= 1) u += fl[(n - 1) * 4 + (c == 0 ? 1 : 3)];
-      if (n < ne) u += fl[n * 4 + (c == 0 ? 0 : 2)];
+    if (n >= 1) u += fl[(n - 1) * 4 + (c == 0 ? 1 : 3)];
+    if (n < ne) u += fl[n * 4 + (c == 0 ? 0 : 2)];
+    A.f[w] = A.dr[4 * n + c] * u;
+  }
+  __threadfence_block();
+  __syncthreads();
+  if (t >= 32) return;
+  const int q = t & 3, ch = q >> 1, ri = q & 1;  // lanes past the fourth repeat the four
+  double* dn = A.dn + (size_t)ch * 4 * nr;
+  const int base = (ch == 0 ? RS_DF_LOAD : RS_DF_TID) + ri;
+  sw::band_sweeps(A.lrec, A.urec, nr, A.f + q, 4, A.y, rsm, t, [&](int node, double U, double V, double F) {
+    if (t >= 4) return;
+    dn[(size_t)(0 + ri) * nr + node] = U;  // dUn
+    dn[(size_t)(2 + ri) * nr + node] = V;  // dVn
+    if (node == nr - 1) {
+      A.scal[base] = F;      // dF
+      A.scal[base + 2] = U;  // dU
     }
-    fbase[(size_t)q * nd + i] = A.dr[i] * u;
-  }
-  __syncthreads();
-  if (t < 4) band_solve_window<6, 12>(ab, VG_LDAB, nd, ipiv, fbase + (size_t)t * nd);
-  __syncthreads();
-  for (int w = t; w < 4 * nd; w += blockDim.x) {
-    const int i = w % nd;
-    fbase[w] = A.dc[i] * fbase[w];
-  }
-  __syncthreads();
-  if (t < 4) {
-    const int ch = t >> 1, ri = t & 1;
-    const double* f = fbase + (size_t)t * nd;
-    const int base = ch == 0 ? RS_DF_LOAD : RS_DF_TID;
-    A.scal[base + ri] = f[4 * (nr - 1) + 2];  // dF
-    A.scal[base + 2 + ri] = f[4 * (nr - 1)];  // dU
-  }
-  for (int w = t; w < 4 * nr; w += blockDim.x) {
-    const int q = w / nr, node = w % nr, ch = q >> 1, ri = q & 1;
-    const double* f = fbase + (size_t)q * nd;
-    double* dn = A.dn + (size_t)ch * 4 * nr;
-    dn[(size_t)(0 + ri) * nr + node] = f[4 * node];      // dUn
-    dn[(size_t)(2 + ri) * nr + node] = f[4 * node + 1];  // dVn
-  }
+  });
 }
 
 // s_rot = N_rot - u_rot (src/vilma_rotation.f90:192-222) from the current m and
@@ -261,7 +238,7 @@ __global__ void k_rot_unit(int nr, int nd, double r_earth, double g_surf, const 
     x[fs] = -r_earth / (4.0 * PI * GRAV_G) * 5.0 * 1.0;
   }
   for (int i = 0; i < nd; ++i) x[i] = R_[i] * x[i];
-  band_solve_strided(A_, VG_LDAB, nd, 6, 12, P_, x, 1);
+  band_solve_window<6, 12>(A_, VG_LDAB, nd, P_, x);
   for (int i = 0; i < nd; ++i) x[i] = C_[i] * x[i];
   surf[t * 2 + 0] = x[fs];  // F(a)
   surf[t * 2 + 1] = x[us];  // U(a)
@@ -287,15 +264,15 @@ static RotArgs rot_args(vg_handle* h) {
   A.sb = h->d_sb.p + 2 * 16;
   A.sc = h->d_sc.p + 2 * 16;
   A.nrm = h->d_nrmc.p + 2 * 4;
-  A.ab = h->d_ab.p;  // degree 2 is the first band record
+  A.lrec = h->d_lrec.p;  // degree 2 is the first band factor
+  A.urec = h->d_urec.p;
   A.dr = h->d_dr.p;
-  A.dc = h->d_dc.p;
-  A.ipiv = h->d_ipiv.p;
   A.mem = h->d_rot_mem.p;
   A.dn = h->d_rot_dn.p;
   A.scal = h->d_rot_sc.p;
   A.f = h->d_rot_f.p;
   A.fl = h->d_rot_fl.p;
+  A.y = h->d_rot_y.p;
   return A;
 }
 
@@ -319,7 +296,8 @@ void rotation_setup(vg_handle* h) {
   h->d_rot_mem.alloc((size_t)2 * 6 * ne * 4);
   h->d_rot_dn.alloc((size_t)2 * 4 * nr);
   h->d_rot_sc.alloc(RS_N);
-  h->d_rot_f.alloc((size_t)4 * nd);
+  h->d_rot_f.alloc(std::max((size_t)8 * nr, (size_t)3 * nd));
+  h->d_rot_y.alloc(sw::scratch(nr));
   h->d_rot_fl.alloc((size_t)16 * ne);
   h->d_rot_rows.alloc((size_t)2 * G.nlat);
   h->d_srot.alloc(G.ng);
@@ -356,32 +334,16 @@ void rotation_setup(vg_handle* h) {
   h->rot_on = true;
 }
 
-// rotation_begin_step (src/vilma_rotation.f90:154-168): drift of both channels
-// shared memory of k_rot_begin
-// (the element contributions always; the band, pivots and right-hand sides
-// when they fit; `staged` says which)
-static size_t rot_smem(const vg_handle* h, int& staged) {
-  const size_t b = (size_t)h->ndof * VG_LDAB * sizeof(double) + (size_t)4 * h->ndof * sizeof(double) +
-                   (size_t)h->ndof * sizeof(int);
-  staged = b <= 200 * 1024 ? 1 : 0;
-  const size_t need = staged ? b : 0;
-  if (need > 48 * 1024) raise_smem_limit((const void*)k_rot_begin, need);
-  return need;
-}
-
 // the drift of both channels from the entering memory
-static void rot_begin_launch(vg_handle* h, const RotArgs& A, size_t sm, int staged, cudaStream_t s) {
+// (rotation_begin_step, src/vilma_rotation.f90:154-168)
+static void rot_begin_launch(vg_handle* h, const RotArgs& A, cudaStream_t s) {
   k_rot_elem<<<(4 * A.ne + ROT_ELEM_THREADS - 1) / ROT_ELEM_THREADS, ROT_ELEM_THREADS, 0, s>>>(A);
-  k_rot_begin<<<1, ROT_THREADS, sm, s>>>(A, staged);
+  k_rot_begin<<<1, ROT_THREADS, 0, s>>>(A);
   h->n_launch += 2;
   VG_CUDA(cudaGetLastError());
 }
 
-void rotation_begin(vg_handle* h) {
-  int staged = 0;
-  const size_t sm = rot_smem(h, staged);
-  rot_begin_launch(h, rot_args(h), sm, staged, h->stream);
-}
+void rotation_begin(vg_handle* h) { rot_begin_launch(h, rot_args(h), h->stream); }
 
 // the rotational sea-level term held across the interval
 void rotation_s_rot(vg_handle* h) {
@@ -418,10 +380,8 @@ void rotation_advance(vg_handle* h, const double* d_sigma, double dt) {
   S.w = G.d_wts.p;
   S.rows = h->d_rot_rows.p;
   const RotArgs A = rot_args(h);
-  int staged = 0;
-  const size_t sm = rot_smem(h, staged);
   for (int k = 0; k < n_sub; ++k) {
-    rot_begin_launch(h, A, sm, staged, s);
+    rot_begin_launch(h, A, s);
     k_rot_solve_commit<<<1, 256, 0, s>>>(A, S);
     ++h->n_launch;
     VG_CUDA(cudaGetLastError());

@@ -9,6 +9,7 @@
 
 #include "vg_device.cuh"
 #include "vg_internal.cuh"
+#include "vg_sweep.cuh"
 
 namespace vg {
 
@@ -333,6 +334,17 @@ __global__ void k_build_band(ElemData ed, int lmax, double* __restrict__ raw, do
     A[(size_t)j * ldab + 20] = (double)(ipiv[(size_t)(l - 2) * n + j] - j);
     rdg[(size_t)(l - 2) * n + j] = A[(size_t)j * ldab + 19];
   }
+}
+
+// The factors as the sweeps read them (vg_sweep.cuh), one thread per (degree,
+// node); zero past the last node.
+__global__ void k_sweep_records(int nr, int nd, const double* __restrict__ ab, const double* __restrict__ dc,
+                                double* __restrict__ lrec, double* __restrict__ urec) {
+  const int n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= nr) return;
+  sw::node_records(ab + (size_t)blockIdx.y * VG_LDAB * nd, VG_LDAB, dc + (size_t)blockIdx.y * nd, nd, n,
+                   lrec + blockIdx.y * sw::lrec_size(nr) + (size_t)n * sw::LN,
+                   urec + blockIdx.y * sw::urec_size(nr) + (size_t)n * sw::UN);
 }
 
 // Degree 1: band part plus the KKT border w (E_uniq weight, src/vilma_radial_fe.f90:425-443,
@@ -820,6 +832,11 @@ void setup_handle(vg_handle* h) {
   k_build_band<<<(lmax - 1 + 31) / 32, 32, 0, s>>>(ed, lmax, raw.p, h->d_ab.p, h->d_dr.p, h->d_dc.p, h->d_ipiv.p,
                                                     h->d_rdiag.p, status.p);
   VG_CUDA(cudaGetLastError());
+  h->d_lrec.alloc((size_t)(lmax - 1) * sw::lrec_size(nr));
+  h->d_urec.alloc((size_t)(lmax - 1) * sw::urec_size(nr));
+  k_sweep_records<<<dim3((nr + 31) / 32, lmax - 1), 32, 0, s>>>(nr, nd, h->d_ab.p, h->d_dc.p, h->d_lrec.p,
+                                                              h->d_urec.p);
+  VG_CUDA(cudaGetLastError());
   // degree 1 (bordered, dense)
   h->ns1 = nd + 1;
   h->kl1 = nd;
@@ -955,7 +972,7 @@ void setup_handle(vg_handle* h) {
   h->d_drift.alloc((size_t)6 * nk);
   h->d_mnorm.alloc((size_t)2 * nk);
   h->d_maxbits.alloc(3);  // two buffer norms + kernel status bits
-  h->d_xs.alloc((size_t)2 * nd * nk);
+  h->d_xs.alloc((size_t)h->ntask * sw::scratch(nr));
   h->d_bh.alloc((size_t)2 * 2 * nr * nk);
   h->d_sc_.alloc(1);
   VG_CUDA(cudaMallocHost(&h->h_sc, sizeof(SleScalars)));

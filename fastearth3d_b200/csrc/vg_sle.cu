@@ -763,7 +763,7 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
   if (drift_pending) {
     VG_CUDA(cudaEventRecord(h->ev_dfork, s));
     VG_CUDA(cudaStreamWaitEvent(h->aux, h->ev_dfork, 0));
-    launch_drift_on(h, h->cur, nullptr, nullptr, h->aux, h->aux2);
+    launch_drift_on(h, h->cur, nullptr, nullptr, h->aux);
     VG_CUDA(cudaEventRecord(h->ev_djoin, h->aux));
   } else {
     launch_drift(h);
