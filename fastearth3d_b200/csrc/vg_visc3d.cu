@@ -173,96 +173,326 @@ constexpr size_t v3_gather_smem() {
 // ------------------------------------------------------------------ GEMMs
 
 // Per-order batched FP64 products (the Legendre stage of the tensor transforms).
-//   mode 0 (synthesis): C[j][n] = sum_{kk < K_m} T_p[mbeg + kk][j] * X[row(m + kk, m)][col_p + n]
+//   MODE 0 (synthesis): C[j][n] = sum_{kk < K_m} T_p[mbeg + kk][j] * X[row(m + kk, m)][col_p + n]
 //                       -> S[((m * nlat + j) * np + p) * ncf + n]
-//   mode 1 (analysis):  C[i][n] = sum_{j} T_p[mbeg + i][j] * S[((m * nlat + j) * np + p) * ncf + n]
+//   MODE 1 (analysis):  C[i][n] = sum_{j} T_p[mbeg + i][j] * S[((m * nlat + j) * np + p) * ncf + n]
 //                       -> R[(row(m + i, m) * np + p) * ncf + n]
-// row(l, m) = kbeg[l] + m for l >= 1, the zero row nk for l = 0.
+// row(l, m) is the slot for l >= 1, the zero row nk for l = 0.
+//
+// The tables have the equatorial symmetry T(l, m; pi - theta) = sig_p (-1)^(l+m)
+// T(l, m; theta) (P, G even, dP/dtheta, H odd), so only the northern rows are
+// summed, the even and odd l + m apart: S_j = E + O, S_mirror = sig (E - O), and
+// in the analysis even (odd) degrees read S_j + (-) sig S_mirror. That halves
+// the work. The sums run on the FP64 matrix instructions (mma m8n8k4: the rate
+// of the FP64 units, 16 FMA a cycle and scheduler, but one operand word per
+// lane and 256 FMA), which keep that rate where register-tiled FMA loops were
+// bound by shared-memory loads and issue.
+// Tile: 4 warps, 64 columns (two 8-column groups a warp) x up to 40 northern
+// rows (40 degrees of each parity in the analysis), both parities: 20 pairs of
+// accumulators a thread, so that three CTAs fit an SM and one's copies, barriers
+// and epilogue run beside the others' products (72 rows and two CTAs: 168 us
+// against 149). K chunks are copied asynchronously three ahead, through the
+// products of the CTA without a break. lmax 128's 65 rows are two tiles of 40
+// and 25.
+// Bound: at lmax 128 with 54 elements 2.1 GFLOP with the symmetry, 2.6 with the
+// tiles' padding (70 us at the FP64 rate), and 346 MB (53 us). Measured 149 us
+// each way, 617 us before (64 x 64 tiles of FMA loops without the symmetry);
+// lmax 256: 3790 -> 880.
 struct GemmArgs {
-  int mode, lmax, nlat, nk, ncf;
+  int lmax, nlat, nk, ncf;
   int nin;  // synthesis input channels per slot row (4 or 6: the gathered channels; np: per product)
   int np;   // products: 6 (spheroidal) or 10 (with the toroidal channels)
-  const int *mbeg, *kbeg;
+  int rt;   // rows per row tile, a multiple of 8
+  int pg;   // products per CTA, a divisor of np
+  const int* mbeg;
   const double* T[10];  // per product: table [lm][j]
   int chan[10];         // synthesis: input channel per product
+  double sig[10];       // table's sign under theta -> pi - theta (times (-1)^(l+m))
   const double* in;
   double* out;
 };
 
-constexpr int GB_M = 64, GB_N = 64, GB_K = 8;
+constexpr int GB_N = 64, GB_R = 5, GB_RT = 8 * GB_R;  // columns, 8-row groups, rows of a CTA tile
+constexpr int GB_K0 = 16, GB_K1 = 8;                  // degrees (both parities), latitudes per chunk
+constexpr int GB_NST = 4;                             // chunk stages: copies run three chunks ahead
+constexpr int GB_PA0 = GB_RT + 2, GB_PB0 = GB_N + 2;  // pitches: 2 pitch = 4 mod 16 doubles, so that the four k of
+constexpr int GB_PA1 = GB_K1 + 2, GB_PB1 = GB_N + 4;  // one parity and four rows fall in distinct banks
+constexpr int GB_ST0 = GB_K0 * (GB_PA0 + GB_PB0);     // doubles per stage
+constexpr int GB_ST1 = 2 * GB_RT * GB_PA1 + 2 * GB_K1 * GB_PB1;
+static_assert((GB_K0 * GB_PA0) % 2 == 0 && (2 * GB_RT * GB_PA1) % 2 == 0, "16-byte copies into the B tiles");
 
-__device__ __forceinline__ int slot_row(const int* kbeg, int l, int m, int nk) { return l >= 1 ? kbeg[l] + m : nk; }
+// slot of (l, m): degrees 1 .. l - 1 hold 2 + .. + l slots
+__device__ __forceinline__ int slot_row(int l, int m, int nk) { return l >= 1 ? l * (l + 1) / 2 - 1 + m : nk; }
 
-__global__ void __launch_bounds__(256) k_v3_gemm(GemmArgs A) {
-  __shared__ double As[GB_K][GB_M + 1];
-  __shared__ double Bs[GB_K][GB_N];
-  const int m = blockIdx.z / A.np, p = blockIdx.z % A.np;
-  const int Km = A.lmax - m + 1;
-  const int rows = (A.mode == 0) ? A.nlat : Km;
-  const int kdim = (A.mode == 0) ? Km : A.nlat;
-  const int r0 = blockIdx.y * GB_M, n0 = blockIdx.x * GB_N;
-  if (r0 >= rows) return;
-  const double* T = A.T[p];
-  const int mb = A.mbeg[m];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 x 16 threads, 4 x 4 outputs each
-  double acc[4][4];
+__device__ __forceinline__ void cp_a16(double* dst, const double* src) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(src) : "memory");
+}
+// the same, zeros where !on (src is then not read; it points at valid memory all the same)
+__device__ __forceinline__ void cp_a8z(double* dst, const double* src, bool on) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(src), "r"(on ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_a16z(double* dst, const double* src, bool on) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+// c (8 x 8) += a (8 x 4) b (4 x 8), FP64; lane t holds a[t / 4][t % 4], b[t % 4][t / 4],
+// c[t / 4][2 (t % 4) + {0, 1}]
+__device__ __forceinline__ void dmma(double2& c, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c.x), "+d"(c.y)
+      : "d"(a), "d"(b));
+}
+
+// One CTA's tile with R row groups of 8 (a compile-time constant: a predicated
+// matrix instruction still takes its cycles).
+template <int MODE, int R>
+__device__ __forceinline__ void gemm_tile(const GemmArgs& A, double* gsm, int m, int p0, int r0, int n0, int nrow) {
+  constexpr int ST = MODE == 0 ? GB_ST0 : GB_ST1;
+  constexpr int KC = MODE == 0 ? GB_K0 : GB_K1;
+  const int Km = A.lmax - m + 1, nh = (A.nlat + 1) / 2;
+  const int kdim = MODE == 0 ? Km : nh;
+  const int mb = A.mbeg[m], nlat = A.nlat, ncf = A.ncf, np = A.np;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, lk = lane & 3;
+  const bool wact = n0 + warp * 16 < ncf;  // the last tile's idle warps only copy
+  const int nch = (kdim + KC - 1) / KC, nq = A.pg * nch;
+  const int bn = 2 * lane;  // this thread's two columns of a B row
+  const bool bon = n0 + bn < ncf;
+  const size_t rowB = MODE == 0 ? (size_t)A.nin * ncf : (size_t)np * ncf;
+  int sp = p0, sc = 0;  // product and chunk staged next
+  auto stage = [&](int q) {
+    if (q < nq) {
+      double* sA = gsm + (q % GB_NST) * ST;
+      const double* T = A.T[sp];
+      if (MODE == 0) {
+        // degrees warp, warp + 4, ..; lanes along the latitudes, then the columns
+        double* dA = sA + warp * GB_PA0 + lane;
+        double* dB = sA + GB_K0 * GB_PA0 + warp * GB_PB0 + bn;
+        int gk = sc * KC + warp, l = m + gk;
+        const double* tA = T + (size_t)(mb + gk) * nlat + r0 + lane;
+        const double* xC = A.in + (size_t)A.chan[sp] * ncf + n0 + bn;
+        const double* xB0 = xC + rowB * A.nk;  // degree 0
+        const double* xB = xC + (ptrdiff_t)rowB * (l * (l + 1) / 2 - 1 + m);
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+        for (int i = 0; i < GB_K0 / 4; ++i) {
+          const bool kon = gk < Km;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-  for (int k0 = 0; k0 < kdim; k0 += GB_K) {
-    // A tile (rows r0.., k k0..): synthesis T[mb + kk][j = r]; analysis T[mb + r][j = kk]
-    for (int t = threadIdx.x; t < GB_K * GB_M; t += 256) {
-      int kk = t / GB_M, r = t % GB_M;
-      int gr = r0 + r, gk = k0 + kk;
-      double v = 0.0;
-      if (gr < rows && gk < kdim)
-        v = (A.mode == 0) ? T[(size_t)(mb + gk) * A.nlat + gr] : T[(size_t)(mb + gr) * A.nlat + gk];
-      As[kk][r] = v;
-    }
-    for (int t = threadIdx.x; t < GB_K * GB_N; t += 256) {
-      int kk = t / GB_N, n = t % GB_N;
-      int gk = k0 + kk, gn = n0 + n;
-      double v = 0.0;
-      if (gk < kdim && gn < A.ncf) {
-        if (A.mode == 0) {
-          int row = slot_row(A.kbeg, m + gk, m, A.nk);
-          v = A.in[(size_t)row * A.nin * A.ncf + (size_t)A.chan[p] * A.ncf + gn];
-        } else {
-          v = A.in[(((size_t)m * A.nlat + gk) * A.np + p) * A.ncf + gn];
+          for (int r = 0; r < 8 * R; r += 32)
+            if (r + 32 <= 8 * R || r + lane < 8 * R) {
+              const bool on = kon && r + lane < nrow;
+              cp_a8z(dA + r, on ? tA + r : T, on);
+            }
+          const bool on = kon && bon;
+          cp_a16z(dB, on ? (l >= 1 ? xB : xB0) : A.in, on);
+          dA += 4 * GB_PA0;
+          tA += 4 * (size_t)nlat;
+          dB += 4 * GB_PB0;
+          xB += rowB * (4 * l + 10);  // slot of l + 4 less slot of l
+          gk += 4;
+          l += 4;
+        }
+      } else {
+        // 8 latitudes of four degrees a warp step, then latitudes warp, warp + 4, .. (and their mirrors)
+        const int k = lane & 7, gj = sc * KC + k;
+        int i = 4 * warp + (lane >> 3);
+        double* dA = sA + i * GB_PA1 + k;
+        const double* tA = T + (size_t)(mb + 2 * r0 + i) * nlat + gj;
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+          const bool on = 2 * r0 + i < Km && gj < nh;
+          cp_a8z(dA, on ? tA : T, on);
+          dA += 16 * GB_PA1;
+          tA += 16 * (size_t)nlat;
+          i += 16;
+        }
+        double* dB = sA + 2 * GB_RT * GB_PA1 + warp * GB_PB1 + bn;
+        const double* xB = A.in + ((size_t)m * nlat * np + sp) * ncf + n0 + bn;
+#pragma unroll
+        for (int u = 0; u < GB_K1 / 4; ++u) {
+          const int j = sc * KC + warp + 4 * u, jm = nlat - 1 - j;  // the mirror row; the equator has none
+          const bool on = j < nh && bon, onm = on && jm != j;
+          cp_a16z(dB, on ? xB + rowB * j : A.in, on);
+          cp_a16z(dB + GB_K1 * GB_PB1, onm ? xB + rowB * jm : A.in, onm);
+          dB += 4 * GB_PB1;
         }
       }
-      Bs[kk][n] = v;
+      if (++sc == nch) {
+        sc = 0;
+        ++sp;
+      }
     }
-    __syncthreads();
+    cp_commit();
+  };
+  double2 E[R][2], O[R][2];
 #pragma unroll
-    for (int kk = 0; kk < GB_K; ++kk) {
-      double a[4], b[4];
+  for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        a[q] = As[kk][ty + 16 * q];
-        b[q] = Bs[kk][tx + 16 * q];
+    for (int t = 0; t < 2; ++t) E[r][t] = O[r][t] = make_double2(0.0, 0.0);
+  for (int q = 0; q < GB_NST - 1; ++q) stage(q);
+  int p = p0, c = 0;
+  for (int q = 0; q < nq; ++q) {
+    cp_wait<GB_NST - 2>();
+    __syncthreads();  // chunk q is in, chunk q - 1's stage is free
+    stage(q + GB_NST - 1);
+    const double* sA = gsm + (q % GB_NST) * ST;
+    const double sg = A.sig[p];
+    if (wact) {
+      const int kleft = kdim - c * KC;
+      if (MODE == 0) {
+        const double* a = sA + 2 * lk * GB_PA0 + lr;
+        const double* b = sA + GB_K0 * GB_PA0 + 2 * lk * GB_PB0 + warp * 16 + lr;
+#pragma unroll
+        for (int ks = 0; ks < GB_K0 / 8; ++ks) {
+          if (ks * 8 >= kleft) break;
+          const double* ak = a + ks * 8 * GB_PA0;
+          const double* bk = b + ks * 8 * GB_PB0;
+          const double be0 = bk[0], be1 = bk[8], bo0 = bk[GB_PB0], bo1 = bk[GB_PB0 + 8];
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const double ae = ak[8 * r], ao = ak[GB_PA0 + 8 * r];
+            dmma(E[r][0], ae, be0);
+            dmma(E[r][1], ae, be1);
+            dmma(O[r][0], ao, bo0);
+            dmma(O[r][1], ao, bo1);
+          }
+        }
+      } else {
+        const double* a = sA + 2 * lr * GB_PA1 + lk;
+        const double* b = sA + 2 * GB_RT * GB_PA1 + lk * GB_PB1 + warp * 16 + lr;
+#pragma unroll
+        for (int ks = 0; ks < GB_K1 / 4; ++ks) {
+          if (ks * 4 >= kleft) break;
+          const double* ak = a + ks * 4;
+          const double* bk = b + ks * 4 * GB_PB1;
+          const double n0v = bk[0], n1v = bk[8], s0 = sg * bk[GB_K1 * GB_PB1], s1 = sg * bk[GB_K1 * GB_PB1 + 8];
+          const double be0 = n0v + s0, be1 = n1v + s1, bo0 = n0v - s0, bo1 = n1v - s1;
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const double ae = ak[16 * r * GB_PA1], ao = ak[(16 * r + 1) * GB_PA1];
+            dmma(E[r][0], ae, be0);
+            dmma(E[r][1], ae, be1);
+            dmma(O[r][0], ao, bo0);
+            dmma(O[r][1], ao, bo1);
+          }
+        }
+      }
+    }
+    if (++c < nch) continue;
+    // the product's outputs, beside the copies of the next one's first chunks
+    if (wact) {
+      const int gn = n0 + warp * 16 + 2 * lk;
+      const bool on1 = gn + 8 < ncf;  // the warp's first column group is on by wact (ncf is even; checked per pair)
+      const bool on0 = gn < ncf;
+      double* o0;
+      double* o1;
+      ptrdiff_t d0, d1;  // per row group
+      if (MODE == 0) {
+        o0 = A.out + (((size_t)m * nlat + r0 + lr) * np + p) * ncf + gn;
+        o1 = A.out + (((size_t)m * nlat + nlat - 1 - r0 - lr) * np + p) * ncf + gn;
+        d0 = 8 * (ptrdiff_t)np * ncf;
+        d1 = -d0;
       }
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+      for (int r = 0; r < R; ++r) {
+        const int row = 8 * r + lr;
+        if (MODE == 0) {
+          if (row < nrow) {
+            const bool mirror = 2 * (r0 + row) != nlat - 1;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) acc[q][u] += a[q] * b[u];
+            for (int t = 0; t < 2; ++t)
+              if (t ? on1 : on0) {
+                const double2 e = E[r][t], o = O[r][t];
+                *reinterpret_cast<double2*>(o0 + 8 * t) = make_double2(e.x + o.x, e.y + o.y);
+                if (mirror)
+                  *reinterpret_cast<double2*>(o1 + 8 * t) = make_double2(sg * (e.x - o.x), sg * (e.y - o.y));
+              }
+          }
+          o0 += d0;
+          o1 += d1;
+        } else if (row < nrow) {
+          const int l = m + 2 * (r0 + row);
+          double* oe = A.out + ((size_t)slot_row(l, m, A.nk) * np + p) * ncf + gn;
+          double* oo = A.out + ((size_t)slot_row(l + 1, m, A.nk) * np + p) * ncf + gn;
+#pragma unroll
+          for (int t = 0; t < 2; ++t)
+            if (t ? on1 : on0) {
+              *reinterpret_cast<double2*>(oe + 8 * t) = E[r][t];
+              if (l < A.lmax) *reinterpret_cast<double2*>(oo + 8 * t) = O[r][t];
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 2; ++t) E[r][t] = O[r][t] = make_double2(0.0, 0.0);
+      }
     }
-    __syncthreads();
+    c = 0;
+    ++p;
   }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    int gr = r0 + ty + 16 * q;
-    if (gr >= rows) continue;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      int gn = n0 + tx + 16 * u;
-      if (gn >= A.ncf) continue;
-      if (A.mode == 0)
-        A.out[(((size_t)m * A.nlat + gr) * A.np + p) * A.ncf + gn] = acc[q][u];
-      else
-        A.out[((size_t)slot_row(A.kbeg, m + gr, m, A.nk) * A.np + p) * A.ncf + gn] = acc[q][u];
+  cp_wait<0>();
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(128, 3) k_v3_gemm(const __grid_constant__ GemmArgs A) {
+  extern __shared__ __align__(16) double gsm[];
+  const int ng = A.np / A.pg, m = blockIdx.z / ng, p0 = (blockIdx.z % ng) * A.pg;
+  const int rows = MODE == 0 ? (A.nlat + 1) / 2 : (A.lmax - m + 2) / 2;  // per parity in the analysis
+  const int r0 = blockIdx.y * A.rt, n0 = blockIdx.x * GB_N;
+  if (r0 >= rows) return;
+  const int nrow = min(A.rt, rows - r0), nr8 = (nrow + 7) >> 3;
+  if (nr8 > 3)
+    gemm_tile<MODE, 5>(A, gsm, m, p0, r0, n0, nrow);
+  else if (nr8 > 1)
+    gemm_tile<MODE, 3>(A, gsm, m, p0, r0, n0, nrow);
+  else
+    gemm_tile<MODE, 1>(A, gsm, m, p0, r0, n0, nrow);
+}
+
+// The per-order products of one stage: mode 0 synthesis, 1 analysis.
+static void launch_gemm(vg_handle* h, GemmArgs A, int mode) {
+  const Grid& G = h->grid;
+  const int rows = mode == 0 ? (G.nlat + 1) / 2 : (G.lmax + 2) / 2;
+  const int rtiles = (rows + GB_RT - 1) / GB_RT;
+  A.rt = ((rows + rtiles - 1) / rtiles + 7) / 8 * 8;
+  // a CTA keeps its pipeline running over as many products as leave enough
+  // CTAs to fill the chip twice
+  const int ct = (A.ncf + GB_N - 1) / GB_N, base = ct * rtiles * G.M;
+  A.pg = 1;
+  for (int d = A.np; d > 1; --d)
+    if (A.np % d == 0 && base * (A.np / d) >= 4 * 148) {
+      A.pg = d;
+      break;
     }
+  const dim3 grid(ct, rtiles, G.M * (A.np / A.pg));
+  const size_t shm = GB_NST * sizeof(double) * (mode == 0 ? GB_ST0 : GB_ST1);
+  if (mode == 0) {
+    raise_smem_limit((const void*)k_v3_gemm<0>, shm);
+    k_v3_gemm<0><<<grid, 128, shm, h->stream>>>(A);
+  } else {
+    raise_smem_limit((const void*)k_v3_gemm<1>, shm);
+    k_v3_gemm<1><<<grid, 128, shm, h->stream>>>(A);
+  }
+  ++h->n_launch;
+  VG_CUDA(cudaGetLastError());
+}
+
+// The tables of the products: synthesis P, D, P, P, G, H (toroidal P, D, G, H)
+// and analysis wP, wD, wP, wP, wG, wH (wD, wP, wG, wH), with their signs under
+// theta -> pi - theta.
+static void gemm_tables(const vg_handle* h, GemmArgs& A, bool weighted) {
+  const Grid& G = h->grid;
+  const double* u[4] = {G.d_plm.p, G.d_dplm.p, h->d_G6.p, h->d_H6.p};
+  const double* w[4] = {h->d_wP.p, h->d_wD.p, h->d_wG.p, h->d_wH.p};
+  const int us[10] = {0, 1, 0, 0, 2, 3, 0, 1, 2, 3}, ws[10] = {0, 1, 0, 0, 2, 3, 1, 0, 2, 3};
+  for (int p = 0; p < A.np; ++p) {
+    const int t = weighted ? ws[p] : us[p];
+    A.T[p] = weighted ? w[t] : u[t];
+    A.sig[p] = (t & 1) ? -1.0 : 1.0;
   }
 }
 
@@ -323,16 +553,6 @@ static void lon_tables_build(vg_handle* h) {
     }
   h->d_lon_tw.upload(tw, h->stream);
   h->d_lon_twt.upload(twt, h->stream);
-}
-
-__device__ __forceinline__ void lon_cp16(void* dst, const void* src) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(src) : "memory");
-}
-__device__ __forceinline__ void lon_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void lon_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
 // synthesis tiles over A (shared, [6 nfl][2 M2], row 6 fl + c): for each
@@ -452,11 +672,11 @@ __device__ __forceinline__ void stage_in(const double* __restrict__ S, double* _
   const int n = M * NS * nft;
   for (int t = threadIdx.x; t < n; t += blockDim.x) {
     const int mq = t / nft, c = t % nft;
-    lon_cp16(X + (size_t)mq * 2 * nft + 2 * c,
+    cp_a16(X + (size_t)mq * 2 * nft + 2 * c,
              S + ((size_t)(mq / NS) * nlat + j) * NQ * ncf + (size_t)(q0 + mq % NS) * ncf + 2 * f0 + 2 * c);
   }
-  lon_commit();
-  lon_wait<0>();
+  cp_commit();
+  cp_wait<0>();
 }
 
 template <int NQ = 6>
@@ -859,32 +1079,22 @@ void visc3d_advance(vg_handle* h, const double* d_sigma, double dt, const double
     VG_CUDA(cudaGetLastError());
   }
   // synthesis
-  const int np = h->tor_on ? 10 : 6;
   GemmArgs S;
-  S.mode = 0;
   S.lmax = G.lmax;
   S.nlat = G.nlat;
   S.nk = h->nk;
   S.ncf = ncf;
   S.nin = h->tor_on ? 6 : 4;
-  S.np = np;
+  S.np = h->tor_on ? 10 : 6;
   S.mbeg = G.d_mbeg.p;
-  S.kbeg = h->d_kbeg.p;
-  const double* st[10] = {G.d_plm.p, G.d_dplm.p, G.d_plm.p, G.d_plm.p, h->d_G6.p,
-                          h->d_H6.p, G.d_plm.p,  G.d_dplm.p, h->d_G6.p, h->d_H6.p};
   const int sc[10] = {0, 1, 1, 2, 3, 3, 4, 4, 5, 5};
-  for (int p = 0; p < np; ++p) {
-    S.T[p] = st[p];
-    S.chan[p] = sc[p];
-  }
+  for (int p = 0; p < S.np; ++p) S.chan[p] = sc[p];
+  gemm_tables(h, S, false);
   S.in = h->d_X.p;
   S.out = h->d_Y.p;
-  dim3 sg((ncf + GB_N - 1) / GB_N, (G.nlat + GB_M - 1) / GB_M, G.M * np);
   {
     PhaseScope pp(h, VG_PH_V3_SYNTH);
-    k_v3_gemm<<<sg, 256, 0, s>>>(S);
-    ++h->n_launch;
-    VG_CUDA(cudaGetLastError());
+    launch_gemm(h, S, 0);
   }
   // longitude pass
   {
@@ -903,19 +1113,12 @@ void visc3d_advance(vg_handle* h, const double* d_sigma, double dt, const double
     VG_CUDA(cudaGetLastError());
   }
   // analysis
-  GemmArgs Aa = S;
-  Aa.mode = 1;
-  const double* at[10] = {h->d_wP.p, h->d_wD.p, h->d_wP.p, h->d_wP.p, h->d_wG.p,
-                          h->d_wH.p, h->d_wD.p, h->d_wP.p, h->d_wG.p, h->d_wH.p};
-  for (int p = 0; p < np; ++p) Aa.T[p] = at[p];
-  Aa.in = h->d_Y.p;
-  Aa.out = h->d_dy.p;
-  dim3 ag((ncf + GB_N - 1) / GB_N, (G.M + GB_M - 1) / GB_M, G.M * np);
+  gemm_tables(h, S, true);
+  S.in = h->d_Y.p;
+  S.out = h->d_dy.p;
   {
     PhaseScope pp(h, VG_PH_V3_ANALYSIS);
-    k_v3_gemm<<<ag, 256, 0, s>>>(Aa);
-    ++h->n_launch;
-    VG_CUDA(cudaGetLastError());
+    launch_gemm(h, S, 1);
   }
   PhaseScope pc(h, VG_PH_V3_SCATTER);
   if (h->tor_on)
@@ -1220,39 +1423,24 @@ void visc3d_adjoint(vg_handle* h, const double* gstore, double dt, const double*
   A.ncf = ncf;
   dim3 gg((h->nk + 31) / 32, (h->ne3d + 7) / 8);
   GemmArgs S;
-  S.mode = 0;
   S.lmax = G.lmax;
   S.nlat = G.nlat;
   S.nk = h->nk;
   S.ncf = ncf;
-  S.nin = tor ? 6 : 4;
+  S.nin = np;
   S.np = np;
   S.mbeg = G.d_mbeg.p;
-  S.kbeg = h->d_kbeg.p;
-  const double* st[10] = {G.d_plm.p, G.d_dplm.p, G.d_plm.p, G.d_plm.p, h->d_G6.p,
-                          h->d_H6.p, G.d_plm.p,  G.d_dplm.p, h->d_G6.p, h->d_H6.p};
-  const double* at[10] = {h->d_wP.p, h->d_wD.p, h->d_wP.p, h->d_wP.p, h->d_wG.p,
-                          h->d_wH.p, h->d_wD.p, h->d_wP.p, h->d_wG.p, h->d_wH.p};
-  const int sc[10] = {0, 1, 1, 2, 3, 3, 4, 4, 5, 5};
-  for (int p = 0; p < np; ++p) {
-    S.T[p] = st[p];
-    S.chan[p] = sc[p];
-  }
-  dim3 sgrid((ncf + GB_N - 1) / GB_N, (G.nlat + GB_M - 1) / GB_M, G.M * np);
   // adjoint chain
   if (tor)
     k_v3_scatter_T<10><<<gg, dim3(32, 8), 0, s>>>(A, lam, h->d_n6.p, h->d_v3a_dyb.p, lam_t);
   else
     k_v3_scatter_T<6><<<gg, dim3(32, 8), 0, s>>>(A, lam, h->d_n6.p, h->d_v3a_dyb.p, nullptr);
-  GemmArgs Ab = S;  // analysis^T: the weighted tables, per-product input rows
-  Ab.nin = np;
-  for (int p = 0; p < np; ++p) {
-    Ab.T[p] = at[p];
-    Ab.chan[p] = p;
-  }
-  Ab.in = h->d_v3a_dyb.p;
-  Ab.out = h->d_v3a_Yb.p;
-  k_v3_gemm<<<sgrid, 256, 0, s>>>(Ab);
+  // analysis^T: the weighted tables, per-product input rows
+  for (int p = 0; p < np; ++p) S.chan[p] = p;
+  gemm_tables(h, S, true);
+  S.in = h->d_v3a_dyb.p;
+  S.out = h->d_v3a_Yb.p;
+  launch_gemm(h, S, 0);
   if (tor) {
     const dim3 lg(G.nlat, (nf + LON_LF_TOR - 1) / LON_LF_TOR);
     k_v3_lon_T<LON_LF_TOR, 10><<<lg, lon_threads(h, LON_LF_TOR), lon_smem(h, LON_LF_TOR, true, 10), s>>>(
@@ -1262,17 +1450,16 @@ void visc3d_adjoint(vg_handle* h, const double* gstore, double dt, const double*
     k_v3_lon_T<LON_LF><<<lg, lon_threads(h, LON_LF), lon_smem(h, LON_LF, true), s>>>(
         gstore, h->d_v3a_Yb.p, G.nlat, G.nphi, nf, dt, h->d_MkPerDt3.p, lon_tables(h), G.d_invsin.p, gradMdt, gw);
   }
-  GemmArgs Sb = S;  // synthesis^T: the unweighted tables, per product out
-  Sb.mode = 1;
-  Sb.in = h->d_v3a_Yb.p;
-  Sb.out = h->d_v3a_Rb.p;
-  dim3 agrid((ncf + GB_N - 1) / GB_N, (G.M + GB_M - 1) / GB_M, G.M * np);
-  k_v3_gemm<<<agrid, 256, 0, s>>>(Sb);
+  // synthesis^T: the unweighted tables, per product out
+  gemm_tables(h, S, false);
+  S.in = h->d_v3a_Yb.p;
+  S.out = h->d_v3a_Rb.p;
+  launch_gemm(h, S, 1);
   if (tor)
     k_v3_gather_T<10><<<gg, dim3(32, 8), 0, s>>>(A, h->d_v3a_Rb.p, lam, lam_new, E, lam_t, lam_t_new, Et);
   else
     k_v3_gather_T<6><<<gg, dim3(32, 8), 0, s>>>(A, h->d_v3a_Rb.p, lam, lam_new, E, nullptr, nullptr, nullptr);
-  h->n_launch += 5;
+  h->n_launch += 3;
   VG_CUDA(cudaGetLastError());
 }
 
