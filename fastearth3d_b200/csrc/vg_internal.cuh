@@ -180,7 +180,8 @@ struct vg_handle {
   vg::DArr<double> d_X, d_Y, d_dy;    // 3-D work buffers: synthesis input, Fourier products, increments
   vg::DArr<double> d_v3a_Yb, d_v3a_dyb, d_v3a_Rb;  // 3-D adjoint: product adjoints
   double* v3_gstore = nullptr;  // when set, the FP64 longitude pass also stores its grid there (adjoint sweeps)
-  vg::DArr<double> d_lon_tw, d_lon_twt;  // FP64 longitude pass: dense twiddle tables (by order, by longitude)
+  vg::DArr<double> d_lon_TM, d_lon_FS, d_lon_FA;  // FP64 longitude pass: twiddle tables and their operand fragments
+  vg::DArr<double> d_lon_tw, d_lon_twt;  // its transpose: dense twiddle tables (by order, by longitude)
   // toroidal degree of freedom (p.toroidal and a genuinely 3-D element;
   // vg_toroidal.cu): memory tmem[buf][((s*2 + ri)*ne + e)*2 + lam][k] with
   // lam 0 = lambda 3, 1 = lambda 4, double-buffered with d_mem (same `cur`)

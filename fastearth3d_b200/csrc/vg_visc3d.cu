@@ -8,7 +8,7 @@
 //   gather    X[k][ch][f][ri] = memory + 2 mu strain (the combined synthesis
 //             input of tau + 2 mu eps), channel 3 pre-scaled by -l(l+1)
 //   synth     per order m, six products over l: P.X0, D.X1, P.X1, P.X2, G.X3,
-//             H.X3 -> S[m][j][p][f][ri] (Fourier coefficients at latitude j)
+//             H.X3 -> S[m, j][p][f][ri] (Fourier coefficients at latitude j)
 //   lon       per latitude: dyadic Fourier coefficients (rr, rt, rp, tt, pp, tp),
 //             inverse DFT to the grid, times -M(theta, phi), forward DFT, the
 //             six analysis inputs (RR, RT, m/sin RP, TT+PP, TT-PP, TP)
@@ -27,6 +27,7 @@
 // (the grid identities of src/vilma_tensor_sh.f90:244-266).
 #include <algorithm>
 #include <cmath>
+#include <initializer_list>
 
 #include "vg_device.cuh"
 #include "vg_internal.cuh"
@@ -95,6 +96,8 @@ struct V3Args {
   // slots, as double bits (the synthesis operand rows' scale groups)
   unsigned long long* gmax = nullptr;
   int lm_rows = 0;  // exact tensor-core path: X rows in lm order (k2lm) instead of slot order
+  // toroidal quadratures 6, 7: 0: wP.(m/sin RT), wD.RP (FP64 path), 1: the other way round (exact path)
+  int tor_swap = 0;
 };
 
 // one thread per (slot k, 3-D element): strain of both histories, 24 values,
@@ -174,8 +177,8 @@ constexpr size_t v3_gather_smem() {
 
 // Per-order batched FP64 products (the Legendre stage of the tensor transforms).
 //   MODE 0 (synthesis): C[j][n] = sum_{kk < K_m} T_p[mbeg + kk][j] * X[row(m + kk, m)][col_p + n]
-//                       -> S[((m * nlat + j) * np + p) * ncf + n]
-//   MODE 1 (analysis):  C[i][n] = sum_{j} T_p[mbeg + i][j] * S[((m * nlat + j) * np + p) * ncf + n]
+//                       -> S[(s_row(m, j) * np + p) * ncf + n]
+//   MODE 1 (analysis):  C[i][n] = sum_{j} T_p[mbeg + i][j] * S[(s_row(m, j) * np + p) * ncf + n]
 //                       -> R[(row(m + i, m) * np + p) * ncf + n]
 // row(l, m) is the slot for l >= 1, the zero row nk for l = 0.
 //
@@ -224,6 +227,15 @@ static_assert((GB_K0 * GB_PA0) % 2 == 0 && (2 * GB_RT * GB_PA1) % 2 == 0, "16-by
 // slot of (l, m): degrees 1 .. l - 1 hold 2 + .. + l slots
 __device__ __forceinline__ int slot_row(int l, int m, int nk) { return l >= 1 ? l * (l + 1) / 2 - 1 + m : nk; }
 
+// Row of (order m, latitude j) in S: eight orders of one latitude lie together.
+// The Legendre products walk the latitudes of one order, the longitude pass the
+// orders of one latitude; with either index outermost the other kernel's rows
+// are 2 MB apart at lmax 128, a page each.
+__host__ __device__ __forceinline__ size_t s_row(int m, int j, int nlat) {
+  return ((size_t)(m >> 3) * nlat + j) * 8 + (m & 7);
+}
+static size_t s_rows(int M, int nlat) { return (size_t)((M + 7) / 8) * 8 * nlat; }
+
 __device__ __forceinline__ void cp_a16(double* dst, const double* src) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(src) : "memory");
@@ -265,7 +277,7 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& A, double* gsm, int m,
   const int nch = (kdim + KC - 1) / KC, nq = A.pg * nch;
   const int bn = 2 * lane;  // this thread's two columns of a B row
   const bool bon = n0 + bn < ncf;
-  const size_t rowB = MODE == 0 ? (size_t)A.nin * ncf : (size_t)np * ncf;
+  const size_t rowB = MODE == 0 ? (size_t)A.nin * ncf : (size_t)8 * np * ncf;  // between degrees, latitudes
   int sp = p0, sc = 0;  // product and chunk staged next
   auto stage = [&](int q) {
     if (q < nq) {
@@ -313,7 +325,7 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& A, double* gsm, int m,
           i += 16;
         }
         double* dB = sA + 2 * GB_RT * GB_PA1 + warp * GB_PB1 + bn;
-        const double* xB = A.in + ((size_t)m * nlat * np + sp) * ncf + n0 + bn;
+        const double* xB = A.in + (s_row(m, 0, nlat) * np + sp) * ncf + n0 + bn;
 #pragma unroll
         for (int u = 0; u < GB_K1 / 4; ++u) {
           const int j = sc * KC + warp + 4 * u, jm = nlat - 1 - j;  // the mirror row; the equator has none
@@ -394,9 +406,9 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& A, double* gsm, int m,
       double* o1;
       ptrdiff_t d0, d1;  // per row group
       if (MODE == 0) {
-        o0 = A.out + (((size_t)m * nlat + r0 + lr) * np + p) * ncf + gn;
-        o1 = A.out + (((size_t)m * nlat + nlat - 1 - r0 - lr) * np + p) * ncf + gn;
-        d0 = 8 * (ptrdiff_t)np * ncf;
+        o0 = A.out + (s_row(m, r0 + lr, nlat) * np + p) * ncf + gn;
+        o1 = A.out + (s_row(m, nlat - 1 - r0 - lr, nlat) * np + p) * ncf + gn;
+        d0 = 64 * (ptrdiff_t)np * ncf;
         d1 = -d0;
       }
 #pragma unroll
@@ -481,16 +493,15 @@ static void launch_gemm(vg_handle* h, GemmArgs A, int mode) {
   VG_CUDA(cudaGetLastError());
 }
 
-// The tables of the products: synthesis P, D, P, P, G, H (toroidal P, D, G, H)
-// and analysis wP, wD, wP, wP, wG, wH (wD, wP, wG, wH), with their signs under
-// theta -> pi - theta.
+// The tables of the products, P, D, P, P, G, H (toroidal P, D, G, H), weighted
+// for the analysis, with their signs under theta -> pi - theta.
 static void gemm_tables(const vg_handle* h, GemmArgs& A, bool weighted) {
   const Grid& G = h->grid;
   const double* u[4] = {G.d_plm.p, G.d_dplm.p, h->d_G6.p, h->d_H6.p};
   const double* w[4] = {h->d_wP.p, h->d_wD.p, h->d_wG.p, h->d_wH.p};
-  const int us[10] = {0, 1, 0, 0, 2, 3, 0, 1, 2, 3}, ws[10] = {0, 1, 0, 0, 2, 3, 1, 0, 2, 3};
+  const int tab[10] = {0, 1, 0, 0, 2, 3, 0, 1, 2, 3};
   for (int p = 0; p < A.np; ++p) {
-    const int t = weighted ? ws[p] : us[p];
+    const int t = tab[p];
     A.T[p] = weighted ? w[t] : u[t];
     A.sig[p] = (t & 1) ? -1.0 : 1.0;
   }
@@ -662,7 +673,7 @@ constexpr int LON_THREADS = 384;
 constexpr int LON_LF = 3;  // fields per CTA: one element's three shape coefficients (two CTAs per SM)
 constexpr int LON_LF_TOR = 3;  // with the toroidal channels: staged in two halves, two CTAs per SM
 
-// the CTA's slice of the products S[m][j][q][f][ri] (fields f0 .. f0 + nft - 1,
+// the CTA's slice of the products S[m, j][q][f][ri] (fields f0 .. f0 + nft - 1,
 // a contiguous run of 2 nft doubles per (m, q)) to and from shared [m][q][2 nft]
 // (16-byte cp.async pieces, all in flight together; ncf and 2 f0 are even)
 // products q0 .. q0 + NS - 1 of the NQ per (m, j), staged as [m][q - q0][2 nft]
@@ -673,7 +684,7 @@ __device__ __forceinline__ void stage_in(const double* __restrict__ S, double* _
   for (int t = threadIdx.x; t < n; t += blockDim.x) {
     const int mq = t / nft, c = t % nft;
     cp_a16(X + (size_t)mq * 2 * nft + 2 * c,
-             S + ((size_t)(mq / NS) * nlat + j) * NQ * ncf + (size_t)(q0 + mq % NS) * ncf + 2 * f0 + 2 * c);
+             S + s_row(mq / NS, j, nlat) * NQ * ncf + (size_t)(q0 + mq % NS) * ncf + 2 * f0 + 2 * c);
   }
   cp_commit();
   cp_wait<0>();
@@ -685,118 +696,499 @@ __device__ __forceinline__ void stage_out(const double* __restrict__ X, double* 
   const int w = 2 * nft, n = M * NQ * w;
   for (int t = threadIdx.x; t < n; t += blockDim.x) {
     const int mq = t / w, c = t % w;
-    S[((size_t)(mq / NQ) * nlat + j) * NQ * ncf + (size_t)(mq % NQ) * ncf + 2 * f0 + c] = X[t];
+    S[s_row(mq / NQ, j, nlat) * NQ * ncf + (size_t)(mq % NQ) * ncf + 2 * f0 + c] = X[t];
   }
 }
 
-// One CTA per (latitude j, LF fields). Dyadic Fourier coefficients from the
-// six synthesis products, synthesis to the grid, times -M(theta_j, phi_i) of
-// the field's element, analysis, and the six analysis inputs, written in place
-// over the synthesis products. With gstore set, the grid before -M dt is also
-// stored, [j][field][component][i], for the adjoint.
-template <int LF, int NQ = 6>
-__global__ void __launch_bounds__(LON_THREADS, 1)
-    k_v3_lon(double* __restrict__ S, int nlat, int nphi, int nf, double dt, const double* __restrict__ Mk3rate,
-             LonTables T, const double* __restrict__ invsin, double* __restrict__ gstore, int trap) {
-  extern __shared__ double sm[];
-  const int j = blockIdx.x, f0 = blockIdx.y * LF;
-  const int nft = min(LF, nf - f0);
-  const int ncf = 2 * nf, half = T.half, wA = 2 * T.M2;
-  double* A = sm;  // [6 LF][2 M2]; [m][q][2 nft] for the analysis inputs
-  double* X = sm + (NQ == 6 ? (size_t)6 * LF * wA : lon_areg(LF, T));  // [6 LF][nphi]; staged products
-  const double is = invsin[j];
-  // 1. the CTA's synthesis products, staged in X as [m][q][2 nft] (contiguous
-  //    runs of 2 nft doubles in S; the spheroidal six, then the toroidal four),
-  //    then the dyadic coefficients rr, rt, rp, tt, pp, tp with the synthesis
-  //    weights (1 at m = 0, 2 above), zero past M
-  stage_in<NQ, 6>(S, X, nlat, ncf, j, f0, nft, T.M);
-  __syncthreads();
-  for (int t = threadIdx.x; t < nft * T.M2; t += blockDim.x) {
-    const int fl = t / T.M2, m = t % T.M2;
-    double pr[6][2];
-    for (int q = 0; q < 6; ++q)
-      for (int ri = 0; ri < 2; ++ri) pr[q][ri] = (m < T.M) ? X[((size_t)m * 6 + q) * 2 * nft + 2 * fl + ri] : 0.0;
-    const double ms = m * is, w = (m == 0) ? 1.0 : 2.0;
-    const double comp[6][2] = {{pr[0][0], pr[0][1]},
-                               {pr[1][0], pr[1][1]},
-                               {-ms * pr[2][1], ms * pr[2][0]},             // i (m / sin) P.X1
-                               {pr[3][0] + pr[4][0], pr[3][1] + pr[4][1]},  // TT + PP
-                               {pr[3][0] - pr[4][0], pr[3][1] - pr[4][1]},  // TT - PP
-                               {-4.0 * pr[5][1], 4.0 * pr[5][0]}};          // 4 i H.X3
-    for (int c = 0; c < 6; ++c) {
-      A[(size_t)(fl * 6 + c) * wA + 2 * m] = w * comp[c][0];
-      A[(size_t)(fl * 6 + c) * wA + 2 * m + 1] = w * comp[c][1];
+// The forward longitude pass: rows r = (product q, field f) of the synthesis
+// products, per latitude the inverse DFT to the grid, times -M(theta_j, phi_i)
+// dt of the field's element, the forward DFT and the analysis inputs, written
+// in place over the products. The rows are rr, rt, i (m/sin) P.X1 = rp, (tt +
+// pp) / 2, (tt - pp) / 2 and tp = 4 i H.X3: -M dt multiplies all six components
+// alike, so tt and pp need not be formed and every row is a transform by
+// itself (the analysis inputs TT + PP and TT - PP are twice rows 3 and 4). With
+// the toroidal channels (TOR) row 1 adds -i (m/sin) P.X4 (product 6), row 2
+// D.X4 (7), row 4 -i H.X5 (9), row 5 G.X5 (8), and each of these rows writes
+// its second analysis input over the product it read: (m/sin) RT in slot 6, RP
+// in 7, TP in 8, TT - PP in 9. With gstore set, the grid before -M dt is also
+// stored, [j][field][row q][i], for the adjoint.
+//
+// Symmetries: phi + pi flips odd orders, -phi flips the sine terms, so with
+// base longitudes i = 0 .. half / 2 and the sums over even and odd m of re cos
+// (Ce, Co) and im sin (Se, So),
+//   g(i) = Ce - Se + Co - So,          g(i + half) = Ce - Se - Co + So,
+//   g(nphi - i) = Ce + Se + Co + So,   g(half - i) = Ce + Se - Co - So
+// (i = 0 and i = half / 2 are their own mirrors), and the forward transform
+// reads the four sign combinations of the base points: four products of about
+// nphi / 4 x nphi / 4 a row each way, half the work of the parity split alone,
+// on the FP64 matrix instructions. The terms m = 0 and i = 0 have cosine 1 and
+// sine 0: they start the accumulators, and the outputs at i = 0 and m = 0 are
+// plain sums, so that at lmax 128 the products are 64 x 64 without a remainder.
+//
+// With half odd (an even lmax on its own grid) the odd orders are the even ones
+// seen from the other end, cos(m phi_i) = (-1)^i cos((half - m) phi_i) and
+// sin(m phi_i) = -(-1)^i sin((half - m) phi_i): with their coefficients stored
+// in the order of half - m and the signs applied on the grid, both parities
+// share two tables (TWIN).
+//
+// Tiles: lon_plan() picks the shape. Persistent CTAs, one per SM, of G groups of
+// warps (four, one a scheduler; eight with G = 1) that work on tiles of their
+// own, so that one group's copies and pointwise work run beside the others'
+// products. A warp holds MT x NW x 4 accumulator tiles; the grid overwrites the
+// coefficients in shared memory. Tables in shared memory (STAB) where they fit
+// beside the groups' 16-row buffers (three groups of four warps with TWIN, two
+// without: nphi up to 258), else their operand fragments from L2, stored in the
+// order the lanes read, eight warps on 32 rows (16 on the largest grids); there
+// TWIN gains nothing (2.98 against 2.86 ms at lmax 256).
+// Bound: at lmax 128, 54 elements 8.4 GFLOP, 230 us at the FP64 rate, and 518 MB,
+// 79 us. Measured 427 us, the products' pipe half busy: the copies, the
+// pointwise pass and the outputs of a group take as long as its products, and
+// three groups do not cover them. One register-tiled FMA kernel with the parity
+// split alone took 1490 us; two groups with four tables 482. lmax 256: 13.9 ->
+// 2.86 ms; lmax 64: 159 -> 62 us.
+struct LonPlan {
+  int M, half, nb;      // orders, half period, base longitudes i = 1 .. nb
+  int Ke, Ko;           // even orders m = 2 .. and odd orders m = 1 ..
+  int kss, ksa;         // four-term steps of the synthesis and the analysis
+  int nts, nta;         // their 8-column tiles
+  int PK, PT, TR;       // pitches of the buffer and of the tables, table rows
+  int G, MT, NW;        // shape (see above)
+  int twin, stab;
+  size_t smem;
+};
+
+struct LonArgs {
+  LonPlan P;
+  int nlat, nphi, nf, trap;
+  double dt;
+  double* S;
+  const double *rate, *invsin;
+  const double *TM, *FS, *FA;  // tables [4 or 2][TR][PT]; fragments of synthesis and analysis [tile][step][table][lane]
+  double* gstore;
+};
+
+static int lon_pitch(int n) {  // the next pitch of 4 or 12 mod 16 doubles: conflict-free fragments
+  while (n % 16 != 4 && n % 16 != 12) ++n;
+  return n;
+}
+
+constexpr size_t LON_SMEM_CTA = 226 * 1024;
+
+static LonPlan lon_plan(const vg_handle* h) {
+  const Grid& G = h->grid;
+  LonPlan P;
+  size_t tab = 0, tile = 0;
+  int nt = 0;
+  auto sizes = [&](bool twin) {
+    P.M = G.M;
+    P.half = G.nphi / 2;
+    P.nb = P.half / 2;
+    P.Ke = (G.M + 1) / 2 - 1;
+    P.Ko = G.M / 2;
+    P.twin = twin;
+    const int K = twin ? P.nb : std::max(P.Ke, P.Ko);
+    P.kss = (K + 3) / 4;
+    P.ksa = (P.nb + 3) / 4;
+    P.nts = (P.nb + 7) / 8;
+    P.nta = (K + 7) / 8;
+    P.PK = lon_pitch(8 * std::max(P.nts, P.nta));
+    P.PT = lon_pitch(8 * P.nts);
+    P.TR = 8 * P.nta;
+    nt = std::max(P.nts, P.nta);
+    tab = (size_t)(twin ? 2 : 4) * P.TR * P.PT * sizeof(double);
+    tile = 16 * (size_t)(4 * P.PK + 2) * sizeof(double) + 16;  // a group's 16-row buffer
+  };
+  P.MT = 2;
+  P.stab = 1;
+  // TWIN where half is odd, the tables then fit and most of the half - m are orders carried
+  sizes(true);
+  if ((P.half & 1) && 4 * P.M > 3 * P.half && nt <= 8 && tab + 3 * tile <= LON_SMEM_CTA) {
+    P.G = 3;
+  } else {
+    sizes(false);
+    if (nt <= 8 && tab + 2 * tile <= LON_SMEM_CTA) {
+      P.G = 2;
+    } else {
+      P.stab = 0;
+      P.G = 1;
+      P.MT = nt <= 16 ? 2 : 1;
     }
   }
-  __syncthreads();
-  if (NQ == 10) {  // Z3: (rt, rp) += e_r x grad_1 = (-i (m/sin) P.X4, D.X4); Z4: (tt, pp, tp) += (-Sh, Sh, Sg)
-    stage_in<NQ, 4>(S, X, nlat, ncf, j, f0, nft, T.M, 6);
-    __syncthreads();
-    for (int t = threadIdx.x; t < nft * T.M; t += blockDim.x) {
-      const int fl = t / T.M, m = t % T.M;
-      double pr[4][2];
-      for (int q = 0; q < 4; ++q)
-        for (int ri = 0; ri < 2; ++ri) pr[q][ri] = X[((size_t)m * 4 + q) * 2 * nft + 2 * fl + ri];
-      const double ms = m * is, w = (m == 0) ? 1.0 : 2.0;
-      const double add[6][2] = {{0.0, 0.0},
-                                {ms * pr[0][1], -ms * pr[0][0]},  // -i (m/sin) P.X4
-                                {pr[1][0], pr[1][1]},             // D.X4
-                                {pr[3][1], -pr[3][0]},            // -i H.X5
-                                {-pr[3][1], pr[3][0]},            // +i H.X5
-                                {pr[2][0], pr[2][1]}};            // G.X5
-      for (int c = 1; c < 6; ++c) {
-        A[(size_t)(fl * 6 + c) * wA + 2 * m] += w * add[c][0];
-        A[(size_t)(fl * 6 + c) * wA + 2 * m + 1] += w * add[c][1];
+  P.NW = P.stab ? (nt <= 4 ? 1 : 2) : nt <= 12 ? 3 : nt <= 16 ? 4 : 6;
+  P.smem = (P.stab ? tab : 0) + (P.G == 1 ? P.MT : P.G) * tile;
+  if (nt > 24 || P.smem > LON_SMEM_CTA) throw Error("visc3d: grid too large for the FP64 longitude pass");
+  return P;
+}
+
+static void lon_plan_tables(vg_handle* h) {
+  const LonPlan P = lon_plan(h);
+  const int nphi = h->grid.nphi;
+  const int ns = P.twin ? 2 : 4;
+  std::vector<double> TM((size_t)ns * P.TR * P.PT, 0.0);
+  for (int s4 = 0; s4 < ns; ++s4)
+    for (int k = 0; k < (P.twin ? P.nb : (s4 & 2) ? P.Ko : P.Ke); ++k)
+      for (int i = 0; i < P.nb; ++i) {
+        const int m = (s4 & 2) ? 2 * k + 1 : 2 * k + 2, t = (int)(((long long)m * (i + 1)) % nphi);
+        const double a = 2.0 * PI * (double)t / (double)nphi;
+        TM[((size_t)s4 * P.TR + k) * P.PT + i] = (s4 & 1) ? std::sin(a) : std::cos(a);
       }
+  h->d_lon_TM.upload(TM, h->stream);
+  if (P.stab) return;
+  std::vector<double> FS((size_t)P.nts * P.kss * ns * 32), FA((size_t)P.nta * P.ksa * ns * 32);
+  auto at = [&](int s4, int k, int i) { return k < P.TR && i < P.PT ? TM[((size_t)s4 * P.TR + k) * P.PT + i] : 0.0; };
+  for (int t = 0; t < P.nts; ++t)
+    for (int ks = 0; ks < P.kss; ++ks)
+      for (int s4 = 0; s4 < ns; ++s4)
+        for (int l = 0; l < 32; ++l)
+          FS[(((size_t)t * P.kss + ks) * ns + s4) * 32 + l] = at(s4, 4 * ks + (l & 3), 8 * t + (l >> 2));
+  for (int t = 0; t < P.nta; ++t)
+    for (int ks = 0; ks < P.ksa; ++ks)
+      for (int s4 = 0; s4 < ns; ++s4)
+        for (int l = 0; l < 32; ++l)
+          FA[(((size_t)t * P.ksa + ks) * ns + s4) * 32 + l] = at(s4, 8 * t + (l >> 2), 4 * ks + (l & 3));
+  if (!FS.empty()) h->d_lon_FS.upload(FS, h->stream);
+  if (!FA.empty()) h->d_lon_FA.upload(FA, h->stream);
+}
+
+// offset of a sum's rows in the buffer: the odd orders' two words off, so that
+// the even and odd coefficients of a row fall in different banks
+__device__ __forceinline__ int lon_sum(int s4, int step) { return s4 * step + (s4 >> 1) * 2; }
+
+// the accumulator tiles of N column tiles t = ng + 4 i: C[mt][i][sum] += buf (rows) x table
+template <int MT, int NW, int N, bool STAB, bool TWIN, bool ANA>
+__device__ __forceinline__ void lon_products(double2 (&C)[MT][NW][4], const double* a, int astep, int arow,
+                                             const double* tab, int TS, int PT, const double* frag, int steps, int ng,
+                                             int lane) {
+  constexpr int NS = TWIN ? 2 : 4;  // tables
+  const int lk = lane & 3, lr = lane >> 2;
+  auto load_b = [&](int ks, double (&b)[N][NS]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int t = ng + 4 * i;
+#pragma unroll
+      for (int s4 = 0; s4 < NS; ++s4)
+        b[i][s4] = STAB ? (ANA ? tab[s4 * TS + (8 * t + lr) * PT + 4 * ks + lk]
+                               : tab[s4 * TS + (4 * ks + lk) * PT + 8 * t + lr])
+                        : __ldg(frag + (((size_t)t * steps + ks) * NS + s4) * 32 + lane);
     }
+  };
+  auto load_a = [&](int ks, double (&av)[MT][4]) {
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int s4 = 0; s4 < 4; ++s4) av[mt][s4] = a[lon_sum(s4, astep) + 8 * mt * arow + 4 * ks];
+  };
+  auto mma = [&](const double (&b)[N][NS], const double (&av)[MT][4]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int s4 = 0; s4 < 4; ++s4)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) dmma(C[mt][i][s4], av[mt][s4], b[i][TWIN ? s4 & 1 : s4]);
+  };
+  // operands one step ahead of the products
+  double b0[N][NS], b1[N][NS], a0[MT][4], a1[MT][4];
+  load_b(0, b0);
+  load_a(0, a0);
+  int ks = 0;
+  for (; ks + 1 < steps; ks += 2) {
+    load_b(ks + 1, b1);
+    load_a(ks + 1, a1);
+    mma(b0, a0);
+    const int nx = min(ks + 2, steps - 1);
+    load_b(nx, b0);
+    load_a(nx, a0);
+    mma(b1, a1);
+  }
+  if (ks < steps) mma(b0, a0);
+}
+
+// the same for a warp's n <= N column tiles (n differs between the warps)
+template <int MT, int NW, int N, bool STAB, bool TWIN, bool ANA>
+__device__ __forceinline__ void lon_products_n(int n, double2 (&C)[MT][NW][4], const double* a, int astep, int arow,
+                                               const double* tab, int TS, int PT, const double* frag, int steps,
+                                               int ng, int lane) {
+  if constexpr (N > 0) {
+    if (n == N)
+      lon_products<MT, NW, N, STAB, TWIN, ANA>(C, a, astep, arow, tab, TS, PT, frag, steps, ng, lane);
+    else
+      lon_products_n<MT, NW, N - 1, STAB, TWIN, ANA>(n, C, a, astep, arow, tab, TS, PT, frag, steps, ng, lane);
+  }
+}
+
+template <int G, int MT, int NW, bool STAB, bool TWIN, bool TOR>
+__global__ void __launch_bounds__(G == 3 ? 384 : 256, 1) k_v3_lon(const __grid_constant__ LonArgs A) {
+  constexpr int GW = G == 1 ? 8 : 4, NMP = GW / 4, ROWS = 8 * MT * NMP, GT = 32 * GW, NQ = TOR ? 10 : 6;
+  constexpr int RG = ROWS / 4, MSTEP = GW / RG;  // staging: groups of four rows, warps on the same group
+  extern __shared__ __align__(16) double lsm[];
+  const LonPlan& P = A.P;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, lk = lane & 3;
+  const int g = warp / GW, wg = warp % GW, ng = wg & 3, mp = wg >> 2, tg = tid % GT;
+  const int PK = P.PK, PT = P.PT, TS = P.TR * P.PT, half = P.half, nphi = A.nphi, M = P.M;
+  const double* tab = STAB ? lsm : A.TM;
+  if (STAB) {
+    for (int t = tid; t < (TWIN ? 1 : 2) * TS; t += 32 * GW * G)
+      reinterpret_cast<double2*>(lsm)[t] = reinterpret_cast<const double2*>(A.TM)[t];
     __syncthreads();
   }
-  // 2. synthesis, times -M dt, and the parity combinations of the analysis
-  lon_synth(A, nft, T, [&](int fl, int i, const double* g1, const double* g2) {
-    const int f = f0 + fl;
-    const double* Mr = Mk3rate + ((size_t)(f / 3) * nlat + j) * nphi;
-    double m1 = Mr[i] * dt, m2 = Mr[i + half] * dt;
-    if (trap) {  // trapezoidal: M / (1 + M/2) (src/vilma_response.f90:1468-1473)
-      m1 = m1 / (1.0 + 0.5 * m1);
-      m2 = m2 / (1.0 + 0.5 * m2);
-    }
-    for (int c = 0; c < 6; ++c) {
-      if (gstore) {
-        double* gs = gstore + (((size_t)j * nf + f) * 6 + c) * nphi;
-        gs[i] = g1[c];
-        gs[i + half] = g2[c];
-      }
-      const double a = -m1 * g1[c], b = -m2 * g2[c];
-      X[(size_t)(fl * 6 + c) * nphi + i] = a + b;
-      X[(size_t)(fl * 6 + c) * nphi + half + i] = a - b;
-    }
-  });
-  __syncthreads();
-  // 3. analysis (F_m = 2 pi / nphi sum_i f_i e^{-i m phi_i}) and the analysis
-  //    inputs RR, RT, m/sin RP, TT + PP, TT - PP, TP
+  const int BS = ROWS * PK;  // one sum's rows
+  double* buf = lsm + (STAB ? (TWIN ? 2 : 4) * TS : 0) + (size_t)g * (4 * BS + 2 + 2 * ROWS);
+  double* z0 = buf + 4 * BS + 2;  // [2][ROWS]: the m = 0 coefficient, then the i = 0 combinations
+  auto bar = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(g + 1), "n"(GT) : "memory"); };
+  const int nrow = 6 * A.nf, nrt = (nrow + ROWS - 1) / ROWS, ntile = A.nlat * nrt;
+  const int srow = NQ * 2 * A.nf;  // doubles per (m, j)
+  const size_t mblock = (size_t)8 * A.nlat * srow;
   const double scl = 2.0 * PI / (double)nphi;
-  lon_anal(X, nft, nphi, T, [&](int fl, int m, const double* re, const double* im) {
-    double F[6][2];
-    for (int c = 0; c < 6; ++c) {
-      F[c][0] = scl * re[c];
-      F[c][1] = scl * im[c];
+  const int nmb = (M + 7) / 8;
+  struct Row {  // what the pointwise pass and the outputs need of a row
+    bool live;
+    int q;
+    const double* rate;
+    double* gs;
+  };
+  for (int tile = blockIdx.x * G + g; tile < ntile; tile += gridDim.x * G) {
+    const int j = tile / nrt, row0 = (tile % nrt) * ROWS;
+    const double is = A.invsin[j];
+    double* Sj = A.S + (size_t)8 * j * srow;  // order m at Sj + (m >> 3) mblock + (m & 7) srow
+    // 1. the rows' coefficients with the synthesis weights (1 at m = 0, 2
+    //    above), even and odd orders apart, zero past M: four rows x eight
+    //    orders a warp step (64-byte runs of the products)
+    {
+      const int r = 4 * (wg % RG) + lk, row = row0 + r, q = row / A.nf;
+      const bool live = row < nrow;
+      const double* src = Sj + lr * srow + 2 * row;
+      const ptrdiff_t part = TOR ? (ptrdiff_t)2 * A.nf * (q == 5 ? 3 : 5) : 0;  // 1 -> 6, 2 -> 7, 4 -> 9, 5 -> 8
+      const bool has = TOR && live && (q == 1 || q == 2 || q >= 4);
+      double* d = buf + r * PK;
+      constexpr int NB = 9 * NW;  // loads in flight together: a whole tile's of the first shape
+      for (int m0 = wg / RG; m0 < nmb; m0 += NB * MSTEP) {
+        double2 z[NB];
+#pragma unroll
+        for (int u = 0; u < NB; ++u) {
+          const int mb = m0 + u * MSTEP;
+          z[u] = make_double2(0.0, 0.0);
+          if (live && 8 * mb + lr < M) z[u] = *reinterpret_cast<const double2*>(src + mb * mblock);
+        }
+#pragma unroll
+        for (int u = 0; u < NB; ++u) {
+          const int mb = m0 + u * MSTEP, m = 8 * mb + lr;
+          if (mb >= nmb) break;
+          const double ms = m * is, w = m == 0 ? 1.0 : 2.0;
+          double2 y = z[u];
+          if (q == 2) y = make_double2(-ms * y.y, ms * y.x);
+          if (q == 5) y = make_double2(-4.0 * y.y, 4.0 * y.x);
+          if (TOR && has && m < M) {
+            const double2 w2 = *reinterpret_cast<const double2*>(src + mb * mblock + part);
+            if (q == 1) {
+              y.x += ms * w2.y;
+              y.y -= ms * w2.x;
+            } else if (q == 4) {
+              y.x += w2.y;
+              y.y -= w2.x;
+            } else {
+              y.x += w2.x;
+              y.y += w2.y;
+            }
+          }
+          if (m == 0) {
+            z0[r] = y.x;
+          } else if (!TWIN || !(m & 1) || m < half) {
+            double* dm = d + lon_sum((m & 1) * 2, BS) + (TWIN && (m & 1) ? (half - m) / 2 - 1 : (m - 1) >> 1);
+            dm[0] = w * y.x;
+            dm[BS] = w * y.y;
+          }
+        }
+      }
+      // the terms of no order staged above: even m < 8 nmb lie at k < 4 nmb - 1,
+      // odd ones at k < 4 nmb (TWIN: at k = (half - m) / 2 - 1)
+      if (wg < RG) {
+        for (int k = 4 * nmb - 1 + lr; k < 4 * P.kss; k += 8) {
+          d[k] = d[BS + k] = 0.0;
+          if (!TWIN && k >= 4 * nmb) d[lon_sum(2, BS) + k] = d[lon_sum(3, BS) + k] = 0.0;
+        }
+        if (TWIN) {
+          for (int k = P.nb + lr; k < 4 * P.kss; k += 8) d[lon_sum(2, BS) + k] = d[lon_sum(3, BS) + k] = 0.0;
+          for (int k = lr; k < (half - 8 * nmb - 1) / 2; k += 8)
+            d[lon_sum(2, BS) + k] = d[lon_sum(3, BS) + k] = 0.0;
+        }
+      }
     }
-    const double ms = m * is;
-    const double out[10][2] = {{F[0][0], F[0][1]},
-                               {F[1][0], F[1][1]},
-                               {ms * F[2][0], ms * F[2][1]},
-                               {F[3][0] + F[4][0], F[3][1] + F[4][1]},
-                               {F[3][0] - F[4][0], F[3][1] - F[4][1]},
-                               {F[5][0], F[5][1]},
-                               {F[2][0], F[2][1]},                      // RP (wD)
-                               {ms * F[1][0], ms * F[1][1]},            // m/sin RT (wP)
-                               {F[5][0], F[5][1]},                      // TP (wG)
-                               {F[3][0] - F[4][0], F[3][1] - F[4][1]}};  // TT - PP (wH)
-    for (int q = 0; q < NQ; ++q)
-      for (int ri = 0; ri < 2; ++ri) A[((size_t)m * NQ + q) * 2 * nft + 2 * fl + ri] = out[q][ri];
-  });
-  __syncthreads();
-  stage_out<NQ>(A, S, nlat, ncf, j, f0, nft, T.M);
+    bar();
+    // 2. the four sums of every row at the base longitudes
+    double2 C[MT][NW][4];
+    const int rw = mp * 8 * MT + lr;  // this lane's first row
+    const double* afrag = buf + rw * PK + lk;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      const double c0 = z0[rw + 8 * mt];
+#pragma unroll
+      for (int i = 0; i < NW; ++i) {
+        C[mt][i][0] = make_double2(c0, c0);
+        C[mt][i][1] = C[mt][i][2] = C[mt][i][3] = make_double2(0.0, 0.0);
+      }
+    }
+    lon_products_n<MT, NW, NW, STAB, TWIN, false>((P.nts - ng + 3) >> 2, C, afrag, BS, PK, tab, TS, PT, A.FS, P.kss, ng, lane);
+    auto row_of = [&](int r) {
+      const int row = row0 + r, q = row / A.nf, f = row - q * A.nf;
+      return Row{row < nrow, q, A.rate + ((size_t)(f / 3) * A.nlat + j) * nphi,
+                 A.gstore ? A.gstore + (((size_t)j * A.nf + f) * 6 + q) * nphi : nullptr};
+    };
+    // M dt at the four points of base longitude i (zero at mirrors that are no points of their own)
+    auto rates = [&](const Row& R, int i, double (&n)[4]) {
+      const bool on = R.live && i <= P.nb, twin = on && i > 0 && 2 * i != half;
+      n[0] = on ? __ldg(R.rate + i) : 0.0;
+      n[1] = on ? __ldg(R.rate + i + half) : 0.0;
+      n[2] = twin ? __ldg(R.rate + nphi - i) : 0.0;
+      n[3] = twin ? __ldg(R.rate + half - i) : 0.0;
+    };
+    auto point = [&](const Row& R, int i, double (&n)[4], double ce, double se, double co, double so, double (&o)[4]) {
+      const double e1 = ce - se, e2 = ce + se, o1 = co - so, o2 = co + so;
+      double a = e1 + o1, b = e1 - o1, c = e2 + o2, d = e2 - o2;
+      if (A.gstore && R.live && i <= P.nb) {
+        R.gs[i] = a;
+        R.gs[i + half] = b;
+        if (i > 0 && 2 * i != half) {
+          R.gs[nphi - i] = c;
+          R.gs[half - i] = d;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        n[u] *= A.dt;
+        if (A.trap) n[u] = n[u] / (1.0 + 0.5 * n[u]);  // M / (1 + M/2) (src/vilma_response.f90:1468-1473)
+      }
+      a *= -n[0];
+      b *= -n[1];
+      c *= -n[2];
+      d *= -n[3];
+      o[0] = (a + b) + (c + d);
+      o[1] = (a + b) - (c + d);
+      o[2] = (a - b) + (c - d);
+      o[3] = (a - b) - (c - d);
+    };
+    // i = 0: the sums themselves, GT / ROWS threads a row (half of them the odd orders)
+    constexpr int XT = GT / ROWS;
+    const int xr = tg / XT, xq = (tg % XT) / (XT / 2), xk = tg % (XT / 2);
+    double x0 = 0.0;
+    {
+      const double* ar = buf + lon_sum(2 * xq, BS) + xr * PK;
+#pragma unroll 8
+      for (int k = xk; k < 4 * P.kss; k += XT / 2) x0 += ar[k];
+#pragma unroll
+      for (int o = XT / 4; o > 0; o >>= 1) x0 += __shfl_xor_sync(0xffffffffu, x0, o);
+    }
+    const double xo = __shfl_xor_sync(0xffffffffu, x0, XT / 2), xz = z0[xr];
+    bar();  // the coefficients are read: the grid goes over them
+    // 3. times -M dt, and the four combinations of the analysis
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      const Row R = row_of(rw + 8 * mt);
+      double n[NW][2][4];
+#pragma unroll
+      for (int i = 0; i < NW; ++i) {
+        const int lon = 8 * (ng + 4 * i) + 2 * lk + 1;
+        rates(R, lon, n[i][0]);
+        rates(R, lon + 1, n[i][1]);
+      }
+#pragma unroll
+      for (int i = 0; i < NW; ++i) {
+        const int t = ng + 4 * i, lon = 8 * t + 2 * lk + 1;
+        if (t >= P.nts) continue;
+        double o0[4], o1[4];
+        // TWIN: (-1)^i on the odd cosine sums, -(-1)^i on the odd sine sums; lon is odd, lon + 1 even
+        constexpr double sg = TWIN ? -1.0 : 1.0;
+        point(R, lon, n[i][0], C[mt][i][0].x, C[mt][i][1].x, sg * C[mt][i][2].x, C[mt][i][3].x, o0);
+        point(R, lon + 1, n[i][1], C[mt][i][0].y, C[mt][i][1].y, C[mt][i][2].y, sg * C[mt][i][3].y, o1);
+        o0[2] *= sg;
+        o1[3] *= sg;
+        double* x = buf + (rw + 8 * mt) * PK + lon - 1;
+        const bool on0 = R.live && lon <= P.nb, on1 = R.live && lon < P.nb;  // zero past the base longitudes
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          *reinterpret_cast<double2*>(x + lon_sum(u, BS)) = make_double2(on0 ? o0[u] : 0.0, on1 ? o1[u] : 0.0);
+      }
+    }
+    if (tg % XT == 0) {
+      const Row R = row_of(xr);
+      double n[4], o[4];
+      rates(R, 0, n);
+      point(R, 0, n, xz + x0, 0.0, xo, 0.0, o);
+      z0[xr] = R.live ? o[0] : 0.0;
+      z0[ROWS + xr] = R.live ? o[2] : 0.0;
+    }
+    bar();
+    // 4. the forward sums of every row
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      const double c0 = z0[rw + 8 * mt], c2 = z0[ROWS + rw + 8 * mt];
+#pragma unroll
+      for (int i = 0; i < NW; ++i) {
+        C[mt][i][0] = make_double2(c0, c0);
+        C[mt][i][2] = make_double2(c2, c2);
+        C[mt][i][1] = C[mt][i][3] = make_double2(0.0, 0.0);
+      }
+    }
+    lon_products_n<MT, NW, NW, STAB, TWIN, true>((P.nta - ng + 3) >> 2, C, afrag, BS, PK, tab, TS, PT, A.FA, P.ksa, ng, lane);
+    x0 = xk == 0 && xq == 0 ? z0[xr] : 0.0;  // m = 0: the sum over the row
+    {
+      const double* ar = buf + xr * PK;
+#pragma unroll 8
+      for (int i = tg % XT; i < 4 * P.ksa; i += XT) x0 += ar[i];
+#pragma unroll
+      for (int o = XT / 2; o > 0; o >>= 1) x0 += __shfl_xor_sync(0xffffffffu, x0, o);
+    }
+    bar();  // the grid is read: the next tile's coefficients go over it
+    // 5. F_m = 2 pi / nphi sum_i f_i e^{-i m phi_i} and the analysis inputs RR,
+    //    RT, m/sin RP, TT + PP, TT - PP, TP (and the toroidal ones)
+    auto emit = [&](const Row& R, double* o0, int m, double re, double im) {
+      if (!R.live || m < 0 || m >= M) return;
+      const double ms = m * is, two = (R.q == 3 || R.q == 4) ? 2.0 * scl : scl;
+      const double2 F = make_double2(two * re, -two * im), Fm = make_double2(ms * F.x, ms * F.y);
+      double* o = o0 + (m >> 3) * mblock + (m & 7) * srow;
+      *reinterpret_cast<double2*>(o) = R.q == 2 ? Fm : F;
+      if (TOR && (R.q == 1 || R.q == 2 || R.q >= 4))
+        *reinterpret_cast<double2*>(o + (ptrdiff_t)2 * A.nf * (R.q == 5 ? 3 : 5)) = R.q == 1 ? Fm : F;
+    };
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      const Row R = row_of(rw + 8 * mt);
+      double* o0 = Sj + 2 * (row0 + rw + 8 * mt);
+#pragma unroll
+      for (int i = 0; i < NW; ++i) {
+        const int t = ng + 4 * i, m = 2 * (8 * t + 2 * lk);
+        if (t >= P.nta) continue;
+        emit(R, o0, TWIN ? half - m - 2 : m + 1, C[mt][i][2].x, C[mt][i][3].x);
+        emit(R, o0, m + 2, C[mt][i][0].x, C[mt][i][1].x);
+        emit(R, o0, TWIN ? half - m - 4 : m + 3, C[mt][i][2].y, C[mt][i][3].y);
+        emit(R, o0, m + 4, C[mt][i][0].y, C[mt][i][1].y);
+      }
+    }
+    if (tg % XT == 0) emit(row_of(xr), Sj + 2 * (row0 + xr), 0, x0, 0.0);
+  }
+}
+
+static void launch_lon(vg_handle* h, LonArgs A) {
+  const bool tor = h->tor_on;
+  void (*k)(const LonArgs) = nullptr;
+#define VG_LON(G_, MT_, NW_, ST_, TW_)                                                                             \
+  if (A.P.G == G_ && A.P.MT == MT_ && A.P.NW == NW_ && A.P.stab == ST_ && A.P.twin == TW_)                           \
+  k = tor ? k_v3_lon<G_, MT_, NW_, ST_ != 0, TW_ != 0, true> : k_v3_lon<G_, MT_, NW_, ST_ != 0, TW_ != 0, false>
+  VG_LON(3, 2, 1, 1, 1);
+  VG_LON(3, 2, 2, 1, 1);
+  VG_LON(2, 2, 1, 1, 0);
+  VG_LON(2, 2, 2, 1, 0);
+  VG_LON(1, 2, 3, 0, 0);
+  VG_LON(1, 2, 4, 0, 0);
+  VG_LON(1, 1, 6, 0, 0);
+#undef VG_LON
+  raise_smem_limit((const void*)k, A.P.smem);
+  int nsm = 0;
+  VG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
+  const int rows = A.P.G == 1 ? 16 * A.P.MT : 16;
+  const long long tiles = (long long)A.nlat * ((6 * A.nf + rows - 1) / rows);
+  k<<<(unsigned)std::min((tiles + A.P.G - 1) / A.P.G, (long long)nsm), A.P.G == 3 ? 384 : 256, A.P.smem, h->stream>>>(A);
+  ++h->n_launch;
+  VG_CUDA(cudaGetLastError());
 }
 
 // shared memory of the longitude pass (forward: adj = 0) and its transpose;
@@ -845,8 +1237,9 @@ __device__ __forceinline__ double v3_scatter_one(const V3Args& A, const T* __res
     if (NQ == 10) {  // lambda 3: (wD.RP + i wP.(m/sin RT)) / J; lambda 4: (wG.TP / 2 + i wH.(TT - PP)) / n4
       const double n4 = 0.25 * nn;
       double t[2][2];
-      t[0][0] = (q[NQ - 4][0] - q[NQ - 3][1]) / J;
-      t[0][1] = (q[NQ - 4][1] + q[NQ - 3][0]) / J;
+      const int d = A.tor_swap ? NQ - 4 : NQ - 3, p = A.tor_swap ? NQ - 3 : NQ - 4;  // wD.RP, wP.(m/sin RT)
+      t[0][0] = (q[d][0] - q[p][1]) / J;
+      t[0][1] = (q[d][1] + q[p][0]) / J;
       t[1][0] = n4 != 0.0 ? (0.5 * q[NQ - 2][0] - q[NQ - 1][1]) / n4 : 0.0;
       t[1][1] = n4 != 0.0 ? (0.5 * q[NQ - 2][1] + q[NQ - 1][0]) / n4 : 0.0;
       for (int ri = 0; ri < 2; ++ri)
@@ -989,9 +1382,10 @@ void visc3d_enable(vg_handle* h, const double* pert) {
   // work buffers and longitude tables of the FP64 path
   const int nf = 3 * h->ne3d, ncf = 2 * nf, nch = h->tor_on ? 6 : 4, np = h->tor_on ? 10 : 6;
   h->d_X.alloc((size_t)(h->nk + 1) * nch * ncf);
-  h->d_Y.alloc((size_t)G.M * G.nlat * np * ncf);
+  h->d_Y.alloc(s_rows(G.M, G.nlat) * np * ncf);
   h->d_dy.alloc((size_t)(h->nk + 1) * np * ncf);
   lon_tables_build(h);
+  lon_plan_tables(h);
   lon_check(h);  // the grid fits the longitude pass (throws otherwise)
   lon_attributes();
   VG_CUDA(cudaStreamSynchronize(s));
@@ -1051,6 +1445,7 @@ void visc3d_advance(vg_handle* h, const double* d_sigma, double dt, const double
       PhaseScope pg(h, VG_PH_V3_GATHER);
       A.gmax = visc3d_oz_gather_max(h);  // zeroes every scale group of the advance
       A.lm_rows = 1;
+      A.tor_swap = 1;
       if (h->tor_on)
         k_v3_gather<double, 6><<<gg, dim3(32, 8), v3_gather_smem<double, 6>(), s>>>(A, h->d_X.p);
       else
@@ -1099,18 +1494,21 @@ void visc3d_advance(vg_handle* h, const double* d_sigma, double dt, const double
   // longitude pass
   {
     PhaseScope pp(h, VG_PH_V3_LON_INV);
-    const dim3 lg(G.nlat, (nf + LON_LF - 1) / LON_LF);
-    if (h->tor_on)
-      k_v3_lon<LON_LF_TOR, 10>
-          <<<dim3(G.nlat, (nf + LON_LF_TOR - 1) / LON_LF_TOR), lon_threads(h, LON_LF_TOR),
-             lon_smem(h, LON_LF_TOR, false, 10), s>>>(h->d_Y.p, G.nlat, G.nphi, nf, dt, h->d_MkPerDt3.p,
-                                                      lon_tables(h), G.d_invsin.p, h->v3_gstore, trap ? 1 : 0);
-    else
-      k_v3_lon<LON_LF><<<lg, lon_threads(h, LON_LF), lon_smem(h, LON_LF, false), s>>>(
-          h->d_Y.p, G.nlat, G.nphi, nf, dt, h->d_MkPerDt3.p, lon_tables(h), G.d_invsin.p, h->v3_gstore,
-          trap ? 1 : 0);
-    ++h->n_launch;
-    VG_CUDA(cudaGetLastError());
+    LonArgs L;
+    L.P = lon_plan(h);
+    L.nlat = G.nlat;
+    L.nphi = G.nphi;
+    L.nf = nf;
+    L.trap = trap ? 1 : 0;
+    L.dt = dt;
+    L.S = h->d_Y.p;
+    L.rate = h->d_MkPerDt3.p;
+    L.invsin = G.d_invsin.p;
+    L.TM = h->d_lon_TM.p;
+    L.FS = h->d_lon_FS.p;
+    L.FA = h->d_lon_FA.p;
+    L.gstore = h->v3_gstore;
+    launch_lon(h, L);
   }
   // analysis
   gemm_tables(h, S, true);
@@ -1164,13 +1562,13 @@ __global__ void __launch_bounds__(256) k_v3_scatter_T(V3Args A, const double* __
     q[5][1] = nn != 0.0 ? 2.0 * L[3][0] / nn : 0.0;
     for (int p = 0; p < 6; ++p)
       for (int ri = 0; ri < 2; ++ri) row[(size_t)p * A.ncf + 2 * f + ri] = q[p][ri];
-    if (NQ == 10) {  // t0 = (q6 - i q7) / J, t1 = (q8 / 2 - i q9) / n4, transposed
+    if (NQ == 10) {  // t0 = (q7 + i q6) / J, t1 = (q8 / 2 + i q9) / n4, transposed
       double T[2][2];
       for (int ri = 0; ri < 2; ++ri)
         for (int lam_ = 0; lam_ < 2; ++lam_) T[lam_][ri] = lam_t[tmem_idx(s3, ri, e, lam_, k, A.ne, A.nk)];
       const double n4 = 0.25 * nn;
-      const double qt[4][2] = {{T[0][0] / J, T[0][1] / J},
-                               {T[0][1] / J, -T[0][0] / J},
+      const double qt[4][2] = {{T[0][1] / J, -T[0][0] / J},
+                               {T[0][0] / J, T[0][1] / J},
                                {n4 != 0.0 ? 0.5 * T[1][0] / n4 : 0.0, n4 != 0.0 ? 0.5 * T[1][1] / n4 : 0.0},
                                {n4 != 0.0 ? T[1][1] / n4 : 0.0, n4 != 0.0 ? -T[1][0] / n4 : 0.0}};
       for (int p = 0; p < 4; ++p)
@@ -1180,7 +1578,7 @@ __global__ void __launch_bounds__(256) k_v3_scatter_T(V3Args A, const double* __
 }
 
 // longitude pass transposed, one CTA per (latitude j, LF fields): the adjoint
-// chain on Yb in place: analysis-input combinations^T, analysis^T (a
+// chain on Yb in place, in the forward pass's rows: analysis-input scales^T, analysis^T (a
 // synthesis with weights 2 pi / nphi), times -M dt, synthesis^T (an analysis
 // with weights 1 at m = 0, 2 above), dyadic components^T; and
 // d J / d (M dt)(j, i) += -sum over components and shapes of G_bar g, g the
@@ -1215,8 +1613,8 @@ __global__ void __launch_bounds__(LON_THREADS, 1)
     const double Fb[6][2] = {{o[0][0], o[0][1]},
                              {o[1][0], o[1][1]},
                              {ms * o[2][0], ms * o[2][1]},
-                             {o[3][0] + o[4][0], o[3][1] + o[4][1]},
-                             {o[3][0] - o[4][0], o[3][1] - o[4][1]},
+                             {2.0 * o[3][0], 2.0 * o[3][1]},  // TT + PP and TT - PP are twice rows 3 and 4
+                             {2.0 * o[4][0], 2.0 * o[4][1]},
                              {o[5][0], o[5][1]}};
     for (int c = 0; c < 6; ++c) {
       A[(size_t)(fl * 6 + c) * wA + 2 * m] = scl * Fb[c][0];
@@ -1224,7 +1622,7 @@ __global__ void __launch_bounds__(LON_THREADS, 1)
     }
   }
   __syncthreads();
-  if (NQ == 10) {  // out6 = F2 (RP), out7 = ms F1, out8 = F5, out9 = F3 - F4, transposed and added
+  if (NQ == 10) {  // out6 = ms F1, out7 = F2 (RP), out8 = F5, out9 = 2 F4, transposed and added
     stage_in<NQ, 4>(Yb, X, nlat, ncf, j, f0, nft, T.M, 6);
     __syncthreads();
     for (int t = threadIdx.x; t < nft * T.M; t += blockDim.x) {
@@ -1234,10 +1632,10 @@ __global__ void __launch_bounds__(LON_THREADS, 1)
         for (int ri = 0; ri < 2; ++ri) o[q][ri] = X[((size_t)m * 4 + q) * 2 * nft + 2 * fl + ri];
       const double ms = m * is;
       const double add[6][2] = {{0.0, 0.0},
-                                {ms * o[1][0], ms * o[1][1]},
-                                {o[0][0], o[0][1]},
-                                {o[3][0], o[3][1]},
-                                {-o[3][0], -o[3][1]},
+                                {ms * o[0][0], ms * o[0][1]},
+                                {o[1][0], o[1][1]},
+                                {0.0, 0.0},
+                                {2.0 * o[3][0], 2.0 * o[3][1]},
                                 {o[2][0], o[2][1]}};
       for (int c = 1; c < 6; ++c) {
         A[(size_t)(fl * 6 + c) * wA + 2 * m] += scl * add[c][0];
@@ -1285,16 +1683,16 @@ __global__ void __launch_bounds__(LON_THREADS, 1)
     const double Sb[6][2] = {{cb[0][0], cb[0][1]},
                              {cb[1][0], cb[1][1]},
                              {ms * cb[2][1], -ms * cb[2][0]},
-                             {cb[3][0] + cb[4][0], cb[3][1] + cb[4][1]},
-                             {cb[3][0] - cb[4][0], cb[3][1] - cb[4][1]},
+                             {cb[3][0], cb[3][1]},
+                             {cb[4][0], cb[4][1]},
                              {4.0 * cb[5][1], -4.0 * cb[5][0]}};
     for (int q = 0; q < 6; ++q)
       for (int ri = 0; ri < 2; ++ri) A[((size_t)m * NQ + q) * 2 * nft + 2 * fl + ri] = Sb[q][ri];
-    if (NQ == 10) {  // P.X4 (rt -= i ms), D.X4 (rp), G.X5 (tp), H.X5 (tt -= i, pp += i), transposed
+    if (NQ == 10) {  // P.X4 (rt -= i ms), D.X4 (rp), G.X5 (tp), H.X5 ((tt - pp) / 2 -= i), transposed
       const double St[4][2] = {{-ms * cb[1][1], ms * cb[1][0]},
                                {cb[2][0], cb[2][1]},
                                {cb[5][0], cb[5][1]},
-                               {-cb[3][1] + cb[4][1], cb[3][0] - cb[4][0]}};
+                               {-cb[4][1], cb[4][0]}};
       for (int q = 0; q < 4; ++q)
         for (int ri = 0; ri < 2; ++ri) A[((size_t)m * NQ + 6 + q) * 2 * nft + 2 * fl + ri] = St[q][ri];
     }
@@ -1377,8 +1775,7 @@ __global__ void __launch_bounds__(256) k_v3_gather_T(V3Args A, const double* __r
 
 static void lon_attributes() {
   for (const void* k :
-       {(const void*)k_v3_lon<LON_LF>, (const void*)k_v3_lon<LON_LF_TOR, 10>, (const void*)k_v3_lon_T<LON_LF>,
-        (const void*)k_v3_lon_T<LON_LF_TOR, 10>})
+       {(const void*)k_v3_lon_T<LON_LF>, (const void*)k_v3_lon_T<LON_LF_TOR, 10>})
     VG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LON_SMEM_MAX));
 }
 
@@ -1392,7 +1789,7 @@ void visc3d_adjoint(vg_handle* h, const double* gstore, double dt, const double*
   const Grid& G = h->grid;
   cudaStream_t s = h->stream;
   const int nf = 3 * h->ne3d, ncf = 2 * nf, np = tor ? 10 : 6;
-  const size_t ny = (size_t)G.M * G.nlat * np * ncf, nr6 = (size_t)(h->nk + 1) * np * ncf;
+  const size_t ny = s_rows(G.M, G.nlat) * np * ncf, nr6 = (size_t)(h->nk + 1) * np * ncf;
   if (h->d_v3a_Yb.n != ny) {
     h->d_v3a_Yb.alloc(ny);
     h->d_v3a_dyb.alloc(nr6);  // slot row nk (degree 0) stays zero

@@ -1,4 +1,4 @@
-"""The FP64 3-D stress products at the edges of their tiles: row tiles of 40
+"""The FP64 3-D stress products and the longitude pass at the edges of their tiles: row tiles of 40
 northern latitudes (one, exactly full, one over), degree and latitude chunks
 with remainders, grids with an equator row and without and with more rows and
 columns than the transform needs, column counts below, at and past a
@@ -45,6 +45,15 @@ def models(lmax, nlat, nphi, counts, toroidal):
     (79, 80, 160, [1, 1, 1, 1], 0),    # 40 northern rows: a full row tile
     (80, 81, 162, [1, 1, 1, 1], 0),    # 41
     (81, 85, 170, [1, 1, 1, 1], 1),    # 43, more rows than the transform needs
+    # longitude tiles: odd half period with most and with few of its orders, tables in shared memory and from L2
+    (24, 25, 50, [1, 2, 1, 1], 0),
+    (20, 21, 66, [1, 1, 1, 1], 1),
+    (32, 33, 66, [1, 1, 1, 1], 1),
+    (47, 48, 100, [1, 1, 1, 1], 0),
+    (66, 67, 134, [1, 1, 1, 1], 0),
+    (30, 31, 262, [1, 1, 1, 1], 1),
+    (20, 21, 390, [1, 1, 1, 1], 0),
+    (16, 17, 520, [1, 1, 1, 1], 0),
 ])
 def test_products_match_oracle_at_tile_edges(lmax, nlat, nphi, counts, toroidal):
     g, o = models(lmax, nlat, nphi, counts, toroidal)
