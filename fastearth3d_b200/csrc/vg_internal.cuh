@@ -209,14 +209,13 @@ struct vg_handle {
       d_C, d_C0, d_C_next, d_dig, d_wcorr, d_Sraw, d_zbed, d_tmp;
   vg::DArr<double> d_F;        // Fourier coefficients (2 * M * nlat * batch)
   vg::DArr<double> d_Gs;       // Legendre sums (2 * M * nlat * batch)
-  vg::DArr<int2> d_sle_chunk;  // fused sea-level loop: Legendre synthesis chunks (m, first l - m)
-  vg::DArr<int> d_sle_cbeg;    // first chunk of each order
-  vg::DArr<double> d_sle_Gp;   // partial Legendre sums (chunk, nlat, 4)
-  int sle_nchunk = 0;
+  vg::DArr<double> d_sle_big;  // the fused sea-level pass's work area where shared memory is too small
+  int sle_mode = 0;     // its kernel variant and dynamic shared memory
+  size_t sle_shm = 0;
   vg::DArr<double> d_sigma, d_ulm, d_nlm;  // spectra (2*nlm)
-  vg::DArr<double> d_rowpart;  // per-row partial sums (8 * nlat)
-  vg::DArr<unsigned int> d_gbar;  // grid barrier of the fused inner loop: count, generation, error
-  int sle_grid = 0;               // CTAs of the cooperative inner-loop launch (one per SM)
+  vg::DArr<double> d_rowpart;  // per-row partial results (9 * nlat)
+  vg::DArr<unsigned int> d_gbar;  // grid barrier of the fused pass: arrivals, finished CTAs, error
+  int sle_grid = 0;               // CTAs of the cooperative launch of the pass (one per SM)
   // counters
   long long n_accept = 0, n_reject = 0, n_solve = 0, n_drift_solved = 0;
   int n_sub_last = 0, n_outer_last = 0, n_inner_last = 0, n_flip_last = 0;

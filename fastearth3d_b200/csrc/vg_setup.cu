@@ -987,7 +987,7 @@ void setup_handle(vg_handle* h) {
   h->d_sigma.alloc((size_t)2 * h->grid.nlm);
   h->d_ulm.alloc((size_t)2 * h->grid.nlm * 2);
   h->d_nlm.alloc((size_t)2 * h->grid.nlm);
-  h->d_rowpart.alloc((size_t)8 * nlat);
+  h->d_rowpart.alloc((size_t)9 * nlat);
   VG_CUDA(cudaStreamSynchronize(s));
 }
 

@@ -7,13 +7,15 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "vg_device.cuh"
 #include "vg_internal.cuh"
 
 namespace vg {
 
-enum { RP_C = 0, RP_DIG, RP_ZETA, RP_CS, RP_DMAX, RP_SMAX, RP_FLIP, RP_MASS, RP_N };
+// per-row partial results
+enum { RP_C = 0, RP_DIG, RP_ZETA, RP_CS, RP_DMAX, RP_DMIN, RP_SMAX, RP_SMIN, RP_MASS, RP_N };
 
 __device__ __forceinline__ double ocean(double topo, double ice) {
   return (topo < 0.0 && RHO_ICE * ice < -RHO_WATER * topo) ? 1.0 : 0.0;
@@ -29,34 +31,30 @@ __global__ void k_ice_interp(int ng, double frac, const double* __restrict__ ice
   dice_now[i] = v - ice_ref[i];
 }
 
-// C0 = ocean_function(topo0, ice - d_ice)  (src/vilma_sle.f90:212)
-__global__ void k_ocean0(int ng, const double* __restrict__ topo0, const double* __restrict__ ice,
-                         const double* __restrict__ dice, double* __restrict__ C0) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < ng) C0[i] = ocean(topo0[i], ice[i] - dice[i]);
-}
-// C = ocean_function(topo0 - rsl, ice)
-__global__ void k_ocean(int ng, const double* __restrict__ topo0, const double* __restrict__ rsl,
-                        const double* __restrict__ ice, double* __restrict__ C) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < ng) C[i] = ocean(topo0[i] - rsl[i], ice[i]);
-}
-
-// grounded-ice increment and the per-row sums of C, dIg, topo0 (C - C0)
-__global__ void k_pass_setup(int nphi, const double* __restrict__ ice, const double* __restrict__ dice,
-                             const double* __restrict__ C, const double* __restrict__ C0,
-                             const double* __restrict__ topo0, double* __restrict__ dig,
-                             double* __restrict__ rowpart, int nlat) {
+// Fields of one pass, a block per row: C0 = ocean_function(topo0, ice - d_ice)
+// (src/vilma_sle.f90:212; once a solve, `set_c0`), the pass's ocean function (C0
+// with a fixed ocean, else ocean_function(topo0 - rsl, ice) in the first pass of a
+// co-convergence iteration, `io1`, and the migrated coastline Cn after it), the
+// grounded-ice increment, and the row sums of C, dIg, topo0 (C - C0)
+__global__ void k_pass_setup(int nphi, int nlat, int set_c0, int io1, int fixed, const double* __restrict__ ice,
+                             const double* __restrict__ dice, const double* __restrict__ topo0,
+                             const double* __restrict__ rsl, const double* __restrict__ Cn, double* __restrict__ C0,
+                             double* __restrict__ C, double* __restrict__ dig, double* __restrict__ rowpart) {
   __shared__ double red[128];
   int j = blockIdx.x;
   double sc = 0.0, sd = 0.0, sz = 0.0;
   for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
     size_t p = (size_t)j * nphi + i;
-    double d = ice[p] * (1.0 - C[p]) - (ice[p] - dice[p]) * (1.0 - C0[p]);
+    const double h = ice[p], h0 = h - dice[p], t0 = topo0[p];
+    const double c0 = set_c0 ? ocean(t0, h0) : C0[p];
+    const double c = fixed ? c0 : io1 ? ocean(t0 - rsl[p], h) : Cn[p];
+    if (set_c0) C0[p] = c0;
+    C[p] = c;
+    double d = h * (1.0 - c) - h0 * (1.0 - c0);
     dig[p] = d;
-    sc += C[p];
+    sc += c;
     sd += d;
-    sz += topo0[p] * (C[p] - C0[p]);
+    sz += t0 * (c - c0);
   }
   sc = block_sum(sc, red);
   sd = block_sum(sd, red);
@@ -68,192 +66,26 @@ __global__ void k_pass_setup(int nphi, const double* __restrict__ ice, const dou
   }
 }
 
-// Surface integral of a row-sum vector, sum_j w_j row_j 2 pi / nphi
-// (src/vilma_sht.f90:184-202), summed in row order like the reference. The
-// finalizer kernels run one block: every thread stages a slice of the terms
-// in shared memory (one coalesced pass), then thread 0 adds them in order.
-// The result is valid in thread 0.
-constexpr int FIN_THREADS = 128, FIN_SEG = 1024;
-__device__ double integrate_rows(const double* row, const double* w, int nlat, double dlon) {
-  __shared__ double term[FIN_SEG];
-  double total = 0.0;
-  for (int j0 = 0; j0 < nlat; j0 += FIN_SEG) {
-    const int n = min(FIN_SEG, nlat - j0);
-    __syncthreads();
-    for (int j = threadIdx.x; j < n; j += blockDim.x) term[j] = w[j0 + j] * row[j0 + j] * dlon;
-    __syncthreads();
-    if (threadIdx.x == 0) {  // in row order; the loads run ahead of the dependent adds
-      int j = 0;
-      for (; j + 8 <= n; j += 8) {
-        double t[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) t[q] = term[j + q];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) total += t[q];
-      }
-      for (; j < n; ++j) total += term[j];
-    }
-  }
-  return total;
-}
-
-// the pass's ocean area, then (with an ocean) its ice and subgrid integrals
-__global__ void k_finalize_pass(SleScalars* sc, const double* __restrict__ rowpart, const double* __restrict__ w,
-                                int nlat, double dlon, int subgrid) {
-  __shared__ double s_c;
-  const double c = integrate_rows(rowpart + RP_C * nlat, w, nlat, dlon);  // valid in thread 0
-  if (threadIdx.x == 0) {
-    sc->C_int = c;
-    s_c = c;
-  }
-  __syncthreads();
-  if (!(s_c > 0.0)) return;  // no ocean: the pass ends here (src/vilma_sle.f90:273-274)
-  const double d = integrate_rows(rowpart + RP_DIG * nlat, w, nlat, dlon);
-  const double z = subgrid ? integrate_rows(rowpart + RP_ZETA * nlat, w, nlat, dlon) : 0.0;
-  if (threadIdx.x == 0) {
-    sc->ice_int = -(RHO_ICE / RHO_WATER) * d;
-    sc->zeta_int = z;
-  }
-}
-__global__ void k_wcorr(const SleScalars* sc, int ng, int subgrid, const double* __restrict__ topo0,
-                        const double* __restrict__ C, const double* __restrict__ C0, double* __restrict__ wcorr) {
-  if (!(sc->C_int > 0.0)) return;  // no ocean
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < ng) wcorr[i] = subgrid ? -RHO_WATER * topo0[i] * (C[i] - C0[i]) : 0.0;
-}
-
-// total surface load (assemble_load, src/vilma_sle.f90:387-403) and its longitude transform
+// the closing load of a solve whose last pass had no ocean: total surface load
+// (assemble_load, src/vilma_sle.f90:387-403), its longitude transform, row sums of C rsl
 __global__ void k_load_fourier(int nphi, int nlat, int M, const double* __restrict__ dig,
                                const double* __restrict__ C, const double* __restrict__ rsl,
                                const double* __restrict__ wcorr, const double* __restrict__ cs,
-                               const double* __restrict__ sn, double* __restrict__ F) {
+                               const double* __restrict__ sn, double* __restrict__ F,
+                               double* __restrict__ rowpart) {
   extern __shared__ double row[];
-  int j = blockIdx.x;
-  for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
-    size_t p = (size_t)j * nphi + i;
-    row[i] = RHO_ICE * dig[p] + RHO_WATER * (C[p] * rsl[p]) + wcorr[p];
-  }
-  __syncthreads();
-  row_fourier_analysis(row, nphi, M, cs, sn, F + (size_t)j * 2, nlat);
-}
-
-// u and N rows from their Legendre sums, Sraw = N - u (+ s_rot), row sum of C Sraw
-__global__ void k_synth_sraw(int nphi, int nlat, int M, const double* __restrict__ G, const double* __restrict__ cs,
-                             const double* __restrict__ sn, const double* __restrict__ C,
-                             const double* __restrict__ srot, double* __restrict__ Sraw,
-                             double* __restrict__ rowpart) {
-  extern __shared__ double sh[];  // Gu[M][2], Gn[M][2]
-  __shared__ double red[128];
-  int j = blockIdx.x;
-  double* Gu = sh;
-  double* Gn = sh + 2 * M;
-  for (int m = threadIdx.x; m < M; m += blockDim.x) {
-    Gu[2 * m] = G[((size_t)m * nlat + j) * 2];
-    Gu[2 * m + 1] = G[((size_t)m * nlat + j) * 2 + 1];
-    Gn[2 * m] = G[(((size_t)M + m) * nlat + j) * 2];
-    Gn[2 * m + 1] = G[(((size_t)M + m) * nlat + j) * 2 + 1];
-  }
-  __syncthreads();
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
-    size_t p = (size_t)j * nphi + i;
-    double u = row_fourier_synth_at(Gu, M, i, nphi, cs, sn);
-    double N = row_fourier_synth_at(Gn, M, i, nphi, cs, sn);
-    double s = N - u;
-    if (srot) s = s + srot[p];
-    Sraw[p] = s;
-    acc += C[p] * s;
-  }
-  acc = block_sum(acc, red);
-  if (threadIdx.x == 0) rowpart[RP_CS * nlat + j] = acc;
-}
-
-__global__ void k_dphi(SleScalars* sc, const double* __restrict__ rowpart, const double* __restrict__ w, int nlat,
-                       double dlon) {
-  const double Cs = integrate_rows(rowpart + RP_CS * nlat, w, nlat, dlon);
-  if (threadIdx.x == 0) {
-    sc->Cs_int = Cs;
-    sc->dphi = (sc->ice_int - Cs + sc->zeta_int) / sc->C_int;
-  }
-}
-
-__global__ void k_rsl_update(int nphi, const SleScalars* __restrict__ sc, const double* __restrict__ Sraw,
-                             const double* __restrict__ C, double* __restrict__ rsl, double* __restrict__ rowpart,
-                             int nlat) {
-  __shared__ double red[128];
-  int j = blockIdx.x;
-  double dphi = sc->dphi, dmax = 0.0, smax = 0.0;
-  for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
-    size_t p = (size_t)j * nphi + i;
-    double rn = Sraw[p] + dphi;
-    dmax = nanmax(dmax, fabs(C[p] * (rn - rsl[p])));
-    rsl[p] = rn;
-    smax = nanmax(smax, fabs(C[p] * rn));
-  }
-  dmax = block_max(dmax, red);
-  smax = block_max(smax, red);
-  if (threadIdx.x == 0) {
-    rowpart[RP_DMAX * nlat + j] = dmax;
-    rowpart[RP_SMAX * nlat + j] = smax;
-  }
-}
-
-__global__ void k_conv(SleScalars* sc, const double* __restrict__ rowpart, int nlat) {
-  __shared__ double red[FIN_THREADS];
-  double dmax = 0.0, smax = 0.0;
-  for (int j = threadIdx.x; j < nlat; j += blockDim.x) {
-    dmax = nanmax(dmax, rowpart[RP_DMAX * nlat + j]);
-    smax = nanmax(smax, rowpart[RP_SMAX * nlat + j]);
-  }
-  dmax = block_max(dmax, red);
-  smax = block_max(smax, red);
-  if (threadIdx.x == 0) {
-    sc->dmax = dmax;
-    sc->smax = smax;
-  }
-}
-
-// migrated coastline and the number of cells that changed state
-__global__ void k_coast(int nphi, const double* __restrict__ topo0, const double* __restrict__ rsl,
-                        const double* __restrict__ ice, const double* __restrict__ C, double* __restrict__ Cn,
-                        double* __restrict__ rowpart, int nlat) {
-  __shared__ double red[128];
-  int j = blockIdx.x;
-  double cnt = 0.0;
-  for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
-    size_t p = (size_t)j * nphi + i;
-    double c = ocean(topo0[p] - rsl[p], ice[p]);
-    Cn[p] = c;
-    cnt += (c != C[p]) ? 1.0 : 0.0;
-  }
-  cnt = block_sum(cnt, red);
-  if (threadIdx.x == 0) rowpart[RP_FLIP * nlat + j] = cnt;
-}
-__global__ void k_flips(SleScalars* sc, const double* __restrict__ rowpart, int nlat) {
-  __shared__ double red[FIN_THREADS];
-  double t = 0.0;  // integer-valued row counts: exact in any order
-  for (int j = threadIdx.x; j < nlat; j += blockDim.x) t += rowpart[RP_FLIP * nlat + j];
-  t = block_sum(t, red);
-  if (threadIdx.x == 0) sc->flips = (int)t;
-}
-
-// row sums of a * b (b may be null: sum of a), into rowpart slot
-__global__ void k_rowsum(int nphi, const double* __restrict__ a, const double* __restrict__ b,
-                         double* __restrict__ out) {
   __shared__ double red[128];
   int j = blockIdx.x;
   double s = 0.0;
   for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
     size_t p = (size_t)j * nphi + i;
-    s += b ? a[p] * b[p] : a[p];
+    row[i] = RHO_ICE * dig[p] + RHO_WATER * (C[p] * rsl[p]) + wcorr[p];
+    s += C[p] * rsl[p];
   }
   s = block_sum(s, red);
-  if (threadIdx.x == 0) out[j] = s;
-}
-__global__ void k_mass(SleScalars* sc, const double* __restrict__ rowpart, const double* __restrict__ w, int nlat,
-                       double dlon) {
-  const double m = integrate_rows(rowpart + RP_MASS * nlat, w, nlat, dlon);
-  if (threadIdx.x == 0) sc->mass_Cs = m - sc->zeta_int;
+  if (threadIdx.x == 0) rowpart[RP_MASS * nlat + j] = s;
+  __syncthreads();
+  row_fourier_analysis(row, nphi, M, cs, sn, F + (size_t)j * 2, nlat);
 }
 
 // z_bed = z_bed_eq - rsl (src/vilma_coupling.f90:428)
@@ -282,36 +114,49 @@ __global__ void k_bsl_rows(int nphi, const double* __restrict__ hi, const double
   }
 }
 
-// ------------------------------------------------------------------ fused inner loop
-// The inner load fixed point of sle_solve (src/vilma_sle.f90:280-340) as one
-// cooperative persistent kernel: one CTA per SM, the convergence test on the
-// device, so no host round trip per iteration. Four grid barriers an
-// iteration:
-//   L  total load of each row and its longitude analysis (the CTA that owns
-//      the row; for the next iteration it runs right after U, on the rows the
-//      CTA has just updated)
-//   A  Legendre analysis + apply, warp per lm                 | barrier
-//   S  Legendre synthesis of u and N, thread per (b, m, j)    | barrier
-//   R  longitude synthesis, Sraw = N - u (+ s_rot), row sums  | barrier
-//   U  mass-conserving dphi (every CTA, rows summed in order by one thread,
-//      so all CTAs agree), rsl update, row maxima, then L     | barrier
-//   convergence (every CTA from the row maxima, the same decision everywhere)
-// The longitude transforms split the half periods (phi + pi flips odd m) and
-// spread each output's sum over several threads, so no thread runs a loop of
-// more than about nphi / 6 terms.
-constexpr int SLE_LCH = 16;  // degrees per Legendre synthesis chunk
+// ------------------------------------------------------------------ fused pass
+// One outer pass of sle_solve (src/vilma_sle.f90:266-352) as one cooperative
+// persistent kernel: the pass integrals, the inner load fixed point with its
+// convergence test on the device, the closing load's spectrum, the migrated
+// coastline and the mass integral. An iteration of the fixed point is two
+// phases with one grid barrier each:
+//   O  the CTA that owns an order: Legendre analysis of the load, the affine
+//      response, Legendre synthesis of N - u (one field: the two differ in the
+//      spectrum already), northern rows with the equatorial symmetry
+//   R  the CTA that owns a row: longitude synthesis, Sraw = N - u (+ s_rot), the
+//      row's part of int C Sraw, the load of rsl = Sraw and its longitude
+//      analysis
+// The mass-conserving dphi is a constant of the grid, so it enters after the
+// fact: the load of rsl = Sraw + dphi is that of Sraw plus dphi times the load of
+// rho_w C, whose spectrum is formed once, and the convergence test
+// max |C (rsl_new - rsl_old)| comes from the row extremes of Sraw_new - rsl_old
+// over the ocean (C is 0 or 1), all known at the one barrier after R.
+//
+// What bounds it: latency. The work of an iteration (0.1 MFLOP an order or a row)
+// is a few hundred FP64 cycles a CTA; the two barriers, the L2 round trips of
+// the exchanged rows and the block barriers inside a phase are the rest. The
+// longitude transforms use the reflection and half-period symmetries (four sums
+// over a quarter of the longitudes), every sum is spread over the 512 threads.
+// Five phases with four barriers, two syntheses and serial row integrals took 254
+// us a pass of eight iterations at lmax 128 (1004 at lmax 256), beside 70 us of
+// small kernels for the integrals, the coastline and the closing load that the
+// pass now holds; it takes 100 us (362). Of an iteration's cycles at lmax 128 the
+// barriers are 4700, O 9000 (order 0, which the others wait for), R 12000.
+constexpr int SLE_THREADS = 512;
 
-struct InnerArgs {
-  int nphi, nlat, M, nlm, nk, lmax, n_inner;
+// pitch of the Legendre functions in shared memory: half warps of two degrees by
+// eight rows read different banks
+__host__ __device__ inline int p_pitch(int nh) { return (nh + 7) / 16 * 16 + 8; }
+
+struct PassArgs {
+  int nphi, nlat, M, nlm, nk, lmax, n_inner, subgrid, fixed;
   double tol, dlon, g;
-  const double *dig, *C, *wcorr, *cs, *sn, *plm, *wts, *gu, *gn, *drift, *srot;
-  const int *lm_m, *lm_l, *lm2k, *mbeg;
-  const int2* chunk;  // Legendre synthesis chunks: (m, first l - m), at most SLE_LCH degrees each
-  const int* cbeg;    // first chunk of each order (M + 1)
-  int nchunk;
-  double *rsl, *F, *sigma, *ulm, *Gp, *Sraw, *rowpart;
+  const double *ice, *topo0, *C0, *dig, *C, *cs, *sn, *plm, *wts, *gu, *gn, *drift, *srot;
+  const int *lm2k, *mbeg;
+  double *wcorr, *rsl, *F, *FC, *sigma, *cst, *D, *Sraw, *Cn, *rowpart, *big;
+  size_t scr;  // doubles of the work area
   SleScalars* sc;
-  unsigned int* bar;  // count, generation, error
+  unsigned int* bar;  // arrivals, finished CTAs, error
   unsigned long long wait_ns;  // bound on a grid barrier's wait (the handle's wait limit, 2 s by default)
 };
 
@@ -321,371 +166,639 @@ __device__ __forceinline__ unsigned long long gtimer_ns() {
   return t;
 }
 
-// Sense-counting grid barrier with a bounded wait. Returns false (in every
-// thread of the CTA) if it timed out or another CTA reported a timeout.
-__device__ bool grid_barrier(unsigned int* bar, unsigned int& gen, unsigned long long wait_ns) {
+// Grid barrier: arrivals counted up to `target`, with a bounded wait. Returns
+// false (in every thread of the CTA) if it timed out or another CTA reported a
+// timeout. What other CTAs wrote before it is read with ld.cg after it.
+__device__ bool grid_barrier(unsigned int* bar, unsigned int& target, unsigned long long wait_ns) {
   __shared__ int s_ok;
   __syncthreads();
+  target += gridDim.x;
   if (threadIdx.x == 0) {
     int ok = 1;
-    volatile unsigned int* vgen = bar + 1;
-    __threadfence();
-    const unsigned int arrived = atomicAdd(bar, 1u);
-    if (arrived == gridDim.x - 1) {
-      bar[0] = 0u;
-      __threadfence();
-      atomicExch(bar + 1, gen + 1u);
-    } else {
-      const unsigned long long t0 = gtimer_ns();
-      while (*vgen == gen) {
-        if (gtimer_ns() - t0 > wait_ns) {
-          atomicExch(bar + 2, 1u);
-          ok = 0;
-          break;
-        }
-        __nanosleep(64);
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    const unsigned long long t0 = gtimer_ns();
+    for (int n = 0;; ++n) {
+      unsigned int v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      if ((int)(v - target) >= 0) break;
+      // the timer is read now and then (each time for a limit too short for that)
+      if ((wait_ns < 10000 || (n & 15) == 15) &&
+          (gtimer_ns() - t0 > wait_ns || *(volatile unsigned int*)(bar + 2))) {
+        atomicExch(bar + 2, 1u);
+        ok = 0;
+        break;
       }
     }
-    __threadfence();
-    if (*(volatile unsigned int*)(bar + 2)) ok = 0;
     s_ok = ok;
   }
-  ++gen;
   __syncthreads();
   return s_ok != 0;
 }
 
-// L for row j: the total surface load and its longitude analysis into F
-// (F_m = 2 pi / nphi sum_i f_i e^{-i m phi_i}; even m read f_i + f_{i+half},
-// odd m f_i - f_{i+half}); tpm threads per order, partial sums in part[2][nthr]
-__device__ __forceinline__ void sle_row_load(const InnerArgs& A, int j, double* sm, double* part) {
-  const int tid = threadIdx.x, nthr = blockDim.x, nphi = A.nphi, M = A.M, half = nphi / 2;
-  const double sc_f = 2.0 * PI / (double)nphi;
-  __syncthreads();
-  for (int i = tid; i < nphi; i += nthr) {
-    const size_t p = (size_t)j * nphi + i;
-    sm[i] = RHO_ICE * A.dig[p] + RHO_WATER * (A.C[p] * A.rsl[p]) + A.wcorr[p];
-  }
-  __syncthreads();
-  const int tpm = max(1, min(8, nthr / M));
-  for (int base = 0; base < M * tpm; base += nthr) {
-    const int u = base + tid, m = u / tpm, q = u % tpm;
-    const bool act = u < M * tpm;
-    double re = 0.0, im = 0.0;
-    if (act) {
-      const double sg = (m & 1) ? -1.0 : 1.0;
-      const int step = (m * tpm) % nphi;
-      int t = (m * q) % nphi;
-      for (int i = q; i < half; i += tpm) {
-        const double v = sm[i] + sg * sm[i + half];
-        re += v * __ldg(&A.cs[t]);
-        im -= v * __ldg(&A.sn[t]);
-        t += step;
-        if (t >= nphi) t -= nphi;
-      }
-    }
-    part[tid] = re;
-    part[nthr + tid] = im;
-    __syncthreads();
-    if (act && q == 0) {
-      double r = 0.0, s2 = 0.0;
-      for (int c = 0; c < tpm; ++c) {
-        r += part[tid + c];
-        s2 += part[nthr + tid + c];
-      }
-      A.F[((size_t)m * A.nlat + j) * 2] = r * sc_f;
-      A.F[((size_t)m * A.nlat + j) * 2 + 1] = s2 * sc_f;
-    }
-    __syncthreads();
-  }
-}
-
 // a grid barrier gave up: record it where the host reads the loop's scalars
-__device__ __forceinline__ void bar_fail(const InnerArgs& A) {
+__device__ __forceinline__ void bar_fail(const PassArgs& A) {
   if (threadIdx.x == 0) A.sc->bar_error = 1;
 }
 
-__global__ void __launch_bounds__(512) k_sle_inner(InnerArgs A) {
-  extern __shared__ double sm[];  // max(nphi, 4 M + 4 nchunk) doubles
-  __shared__ double red[512];
-  __shared__ double part[4 * 512];
-  __shared__ double s_val;
-  __shared__ int s_stop;
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  const int lane = tid & 31, wid = tid >> 5, nw = nthr >> 5;
-  const int nphi = A.nphi, nlat = A.nlat, M = A.M, nlm = A.nlm, half = nphi / 2;
-  unsigned int gen = 0;
-  if (!(A.sc->C_int > 0.0)) return;  // no ocean: nothing to redistribute (every CTA reads the same value)
-  // L of the first iteration
-  for (int j = blockIdx.x; j < nlat; j += gridDim.x) sle_row_load(A, j, sm, part);
-  if (!grid_barrier(A.bar, gen, A.wait_ns)) return bar_fail(A);
-  for (int it = 1; it <= A.n_inner; ++it) {
-    // A. Legendre analysis (warp per lm, four lm of a warp at once) and the
-    //    affine response u, N
-    for (int lm0 = blockIdx.x * nw + wid; lm0 < nlm; lm0 += 4 * gridDim.x * nw) {
-      constexpr int U4 = 4;
-      double re[U4], im[U4];
-      int lmv[U4];
-      const double* Fm[U4];
-      const double* P[U4];
+// sum_j w_j row_j 2 pi / nphi (src/vilma_sht.f90:184-202) by one warp, the same
+// value in every lane and CTA
+__device__ __forceinline__ double warp_rows(const double* row, const double* w, int nlat, double dlon) {
+  double s = 0.0;
+  for (int j0 = threadIdx.x & 31; j0 < nlat; j0 += 256) {
+    double t[8];
 #pragma unroll
-      for (int u = 0; u < U4; ++u) {
-        lmv[u] = lm0 + u * gridDim.x * nw;
-        const int lmc = min(lmv[u], nlm - 1);  // past the end: a valid row, result unused
-        Fm[u] = A.F + ((size_t)A.lm_m[lmc] * nlat) * 2;
-        P[u] = A.plm + (size_t)lmc * nlat;
-        re[u] = 0.0;
-        im[u] = 0.0;
-      }
-      for (int j = lane; j < nlat; j += 32) {
-        const double w = A.wts[j];
+    for (int u = 0; u < 8; ++u) t[u] = j0 + 32 * u < nlat ? w[j0 + 32 * u] * __ldcg(row + j0 + 32 * u) * dlon : 0.0;
 #pragma unroll
-        for (int u = 0; u < U4; ++u) {
-          const double wp = w * P[u][j];
-          re[u] += wp * Fm[u][2 * j];
-          im[u] += wp * Fm[u][2 * j + 1];
-        }
-      }
+    for (int u = 0; u < 8; ++u) s += t[u];
+  }
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+// largest value of a warp, in every lane, by two integer reductions on the
+// order-preserving bit pattern (a positive NaN counts as the largest)
+__device__ __forceinline__ double warp_max(double v) {
+  const long long b = __double_as_longlong(v);
+  const unsigned long long k = (unsigned long long)b ^ (b < 0 ? ~0ull : 1ull << 63);
+  const unsigned int hi = (unsigned int)(k >> 32);
+  const unsigned int H = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned int L = __reduce_max_sync(0xffffffffu, hi == H ? (unsigned int)k : 0u);
+  const unsigned long long r = ((unsigned long long)H << 32) | L;
+  return __longlong_as_double((long long)(r ^ ((r >> 63) ? 1ull << 63 : ~0ull)));
+}
+
+// twiddle table in shared memory, skewed so that strides of 2, 4 and 8 entries
+// fall in different banks
+__device__ __forceinline__ int tw_at(int t) { return t + (t >> 3); }
+
+// Longitudes of base longitude i: i, i + half, nphi - i, half - i (nphi odd: i
+// and nphi - i only); the last two only where they are points of their own
+struct Lon {
+  int nphi, half, nbase;
+  bool even;
+  __device__ __forceinline__ Lon(int n) : nphi(n), half(n / 2), nbase(n % 2 ? (n + 1) / 2 : n / 4 + 1), even(n % 2 == 0) {}
+  __device__ __forceinline__ int at(int i, int pt) const {
+    return pt == 0 ? i : pt == 1 ? i + half : pt == 2 ? nphi - i : half - i;
+  }
+  __device__ __forceinline__ bool has(int i, int pt) const {
+    if (pt == 0) return true;
+    if (!even) return pt == 2 && i > 0;
+    return pt == 1 || (i > 0 && 2 * i != half);
+  }
+};
+
+// This thread's share of a longitude sum over `n` outputs with Q parts each:
+// part q of output o, the twiddle index t0 of its first term and the step between
+// its terms (a term advances the index by o, `mul` terms of other parts between)
+struct Share {
+  int Q, q, o, t0, step;
+  __device__ __forceinline__ Share(int n, int mul, int nphi, int u) {
+    Q = max(1, min(16, SLE_THREADS / n));
+    q = u / n;
+    o = u - q * n;
+    t0 = (int)(((unsigned)(mul * q) * (unsigned)o) % (unsigned)nphi);
+    step = (int)(((unsigned)(mul * Q) * (unsigned)o) % (unsigned)nphi);
+  }
+};
+
+struct PassSmem {  // carved from the dynamic shared memory
+  double2 *tw, *Gd, *Fe, *dl;  // twiddles; a row's spectrum; an order's rows [4][nh]; its degrees
+  double *X, *L;               // per base longitude four values; a row of the grid
+};
+
+// F(m) = 2 pi / nphi sum_i L_i e^{-i m phi_i} of the row in S.L, to out[m stride]
+__device__ __forceinline__ void row_analysis(const Lon& G, int M, const PassSmem& S, const Share& A0, double* part,
+                                             double2* out, int stride) {
+  const int tid = threadIdx.x;
+  for (int i = tid; i < G.nbase; i += SLE_THREADS) {
+    double v[4];
 #pragma unroll
-      for (int u = 0; u < U4; ++u)
-        for (int o = 16; o > 0; o >>= 1) {
-          re[u] += __shfl_down_sync(0xffffffffu, re[u], o);
-          im[u] += __shfl_down_sync(0xffffffffu, im[u], o);
-        }
-      // lanes 0..3 write lm u (the sums are in lane 0; broadcast them)
-#pragma unroll
-      for (int u = 0; u < U4; ++u) {
-        re[u] = __shfl_sync(0xffffffffu, re[u], 0);
-        im[u] = __shfl_sync(0xffffffffu, im[u], 0);
-      }
-      if (lane < U4) {
-        double r = re[0], i2 = im[0];
-#pragma unroll
-        for (int u = 1; u < U4; ++u)
-          if (lane == u) {
-            r = re[u];
-            i2 = im[u];
-          }
-        const int lm = lmv[lane];
-        if (lm < nlm) {
-          A.sigma[2 * lm] = r;
-          A.sigma[2 * lm + 1] = i2;
-          const int l = A.lm_l[lm];
-          double* uu = A.ulm;
-          double* n = A.ulm + 2 * (size_t)nlm;
-          if (l == 0) {
-            uu[2 * lm] = A.gu[0] * r;
-            uu[2 * lm + 1] = A.gu[0] * i2;
-            n[2 * lm] = A.gn[0] * r;
-            n[2 * lm + 1] = A.gn[0] * i2;
-          } else {
-            const int k = A.lm2k[lm];
-            uu[2 * lm] = A.gu[l] * r + A.drift[(size_t)0 * A.nk + k];
-            uu[2 * lm + 1] = A.gu[l] * i2 + A.drift[(size_t)1 * A.nk + k];
-            n[2 * lm] = A.gn[l] * r - A.drift[(size_t)2 * A.nk + k] / A.g;
-            n[2 * lm + 1] = A.gn[l] * i2 - A.drift[(size_t)3 * A.nk + k] / A.g;
-          }
-        }
-      }
+    for (int pt = 0; pt < 4; ++pt) v[pt] = G.has(i, pt) ? S.L[G.at(i, pt)] : 0.0;
+    double4 x;
+    if (G.even) {
+      const double ab = v[0] + v[1], am = v[0] - v[1], cd = v[2] + v[3], cm = v[2] - v[3];
+      x = make_double4(ab + cd, ab - cd, am + cm, am - cm);
+    } else {
+      x = make_double4(v[0] + v[2], v[0] - v[2], v[0] + v[2], v[0] - v[2]);
     }
-    if (!grid_barrier(A.bar, gen, A.wait_ns)) return bar_fail(A);
-    // S. Legendre synthesis of u and N in chunks of at most SLE_LCH degrees: a
-    //    thread per (chunk, j), partial sums Gp[j][chunk][u re, u im, N re, N im]
-    //    (one 32-byte sector per thread; a row's partials contiguous)
-    for (int t = blockIdx.x * nthr + tid; t < A.nchunk * nlat; t += gridDim.x * nthr) {
-      const int c = t / nlat, j = t % nlat;
-      const int2 ch = A.chunk[c];
-      const int n = min(SLE_LCH, A.lmax - ch.x + 1 - ch.y);
-      const int lm = A.mbeg[ch.x] + ch.y;
-      const double* pc = A.plm + (size_t)lm * nlat + j;
-      const double* qu = A.ulm + 2 * (size_t)lm;
-      const double* qn = A.ulm + 2 * ((size_t)nlm + lm);
-      double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+    reinterpret_cast<double2*>(S.X)[2 * i] = make_double2(x.x, x.y);
+    reinterpret_cast<double2*>(S.X)[2 * i + 1] = make_double2(x.z, x.w);
+  }
+  __syncthreads();
+  const int Q = A0.Q;
+  const double sc = 2.0 * PI / (double)G.nphi;
+  for (int base = 0; base < M * Q; base += SLE_THREADS) {
+    const Share sh = base ? Share(M, 1, G.nphi, base + tid) : A0;
+    const int m = sh.o;
+    double re = 0.0, im = 0.0;
+    if (base + tid < M * Q) {
+      const double2* x = reinterpret_cast<const double2*>(S.X) + (m & 1);
+      int t = sh.t0;
 #pragma unroll 4
-      for (int q = 0; q < n; ++q) {
-        const double p = pc[(size_t)q * nlat];
-        a0 += qu[2 * q] * p;
-        a1 += qu[2 * q + 1] * p;
-        a2 += qn[2 * q] * p;
-        a3 += qn[2 * q + 1] * p;
+      for (int i = sh.q; i < G.nbase; i += Q) {
+        const double2 w = S.tw[tw_at(t)], v = x[2 * i];
+        re = fma(v.x, w.x, re);
+        im = fma(-v.y, w.y, im);
+        t += sh.step;
+        if (t >= G.nphi) t -= G.nphi;
       }
-      double* o = A.Gp + ((size_t)j * A.nchunk + c) * 4;
-      o[0] = a0;
-      o[1] = a1;
-      o[2] = a2;
-      o[3] = a3;
     }
-    if (!grid_barrier(A.bar, gen, A.wait_ns)) return bar_fail(A);
-    // R. longitude synthesis (g(i) = G_0 + 2 sum_m Re G_m e^{i m phi_i}, even and
-    //    odd m apart, tpi threads per longitude pair (i, i + half)),
-    //    Sraw = N - u (+ s_rot), row sums of C Sraw
-    for (int j = blockIdx.x; j < nlat; j += gridDim.x) {
-      double* Gu = sm;
-      double* Gn = sm + 2 * M;
-      double* gp = sm + 4 * M;  // the row's partial sums, staged
+    if (Q == 1) {
+      if (base + tid < M) __stcg(out + (size_t)m * stride, make_double2(re * sc, im * sc));
+    } else {
+      part[2 * tid] = re;
+      part[2 * tid + 1] = im;
       __syncthreads();
-      for (int t = tid; t < 4 * A.nchunk; t += nthr) gp[t] = A.Gp[(size_t)j * A.nchunk * 4 + t];
-      __syncthreads();
-      for (int m = tid; m < M; m += nthr) {  // the order's chunks summed in order
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-        for (int c = A.cbeg[m]; c < A.cbeg[m + 1]; ++c) {
-          const double* o = gp + 4 * c;
-          a0 += o[0];
-          a1 += o[1];
-          a2 += o[2];
-          a3 += o[3];
+      if (tid < M) {
+        for (int c = 1; c < Q; ++c) {
+          re += part[2 * (tid + c * M)];
+          im += part[2 * (tid + c * M) + 1];
         }
-        Gu[2 * m] = a0;
-        Gu[2 * m + 1] = a1;
-        Gn[2 * m] = a2;
-        Gn[2 * m + 1] = a3;
+        __stcg(out + (size_t)m * stride, make_double2(re * sc, im * sc));
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// A CTA with one order keeps that order's Legendre functions (northern rows) in
+// shared memory (MODE 1), where they fit: the barriers invalidate L1, so read
+// through it (MODE 0) they come from L2 in each iteration (106 us a pass at lmax
+// 128 and 77 at lmax 85, against 100 and 76). MODE 2, a grid whose
+// work area does not fit in shared memory: the work area is A.scr doubles a CTA of
+// global memory.
+template <int MODE>
+__global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
+  extern __shared__ __align__(16) double dyn[];
+  double* const sm = MODE == 2 ? A.big + (size_t)blockIdx.x * A.scr : dyn;
+  __shared__ __align__(16) double part[4 * SLE_THREADS];
+  __shared__ double s_w[5][SLE_THREADS / 32];
+  __shared__ double s_int[3], s_red[5];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int nphi = A.nphi, nlat = A.nlat, M = A.M, nh = (nlat + 1) / 2;
+  const Lon G(nphi);
+  PassSmem S;
+  S.tw = reinterpret_cast<double2*>(sm);
+  S.Gd = S.tw + tw_at(nphi) + 1;  // the rows' phase
+  S.X = reinterpret_cast<double*>(S.Gd + M);
+  S.L = S.X + 4 * G.nbase;
+  S.Fe = S.Gd;  // the orders' phase: the same space
+  S.dl = S.Fe + 4 * nh;
+  const int pp = p_pitch(nh);
+  double* const Ps = sm + A.scr;
+  double* const Ks = Ps + (size_t)(A.lmax + 1) * pp;  // [degree][6], see below
+  if (MODE == 1 && blockIdx.x < M) {
+    const int m = blockIdx.x;
+    for (int x = tid; x < A.lmax - m + 1; x += SLE_THREADS) {
+      Ks[6 * x + 4] = A.gu[m + x];
+      Ks[6 * x + 5] = A.gn[m + x];
+    }
+    for (int u = tid; u < (A.lmax - m + 1) * nh; u += SLE_THREADS) {
+      const int x = u / nh, j = u - x * nh;
+      Ps[(size_t)x * pp + j] = A.plm[(size_t)(A.mbeg[m] + x) * nlat + j];
+    }
+  }
+  const Share ss(G.nbase, 2, nphi, tid), sa(M, 1, nphi, tid);
+  unsigned int target = 0;
+  // the pass integrals, in every CTA from the row sums of the setup
+  if (wid < 3) {
+    const double v = warp_rows(A.rowpart + (wid == 0 ? RP_C : wid == 1 ? RP_DIG : RP_ZETA) * nlat, A.wts, nlat, A.dlon);
+    if (lane == 0) s_int[wid] = v;
+  }
+  for (int t = tid; t < nphi; t += SLE_THREADS) S.tw[tw_at(t)] = make_double2(A.cs[t], A.sn[t]);
+  __syncthreads();
+  const double C_int = s_int[0], ice_int = -(RHO_ICE / RHO_WATER) * s_int[1];
+  const double zeta_int = A.subgrid ? s_int[2] : 0.0;
+  if (blockIdx.x == 0 && tid == 0) {
+    A.sc->C_int = C_int;
+    A.sc->flips = 0;
+    A.sc->n_inner = 0;
+    if (C_int > 0.0) {
+      A.sc->ice_int = ice_int;
+      A.sc->zeta_int = zeta_int;
+    }
+  }
+  if (!(C_int > 0.0)) return;  // no ocean: nothing to redistribute (the same value in every CTA)
+  double2* F = reinterpret_cast<double2*>(A.F);    // [m][j]
+  double2* FC = reinterpret_cast<double2*>(A.FC);  // of the load rho_w C
+  double2* D = reinterpret_cast<double2*>(A.D);    // [j][m], twice the coefficient above m = 0
+  // the subgrid load, the load of the entering rsl and that of rho_w C
+  for (int j = blockIdx.x; j < nlat; j += gridDim.x) {
+    for (int i = tid; i < nphi; i += SLE_THREADS) {
+      const size_t p = (size_t)j * nphi + i;
+      const double c = A.C[p], wc = A.subgrid ? -RHO_WATER * A.topo0[p] * (c - A.C0[p]) : 0.0;
+      A.wcorr[p] = wc;
+      S.L[i] = RHO_ICE * A.dig[p] + RHO_WATER * (c * A.rsl[p]) + wc;
+    }
+    __syncthreads();
+    row_analysis(G, M, S, sa, part, F + j, nlat);
+    for (int i = tid; i < nphi; i += SLE_THREADS) S.L[i] = RHO_WATER * A.C[(size_t)j * nphi + i];
+    __syncthreads();
+    row_analysis(G, M, S, sa, part, FC + j, nlat);
+  }
+  if (!grid_barrier(A.bar, target, A.wait_ns)) return bar_fail(A);
+  double dphi = 0.0;  // of the last iteration done
+  bool done = A.n_inner < 1;
+  for (int it = 1;; ++it) {
+    // the last warps: the row results of the previous iteration (the same in every
+    // CTA), beside the other warps' first loads of O
+    if (it > 1 && wid >= SLE_THREADS / 32 - 5) {
+      const int k = wid - (SLE_THREADS / 32 - 5);
+      if (k == 0) {
+        const double v = warp_rows(A.rowpart + RP_CS * nlat, A.wts, nlat, A.dlon);
+        if (lane == 0) s_red[0] = v;
+      } else {
+        const double* r = A.rowpart + (k == 1 ? RP_DMAX : k == 2 ? RP_DMIN : k == 3 ? RP_SMAX : RP_SMIN) * nlat;
+        double v = -HUGE_VAL;  // minima are kept negated
+        for (int j0 = lane; j0 < nlat; j0 += 256) {
+          double t[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) t[u] = j0 + 32 * u < nlat ? __ldcg(r + j0 + 32 * u) : -HUGE_VAL;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) v = fmax(v, t[u]);
+        }
+        v = warp_max(v);
+        if (lane == 0) s_red[k] = v;
+      }
+    }
+    // ---- O: orders of this CTA; once done, only the closing load's spectrum
+    for (int m = blockIdx.x, first = 1; first || m < M; m += gridDim.x, first = 0) {
+      const int nl = m < M ? A.lmax - m + 1 : 0, lm0 = A.mbeg[min(m, M - 1)];
+      for (int u = tid; u < (nl ? (it > 1 ? nh : 2 * nh) : 0); u += SLE_THREADS) {
+        const int f = u >= nh, j = u - f * nh, jm = nlat - 1 - j;  // f: of rho_w C, the first time only
+        const double2* src = (f ? FC : F) + (size_t)m * nlat;
+        const double2 a = __ldcg(src + j), b = jm != j ? __ldcg(src + jm) : make_double2(0.0, 0.0);
+        const double w = A.wts[j];
+        S.Fe[(2 * f) * nh + j] = make_double2(w * (a.x + b.x), w * (a.y + b.y));
+        S.Fe[(2 * f + 1) * nh + j] = make_double2(w * (a.x - b.x), w * (a.y - b.y));
       }
       __syncthreads();
-      const int tpi = max(1, min(8, nthr / half));
-      double acc = 0.0;
-      for (int base = 0; base < half * tpi; base += nthr) {
-        const int u = base + tid, i = u / tpi, q = u % tpi;
-        const bool act = u < half * tpi;
-        double ue = 0.0, uo = 0.0, ne = 0.0, no = 0.0;
-        if (act) {
-          int t = (i * (1 + q)) % nphi;
-          const int step = (i * tpi) % nphi;
-          for (int m = 1 + q; m < M; m += tpi) {
-            const double c = __ldg(&A.cs[t]), sn = __ldg(&A.sn[t]);
-            const double vu = Gu[2 * m] * c - Gu[2 * m + 1] * sn;
-            const double vn = Gn[2 * m] * c - Gn[2 * m + 1] * sn;
-            if (m & 1) {
-              uo += vu;
-              no += vn;
-            } else {
-              ue += vu;
-              ne += vn;
+      if (it > 1 && first) {
+        // dphi and the convergence test (src/vilma_sle.f90:320-338); NaN anywhere in
+        // Sraw is in Cs, hence in dphi and in both maxima
+        const double Cs = s_red[0];
+        dphi = (ice_int - Cs + zeta_int) / C_int;
+        const double dmax = nanmax(fabs(s_red[1] + dphi), fabs(dphi - s_red[2]));
+        const double smax = nanmax(fabs(s_red[3] + dphi), fabs(dphi - s_red[4]));
+        done = dmax <= A.tol * fmax(smax, TINY) || it > A.n_inner;
+        if (blockIdx.x == 0 && tid == 0) {
+          A.sc->Cs_int = Cs;
+          A.sc->dphi = dphi;
+          A.sc->dmax = dmax;
+          A.sc->smax = smax;
+          A.sc->n_inner = it - 1;
+        }
+      }
+      if (nl == 0) break;
+      // analysis: eight lanes a degree, up to three degrees a thread
+      constexpr int W = 8, NX = SLE_THREADS / W, NV = 3;
+      const int lw = lane & (W - 1);
+      for (int x0 = 0; x0 < nl; x0 += NV * NX) {
+        const int xa = x0 + tid / W, nv = min(NV, (nl - x0 + NX - 1) / NX);
+        // lane v < nv closes degree xa + v NX: the spectrum of rho_w C and the drift's
+        // part of N - u, both kept from the first iteration, and the response factors
+        const int xk = xa + lw * NX, lmk = lm0 + xk;
+        const bool mine = lw < nv && xk < nl;
+        double kc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        if (mine && MODE != 1) {
+          kc[4] = A.gu[m + xk];
+          kc[5] = A.gn[m + xk];
+        }
+        if (mine && it == 1) {
+          if (m + xk > 0) {
+            const int k = A.lm2k[lmk];
+            kc[2] = -(A.drift[(size_t)2 * A.nk + k] / A.g) - A.drift[k];
+            kc[3] = -(A.drift[(size_t)3 * A.nk + k] / A.g) - A.drift[(size_t)A.nk + k];
+          }
+        } else if (mine && MODE != 1) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) kc[c] = A.cst[4 * (size_t)lmk + c];
+        }
+        double re[NV] = {}, im[NV] = {}, rc[NV] = {}, ic[NV] = {};
+        const double* P[NV];
+        const double2* fe[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          const int x = min(xa + v * NX, nl - 1);  // past the end: a valid row, result unused
+          P[v] = MODE == 1 ? Ps + (size_t)x * pp : A.plm + (size_t)(lm0 + x) * nlat;
+          fe[v] = S.Fe + (x & 1) * nh;
+        }
+        auto sums = [&](auto NVc, auto FIRST) {
+#pragma unroll 3
+          for (int j = lw; j < nh; j += W) {
+#pragma unroll
+            for (int v = 0; v < NVc.value; ++v) {
+              const double p = MODE == 1 ? P[v][j] : __ldg(P[v] + j);
+              const double2 f = fe[v][j];
+              re[v] = fma(p, f.x, re[v]);
+              im[v] = fma(p, f.y, im[v]);
+              if (FIRST.value) {
+                const double2 c = fe[v][2 * nh + j];
+                rc[v] = fma(p, c.x, rc[v]);
+                ic[v] = fma(p, c.y, ic[v]);
+              }
             }
-            t += step;
+          }
+#pragma unroll
+          for (int o = W / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int v = 0; v < NVc.value; ++v) {
+              re[v] += __shfl_xor_sync(0xffffffffu, re[v], o);
+              im[v] += __shfl_xor_sync(0xffffffffu, im[v], o);
+              if (FIRST.value) {
+                rc[v] += __shfl_xor_sync(0xffffffffu, rc[v], o);
+                ic[v] += __shfl_xor_sync(0xffffffffu, ic[v], o);
+              }
+            }
+        };
+        using std::integral_constant;
+        if (it == 1) {
+          sums(integral_constant<int, 3>(), integral_constant<bool, true>());
+        } else if (nv == 3) {
+          sums(integral_constant<int, 3>(), integral_constant<bool, false>());
+        } else if (nv == 2) {
+          sums(integral_constant<int, 2>(), integral_constant<bool, false>());
+        } else {
+          sums(integral_constant<int, 1>(), integral_constant<bool, false>());
+        }
+        if (mine) {
+          double sr = lw == 0 ? re[0] : lw == 1 ? re[1] : re[2], si = lw == 0 ? im[0] : lw == 1 ? im[1] : im[2];
+          if (it == 1) {
+            kc[0] = lw == 0 ? rc[0] : lw == 1 ? rc[1] : rc[2];
+            kc[1] = lw == 0 ? ic[0] : lw == 1 ? ic[1] : ic[2];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) (MODE == 1 ? Ks + 6 * xk : A.cst + 4 * (size_t)lmk)[c] = kc[c];
+          } else if (MODE == 1) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) kc[c] = Ks[6 * xk + c];
+          }
+          if (MODE == 1) {
+            kc[4] = Ks[6 * xk + 4];
+            kc[5] = Ks[6 * xk + 5];
+          }
+          if (it > 1) {
+            sr = fma(dphi, kc[0], sr);
+            si = fma(dphi, kc[1], si);
+          }
+          if (done) {
+            A.sigma[2 * lmk] = sr;
+            A.sigma[2 * lmk + 1] = si;
+          }
+          S.dl[xk] = make_double2((kc[5] * sr - kc[4] * sr) + kc[2], (kc[5] * si - kc[4] * si) + kc[3]);
+        }
+      }
+      __syncthreads();
+      if (done) continue;
+      // synthesis: a thread per (northern row, part of the degree pairs)
+      const int Q = max(1, min(16, SLE_THREADS / nh));
+      for (int base = 0; base < nh * Q; base += SLE_THREADS) {
+        const int u = base + tid, q = u / nh, j = u - q * nh;
+        double er = 0.0, ei = 0.0, orr = 0.0, oi = 0.0;
+        if (u < nh * Q) {
+          const double* P = MODE == 1 ? Ps + j : A.plm + (size_t)lm0 * nlat + j;
+          const int pt = MODE == 1 ? pp : nlat;
+#pragma unroll 4
+          for (int x = 2 * q; x < nl; x += 2 * Q) {
+            const double p = MODE == 1 ? P[(size_t)x * pt] : __ldg(P + (size_t)x * pt);
+            const double2 d = S.dl[x];
+            er = fma(p, d.x, er);
+            ei = fma(p, d.y, ei);
+            if (x + 1 < nl) {
+              const double p1 = MODE == 1 ? P[(size_t)(x + 1) * pt] : __ldg(P + (size_t)(x + 1) * pt);
+              const double2 d1 = S.dl[x + 1];
+              orr = fma(p1, d1.x, orr);
+              oi = fma(p1, d1.y, oi);
+            }
+          }
+        }
+        if (Q > 1) {
+          reinterpret_cast<double2*>(part)[2 * tid] = make_double2(er, ei);
+          reinterpret_cast<double2*>(part)[2 * tid + 1] = make_double2(orr, oi);
+          __syncthreads();
+        }
+        if (Q > 1 ? tid < nh : u < nh) {
+          for (int c = 1; c < Q; ++c) {
+            const double2 e = reinterpret_cast<const double2*>(part)[2 * (tid + c * nh)];
+            const double2 o = reinterpret_cast<const double2*>(part)[2 * (tid + c * nh) + 1];
+            er += e.x;
+            ei += e.y;
+            orr += o.x;
+            oi += o.y;
+          }
+          const double w = m == 0 ? 1.0 : 2.0;
+          const int jm = nlat - 1 - j;
+          __stcg(D + (size_t)j * M + m, make_double2(w * (er + orr), w * (ei + oi)));
+          if (jm != j) __stcg(D + (size_t)jm * M + m, make_double2(w * (er - orr), w * (ei - oi)));
+        }
+      }
+      __syncthreads();
+    }
+    if (done) break;
+    if (!grid_barrier(A.bar, target, A.wait_ns)) return bar_fail(A);
+    // ---- R: rows of this CTA
+    for (int j = blockIdx.x; j < nlat; j += gridDim.x) {
+      const size_t row = (size_t)j * nphi;
+      for (int m = tid; m < M; m += SLE_THREADS) S.Gd[m] = __ldcg(D + (size_t)j * M + m);
+      // this thread's first grid point, on its way while the sums are formed
+      double pc = 0.0, pd = 0.0, pw = 0.0, po = 0.0, pr = 0.0;
+      auto fetch = [&](int u) {
+        const int i = u >> 2, pt = u & 3;
+        if (i < G.nbase && G.has(i, pt)) {
+          const size_t p = row + G.at(i, pt);
+          pc = A.C[p];
+          pd = A.dig[p];
+          pw = A.wcorr[p];
+          po = it == 1 ? A.rsl[p] : A.Sraw[p];
+          pr = A.srot ? A.srot[p] : 0.0;
+        }
+      };
+      fetch(tid);
+      __syncthreads();
+      const int Q = ss.Q;
+      for (int base = 0; base < G.nbase * Q; base += SLE_THREADS) {
+        const Share sh = base ? Share(G.nbase, 2, nphi, base + tid) : ss;
+        const int i = sh.o;
+        double ce = 0.0, se = 0.0, co = 0.0, so = 0.0;
+        if (base + tid < G.nbase * Q) {
+          int t = sh.t0;
+#pragma unroll 2
+          for (int m = 2 * sh.q; m < M; m += 2 * Q) {
+            const double2 w = S.tw[tw_at(t)], v = S.Gd[m];
+            ce = fma(v.x, w.x, ce);
+            se = fma(v.y, w.y, se);
+            if (m + 1 < M) {
+              int t1 = t + i;
+              if (t1 >= nphi) t1 -= nphi;
+              const double2 w1 = S.tw[tw_at(t1)], v1 = S.Gd[m + 1];
+              co = fma(v1.x, w1.x, co);
+              so = fma(v1.y, w1.y, so);
+            }
+            t += sh.step;
             if (t >= nphi) t -= nphi;
           }
         }
-        part[tid] = ue;
-        part[nthr + tid] = uo;
-        part[2 * nthr + tid] = ne;
-        part[3 * nthr + tid] = no;
-        __syncthreads();
-        if (act && q == 0) {
-          double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-          for (int c = 0; c < tpi; ++c) {
-            a0 += part[tid + c];
-            a1 += part[nthr + tid + c];
-            a2 += part[2 * nthr + tid + c];
-            a3 += part[3 * nthr + tid + c];
+        if (Q == 1) {
+          if (base + tid < G.nbase) {
+            reinterpret_cast<double2*>(S.X)[2 * i] = make_double2(ce, se);
+            reinterpret_cast<double2*>(S.X)[2 * i + 1] = make_double2(co, so);
           }
-          const double u1 = Gu[0] + 2.0 * (a0 + a1), u2 = Gu[0] + 2.0 * (a0 - a1);
-          const double n1 = Gn[0] + 2.0 * (a2 + a3), n2 = Gn[0] + 2.0 * (a2 - a3);
-          const size_t p1 = (size_t)j * nphi + i, p2 = p1 + half;
-          double s1 = n1 - u1, s2 = n2 - u2;
-          if (A.srot) {
-            s1 = s1 + A.srot[p1];
-            s2 = s2 + A.srot[p2];
-          }
-          A.Sraw[p1] = s1;
-          A.Sraw[p2] = s2;
-          acc += A.C[p1] * s1 + A.C[p2] * s2;
-        }
-        __syncthreads();
-      }
-      acc = block_sum(acc, red);
-      if (tid == 0) A.rowpart[RP_CS * nlat + j] = acc;
-    }
-    if (!grid_barrier(A.bar, gen, A.wait_ns)) return bar_fail(A);
-    // U. dphi in every CTA (rows in order by thread 0: the same value everywhere)
-    {
-      const double Cs = integrate_rows(A.rowpart + RP_CS * nlat, A.wts, nlat, A.dlon);
-      if (tid == 0) {
-        const double dphi = (A.sc->ice_int - Cs + A.sc->zeta_int) / A.sc->C_int;
-        s_val = dphi;
-        if (blockIdx.x == 0) {
-          A.sc->Cs_int = Cs;
-          A.sc->dphi = dphi;
+        } else {
+          part[tid] = ce;
+          part[SLE_THREADS + tid] = se;
+          part[2 * SLE_THREADS + tid] = co;
+          part[3 * SLE_THREADS + tid] = so;
         }
       }
       __syncthreads();
-    }
-    const double dphi = s_val;
-    for (int j = blockIdx.x; j < nlat; j += gridDim.x) {
-      double dmax = 0.0, smax = 0.0;
-      for (int i = tid; i < nphi; i += nthr) {
-        const size_t p = (size_t)j * nphi + i;
-        const double rn = A.Sraw[p] + dphi;
-        dmax = nanmax(dmax, fabs(A.C[p] * (rn - A.rsl[p])));
-        A.rsl[p] = rn;
-        smax = nanmax(smax, fabs(A.C[p] * rn));
+      if (Q > 1) {
+        for (int u = tid; u < 4 * G.nbase; u += SLE_THREADS) {
+          const int s4 = u / G.nbase, i = u - s4 * G.nbase;
+          double v = 0.0;
+#pragma unroll 4
+          for (int c = 0; c < Q; ++c) v += part[s4 * SLE_THREADS + c * G.nbase + i];
+          S.X[4 * i + s4] = v;
+        }
+        __syncthreads();
       }
-      dmax = block_max_w(dmax, red);
-      smax = block_max_w(smax, red);
-      if (tid == 0) {
-        A.rowpart[RP_DMAX * nlat + j] = dmax;
-        A.rowpart[RP_SMAX * nlat + j] = smax;
-      }
-      sle_row_load(A, j, sm, part);  // L of the next iteration (unused if this one converged)
-    }
-    if (!grid_barrier(A.bar, gen, A.wait_ns)) return bar_fail(A);
-    // convergence (src/vilma_sle.f90:330-338), the same decision in every CTA
-    {
-      double dmax = 0.0, smax = 0.0;
-      for (int j = tid; j < nlat; j += nthr) {
-        dmax = nanmax(dmax, A.rowpart[RP_DMAX * nlat + j]);
-        smax = nanmax(smax, A.rowpart[RP_SMAX * nlat + j]);
-      }
-      dmax = block_max_w(dmax, red);
-      smax = block_max_w(smax, red);
-      if (tid == 0) {
-        s_stop = (dmax <= A.tol * fmax(smax, TINY)) ? 1 : 0;
-        if (blockIdx.x == 0) {
-          A.sc->dmax = dmax;
-          A.sc->smax = smax;
-          A.sc->n_inner = it;
+      double acc = 0.0, dmx = -HUGE_VAL, dmn = -HUGE_VAL, smx = -HUGE_VAL, smn = -HUGE_VAL;  // minima negated
+      for (int u = tid; u < 4 * G.nbase; u += SLE_THREADS) {
+        if (u != tid) fetch(u);
+        const int i = u >> 2, pt = u & 3;
+        if (!G.has(i, pt)) continue;
+        const double2 e = reinterpret_cast<const double2*>(S.X)[2 * i], o = reinterpret_cast<const double2*>(S.X)[2 * i + 1];
+        const double ev = pt < 2 ? e.x - e.y : e.x + e.y, ov = pt < 2 ? o.x - o.y : o.x + o.y;
+        double v = (pt & 1) ? ev - ov : ev + ov;
+        v += pr;
+        const size_t p = row + G.at(i, pt);
+        A.Sraw[p] = v;
+        S.L[G.at(i, pt)] = RHO_ICE * pd + RHO_WATER * (pc * v) + pw;
+        acc += pc * v;
+        if (pc != 0.0) {
+          const double d = it == 1 ? v - po : v - (po + dphi);
+          dmx = fmax(dmx, d);
+          dmn = fmax(dmn, -d);
+          smx = fmax(smx, v);
+          smn = fmax(smn, -v);
         }
       }
+      if (wid * 32 < 4 * G.nbase) {
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        dmx = warp_max(dmx);
+        dmn = warp_max(dmn);
+        smx = warp_max(smx);
+        smn = warp_max(smn);
+      }
+      if (lane == 0) {
+        s_w[0][wid] = acc;
+        s_w[1][wid] = dmx;
+        s_w[2][wid] = dmn;
+        s_w[3][wid] = smx;
+        s_w[4][wid] = smn;
+      }
       __syncthreads();
-      if (s_stop) break;
+      // the last warps add up the row's results while the others fold its load
+      if (wid >= SLE_THREADS / 32 - 5) {
+        const int k = wid - (SLE_THREADS / 32 - 5);
+        double v = lane < SLE_THREADS / 32 ? s_w[k][lane] : k ? -HUGE_VAL : 0.0;
+        if (k == 0) {
+          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        } else {
+          v = warp_max(v);
+        }
+        const int slot = k == 0 ? RP_CS : k == 1 ? RP_DMAX : k == 2 ? RP_DMIN : k == 3 ? RP_SMAX : RP_SMIN;
+        if (lane == 0) __stcg(A.rowpart + slot * nlat + j, v);
+      }
+      row_analysis(G, M, S, sa, part, F + j, nlat);
     }
+    if (!grid_barrier(A.bar, target, A.wait_ns)) return bar_fail(A);
+  }
+  // ---- rsl, the migrated coastline and the mass integral of the CTA's rows
+  int flips = 0;
+  for (int j = blockIdx.x; j < nlat; j += gridDim.x) {
+    double acc = 0.0;
+    for (int i = tid; i < nphi; i += SLE_THREADS) {
+      const size_t p = (size_t)j * nphi + i;
+      const double c = A.C[p];
+      double r = A.rsl[p];
+      if (A.n_inner >= 1) {
+        r = A.Sraw[p] + dphi;
+        A.rsl[p] = r;
+      }
+      acc += c * r;
+      if (!A.fixed) {
+        const double cn = ocean(A.topo0[p] - r, A.ice[p]);
+        A.Cn[p] = cn;
+        flips += cn != c ? 1 : 0;
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    __syncthreads();
+    if (lane == 0) s_w[0][wid] = acc;
+    __syncthreads();
+    if (tid == 0) {
+      for (int c = 1; c < SLE_THREADS / 32; ++c) acc += s_w[0][c];
+      __stcg(A.rowpart + RP_MASS * nlat + j, acc);
+    }
+  }
+  flips = __reduce_add_sync(0xffffffffu, flips);
+  if (lane == 0 && flips) atomicAdd(&A.sc->flips, flips);
+  // the CTA that finishes last adds the rows' mass
+  __shared__ int s_last;
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(A.bar + 1, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (s_last && wid == 0) {
+    const double v = warp_rows(A.rowpart + RP_MASS * nlat, A.wts, nlat, A.dlon);
+    if (lane == 0) A.sc->mass_Cs = v - zeta_int;
   }
 }
 
-// dynamic shared memory of the fused loop: the row (nphi) or, in R, the
-// Fourier sums (4 M) and the row's staged partial sums (4 chunks)
-static size_t sle_inner_smem(const vg_handle* h) {
-  const Grid& G = h->grid;
-  int nch = 0;
-  for (int m = 0; m < G.M; ++m) nch += (G.lmax - m + SLE_LCH) / SLE_LCH;
-  return (size_t)std::max(G.nphi, 4 * G.M + 4 * nch) * sizeof(double);
+// doubles of a CTA's work area: the twiddles, then the larger of the two phases
+static size_t sle_pass_scratch(const Grid& G) {
+  const size_t nbase = G.nphi % 2 ? (G.nphi + 1) / 2 : G.nphi / 4 + 1, nh = (G.nlat + 1) / 2;
+  const size_t rows = 2 * (size_t)G.M + 4 * nbase + G.nphi, orders = 2 * (4 * nh + G.lmax + 1);
+  return 2 * (size_t)(G.nphi + (G.nphi >> 3) + 1) + (std::max(rows, orders) + 1) / 2 * 2;
 }
 
-static void launch_inner_loop(vg_handle* h) {
+// int C rsl - zeta of that load
+__global__ void k_mass(SleScalars* sc, const double* __restrict__ rowpart, const double* __restrict__ w, int nlat,
+                       double dlon) {
+  const double m = warp_rows(rowpart + RP_MASS * nlat, w, nlat, dlon);
+  if (threadIdx.x == 0) sc->mass_Cs = m - sc->zeta_int;
+}
+
+static const void* pass_kernel(int mode) {
+  return mode == 2 ? (const void*)k_sle_pass<2> : mode == 1 ? (const void*)k_sle_pass<1> : (const void*)k_sle_pass<0>;
+}
+
+static void launch_pass(vg_handle* h) {
   const Grid& G = h->grid;
   cudaStream_t s = h->stream;
+  const size_t scr = sle_pass_scratch(G);
   if (h->sle_grid == 0) {
-    int dev = 0, nsm = 0, per_sm = 0;
+    int dev = 0, nsm = 0, per_sm = 0, lim = 0;
     VG_CUDA(cudaGetDevice(&dev));
     VG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const size_t shm = sle_inner_smem(h);
-    raise_smem_limit((const void*)k_sle_inner, shm);
-    VG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sle_inner, 512, shm));
+    VG_CUDA(cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    cudaFuncAttributes fa;
+    VG_CUDA(cudaFuncGetAttributes(&fa, pass_kernel(0)));
+    const size_t room = (size_t)lim - fa.sharedSizeBytes, psz = (size_t)(p_pitch((G.nlat + 1) / 2) + 6) * (G.lmax + 1);
+    const int ctas = h->p.sle_ctas > 0 ? std::min(h->p.sle_ctas, nsm) : nsm;
+    h->sle_mode = scr * sizeof(double) > room ? 2 : G.M <= ctas && (scr + psz) * sizeof(double) <= room ? 1 : 0;
+    h->sle_shm = h->sle_mode == 2 ? 0 : (scr + (h->sle_mode == 1 ? psz : 0)) * sizeof(double);
+    const void* fn = pass_kernel(h->sle_mode);
+    if (h->sle_shm) raise_smem_limit(fn, h->sle_shm);
+    VG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, SLE_THREADS, h->sle_shm));
     if (per_sm < 1) throw Error("sle_solve: the fused inner loop does not fit on an SM");
     h->sle_grid = h->p.sle_ctas > 0 ? std::min(h->p.sle_ctas, nsm * per_sm) : nsm;
     h->d_gbar.alloc(4);
-    std::vector<int2> chunk;
-    std::vector<int> cbeg(G.M + 1);
-    for (int m = 0; m < G.M; ++m) {
-      cbeg[m] = (int)chunk.size();
-      for (int l0 = 0; l0 < G.lmax - m + 1; l0 += SLE_LCH) chunk.push_back(make_int2(m, l0));
-    }
-    cbeg[G.M] = (int)chunk.size();
-    h->sle_nchunk = (int)chunk.size();
-    h->d_sle_chunk.upload(chunk, s);
-    h->d_sle_cbeg.upload(cbeg, s);
-    h->d_sle_Gp.alloc((size_t)h->sle_nchunk * G.nlat * 4);
+    if (h->sle_mode == 2) h->d_sle_big.alloc(scr * (size_t)h->sle_grid);
   }
-  InnerArgs A;
+  PassArgs A;
   A.nphi = G.nphi;
   A.nlat = G.nlat;
   A.M = G.M;
@@ -693,12 +806,16 @@ static void launch_inner_loop(vg_handle* h) {
   A.nk = h->nk;
   A.lmax = G.lmax;
   A.n_inner = h->p.sle_n_inner;
+  A.subgrid = h->p.sle_subgrid;
+  A.fixed = h->p.sle_fixed_ocean;
   A.tol = h->p.sle_tol;
   A.dlon = 2.0 * PI / (double)G.nphi;
   A.g = h->g;
+  A.ice = h->d_ice_now.p;
+  A.topo0 = h->d_z_bed_eq.p;
+  A.C0 = h->d_C0.p;
   A.dig = h->d_dig.p;
   A.C = h->d_C.p;
-  A.wcorr = h->d_wcorr.p;
   A.cs = G.d_cos.p;
   A.sn = G.d_sin.p;
   A.plm = G.d_plm.p;
@@ -707,27 +824,27 @@ static void launch_inner_loop(vg_handle* h) {
   A.gn = h->d_gn.p;
   A.drift = h->d_drift.p;
   A.srot = (h->rot_on || h->srot_ext) ? h->d_srot.p : nullptr;
-  A.lm_m = G.d_lm_m.p;
-  A.lm_l = G.d_lm_l.p;
   A.lm2k = h->d_lm2k.p;
   A.mbeg = G.d_mbeg.p;
+  A.wcorr = h->d_wcorr.p;
   A.rsl = h->d_rsl.p;
   A.F = h->d_F.p;
+  A.FC = h->d_F.p + (size_t)2 * G.M * G.nlat;
   A.sigma = h->d_sigma.p;
-  A.ulm = h->d_ulm.p;
-  A.chunk = h->d_sle_chunk.p;
-  A.cbeg = h->d_sle_cbeg.p;
-  A.nchunk = h->sle_nchunk;
-  A.Gp = h->d_sle_Gp.p;
+  A.cst = h->d_ulm.p;
+  A.D = h->d_Gs.p;
   A.Sraw = h->d_Sraw.p;
+  A.Cn = h->d_C_next.p;
   A.rowpart = h->d_rowpart.p;
   A.sc = h->d_sc_.p;
+  A.big = h->sle_mode == 2 ? h->d_sle_big.p : nullptr;
+  A.scr = scr;
   A.bar = h->d_gbar.p;
   A.wait_ns = h->wait_ns;
   VG_CUDA(cudaMemsetAsync(h->d_gbar.p, 0, 4 * sizeof(unsigned int), s));
-  const size_t shm = sle_inner_smem(h);
   void* args[] = {&A};
-  VG_CUDA(cudaLaunchCooperativeKernel((const void*)k_sle_inner, dim3(h->sle_grid), dim3(512), args, shm, s));
+  VG_CUDA(cudaLaunchCooperativeKernel(pass_kernel(h->sle_mode), dim3(h->sle_grid), dim3(SLE_THREADS), args,
+                                      h->sle_shm, s));
   ++h->n_launch;
 }
 
@@ -752,7 +869,6 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
   double* rp = h->d_rowpart.p;
   const int eb = 256, eg = (ng + eb - 1) / eb;
   if (!p.sle_warm_start) VG_CUDA(cudaMemsetAsync(h->d_rsl.p, 0, ng * sizeof(double), s));
-  VG_CUDA(cudaMemsetAsync(h->d_wcorr.p, 0, ng * sizeof(double), s));
   VG_CUDA(cudaMemsetAsync(sc, 0, sizeof(SleScalars), s));
   const bool trap = p.scheme == VG_SCHEME_TRAP && !report_only;
   // response_begin_step. Forward Euler without the toroidal channel: the drift
@@ -772,7 +888,6 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
     if (drift_pending) VG_CUDA(cudaStreamWaitEvent(s, h->ev_djoin, 0));
     drift_pending = false;
   };
-  k_ocean0<<<eg, eb, 0, s>>>(ng, h->d_z_bed_eq.p, h->d_ice_now.p, h->d_dice_now.p, h->d_C0.p); ++h->n_launch;
   // the sea-level <-> memory co-convergence (src/vilma_sle.f90:218-365): one
   // pass for forward Euler; trapezoid endpoint passes until the surface drift
   // settles for the trapezoidal scheme
@@ -780,34 +895,24 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
   const int n_mem = trap ? std::max(1, p.sle_max_mem_iter) : 1;
   h->n_inner_last = 0;
   h->n_flip_last = 0;
+  bool ocean_seen = false;  // a pass with an ocean has written the subgrid load
   for (int im = 1; im <= n_mem; ++im) {
+  bool closed = false;  // the last pass left the closing load's spectrum and the mass integral
   for (int io = 1; io <= p.sle_n_outer; ++io) {
-    if (p.sle_fixed_ocean) {
-      if (io == 1) VG_CUDA(cudaMemcpyAsync(h->d_C.p, h->d_C0.p, ng * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    } else if (io == 1) {
-      k_ocean<<<eg, eb, 0, s>>>(ng, h->d_z_bed_eq.p, h->d_rsl.p, h->d_ice_now.p, h->d_C.p); ++h->n_launch;
-    } else {
-      VG_CUDA(cudaMemcpyAsync(h->d_C.p, h->d_C_next.p, ng * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    }
-    k_pass_setup<<<nlat, 128, 0, s>>>(nphi, h->d_ice_now.p, h->d_dice_now.p, h->d_C.p, h->d_C0.p, h->d_z_bed_eq.p,
-                                      h->d_dig.p, rp, nlat); ++h->n_launch;
-    // no host round trip before the inner loop: with no ocean (C_int <= 0) the
-    // kernels below return at once and the pass ends after the one read
-    k_finalize_pass<<<1, FIN_THREADS, 0, s>>>(sc, rp, G.d_wts.p, nlat, dlon, p.sle_subgrid); ++h->n_launch;
-    k_wcorr<<<eg, eb, 0, s>>>(sc, ng, p.sle_subgrid, h->d_z_bed_eq.p, h->d_C.p, h->d_C0.p, h->d_wcorr.p);
-    ++h->n_launch;
+    k_pass_setup<<<nlat, 128, 0, s>>>(nphi, nlat, im == 1 && io == 1, io == 1, p.sle_fixed_ocean, h->d_ice_now.p,
+                                      h->d_dice_now.p, h->d_z_bed_eq.p, h->d_rsl.p, h->d_C_next.p, h->d_C0.p,
+                                      h->d_C.p, h->d_dig.p, rp); ++h->n_launch;
     join_drift();
+    // no host round trip before the pass: with no ocean (C_int <= 0) it returns
+    // at once and the solve ends after the one read
     {
       PhaseScope ps(h, VG_PH_SLE);
-      launch_inner_loop(h);
-    }
-    if (!p.sle_fixed_ocean) {  // the coastline test of this pass, read with the loop's scalars
-      k_coast<<<nlat, 128, 0, s>>>(nphi, h->d_z_bed_eq.p, h->d_rsl.p, h->d_ice_now.p, h->d_C.p, h->d_C_next.p,
-                                   rp, nlat); ++h->n_launch;
-      k_flips<<<1, FIN_THREADS, 0, s>>>(sc, rp, nlat); ++h->n_launch;
+      launch_pass(h);
     }
     read_scalars(h);
     if (h->sle_tape) tape_pass(h, h->h_sc->C_int, h->h_sc->n_inner);
+    closed = h->h_sc->C_int > 0.0;
+    ocean_seen |= closed;
     if (h->h_sc->C_int <= 0.0) break;  // no ocean: nothing to redistribute
     if (h->h_sc->bar_error) throw Error("sle_solve: grid barrier of the fused inner loop timed out");
     h->n_inner_last = h->h_sc->n_inner;
@@ -817,10 +922,16 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
     if (h->h_sc->flips == 0) break;
   }
   join_drift();  // (already joined unless the pass loop was empty)
-  // closing load, its analysis, and the memory advance (src/vilma_sle.f90:353-358)
-  k_load_fourier<<<nlat, 128, nphi * sizeof(double), s>>>(nphi, nlat, M, h->d_dig.p, h->d_C.p, h->d_rsl.p,
-                                                          h->d_wcorr.p, G.d_cos.p, G.d_sin.p, h->d_F.p); ++h->n_launch;
-  legendre_analysis_dev(h, h->d_F.p, 1, h->d_sigma.p);
+  // the closing load's spectrum (from the pass, unless that had no ocean) and the
+  // memory advance (src/vilma_sle.f90:353-358)
+  if (!closed) {
+    if (!ocean_seen) VG_CUDA(cudaMemsetAsync(h->d_wcorr.p, 0, ng * sizeof(double), s));
+    k_load_fourier<<<nlat, 128, nphi * sizeof(double), s>>>(nphi, nlat, M, h->d_dig.p, h->d_C.p, h->d_rsl.p,
+                                                            h->d_wcorr.p, G.d_cos.p, G.d_sin.p, h->d_F.p, rp);
+    k_mass<<<1, 32, 0, s>>>(sc, rp, G.d_wts.p, nlat, dlon);
+    h->n_launch += 2;
+    legendre_analysis_dev(h, h->d_F.p, 1, h->d_sigma.p);
+  }
   if (report_only) break;
   if (!trap) {
     advance_memory(h, h->d_sigma.p, dt);
@@ -829,8 +940,6 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
   if (trap_endpoint_pass(h, dt)) break;
   }
   if (trap) trap_finalize(h, dt);
-  k_rowsum<<<nlat, 128, 0, s>>>(nphi, h->d_C.p, h->d_rsl.p, rp + RP_MASS * nlat); ++h->n_launch;
-  k_mass<<<1, FIN_THREADS, 0, s>>>(sc, rp, G.d_wts.p, nlat, dlon); ++h->n_launch;
 }
 
 // solid_earth_update without rotation; d_ice1 is the interval-end ice on the device

@@ -1,0 +1,71 @@
+"""The fused sea-level pass at the edges of its work split: grids with and
+without an equator row, even, twice-odd and odd longitude counts, one order and
+several a CTA (more orders than CTAs; three CTAs for everything), a work area
+larger than shared memory, a fixed coastline, the subgrid load, one inner
+iteration, a solve with no ocean; GPU = oracle with test_gpu_parity.py's
+tolerances, the same iteration counts, and the same result whatever the CTAs."""
+import numpy as np
+import pytest
+
+from fastearth3d_b200 import lib as vlib
+from fastearth3d_b200 import synth
+from oracle import orc
+from parity_util import check_models
+
+pytestmark = pytest.mark.gpu
+
+
+def fields(nlat, nphi, ocean):
+    lat = np.linspace(0.0, np.pi, nlat + 2)[1:-1, None]
+    lon = 2 * np.pi * np.arange(nphi)[None] / nphi
+    topo = -900.0 + 2300.0 * np.sin(lon + 0.4) * np.sin(lat) ** 2 + 700.0 * np.cos(2 * lat)
+    topo = topo + 350.0 * np.cos(2 * lon - 1.0) * np.sin(lat)
+    if not ocean:
+        topo = np.abs(topo) + 50.0
+    ice = 2100.0 * np.exp(-((lat - 0.7) ** 2 + 0.4 * (1 - np.cos(lon - 1.1))) / 0.08)
+    return topo.reshape(-1), ice.reshape(-1)
+
+
+def run(lmax, nlat, nphi, opts, ctas=0, gpu=True, ocean=True):
+    mk, model = (vlib, vlib.Model) if gpu else (orc, orc.Oracle)
+    p = mk.default_params()
+    p.lmax, p.nlat, p.nphi = lmax, nlat, nphi
+    for i, c in enumerate([1, 2, 2, 1]):
+        p.ne_layer[i] = c
+    for k, v in opts.items():
+        setattr(p, k, v)
+    if gpu:
+        p.sle_ctas = ctas
+    m = model(p)
+    topo, ice = fields(nlat, nphi, ocean)
+    m.set_reference(topo, 0.25 * ice)
+    for f in (0.5, 1.0, 0.6):
+        m.update(f * ice, 150.0)
+    return m
+
+
+@pytest.mark.parametrize("lmax,nlat,nphi,opts", [
+    (2, 3, 6, {}),
+    (5, 6, 12, {"sle_subgrid": 1}),
+    (7, 9, 15, {}),
+    (16, 17, 34, {"sle_fixed_ocean": 1}),
+    (21, 24, 46, {"sle_n_inner": 1}),
+    (33, 40, 76, {"sle_n_outer": 1}),
+    (150, 151, 302, {}),
+    (4, 7000, 10, {}),
+])
+def test_pass_matches_oracle(lmax, nlat, nphi, opts):
+    g, o = run(lmax, nlat, nphi, opts), run(lmax, nlat, nphi, opts, gpu=False)
+    check_models(g, o)
+    assert g.info().n_inner_last == o.info().n_inner_last
+
+
+def test_no_ocean_matches_oracle():
+    g, o = run(12, 13, 26, {}, ocean=False), run(12, 13, 26, {}, gpu=False, ocean=False)
+    check_models(g, o)
+
+
+def test_result_does_not_depend_on_the_ctas():
+    a, b = run(33, 40, 76, {}), run(33, 40, 76, {}, ctas=3)
+    for x, y in zip(a.fields(), b.fields()):
+        assert np.array_equal(x, y)
