@@ -146,8 +146,6 @@ int vg_create(const vg_params* p, vg_handle** out) {
     VG_CUDA(cudaStreamCreateWithFlags(&h->aux, cudaStreamNonBlocking));
     VG_CUDA(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
     VG_CUDA(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
-    VG_CUDA(cudaEventCreateWithFlags(&h->ev_dfork, cudaEventDisableTiming));
-    VG_CUDA(cudaEventCreateWithFlags(&h->ev_djoin, cudaEventDisableTiming));
     vg::setup_handle(h);
     if (h->p.rotation) vg::rotation_setup(h);
     if (h->p.scheme == VG_SCHEME_TRAP) vg::trap_setup(h);
@@ -168,7 +166,7 @@ int vg_destroy(vg_handle* h) {
   if (h->aux) cudaStreamSynchronize(h->aux);
   if (h->h_sc) cudaFreeHost(h->h_sc);
   cudaStream_t s = h->stream, a = h->aux;
-  cudaEvent_t ev[4] = {h->ev_fork, h->ev_join, h->ev_dfork, h->ev_djoin};
+  cudaEvent_t ev[2] = {h->ev_fork, h->ev_join};
   delete h;
   for (cudaEvent_t e : ev)
     if (e) cudaEventDestroy(e);
@@ -639,7 +637,7 @@ int vg_set_fields(vg_handle* h, const double* h_ice, const double* rsl, const do
     if (rsl) h->d_rsl.upload(rsl, ng, s);
     if (z_bed) h->d_zbed.upload(z_bed, ng, s);
     if (C) h->d_C.upload(C, ng, s);
-    vg::update_bsl(h);
+    vg::finish_step(h, nullptr);
   });
 }
 

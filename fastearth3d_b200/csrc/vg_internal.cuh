@@ -93,6 +93,8 @@ struct SleScalars {
   int flips, n_inner;  // coastline flips; inner iterations done by the fused loop
   int bar_error;       // a grid barrier of the fused loop gave up
   unsigned long long mem_norm_bits;  // max |memory| of the state the last advance wrote
+  unsigned long long stage_status;   // status bits of its tensor-core stages
+  double bsl;                        // barystatic sea level at the end of the interval
 };
 
 // Phase timers, the device counterpart of the reference's [PROFILE] buckets
@@ -133,7 +135,6 @@ struct vg_handle {
   // drift beside the sea-level pass setup, joined before the fused loop reads it
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  cudaEvent_t ev_dfork = nullptr, ev_djoin = nullptr;
   // sizes
   int nr = 0, ne = 0, ndof = 0, nk = 0, ne3d = 0;
   int kl = 0, ku = 0, kv = 0, ldab = 0;  // band of degrees >= 2
@@ -214,6 +215,7 @@ struct vg_handle {
   size_t sle_shm = 0;
   vg::DArr<double> d_sigma, d_ulm, d_nlm;  // spectra (2*nlm)
   vg::DArr<double> d_rowpart;  // per-row partial results (9 * nlat)
+  vg::DArr<unsigned int> d_end_count;  // rows that k_step_end has finished
   vg::DArr<unsigned int> d_gbar;  // grid barrier of the fused pass: arrivals, finished CTAs, error
   int sle_grid = 0;               // CTAs of the cooperative launch of the pass (one per SM)
   // counters
@@ -262,7 +264,6 @@ void build_grid(Grid& G, int lmax, int nlat, int nphi, cudaStream_t s);
 // (nullptr: the handle's dUn, dVn) and the surface drift
 void launch_drift(vg_handle* h, int buf = -1, double* dUn = nullptr, double* dVn = nullptr, double* dWn = nullptr);
 // the same without the toroidal drift, on stream s
-void launch_drift_on(vg_handle* h, int buf, double* dUn, double* dVn, cudaStream_t s);
 // memory advance of one step (3-D elements pseudo-spectrally, the others per
 // slot), current buffer -> the other one, with the strain of (sigma, dUn,
 // dVn) (nullptr: the handle's drift), and the next buffer's per-slot norms and
@@ -283,7 +284,8 @@ void sht_synthesis_dev(vg_handle* h, const double* d_q, double* d_f, int batch);
 // SLE + stepper (vg_sle.cu)
 void sle_solve_dev(vg_handle* h, double dt, bool report_only);
 void update_dev(vg_handle* h, const double* d_ice1, double dt_yr);
-void update_bsl(vg_handle* h);
+void finish_step(vg_handle* h, const double* d_ice1);
+double checked_norm(unsigned long long bits, unsigned long long status);
 // 3-D (vg_visc3d.cu)
 void visc3d_enable(vg_handle* h, const double* pert_host);
 // 3-D memory advance (current buffer -> the other one), folding the new

@@ -199,7 +199,10 @@ __global__ void __launch_bounds__(32) k_drift_solve(DriftArgs A) {
                   });
 }
 
-void launch_drift_on(vg_handle* h, int buf, double* dUn, double* dVn, cudaStream_t s) {
+void launch_drift(vg_handle* h, int buf, double* dUn, double* dVn, double* dWn) {
+  PhaseScope ps(h, VG_PH_DRIFT);
+  if (buf < 0) buf = h->cur;
+  cudaStream_t s = h->stream;
   DriftArgs A;
   A.mem = h->d_mem[buf].p;
   A.mnorm = h->d_mnorm.p + (size_t)buf * h->nk;
@@ -232,12 +235,6 @@ void launch_drift_on(vg_handle* h, int buf, double* dUn, double* dVn, cudaStream
   k_drift_solve<<<h->ntask + deg1_tasks(h->nr), 32, sw::SMEM * sizeof(double), s>>>(A);
   ++h->n_launch;
   VG_CUDA(cudaGetLastError());
-}
-
-void launch_drift(vg_handle* h, int buf, double* dUn, double* dVn, double* dWn) {
-  PhaseScope ps(h, VG_PH_DRIFT);
-  if (buf < 0) buf = h->cur;
-  launch_drift_on(h, buf, dUn, dVn, h->stream);
   if (h->tor_on) launch_drift_tor(h, buf, dWn);  // its own forcing, its own operator
 }
 
@@ -336,13 +333,26 @@ __global__ void __launch_bounds__(256) k_advance_1d(const double* __restrict__ m
   }
 }
 
-// global max of the per-slot norms of one buffer
-__global__ void k_norm_max(const double* __restrict__ mnorm, int nk, unsigned long long* __restrict__ maxbits) {
-  __shared__ double red[1024];
+// global max of the per-slot norms of one buffer; beside the step's scalars, with
+// the status of the tensor-core stages, it needs no copy of its own
+__global__ void k_norm_max(const double* __restrict__ mnorm, int nk, unsigned long long* __restrict__ maxbits,
+                           const unsigned long long* __restrict__ status, SleScalars* __restrict__ sc) {
+  __shared__ double red[32];
   double v = 0.0;
   for (int k = threadIdx.x; k < nk; k += blockDim.x) v = nanmax(v, mnorm[k]);
-  v = block_max(v, red);
-  if (threadIdx.x == 0) *maxbits = (unsigned long long)__double_as_longlong(v);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  v = red[threadIdx.x];  // 32 warps
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if (threadIdx.x == 0) {
+    *maxbits = (unsigned long long)__double_as_longlong(v);
+    sc->mem_norm_bits = (unsigned long long)__double_as_longlong(v);
+    sc->stage_status = *status;
+  }
 }
 
 // Memory advance of one step, current buffer -> the other one: the 3-D
@@ -381,42 +391,54 @@ void advance_memory(vg_handle* h, const double* d_sigma, double dt, const double
     if (v3) visc3d_advance(h, d_sigma, dt, dUn, dVn, trap, dWn);
     spectral(h->stream);
   }
-  k_norm_max<<<1, 1024, 0, h->stream>>>(mn, h->nk, h->d_maxbits.p + nxt);
+  k_norm_max<<<1, 1024, 0, h->stream>>>(mn, h->nk, h->d_maxbits.p + nxt, h->d_maxbits.p + 2, h->d_sc_.p);
   ++h->n_launch;
   VG_CUDA(cudaGetLastError());
 }
 
-// per-slot norm and global max of one buffer (after vg_set_state / reset)
-__global__ void k_mem_norm(const double* __restrict__ mem, int ne, int nk, double* __restrict__ mnorm) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
+// per-slot norms of one buffer (after vg_set_state / reset), folded into zeros:
+// NORM_Q planes a thread, so that the read of the memory is spread over the chip
+// (one thread a slot ran at 1% of the bandwidth: 73 us at lmax 85, 6 now)
+constexpr int NORM_Q = 32;
+__global__ void k_mem_norm(const double* __restrict__ mem, int nq, int nk, double* __restrict__ mnorm) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nk) return;
   double amax = 0.0;
-  for (int q = 0; q < 6 * ne * 4; ++q) amax = nanmax(amax, fabs(mem[(size_t)q * nk + k]));
-  mnorm[k] = amax;
+  const int q1 = min(nq, (int)(blockIdx.y + 1) * NORM_Q);
+#pragma unroll 8
+  for (int q = blockIdx.y * NORM_Q; q < q1; ++q) amax = nanmax(amax, fabs(mem[(size_t)q * nk + k]));
+  atomic_max_bits(reinterpret_cast<unsigned long long*>(mnorm) + k, amax);
 }
 
 void compute_mem_norm(vg_handle* h, int buf) {
   double* mn = h->d_mnorm.p + (size_t)buf * h->nk;
-  k_mem_norm<<<(h->nk + 255) / 256, 256, 0, h->stream>>>(h->d_mem[buf].p, h->ne, h->nk, mn);
+  const int nq = 6 * h->ne * 4;
+  VG_CUDA(cudaMemsetAsync(mn, 0, h->nk * sizeof(double), h->stream));
+  k_mem_norm<<<dim3((h->nk + 127) / 128, (nq + NORM_Q - 1) / NORM_Q), 128, 0, h->stream>>>(h->d_mem[buf].p, nq, h->nk,
+                                                                                         mn);
   VG_CUDA(cudaGetLastError());
   if (h->tor_on) mem_norm_tor(h, buf, mn);
-  k_norm_max<<<1, 1024, 0, h->stream>>>(mn, h->nk, h->d_maxbits.p + buf);
+  k_norm_max<<<1, 1024, 0, h->stream>>>(mn, h->nk, h->d_maxbits.p + buf, h->d_maxbits.p + 2, h->d_sc_.p);
   VG_CUDA(cudaGetLastError());
+}
+
+double checked_norm(unsigned long long bits, unsigned long long status) {
+  if (status != 0) {
+    char msg[160];
+    std::snprintf(msg, sizeof(msg), "tensor-core stage wait timed out (status bits 0x%llx); results are invalid",
+                  status);
+    throw Error(msg);
+  }
+  double v;
+  std::memcpy(&v, &bits, sizeof(v));
+  return v;
 }
 
 double read_mem_norm(vg_handle* h, int buf) {
   unsigned long long bits[3] = {0, 0, 0};
   VG_CUDA(cudaMemcpyAsync(bits, h->d_maxbits.p, sizeof(bits), cudaMemcpyDeviceToHost, h->stream));
   VG_CUDA(cudaStreamSynchronize(h->stream));
-  if (bits[2] != 0) {
-    char msg[160];
-    std::snprintf(msg, sizeof(msg), "tensor-core stage wait timed out (status bits 0x%llx); results are invalid",
-                  bits[2]);
-    throw Error(msg);
-  }
-  double v;
-  std::memcpy(&v, &bits[buf], sizeof(v));
-  return v;
+  return checked_norm(bits[buf], bits[2]);
 }
 
 }  // namespace vg

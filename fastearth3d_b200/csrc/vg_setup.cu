@@ -975,6 +975,7 @@ void setup_handle(vg_handle* h) {
   h->d_xs.alloc((size_t)h->ntask * sw::scratch(nr));
   h->d_bh.alloc((size_t)2 * 2 * nr * nk);
   h->d_sc_.alloc(1);
+  VG_CUDA(cudaMemsetAsync(h->d_sc_.p, 0, sizeof(SleScalars), s));
   VG_CUDA(cudaMallocHost(&h->h_sc, sizeof(SleScalars)));
   std::memset(h->h_sc, 0, sizeof(SleScalars));
   const int ng = h->grid.ng, M = h->grid.M, nlat = h->grid.nlat;
@@ -988,6 +989,8 @@ void setup_handle(vg_handle* h) {
   h->d_ulm.alloc((size_t)2 * h->grid.nlm * 2);
   h->d_nlm.alloc((size_t)2 * h->grid.nlm);
   h->d_rowpart.alloc((size_t)9 * nlat);
+  h->d_end_count.alloc(1);
+  VG_CUDA(cudaMemsetAsync(h->d_end_count.p, 0, sizeof(unsigned int), s));
   VG_CUDA(cudaStreamSynchronize(s));
 }
 

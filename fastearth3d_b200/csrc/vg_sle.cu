@@ -21,11 +21,15 @@ __device__ __forceinline__ double ocean(double topo, double ice) {
   return (topo < 0.0 && RHO_ICE * ice < -RHO_WATER * topo) ? 1.0 : 0.0;
 }
 
+// the ice at a fraction of the interval and its change from the reference; with
+// rsl_n the entering rsl is kept there for a rejected step
 __global__ void k_ice_interp(int ng, double frac, const double* __restrict__ ice0, const double* __restrict__ ice1,
                              const double* __restrict__ ice_ref, double* __restrict__ ice_now,
-                             double* __restrict__ dice_now) {
+                             double* __restrict__ dice_now, const double* __restrict__ rsl,
+                             double* __restrict__ rsl_n) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ng) return;
+  if (rsl_n) rsl_n[i] = rsl[i];
   double v = ice0[i] + frac * (ice1[i] - ice0[i]);
   ice_now[i] = v;
   dice_now[i] = v - ice_ref[i];
@@ -35,13 +39,16 @@ __global__ void k_ice_interp(int ng, double frac, const double* __restrict__ ice
 // (src/vilma_sle.f90:212; once a solve, `set_c0`), the pass's ocean function (C0
 // with a fixed ocean, else ocean_function(topo0 - rsl, ice) in the first pass of a
 // co-convergence iteration, `io1`, and the migrated coastline Cn after it), the
-// grounded-ice increment, and the row sums of C, dIg, topo0 (C - C0)
+// grounded-ice increment, and the row sums of C, dIg, topo0 (C - C0). The first
+// pass of a solve also clears the solve's scalars.
 __global__ void k_pass_setup(int nphi, int nlat, int set_c0, int io1, int fixed, const double* __restrict__ ice,
                              const double* __restrict__ dice, const double* __restrict__ topo0,
                              const double* __restrict__ rsl, const double* __restrict__ Cn, double* __restrict__ C0,
-                             double* __restrict__ C, double* __restrict__ dig, double* __restrict__ rowpart) {
-  __shared__ double red[128];
+                             double* __restrict__ C, double* __restrict__ dig, double* __restrict__ rowpart,
+                             SleScalars* __restrict__ scal) {
+  __shared__ double red[32];
   int j = blockIdx.x;
+  if (set_c0 && j == 0 && threadIdx.x == 0) *scal = SleScalars{};
   double sc = 0.0, sd = 0.0, sz = 0.0;
   for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
     size_t p = (size_t)j * nphi + i;
@@ -56,9 +63,9 @@ __global__ void k_pass_setup(int nphi, int nlat, int set_c0, int io1, int fixed,
     sd += d;
     sz += t0 * (c - c0);
   }
-  sc = block_sum(sc, red);
-  sd = block_sum(sd, red);
-  sz = block_sum(sz, red);
+  sc = block_sum_w(sc, red);
+  sd = block_sum_w(sd, red);
+  sz = block_sum_w(sz, red);
   if (threadIdx.x == 0) {
     rowpart[RP_C * nlat + j] = sc;
     rowpart[RP_DIG * nlat + j] = sd;
@@ -79,38 +86,59 @@ __global__ void k_load_fourier(int nphi, int nlat, int M, const double* __restri
   double s = 0.0;
   for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
     size_t p = (size_t)j * nphi + i;
-    row[i] = RHO_ICE * dig[p] + RHO_WATER * (C[p] * rsl[p]) + wcorr[p];
+    row[i] = RHO_ICE * dig[p] + RHO_WATER * (C[p] * rsl[p]) + (wcorr ? wcorr[p] : 0.0);
     s += C[p] * rsl[p];
   }
-  s = block_sum(s, red);
+  s = block_sum_w(s, red);
   if (threadIdx.x == 0) rowpart[RP_MASS * nlat + j] = s;
   __syncthreads();
   row_fourier_analysis(row, nphi, M, cs, sn, F + (size_t)j * 2, nlat);
 }
 
-// z_bed = z_bed_eq - rsl (src/vilma_coupling.f90:428)
-__global__ void k_zbed(int ng, const double* __restrict__ zeq, const double* __restrict__ rsl,
-                       double* __restrict__ zb) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < ng) zb[i] = zeq[i] - rsl[i];
-}
-// row sums of C and of h_ice (1 - C) - h_ice_eq (1 - C0), for update_bsl
-__global__ void k_bsl_rows(int nphi, const double* __restrict__ hi, const double* __restrict__ hq,
-                           const double* __restrict__ C, const double* __restrict__ C0, double* __restrict__ rowpart,
-                           int nlat) {
-  __shared__ double red[128];
+// End of an interval, a block per row: with ice1 the ice becomes the interval's
+// end value and z_bed = z_bed_eq - rsl (src/vilma_coupling.f90:428); then update_bsl
+// (src/vilma_coupling.f90:572-597) from the row sums of C and of
+// h_ice (1 - C) - h_ice_eq (1 - C0), added up by the block that finishes last
+__global__ void k_step_end(int nphi, int nlat, double dlon, const double* __restrict__ ice1,
+                           const double* __restrict__ zeq, const double* __restrict__ rsl, double* __restrict__ zb,
+                           double* __restrict__ hi, const double* __restrict__ hq, const double* __restrict__ C,
+                           const double* __restrict__ C0, const double* __restrict__ w, double* __restrict__ rowpart,
+                           SleScalars* __restrict__ scal, unsigned int* __restrict__ done) {
+  __shared__ double red[32];
+  __shared__ int s_last;
   int j = blockIdx.x;
   double sc = 0.0, st = 0.0;
   for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
     size_t p = (size_t)j * nphi + i;
+    const double h = ice1 ? ice1[p] : hi[p];
+    if (ice1) {
+      hi[p] = h;
+      zb[p] = zeq[p] - rsl[p];
+    }
     sc += C[p];
-    st += hi[p] * (1.0 - C[p]) - hq[p] * (1.0 - C0[p]);
+    st += h * (1.0 - C[p]) - hq[p] * (1.0 - C0[p]);
   }
-  sc = block_sum(sc, red);
-  st = block_sum(st, red);
+  sc = block_sum_w(sc, red);
+  st = block_sum_w(st, red);
   if (threadIdx.x == 0) {
     rowpart[RP_C * nlat + j] = sc;
     rowpart[RP_DIG * nlat + j] = st;
+    __threadfence();
+    s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!s_last) return;
+  double c = 0.0, t = 0.0;
+  for (int q = threadIdx.x; q < nlat; q += blockDim.x) {
+    c += w[q] * __ldcg(rowpart + RP_C * nlat + q) * dlon;
+    t += w[q] * __ldcg(rowpart + RP_DIG * nlat + q) * dlon;
+  }
+  c = block_sum_w(c, red);
+  t = block_sum_w(t, red);
+  if (threadIdx.x == 0) {
+    scal->bsl = c > 0.0 ? -(RHO_ICE / RHO_WATER) * t / c : 0.0;
+    *done = 0u;
   }
 }
 
@@ -376,6 +404,8 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
     if (C_int > 0.0) {
       A.sc->ice_int = ice_int;
       A.sc->zeta_int = zeta_int;
+    } else {
+      A.sc->mass_Cs = -A.sc->zeta_int;  // int C rsl is zero
     }
   }
   if (!(C_int > 0.0)) return;  // no ocean: nothing to redistribute (the same value in every CTA)
@@ -742,7 +772,7 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
   }
   flips = __reduce_add_sync(0xffffffffu, flips);
   if (lane == 0 && flips) atomicAdd(&A.sc->flips, flips);
-  // the CTA that finishes last adds the rows' mass
+  // the CTA that finishes last adds the rows' mass and resets the barrier
   __shared__ int s_last;
   __syncthreads();
   if (tid == 0) {
@@ -753,7 +783,10 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
   __syncthreads();
   if (s_last && wid == 0) {
     const double v = warp_rows(A.rowpart + RP_MASS * nlat, A.wts, nlat, A.dlon);
-    if (lane == 0) A.sc->mass_Cs = v - zeta_int;
+    if (lane == 0) {
+      A.sc->mass_Cs = v - zeta_int;
+      A.bar[0] = A.bar[1] = 0u;
+    }
   }
 }
 
@@ -795,7 +828,8 @@ static void launch_pass(vg_handle* h) {
     VG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, SLE_THREADS, h->sle_shm));
     if (per_sm < 1) throw Error("sle_solve: the fused inner loop does not fit on an SM");
     h->sle_grid = h->p.sle_ctas > 0 ? std::min(h->p.sle_ctas, nsm * per_sm) : nsm;
-    h->d_gbar.alloc(4);
+    if (!h->d_gbar.p) h->d_gbar.alloc(4);
+    VG_CUDA(cudaMemsetAsync(h->d_gbar.p, 0, 4 * sizeof(unsigned int), s));  // later: by the last CTA of each launch
     if (h->sle_mode == 2) h->d_sle_big.alloc(scr * (size_t)h->sle_grid);
   }
   PassArgs A;
@@ -841,7 +875,6 @@ static void launch_pass(vg_handle* h) {
   A.scr = scr;
   A.bar = h->d_gbar.p;
   A.wait_ns = h->wait_ns;
-  VG_CUDA(cudaMemsetAsync(h->d_gbar.p, 0, 4 * sizeof(unsigned int), s));
   void* args[] = {&A};
   VG_CUDA(cudaLaunchCooperativeKernel(pass_kernel(h->sle_mode), dim3(h->sle_grid), dim3(SLE_THREADS), args,
                                       h->sle_shm, s));
@@ -869,25 +902,9 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
   double* rp = h->d_rowpart.p;
   const int eb = 256, eg = (ng + eb - 1) / eb;
   if (!p.sle_warm_start) VG_CUDA(cudaMemsetAsync(h->d_rsl.p, 0, ng * sizeof(double), s));
-  VG_CUDA(cudaMemsetAsync(sc, 0, sizeof(SleScalars), s));
+  if (p.sle_n_outer < 1) VG_CUDA(cudaMemsetAsync(sc, 0, sizeof(SleScalars), s));  // (else by the first pass)
   const bool trap = p.scheme == VG_SCHEME_TRAP && !report_only;
-  // response_begin_step. Forward Euler without the toroidal channel: the drift
-  // (its degree 1 beside the band sweeps) runs on the second stream while this
-  // stream sets up the first pass (ocean function, row integrals: none of the
-  // drift's buffers), and is joined before the fused loop reads it.
-  bool drift_pending = !trap && !h->tor_on && !h->prof.on;
-  if (drift_pending) {
-    VG_CUDA(cudaEventRecord(h->ev_dfork, s));
-    VG_CUDA(cudaStreamWaitEvent(h->aux, h->ev_dfork, 0));
-    launch_drift_on(h, h->cur, nullptr, nullptr, h->aux);
-    VG_CUDA(cudaEventRecord(h->ev_djoin, h->aux));
-  } else {
-    launch_drift(h);
-  }
-  auto join_drift = [&]() {
-    if (drift_pending) VG_CUDA(cudaStreamWaitEvent(s, h->ev_djoin, 0));
-    drift_pending = false;
-  };
+  launch_drift(h);  // response_begin_step
   // the sea-level <-> memory co-convergence (src/vilma_sle.f90:218-365): one
   // pass for forward Euler; trapezoid endpoint passes until the surface drift
   // settles for the trapezoidal scheme
@@ -901,8 +918,7 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
   for (int io = 1; io <= p.sle_n_outer; ++io) {
     k_pass_setup<<<nlat, 128, 0, s>>>(nphi, nlat, im == 1 && io == 1, io == 1, p.sle_fixed_ocean, h->d_ice_now.p,
                                       h->d_dice_now.p, h->d_z_bed_eq.p, h->d_rsl.p, h->d_C_next.p, h->d_C0.p,
-                                      h->d_C.p, h->d_dig.p, rp); ++h->n_launch;
-    join_drift();
+                                      h->d_C.p, h->d_dig.p, rp, sc); ++h->n_launch;
     // no host round trip before the pass: with no ocean (C_int <= 0) it returns
     // at once and the solve ends after the one read
     {
@@ -914,22 +930,27 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
     closed = h->h_sc->C_int > 0.0;
     ocean_seen |= closed;
     if (h->h_sc->C_int <= 0.0) break;  // no ocean: nothing to redistribute
-    if (h->h_sc->bar_error) throw Error("sle_solve: grid barrier of the fused inner loop timed out");
+    if (h->h_sc->bar_error) {
+      h->sle_grid = 0;  // the barrier's counters are set up again before the next launch
+      throw Error("sle_solve: grid barrier of the fused inner loop timed out");
+    }
     h->n_inner_last = h->h_sc->n_inner;
     h->n_outer_last = io;
     if (p.sle_fixed_ocean) break;
     h->n_flip_last = h->h_sc->flips;
     if (h->h_sc->flips == 0) break;
   }
-  join_drift();  // (already joined unless the pass loop was empty)
   // the closing load's spectrum (from the pass, unless that had no ocean) and the
   // memory advance (src/vilma_sle.f90:353-358)
   if (!closed) {
-    if (!ocean_seen) VG_CUDA(cudaMemsetAsync(h->d_wcorr.p, 0, ng * sizeof(double), s));
     k_load_fourier<<<nlat, 128, nphi * sizeof(double), s>>>(nphi, nlat, M, h->d_dig.p, h->d_C.p, h->d_rsl.p,
-                                                            h->d_wcorr.p, G.d_cos.p, G.d_sin.p, h->d_F.p, rp);
-    k_mass<<<1, 32, 0, s>>>(sc, rp, G.d_wts.p, nlat, dlon);
-    h->n_launch += 2;
+                                                            ocean_seen ? h->d_wcorr.p : nullptr, G.d_cos.p,
+                                                            G.d_sin.p, h->d_F.p, rp);
+    ++h->n_launch;
+    if (p.sle_n_outer < 1) {
+      k_mass<<<1, 32, 0, s>>>(sc, rp, G.d_wts.p, nlat, dlon);
+      ++h->n_launch;
+    }
     legendre_analysis_dev(h, h->d_F.p, 1, h->d_sigma.p);
   }
   if (report_only) break;
@@ -968,16 +989,16 @@ void update_dev(vg_handle* h, const double* d_ice1, double dt_yr) {
   };
   if (span <= 0.0) {
     k_ice_interp<<<eg, eb, 0, s>>>(ng, 0.0, h->d_h_ice.p, h->d_h_ice.p, h->d_h_ice_eq.p, h->d_ice_now.p,
-                                   h->d_dice_now.p); ++h->n_launch;
+                                   h->d_dice_now.p, nullptr, nullptr); ++h->n_launch;
     sle_solve_dev(h, 0.0, true);
     h->worst_mass_resid = mass_resid();
   } else if (p.scheme == VG_SCHEME_TRAP) {
     // implicit branch (src/vilma_timestep.f90:229-307): step doubling around
     // each trial step, accept / reject against rtol, atol; dt_try carried
     // across intervals
-    auto solve_at = [&](double t_eval, double dts) {
+    auto solve_at = [&](double t_eval, double dts, double* keep_rsl) {
       k_ice_interp<<<eg, eb, 0, s>>>(ng, (t_eval - t0) / span, h->d_h_ice.p, d_ice1, h->d_h_ice_eq.p,
-                                     h->d_ice_now.p, h->d_dice_now.p); ++h->n_launch;
+                                     h->d_ice_now.p, h->d_dice_now.p, h->d_rsl.p, keep_rsl); ++h->n_launch;
       VG_CUDA(cudaGetLastError());
       h->n_solve++;
       sle_solve_dev(h, dts, false);
@@ -985,7 +1006,7 @@ void update_dev(vg_handle* h, const double* d_ice1, double dt_yr) {
     };
     if (!h->sigma_primed) {  // seed sigma_n: a report-only solve at t0 (:234-241)
       k_ice_interp<<<eg, eb, 0, s>>>(ng, 0.0, h->d_h_ice.p, h->d_h_ice.p, h->d_h_ice_eq.p, h->d_ice_now.p,
-                                     h->d_dice_now.p); ++h->n_launch;
+                                     h->d_dice_now.p, nullptr, nullptr); ++h->n_launch;
       sle_solve_dev(h, 0.0, true);
       trap_prime(h);
     }
@@ -997,14 +1018,13 @@ void update_dev(vg_handle* h, const double* d_ice1, double dt_yr) {
       if (t >= t1 - 1.0e-9 * span) break;
       const double dts = std::min(h->dt_try, t1 - t);
       const bool at_floor = p.dt_min > 0.0 && dts <= p.dt_min * (1.0 + 1.0e-9);
-      VG_CUDA(cudaMemcpyAsync(h->d_rsl_n.p, h->d_rsl.p, ng * sizeof(double), cudaMemcpyDeviceToDevice, s));
       trap_save(h);
-      solve_at(t + dts, dts);  // coarse
+      solve_at(t + dts, dts, h->d_rsl_n.p);  // coarse
       trap_stash_coarse(h);
       trap_restore(h);
       VG_CUDA(cudaMemcpyAsync(h->d_rsl.p, h->d_rsl_n.p, ng * sizeof(double), cudaMemcpyDeviceToDevice, s));
-      solve_at(t + 0.5 * dts, 0.5 * dts);  // fine
-      solve_at(t + dts, 0.5 * dts);
+      solve_at(t + 0.5 * dts, 0.5 * dts, nullptr);  // fine
+      solve_at(t + dts, 0.5 * dts, nullptr);
       double err_inf = 0.0, tau_inf = 0.0;
       trap_coarse_fine_error(h, err_inf, tau_inf);
       const double errsc = (err_inf / ricfac) / (p.atol + p.rtol * tau_inf);
@@ -1044,18 +1064,17 @@ void update_dev(vg_handle* h, const double* d_ice1, double dt_yr) {
     while (true) {
       if (t >= t1 - 1.0e-9 * span) break;
       dtc = std::min(dtc, t1 - t);
-      VG_CUDA(cudaMemcpyAsync(h->d_rsl_n.p, h->d_rsl.p, ng * sizeof(double), cudaMemcpyDeviceToDevice, s));
       double tau0 = h->mem_norm;
       double frac = (t + dtc - t0) / span;
       k_ice_interp<<<eg, eb, 0, s>>>(ng, frac, h->d_h_ice.p, d_ice1, h->d_h_ice_eq.p, h->d_ice_now.p,
-                                     h->d_dice_now.p); ++h->n_launch;
+                                     h->d_dice_now.p, h->d_rsl.p, h->d_rsl_n.p); ++h->n_launch;
       VG_CUDA(cudaGetLastError());
       h->n_solve++;
       if (h->sle_tape) tape_attempt_begin(h, frac, dtc);
       sle_solve_dev(h, dtc, false);
       int nxt = 1 - h->cur;
-      VG_CUDA(cudaMemcpyAsync(h->h_sc, h->d_sc_.p, sizeof(SleScalars), cudaMemcpyDeviceToHost, s));
-      double err_inf = read_mem_norm(h, nxt);  // synchronises: the scalars are in as well
+      read_scalars(h);  // the pass's results and the norm and status that the advance left beside them
+      double err_inf = checked_norm(h->h_sc->mem_norm_bits, h->h_sc->stage_status);
       h->worst_mass_resid = std::max(h->worst_mass_resid, mass_resid_read());
       bool finite = err_inf <= HUGE_;
       double scale = std::max(tau0, tau_run);
@@ -1080,31 +1099,20 @@ void update_dev(vg_handle* h, const double* d_ice1, double dt_yr) {
   }
   // polar motion to the interval end under the converged load (:411-421)
   if (h->rot_on) rotation_advance(h, h->d_sigma.p, span);
-  VG_CUDA(cudaMemcpyAsync(h->d_h_ice.p, d_ice1, ng * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  k_zbed<<<eg, eb, 0, s>>>(ng, h->d_z_bed_eq.p, h->d_rsl.p, h->d_zbed.p); ++h->n_launch;
-  VG_CUDA(cudaGetLastError());
   h->time_yr += dt_yr;
   h->time_s = h->time_yr * SEC_PER_YEAR;  // not the sub-steps' sum: a restart's clock (seconds) gives time_yr back
-  update_bsl(h);
+  finish_step(h, d_ice1);
 }
 
-// src/vilma_coupling.f90:572-597 update_bsl
-void update_bsl(vg_handle* h) {
+void finish_step(vg_handle* h, const double* d_ice1) {
   const Grid& G = h->grid;
-  const int nlat = G.nlat, nphi = G.nphi;
-  cudaStream_t s = h->stream;
-  double* rp = h->d_rowpart.p;
-  k_bsl_rows<<<nlat, 128, 0, s>>>(nphi, h->d_h_ice.p, h->d_h_ice_eq.p, h->d_C.p, h->d_C0.p, rp, nlat); ++h->n_launch;
+  k_step_end<<<G.nlat, 128, 0, h->stream>>>(G.nphi, G.nlat, 2.0 * PI / (double)G.nphi, d_ice1, h->d_z_bed_eq.p,
+                                            h->d_rsl.p, h->d_zbed.p, h->d_h_ice.p, h->d_h_ice_eq.p, h->d_C.p,
+                                            h->d_C0.p, G.d_wts.p, h->d_rowpart.p, h->d_sc_.p, h->d_end_count.p);
+  ++h->n_launch;
   VG_CUDA(cudaGetLastError());
-  std::vector<double> rows((size_t)RP_N * nlat);
-  VG_CUDA(cudaMemcpyAsync(rows.data(), rp, rows.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
-  VG_CUDA(cudaStreamSynchronize(s));
-  double dlon = 2.0 * PI / (double)nphi, c_int = 0.0, t_int = 0.0;
-  for (int j = 0; j < nlat; ++j) {
-    c_int += G.wts[j] * rows[RP_C * nlat + j] * dlon;
-    t_int += G.wts[j] * rows[RP_DIG * nlat + j] * dlon;
-  }
-  h->bsl = c_int > 0.0 ? -(RHO_ICE / RHO_WATER) * t_int / c_int : 0.0;
+  read_scalars(h);
+  h->bsl = h->h_sc->bsl;
 }
 
 }  // namespace vg
