@@ -34,6 +34,7 @@
 
 #include "vg_device.cuh"
 #include "vg_internal.cuh"
+#include "vg_sle_pass.cuh"
 
 namespace vg {
 
@@ -548,59 +549,187 @@ __global__ void k_c_bytes(int ng, const double* __restrict__ C, unsigned char* _
   if (i < ng) out[i] = C[i] != 0.0 ? 1 : 0;
 }
 
-// per-row sums of lam
-__global__ void k_rev_rows(int nphi, const double* __restrict__ lam, double* __restrict__ rows) {
-  __shared__ double red[128];
-  const int j = blockIdx.x;
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < nphi; i += blockDim.x) acc += lam[(size_t)j * nphi + i];
-  acc = block_sum(acc, red);
-  if (threadIdx.x == 0) rows[j] = acc;
-}
+// The adjoint of one pass's inner iterations, K of them in reverse, as one
+// cooperative kernel with the two phases of the sea-level pass: lam, the adjoint
+// of the pass's final rsl, becomes that of its starting rsl; digbar accumulates
+// rho_i load_bar and surf_bar the surface drift's adjoints. An iteration:
+//   dphi_bar = sum lam, <C Sraw>_bar = -dphi_bar / <C>
+//   Sraw_bar = lam + <C Sraw>_bar C w_j dlon
+//   q_bar = Synth^T Sraw_bar = (c_m / dlon) A(Sraw_bar / w_j): the spectrum of
+//           C w_j dlon over w_j is formed once, that of lam / w_j is the
+//           Legendre sum of lam's rows without the quadrature weights
+//   apply^T: sigma_bar = (gn - gu) q_bar, dUa_bar -= q_bar, dFa_bar -= q_bar / g
+//   load_bar = A^T sigma_bar = dlon w_j Synth(sigma_bar / c_m)
+//   lam = rho_w C load_bar, digbar += rho_i load_bar
+// and at the end of the pass ice_now_bar = (1 - C) (digbar - (rho_i / rho_w)
+// ice_int_bar w_j dlon), ice_int_bar the sum of dphi_bar / <C>, into the adjoints
+// of this interval's end ice (frac) and of the previous interval's (1 - frac).
+// Bound by latency like the pass itself: nine kernels an iteration took 40 us and
+// their launches at lmax 64, this takes 11.
+struct RevArgs : PassBase {
+  int nk, K, fresh;  // fresh: digbar starts at zero
+  double C_int, g, frac;
+  const unsigned char* C;
+  const double *gu, *gn;
+  const int* lm2k;
+  double *lam, *digbar, *surf_bar, *gi1, *gi0;
+};
 
-// dphi_bar = sum of lam (rows in order): scal[0] = <C Sraw>_bar = -dphi_bar / <C>,
-// scal[1] += ice_int_bar = dphi_bar / <C>
-__global__ void k_rev_scal(int nlat, const double* __restrict__ rows, double C_int, double* __restrict__ scal) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  double acc = 0.0;
-  for (int j = 0; j < nlat; ++j) acc += rows[j];
-  scal[0] = -acc / C_int;
-  scal[1] += acc / C_int;
-}
-
-// Sraw_bar = lam + scal[0] C w_j dlon, divided by w_j for the analysis that
-// forms the synthesis transpose
-__global__ void k_rev_y(int ng, int nphi, const double* __restrict__ lam, const unsigned char* __restrict__ C,
-                        const double* __restrict__ wts, double dlon, const double* __restrict__ scal,
-                        double* __restrict__ out) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= ng) return;
-  const double w = wts[p / nphi];
-  out[p] = (lam[p] + (C[p] ? scal[0] * w * dlon : 0.0)) / w;
-}
-
-// q_bar = (c_m / sc) q (the synthesis transpose of Sraw_bar, q the analysis of
-// Sraw_bar / w_j); apply^T: sigma_bar = (gn - gu) q_bar, the surface drift
-// adjoints dUa_bar -= q_bar, dFa_bar -= q_bar / g; out = sigma_bar / c_m for
-// the synthesis that forms the analysis transpose
-__global__ void k_rev_apply(int nlm, int nk, double g, double sc, const int* __restrict__ lm_l,
-                            const int* __restrict__ lm_m, const int* __restrict__ lm2k, const double* __restrict__ gu,
-                            const double* __restrict__ gn, const double* __restrict__ q, double* __restrict__ surf_bar,
-                            double* __restrict__ out) {
-  const int lm = blockIdx.x * blockDim.x + threadIdx.x;
-  if (lm >= nlm) return;
-  const int l = lm_l[lm], m = lm_m[lm];
-  const double cm = (m == 0) ? 1.0 : 2.0;
-  const double qr = q[2 * lm] * cm / sc, qi = (m == 0) ? 0.0 : q[2 * lm + 1] * cm / sc;
-  const double gd = gn[l] - gu[l];
-  out[2 * lm] = gd * qr / cm;
-  out[2 * lm + 1] = gd * qi / cm;
-  if (l == 0) return;
-  const int k = lm2k[lm];
-  surf_bar[(size_t)0 * nk + k] -= qr;
-  surf_bar[(size_t)1 * nk + k] -= qi;
-  surf_bar[(size_t)2 * nk + k] -= qr / g;
-  surf_bar[(size_t)3 * nk + k] -= qi / g;
+template <int MODE>
+__global__ void __launch_bounds__(SLE_THREADS) k_sle_rev(RevArgs A) {
+  extern __shared__ __align__(16) double dyn[];
+  double* const sm = MODE == 2 ? A.big + (size_t)blockIdx.x * A.scr : dyn;
+  __shared__ __align__(16) double part[4 * SLE_THREADS];
+  __shared__ double s_w[SLE_THREADS / 32];
+  __shared__ double s_sum;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int nphi = A.nphi, nlat = A.nlat, M = A.M;
+  const Pass<MODE> S(A, sm, part);
+  const Lon& G = S.G;
+  double2* F = reinterpret_cast<double2*>(A.F);
+  double2* FC = reinterpret_cast<double2*>(A.FC);
+  unsigned int target = 0;
+  // the row sum of the threads' values, to the row's slot (the first warp writes)
+  auto row_sum = [&](double v, int j) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if (lane == 0) s_w[wid] = v;
+    __syncthreads();
+    if (wid == 0) {
+      v = lane < SLE_THREADS / 32 ? s_w[lane] : 0.0;
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) __stcg(A.rowpart + j, v);
+    }
+  };
+  auto ice_bar = [&](size_t p, double d) {
+    A.gi1[p] += A.frac * d;
+    if (A.gi0) A.gi0[p] += (1.0 - A.frac) * d;
+  };
+  if (A.K == 0) {
+    for (int j = blockIdx.x; j < nlat; j += gridDim.x)
+      for (int i = tid; i < nphi; i += SLE_THREADS) {
+        const size_t p = (size_t)j * nphi + i;
+        if (!A.C[p]) ice_bar(p, A.fresh ? 0.0 : A.digbar[p]);
+      }
+    return;
+  }
+  for (int j = blockIdx.x; j < nlat; j += gridDim.x) {
+    double acc = 0.0;
+    for (int i = tid; i < nphi; i += SLE_THREADS) {
+      const double v = A.lam[(size_t)j * nphi + i];
+      S.L[i] = v;
+      acc += v;
+    }
+    row_sum(acc, j);
+    S.row_analysis(F + j, nlat);
+    for (int i = tid; i < nphi; i += SLE_THREADS) S.L[i] = A.C[(size_t)j * nphi + i] ? 1.0 : 0.0;
+    __syncthreads();
+    S.row_analysis(FC + j, nlat);
+  }
+  if (!grid_barrier(A.bar, target, A.wait_ns)) return bar_fail(A);
+  double int_bar = 0.0;
+  for (int it = 1;; ++it) {
+    // the last warp: sum of lam, beside the other warps' first loads of O
+    if (wid == SLE_THREADS / 32 - 1) {
+      double v = 0.0;
+      for (int j0 = lane; j0 < nlat; j0 += 256) {
+        double t[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t[u] = j0 + 32 * u < nlat ? __ldcg(A.rowpart + j0 + 32 * u) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v += t[u];
+      }
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) s_sum = v;
+    }
+    double cs_bar = 0.0;
+    for (int m = blockIdx.x, first = 1; first || m < M; m += gridDim.x, first = 0) {
+      const int nl = m < M ? A.lmax - m + 1 : 0, lm0 = A.mbeg[min(m, M - 1)];
+      if (nl) S.order_fold(A, m, it == 1, true);
+      __syncthreads();
+      if (first) {
+        cs_bar = -s_sum / A.C_int;
+        int_bar -= cs_bar;
+      }
+      if (nl == 0) break;
+      // kc: the spectrum of C, and the sum of q_bar over the iterations
+      const double cm = m == 0 ? 1.0 : 2.0;
+      S.order_analysis(
+          A, nl, lm0, it == 1,
+          [&](int x, double* kc) {
+            if (MODE != 1 && it > 1) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c) kc[c] = A.cst[4 * (size_t)(lm0 + x) + c];
+            }
+          },
+          [&](int x, double sr, double si, double cr, double ci, double* kc) {
+            double* keep = MODE == 1 ? S.Ks + 6 * x : A.cst + 4 * (size_t)(lm0 + x);
+            if (it == 1) {
+              kc[0] = cr;
+              kc[1] = ci;
+              keep[0] = cr;
+              keep[1] = ci;
+            } else if (MODE == 1) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c) kc[c] = keep[c];
+            }
+            const double t = cs_bar * A.dlon;
+            const double qr = fma(t, kc[0], sr) * cm / A.dlon, qi = m == 0 ? 0.0 : fma(t, kc[1], si) * cm / A.dlon;
+            const double tr = kc[2] + qr, ti = kc[3] + qi;
+            const int l = m + x;
+            if (it < A.K) {
+              keep[2] = tr;
+              keep[3] = ti;
+            } else if (l > 0) {
+              const int k = A.lm2k[lm0 + x];
+              A.surf_bar[k] -= tr;
+              A.surf_bar[(size_t)1 * A.nk + k] -= ti;
+              A.surf_bar[(size_t)2 * A.nk + k] -= tr / A.g;
+              A.surf_bar[(size_t)3 * A.nk + k] -= ti / A.g;
+            }
+            const double gd = A.gn[l] - A.gu[l];
+            S.dl[x] = make_double2(gd * qr / cm, gd * qi / cm);
+          });
+      __syncthreads();
+      S.order_synthesis(A, m, nl, lm0);
+      __syncthreads();
+    }
+    if (!grid_barrier(A.bar, target, A.wait_ns)) return bar_fail(A);
+    const bool last = it == A.K;
+    for (int j = blockIdx.x; j < nlat; j += gridDim.x) {
+      const size_t row = (size_t)j * nphi;
+      const double w = A.wts[j];
+      for (int m = tid; m < M; m += SLE_THREADS) S.Gd[m] = __ldcg(reinterpret_cast<const double2*>(A.D) + (size_t)j * M + m);
+      __syncthreads();
+      S.row_synthesis();
+      double acc = 0.0;
+      for (int u = tid; u < 4 * G.nbase; u += SLE_THREADS) {
+        const int i = u >> 2, pt = u & 3;
+        if (!G.has(i, pt)) continue;
+        const size_t p = row + G.at(i, pt);
+        const bool c = A.C[p] != 0;
+        const double d0 = it == 1 && A.fresh ? 0.0 : A.digbar[p];
+        const double lb = A.dlon * w * S.value(i, pt), v = c ? RHO_WATER * lb : 0.0, d = d0 + RHO_ICE * lb;
+        if (last) {
+          A.lam[p] = v;
+          if (!c) ice_bar(p, d - (RHO_ICE / RHO_WATER) * int_bar * w * A.dlon);
+        } else {
+          A.digbar[p] = d;
+          S.L[G.at(i, pt)] = v;
+          acc += v;
+        }
+      }
+      if (last) {
+        __syncthreads();  // the row's sums are read
+        continue;
+      }
+      row_sum(acc, j);
+      S.row_analysis(F + j, nlat);
+    }
+    if (last) break;
+    if (!grid_barrier(A.bar, target, A.wait_ns)) return bar_fail(A);
+  }
+  if (pass_last(A.bar) && tid == 0) A.bar[0] = A.bar[1] = 0u;
 }
 
 // s / c_m (the closing load's sigma_bar, ahead of the analysis transpose)
@@ -624,20 +753,6 @@ __global__ void k_rev_load(int ng, int nphi, const double* __restrict__ g, const
   const double v = C[p] ? RHO_WATER * lb : 0.0;
   lam_out[p] = add ? lam_out[p] + v : v;
   digbar[p] += RHO_ICE * lb;
-}
-
-// the end of a pass: ice_now_bar = (1 - C) (digbar - (rho_i / rho_w) ice_int_bar
-// w_j dlon), into the adjoints of this interval's end ice (frac) and of the
-// previous interval's (1 - frac; none for the first interval of the call)
-__global__ void k_rev_ice(int ng, int nphi, const unsigned char* __restrict__ C, const double* __restrict__ digbar,
-                          const double* __restrict__ wts, double dlon, const double* __restrict__ scal, int with_int,
-                          double frac, double* __restrict__ gi1, double* __restrict__ gi0) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= ng || C[p]) return;
-  double d = digbar[p];
-  if (with_int) d -= (RHO_ICE / RHO_WATER) * scal[1] * wts[p / nphi] * dlon;
-  gi1[p] += frac * d;
-  if (gi0) gi0[p] += (1.0 - frac) * d;
 }
 
 // sum over the 3-D elements' grids (n3 fields of ng) into y, divided by w_j
@@ -703,7 +818,7 @@ struct AdjWork {
   // spectral work arrays, d J / d ice, the tape
   DArr<double> ice, ck_rsl, ck_hice;
   DriverSnap entry;
-  DArr<double> rA, rB, digbar, ybuf, gbuf, obuf, sbuf, scal, rows, gice;
+  DArr<double> rA, digbar, ybuf, gbuf, obuf, gice;
   SleTape tape;
 };
 
@@ -1139,39 +1254,36 @@ void sle_interval(vg_handle* h, AdjWork& W, int n, double dt_yr, int nsite) {
   VG_CUDA(cudaGetLastError());
 }
 
-// One pass's adjoint iterations (the pass's K inner iterations in reverse)
-// from rb, the adjoint of the pass's final r, to the adjoint of its starting
-// r (left in rb); digbar and scal[1] (ice_int_bar) accumulate, surf_bar too.
-void rev_pass(vg_handle* h, AdjWork& W, const unsigned char* C, const TapePass& P, double*& rb, double*& rb2) {
-  const Grid& G = h->grid;
-  const int ng = G.ng, nphi = G.nphi, nlat = G.nlat, nlm = G.nlm;
-  const double dlon = 2.0 * PI / (double)nphi, sc = dlon;
-  cudaStream_t s = h->stream;
-  const int eg = (ng + 255) / 256, lg = (nlm + 255) / 256;
-  for (int k = 0; k < P.K; ++k) {
-    k_rev_rows<<<nlat, 128, 0, s>>>(nphi, rb, W.rows.p);
-    k_rev_scal<<<1, 32, 0, s>>>(nlat, W.rows.p, P.C_int, W.scal.p);
-    k_rev_y<<<eg, 256, 0, s>>>(ng, nphi, rb, C, G.d_wts.p, dlon, W.scal.p, W.ybuf.p);
-    h->n_launch += 3;
-    VG_CUDA(cudaGetLastError());
-    sht_analysis_dev(h, W.ybuf.p, W.obuf.p, 1);
-    k_rev_apply<<<lg, 256, 0, s>>>(nlm, h->nk, h->g, sc, G.d_lm_l.p, G.d_lm_m.p, h->d_lm2k.p, h->d_gu.p, h->d_gn.p,
-                                   W.obuf.p, W.surf_bar.p, W.sbuf.p);
-    ++h->n_launch;
-    VG_CUDA(cudaGetLastError());
-    sht_synthesis_dev(h, W.sbuf.p, W.gbuf.p, 1);
-    k_rev_load<<<eg, 256, 0, s>>>(ng, nphi, W.gbuf.p, G.d_wts.p, sc, C, 0, rb2, W.digbar.p);
-    ++h->n_launch;
-    VG_CUDA(cudaGetLastError());
-    std::swap(rb, rb2);
-  }
+// One pass's adjoint: rb from the adjoint of the pass's final rsl to that of its
+// starting rsl, surf_bar and the ice adjoints accumulate
+void rev_pass(vg_handle* h, AdjWork& W, const unsigned char* C, const TapePass& P, bool fresh, double frac, double* gi1,
+              double* gi0, double* rb) {
+  static const void* const kernel[3] = {(const void*)k_sle_rev<0>, (const void*)k_sle_rev<1>,
+                                        (const void*)k_sle_rev<2>};
+  RevArgs A;
+  pass_base(h, A);  // (the forward has planned the passes)
+  A.nk = h->nk;
+  A.K = P.K;
+  A.fresh = fresh;
+  A.C_int = P.C_int;
+  A.g = h->g;
+  A.frac = frac;
+  A.C = C;
+  A.gu = h->d_gu.p;
+  A.gn = h->d_gn.p;
+  A.lm2k = h->d_lm2k.p;
+  A.lam = rb;
+  A.digbar = W.digbar.p;
+  A.surf_bar = W.surf_bar.p;
+  A.gi1 = gi1;
+  A.gi0 = gi0;
+  pass_launch(h, kernel, &A);
 }
 
 // the reverse of one accepted sub-step: lam = the memory adjoint after it,
 // rb = the adjoint of its final rsl; on return lam = the adjoint before it,
 // rb = the adjoint of the rsl it started from
-void rev_substep(vg_handle* h, AdjWork& W, const TapeSub& sb, double dt_ref, bool warm, double*& rb,
-                 double*& rb2) {
+void rev_substep(vg_handle* h, AdjWork& W, const TapeSub& sb, double dt_ref, bool warm, double* rb) {
   const Grid& G = h->grid;
   const int ng = G.ng, nphi = G.nphi, nlm = G.nlm;
   const size_t n2 = 2 * (size_t)nlm;
@@ -1200,13 +1312,7 @@ void rev_substep(vg_handle* h, AdjWork& W, const TapeSub& sb, double dt_ref, boo
   for (int io = sb.npass - 1; io >= 0; --io) {
     const TapePass& P = T.passes[sb.pass0 + io];
     const unsigned char* C = T.cb.p + (size_t)(sb.pass0 + io) * ng;
-    if (io != sb.npass - 1) VG_CUDA(cudaMemsetAsync(W.digbar.p, 0, (size_t)ng * sizeof(double), s));
-    VG_CUDA(cudaMemsetAsync(W.scal.p, 0, 2 * sizeof(double), s));
-    rev_pass(h, W, C, P, rb, rb2);
-    k_rev_ice<<<eg, 256, 0, s>>>(ng, nphi, C, W.digbar.p, G.d_wts.p, dlon, W.scal.p, P.K > 0 ? 1 : 0, sb.frac, gi1,
-                                 gi0);
-    ++h->n_launch;
-    VG_CUDA(cudaGetLastError());
+    rev_pass(h, W, C, P, io != sb.npass - 1, sb.frac, gi1, gi0, rb);
   }
   // the first pass started from the previous sub-step's rsl (warm start) or from zero
   if (!warm) VG_CUDA(cudaMemsetAsync(rb, 0, (size_t)ng * sizeof(double), s));
@@ -1323,14 +1429,10 @@ double sle_misfit_grad_dev(vg_handle* h, int nsteps, double dt_yr, const double*
   // reverse sweep
   reverse_prepare(h, W);
   ensure(W.rA, ng);
-  ensure(W.rB, ng);
   ensure(W.digbar, ng);
   ensure(W.ybuf, ng);
   ensure(W.gbuf, ng);
   ensure(W.obuf, 2 * (size_t)G.nlm);
-  ensure(W.sbuf, 2 * (size_t)G.nlm);
-  ensure(W.scal, 2);
-  ensure(W.rows, (size_t)G.nlat);
   ensure(W.gice, (size_t)nsteps * ng);
   VG_CUDA(cudaMemsetAsync(W.lam.p, 0, S * sizeof(double), s));
   VG_CUDA(cudaMemsetAsync(W.rA.p, 0, ng * sizeof(double), s));
@@ -1340,7 +1442,6 @@ double sle_misfit_grad_dev(vg_handle* h, int nsteps, double dt_yr, const double*
     VG_CUDA(cudaMemsetAsync(W.gradMdt.p, 0, (size_t)h->ne3d * ng * sizeof(double), s));
   }
   double* rb = W.rA.p;
-  double* rb2 = W.rB.p;
   const bool warm = h->p.sle_warm_start != 0;
   for (int c = nck - 1; c >= 0; --c) {
     if (c != nck - 1) {
@@ -1353,7 +1454,7 @@ double sle_misfit_grad_dev(vg_handle* h, int nsteps, double dt_yr, const double*
       k_site_scatter<<<1, 32, 0, s>>>(nsite, W.site.p, W.resid.p + (size_t)n * nsite, rb);
       ++h->n_launch;
       VG_CUDA(cudaGetLastError());
-      for (; q >= 0 && T.subs[q].n == n; --q) rev_substep(h, W, T.subs[q], dt_ref, warm, rb, rb2);
+      for (; q >= 0 && T.subs[q].n == n; --q) rev_substep(h, W, T.subs[q], dt_ref, warm, rb);
     }
     if (q != -1) throw Error("vg_sle_misfit_grad: the recorded sub-steps do not match the segment's intervals");
   }
@@ -1393,7 +1494,7 @@ double sle_misfit_grad_dev(vg_handle* h, int nsteps, double dt_yr, const double*
       std::fill(grad_pert_lm, grad_pert_lm + n2, 0.0);
     }
   }
-  VG_CUDA(cudaStreamSynchronize(s));
+  check_pass_barrier(h);
   guard.restore();
   return J;
 }

@@ -7,15 +7,12 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <type_traits>
 
 #include "vg_device.cuh"
 #include "vg_internal.cuh"
+#include "vg_sle_pass.cuh"
 
 namespace vg {
-
-// per-row partial results
-enum { RP_C = 0, RP_DIG, RP_ZETA, RP_CS, RP_DMAX, RP_DMIN, RP_SMAX, RP_SMIN, RP_MASS, RP_N };
 
 __device__ __forceinline__ double ocean(double topo, double ice) {
   return (topo < 0.0 && RHO_ICE * ice < -RHO_WATER * topo) ? 1.0 : 0.0;
@@ -170,191 +167,14 @@ __global__ void k_step_end(int nphi, int nlat, double dlon, const double* __rest
 // small kernels for the integrals, the coastline and the closing load that the
 // pass now holds; it takes 100 us (362). Of an iteration's cycles at lmax 128 the
 // barriers are 4700, O 9000 (order 0, which the others wait for), R 12000.
-constexpr int SLE_THREADS = 512;
-
-// pitch of the Legendre functions in shared memory: half warps of two degrees by
-// eight rows read different banks
-__host__ __device__ inline int p_pitch(int nh) { return (nh + 7) / 16 * 16 + 8; }
-
-struct PassArgs {
-  int nphi, nlat, M, nlm, nk, lmax, n_inner, subgrid, fixed;
-  double tol, dlon, g;
-  const double *ice, *topo0, *C0, *dig, *C, *cs, *sn, *plm, *wts, *gu, *gn, *drift, *srot;
-  const int *lm2k, *mbeg;
-  double *wcorr, *rsl, *F, *FC, *sigma, *cst, *D, *Sraw, *Cn, *rowpart, *big;
-  size_t scr;  // doubles of the work area
-  SleScalars* sc;
-  unsigned int* bar;  // arrivals, finished CTAs, error
-  unsigned long long wait_ns;  // bound on a grid barrier's wait (the handle's wait limit, 2 s by default)
+struct PassArgs : PassBase {
+  int nk, n_inner, subgrid, fixed;
+  double tol, g;
+  const double *ice, *topo0, *C0, *dig, *C, *gu, *gn, *drift, *srot;
+  const int* lm2k;
+  double *wcorr, *rsl, *sigma, *Sraw, *Cn;
 };
 
-__device__ __forceinline__ unsigned long long gtimer_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Grid barrier: arrivals counted up to `target`, with a bounded wait. Returns
-// false (in every thread of the CTA) if it timed out or another CTA reported a
-// timeout. What other CTAs wrote before it is read with ld.cg after it.
-__device__ bool grid_barrier(unsigned int* bar, unsigned int& target, unsigned long long wait_ns) {
-  __shared__ int s_ok;
-  __syncthreads();
-  target += gridDim.x;
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-    const unsigned long long t0 = gtimer_ns();
-    for (int n = 0;; ++n) {
-      unsigned int v;
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-      if ((int)(v - target) >= 0) break;
-      // the timer is read now and then (each time for a limit too short for that)
-      if ((wait_ns < 10000 || (n & 15) == 15) &&
-          (gtimer_ns() - t0 > wait_ns || *(volatile unsigned int*)(bar + 2))) {
-        atomicExch(bar + 2, 1u);
-        ok = 0;
-        break;
-      }
-    }
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
-
-// a grid barrier gave up: record it where the host reads the loop's scalars
-__device__ __forceinline__ void bar_fail(const PassArgs& A) {
-  if (threadIdx.x == 0) A.sc->bar_error = 1;
-}
-
-// sum_j w_j row_j 2 pi / nphi (src/vilma_sht.f90:184-202) by one warp, the same
-// value in every lane and CTA
-__device__ __forceinline__ double warp_rows(const double* row, const double* w, int nlat, double dlon) {
-  double s = 0.0;
-  for (int j0 = threadIdx.x & 31; j0 < nlat; j0 += 256) {
-    double t[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) t[u] = j0 + 32 * u < nlat ? w[j0 + 32 * u] * __ldcg(row + j0 + 32 * u) * dlon : 0.0;
-#pragma unroll
-    for (int u = 0; u < 8; ++u) s += t[u];
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  return s;
-}
-
-// largest value of a warp, in every lane, by two integer reductions on the
-// order-preserving bit pattern (a positive NaN counts as the largest)
-__device__ __forceinline__ double warp_max(double v) {
-  const long long b = __double_as_longlong(v);
-  const unsigned long long k = (unsigned long long)b ^ (b < 0 ? ~0ull : 1ull << 63);
-  const unsigned int hi = (unsigned int)(k >> 32);
-  const unsigned int H = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned int L = __reduce_max_sync(0xffffffffu, hi == H ? (unsigned int)k : 0u);
-  const unsigned long long r = ((unsigned long long)H << 32) | L;
-  return __longlong_as_double((long long)(r ^ ((r >> 63) ? 1ull << 63 : ~0ull)));
-}
-
-// twiddle table in shared memory, skewed so that strides of 2, 4 and 8 entries
-// fall in different banks
-__device__ __forceinline__ int tw_at(int t) { return t + (t >> 3); }
-
-// Longitudes of base longitude i: i, i + half, nphi - i, half - i (nphi odd: i
-// and nphi - i only); the last two only where they are points of their own
-struct Lon {
-  int nphi, half, nbase;
-  bool even;
-  __device__ __forceinline__ Lon(int n) : nphi(n), half(n / 2), nbase(n % 2 ? (n + 1) / 2 : n / 4 + 1), even(n % 2 == 0) {}
-  __device__ __forceinline__ int at(int i, int pt) const {
-    return pt == 0 ? i : pt == 1 ? i + half : pt == 2 ? nphi - i : half - i;
-  }
-  __device__ __forceinline__ bool has(int i, int pt) const {
-    if (pt == 0) return true;
-    if (!even) return pt == 2 && i > 0;
-    return pt == 1 || (i > 0 && 2 * i != half);
-  }
-};
-
-// This thread's share of a longitude sum over `n` outputs with Q parts each:
-// part q of output o, the twiddle index t0 of its first term and the step between
-// its terms (a term advances the index by o, `mul` terms of other parts between)
-struct Share {
-  int Q, q, o, t0, step;
-  __device__ __forceinline__ Share(int n, int mul, int nphi, int u) {
-    Q = max(1, min(16, SLE_THREADS / n));
-    q = u / n;
-    o = u - q * n;
-    t0 = (int)(((unsigned)(mul * q) * (unsigned)o) % (unsigned)nphi);
-    step = (int)(((unsigned)(mul * Q) * (unsigned)o) % (unsigned)nphi);
-  }
-};
-
-struct PassSmem {  // carved from the dynamic shared memory
-  double2 *tw, *Gd, *Fe, *dl;  // twiddles; a row's spectrum; an order's rows [4][nh]; its degrees
-  double *X, *L;               // per base longitude four values; a row of the grid
-};
-
-// F(m) = 2 pi / nphi sum_i L_i e^{-i m phi_i} of the row in S.L, to out[m stride]
-__device__ __forceinline__ void row_analysis(const Lon& G, int M, const PassSmem& S, const Share& A0, double* part,
-                                             double2* out, int stride) {
-  const int tid = threadIdx.x;
-  for (int i = tid; i < G.nbase; i += SLE_THREADS) {
-    double v[4];
-#pragma unroll
-    for (int pt = 0; pt < 4; ++pt) v[pt] = G.has(i, pt) ? S.L[G.at(i, pt)] : 0.0;
-    double4 x;
-    if (G.even) {
-      const double ab = v[0] + v[1], am = v[0] - v[1], cd = v[2] + v[3], cm = v[2] - v[3];
-      x = make_double4(ab + cd, ab - cd, am + cm, am - cm);
-    } else {
-      x = make_double4(v[0] + v[2], v[0] - v[2], v[0] + v[2], v[0] - v[2]);
-    }
-    reinterpret_cast<double2*>(S.X)[2 * i] = make_double2(x.x, x.y);
-    reinterpret_cast<double2*>(S.X)[2 * i + 1] = make_double2(x.z, x.w);
-  }
-  __syncthreads();
-  const int Q = A0.Q;
-  const double sc = 2.0 * PI / (double)G.nphi;
-  for (int base = 0; base < M * Q; base += SLE_THREADS) {
-    const Share sh = base ? Share(M, 1, G.nphi, base + tid) : A0;
-    const int m = sh.o;
-    double re = 0.0, im = 0.0;
-    if (base + tid < M * Q) {
-      const double2* x = reinterpret_cast<const double2*>(S.X) + (m & 1);
-      int t = sh.t0;
-#pragma unroll 4
-      for (int i = sh.q; i < G.nbase; i += Q) {
-        const double2 w = S.tw[tw_at(t)], v = x[2 * i];
-        re = fma(v.x, w.x, re);
-        im = fma(-v.y, w.y, im);
-        t += sh.step;
-        if (t >= G.nphi) t -= G.nphi;
-      }
-    }
-    if (Q == 1) {
-      if (base + tid < M) __stcg(out + (size_t)m * stride, make_double2(re * sc, im * sc));
-    } else {
-      part[2 * tid] = re;
-      part[2 * tid + 1] = im;
-      __syncthreads();
-      if (tid < M) {
-        for (int c = 1; c < Q; ++c) {
-          re += part[2 * (tid + c * M)];
-          im += part[2 * (tid + c * M) + 1];
-        }
-        __stcg(out + (size_t)m * stride, make_double2(re * sc, im * sc));
-      }
-    }
-  }
-  __syncthreads();
-}
-
-// A CTA with one order keeps that order's Legendre functions (northern rows) in
-// shared memory (MODE 1), where they fit: the barriers invalidate L1, so read
-// through it (MODE 0) they come from L2 in each iteration (106 us a pass at lmax
-// 128 and 77 at lmax 85, against 100 and 76). MODE 2, a grid whose
-// work area does not fit in shared memory: the work area is A.scr doubles a CTA of
-// global memory.
 template <int MODE>
 __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
   extern __shared__ __align__(16) double dyn[];
@@ -363,37 +183,20 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
   __shared__ double s_w[5][SLE_THREADS / 32];
   __shared__ double s_int[3], s_red[5];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int nphi = A.nphi, nlat = A.nlat, M = A.M, nh = (nlat + 1) / 2;
-  const Lon G(nphi);
-  PassSmem S;
-  S.tw = reinterpret_cast<double2*>(sm);
-  S.Gd = S.tw + tw_at(nphi) + 1;  // the rows' phase
-  S.X = reinterpret_cast<double*>(S.Gd + M);
-  S.L = S.X + 4 * G.nbase;
-  S.Fe = S.Gd;  // the orders' phase: the same space
-  S.dl = S.Fe + 4 * nh;
-  const int pp = p_pitch(nh);
-  double* const Ps = sm + A.scr;
-  double* const Ks = Ps + (size_t)(A.lmax + 1) * pp;  // [degree][6], see below
-  if (MODE == 1 && blockIdx.x < M) {
-    const int m = blockIdx.x;
-    for (int x = tid; x < A.lmax - m + 1; x += SLE_THREADS) {
-      Ks[6 * x + 4] = A.gu[m + x];
-      Ks[6 * x + 5] = A.gn[m + x];
+  const int nphi = A.nphi, nlat = A.nlat, M = A.M;
+  const Pass<MODE> S(A, sm, part);
+  const Lon& G = S.G;
+  if (MODE == 1 && blockIdx.x < M)
+    for (int x = tid; x < A.lmax - (int)blockIdx.x + 1; x += SLE_THREADS) {
+      S.Ks[6 * x + 4] = A.gu[blockIdx.x + x];
+      S.Ks[6 * x + 5] = A.gn[blockIdx.x + x];
     }
-    for (int u = tid; u < (A.lmax - m + 1) * nh; u += SLE_THREADS) {
-      const int x = u / nh, j = u - x * nh;
-      Ps[(size_t)x * pp + j] = A.plm[(size_t)(A.mbeg[m] + x) * nlat + j];
-    }
-  }
-  const Share ss(G.nbase, 2, nphi, tid), sa(M, 1, nphi, tid);
   unsigned int target = 0;
   // the pass integrals, in every CTA from the row sums of the setup
   if (wid < 3) {
     const double v = warp_rows(A.rowpart + (wid == 0 ? RP_C : wid == 1 ? RP_DIG : RP_ZETA) * nlat, A.wts, nlat, A.dlon);
     if (lane == 0) s_int[wid] = v;
   }
-  for (int t = tid; t < nphi; t += SLE_THREADS) S.tw[tw_at(t)] = make_double2(A.cs[t], A.sn[t]);
   __syncthreads();
   const double C_int = s_int[0], ice_int = -(RHO_ICE / RHO_WATER) * s_int[1];
   const double zeta_int = A.subgrid ? s_int[2] : 0.0;
@@ -409,9 +212,8 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
     }
   }
   if (!(C_int > 0.0)) return;  // no ocean: nothing to redistribute (the same value in every CTA)
-  double2* F = reinterpret_cast<double2*>(A.F);    // [m][j]
+  double2* F = reinterpret_cast<double2*>(A.F);
   double2* FC = reinterpret_cast<double2*>(A.FC);  // of the load rho_w C
-  double2* D = reinterpret_cast<double2*>(A.D);    // [j][m], twice the coefficient above m = 0
   // the subgrid load, the load of the entering rsl and that of rho_w C
   for (int j = blockIdx.x; j < nlat; j += gridDim.x) {
     for (int i = tid; i < nphi; i += SLE_THREADS) {
@@ -421,10 +223,10 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
       S.L[i] = RHO_ICE * A.dig[p] + RHO_WATER * (c * A.rsl[p]) + wc;
     }
     __syncthreads();
-    row_analysis(G, M, S, sa, part, F + j, nlat);
+    S.row_analysis(F + j, nlat);
     for (int i = tid; i < nphi; i += SLE_THREADS) S.L[i] = RHO_WATER * A.C[(size_t)j * nphi + i];
     __syncthreads();
-    row_analysis(G, M, S, sa, part, FC + j, nlat);
+    S.row_analysis(FC + j, nlat);
   }
   if (!grid_barrier(A.bar, target, A.wait_ns)) return bar_fail(A);
   double dphi = 0.0;  // of the last iteration done
@@ -454,14 +256,7 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
     // ---- O: orders of this CTA; once done, only the closing load's spectrum
     for (int m = blockIdx.x, first = 1; first || m < M; m += gridDim.x, first = 0) {
       const int nl = m < M ? A.lmax - m + 1 : 0, lm0 = A.mbeg[min(m, M - 1)];
-      for (int u = tid; u < (nl ? (it > 1 ? nh : 2 * nh) : 0); u += SLE_THREADS) {
-        const int f = u >= nh, j = u - f * nh, jm = nlat - 1 - j;  // f: of rho_w C, the first time only
-        const double2* src = (f ? FC : F) + (size_t)m * nlat;
-        const double2 a = __ldcg(src + j), b = jm != j ? __ldcg(src + jm) : make_double2(0.0, 0.0);
-        const double w = A.wts[j];
-        S.Fe[(2 * f) * nh + j] = make_double2(w * (a.x + b.x), w * (a.y + b.y));
-        S.Fe[(2 * f + 1) * nh + j] = make_double2(w * (a.x - b.x), w * (a.y - b.y));
-      }
+      if (nl) S.order_fold(A, m, it == 1, false);
       __syncthreads();
       if (it > 1 && first) {
         // dphi and the convergence test (src/vilma_sle.f90:320-338); NaN anywhere in
@@ -480,147 +275,54 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
         }
       }
       if (nl == 0) break;
-      // analysis: eight lanes a degree, up to three degrees a thread
-      constexpr int W = 8, NX = SLE_THREADS / W, NV = 3;
-      const int lw = lane & (W - 1);
-      for (int x0 = 0; x0 < nl; x0 += NV * NX) {
-        const int xa = x0 + tid / W, nv = min(NV, (nl - x0 + NX - 1) / NX);
-        // lane v < nv closes degree xa + v NX: the spectrum of rho_w C and the drift's
-        // part of N - u, both kept from the first iteration, and the response factors
-        const int xk = xa + lw * NX, lmk = lm0 + xk;
-        const bool mine = lw < nv && xk < nl;
-        double kc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        if (mine && MODE != 1) {
-          kc[4] = A.gu[m + xk];
-          kc[5] = A.gn[m + xk];
-        }
-        if (mine && it == 1) {
-          if (m + xk > 0) {
-            const int k = A.lm2k[lmk];
-            kc[2] = -(A.drift[(size_t)2 * A.nk + k] / A.g) - A.drift[k];
-            kc[3] = -(A.drift[(size_t)3 * A.nk + k] / A.g) - A.drift[(size_t)A.nk + k];
-          }
-        } else if (mine && MODE != 1) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) kc[c] = A.cst[4 * (size_t)lmk + c];
-        }
-        double re[NV] = {}, im[NV] = {}, rc[NV] = {}, ic[NV] = {};
-        const double* P[NV];
-        const double2* fe[NV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-          const int x = min(xa + v * NX, nl - 1);  // past the end: a valid row, result unused
-          P[v] = MODE == 1 ? Ps + (size_t)x * pp : A.plm + (size_t)(lm0 + x) * nlat;
-          fe[v] = S.Fe + (x & 1) * nh;
-        }
-        auto sums = [&](auto NVc, auto FIRST) {
-#pragma unroll 3
-          for (int j = lw; j < nh; j += W) {
-#pragma unroll
-            for (int v = 0; v < NVc.value; ++v) {
-              const double p = MODE == 1 ? P[v][j] : __ldg(P[v] + j);
-              const double2 f = fe[v][j];
-              re[v] = fma(p, f.x, re[v]);
-              im[v] = fma(p, f.y, im[v]);
-              if (FIRST.value) {
-                const double2 c = fe[v][2 * nh + j];
-                rc[v] = fma(p, c.x, rc[v]);
-                ic[v] = fma(p, c.y, ic[v]);
-              }
+      // kc: the spectrum of rho_w C and the drift's part of N - u, both kept from the
+      // first iteration, and the response factors
+      S.order_analysis(
+          A, nl, lm0, it == 1,
+          [&](int x, double* kc) {
+            if (MODE != 1) {
+              kc[4] = A.gu[m + x];
+              kc[5] = A.gn[m + x];
             }
-          }
-#pragma unroll
-          for (int o = W / 2; o > 0; o >>= 1)
-#pragma unroll
-            for (int v = 0; v < NVc.value; ++v) {
-              re[v] += __shfl_xor_sync(0xffffffffu, re[v], o);
-              im[v] += __shfl_xor_sync(0xffffffffu, im[v], o);
-              if (FIRST.value) {
-                rc[v] += __shfl_xor_sync(0xffffffffu, rc[v], o);
-                ic[v] += __shfl_xor_sync(0xffffffffu, ic[v], o);
+            if (it == 1) {
+              if (m + x > 0) {
+                const int k = A.lm2k[lm0 + x];
+                kc[2] = -(A.drift[(size_t)2 * A.nk + k] / A.g) - A.drift[k];
+                kc[3] = -(A.drift[(size_t)3 * A.nk + k] / A.g) - A.drift[(size_t)A.nk + k];
               }
+            } else if (MODE != 1) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c) kc[c] = A.cst[4 * (size_t)(lm0 + x) + c];
             }
-        };
-        using std::integral_constant;
-        if (it == 1) {
-          sums(integral_constant<int, 3>(), integral_constant<bool, true>());
-        } else if (nv == 3) {
-          sums(integral_constant<int, 3>(), integral_constant<bool, false>());
-        } else if (nv == 2) {
-          sums(integral_constant<int, 2>(), integral_constant<bool, false>());
-        } else {
-          sums(integral_constant<int, 1>(), integral_constant<bool, false>());
-        }
-        if (mine) {
-          double sr = lw == 0 ? re[0] : lw == 1 ? re[1] : re[2], si = lw == 0 ? im[0] : lw == 1 ? im[1] : im[2];
-          if (it == 1) {
-            kc[0] = lw == 0 ? rc[0] : lw == 1 ? rc[1] : rc[2];
-            kc[1] = lw == 0 ? ic[0] : lw == 1 ? ic[1] : ic[2];
+          },
+          [&](int x, double sr, double si, double cr, double ci, double* kc) {
+            const int lm = lm0 + x;
+            if (it == 1) {
+              kc[0] = cr;
+              kc[1] = ci;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) (MODE == 1 ? Ks + 6 * xk : A.cst + 4 * (size_t)lmk)[c] = kc[c];
-          } else if (MODE == 1) {
+              for (int c = 0; c < 4; ++c) (MODE == 1 ? S.Ks + 6 * x : A.cst + 4 * (size_t)lm)[c] = kc[c];
+            } else if (MODE == 1) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) kc[c] = Ks[6 * xk + c];
-          }
-          if (MODE == 1) {
-            kc[4] = Ks[6 * xk + 4];
-            kc[5] = Ks[6 * xk + 5];
-          }
-          if (it > 1) {
-            sr = fma(dphi, kc[0], sr);
-            si = fma(dphi, kc[1], si);
-          }
-          if (done) {
-            A.sigma[2 * lmk] = sr;
-            A.sigma[2 * lmk + 1] = si;
-          }
-          S.dl[xk] = make_double2((kc[5] * sr - kc[4] * sr) + kc[2], (kc[5] * si - kc[4] * si) + kc[3]);
-        }
-      }
+              for (int c = 0; c < 4; ++c) kc[c] = S.Ks[6 * x + c];
+            }
+            if (MODE == 1) {
+              kc[4] = S.Ks[6 * x + 4];
+              kc[5] = S.Ks[6 * x + 5];
+            }
+            if (it > 1) {
+              sr = fma(dphi, kc[0], sr);
+              si = fma(dphi, kc[1], si);
+            }
+            if (done) {
+              A.sigma[2 * lm] = sr;
+              A.sigma[2 * lm + 1] = si;
+            }
+            S.dl[x] = make_double2((kc[5] * sr - kc[4] * sr) + kc[2], (kc[5] * si - kc[4] * si) + kc[3]);
+          });
       __syncthreads();
       if (done) continue;
-      // synthesis: a thread per (northern row, part of the degree pairs)
-      const int Q = max(1, min(16, SLE_THREADS / nh));
-      for (int base = 0; base < nh * Q; base += SLE_THREADS) {
-        const int u = base + tid, q = u / nh, j = u - q * nh;
-        double er = 0.0, ei = 0.0, orr = 0.0, oi = 0.0;
-        if (u < nh * Q) {
-          const double* P = MODE == 1 ? Ps + j : A.plm + (size_t)lm0 * nlat + j;
-          const int pt = MODE == 1 ? pp : nlat;
-#pragma unroll 4
-          for (int x = 2 * q; x < nl; x += 2 * Q) {
-            const double p = MODE == 1 ? P[(size_t)x * pt] : __ldg(P + (size_t)x * pt);
-            const double2 d = S.dl[x];
-            er = fma(p, d.x, er);
-            ei = fma(p, d.y, ei);
-            if (x + 1 < nl) {
-              const double p1 = MODE == 1 ? P[(size_t)(x + 1) * pt] : __ldg(P + (size_t)(x + 1) * pt);
-              const double2 d1 = S.dl[x + 1];
-              orr = fma(p1, d1.x, orr);
-              oi = fma(p1, d1.y, oi);
-            }
-          }
-        }
-        if (Q > 1) {
-          reinterpret_cast<double2*>(part)[2 * tid] = make_double2(er, ei);
-          reinterpret_cast<double2*>(part)[2 * tid + 1] = make_double2(orr, oi);
-          __syncthreads();
-        }
-        if (Q > 1 ? tid < nh : u < nh) {
-          for (int c = 1; c < Q; ++c) {
-            const double2 e = reinterpret_cast<const double2*>(part)[2 * (tid + c * nh)];
-            const double2 o = reinterpret_cast<const double2*>(part)[2 * (tid + c * nh) + 1];
-            er += e.x;
-            ei += e.y;
-            orr += o.x;
-            oi += o.y;
-          }
-          const double w = m == 0 ? 1.0 : 2.0;
-          const int jm = nlat - 1 - j;
-          __stcg(D + (size_t)j * M + m, make_double2(w * (er + orr), w * (ei + oi)));
-          if (jm != j) __stcg(D + (size_t)jm * M + m, make_double2(w * (er - orr), w * (ei - oi)));
-        }
-      }
+      S.order_synthesis(A, m, nl, lm0);
       __syncthreads();
     }
     if (done) break;
@@ -628,7 +330,7 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
     // ---- R: rows of this CTA
     for (int j = blockIdx.x; j < nlat; j += gridDim.x) {
       const size_t row = (size_t)j * nphi;
-      for (int m = tid; m < M; m += SLE_THREADS) S.Gd[m] = __ldcg(D + (size_t)j * M + m);
+      for (int m = tid; m < M; m += SLE_THREADS) S.Gd[m] = __ldcg(reinterpret_cast<const double2*>(A.D) + (size_t)j * M + m);
       // this thread's first grid point, on its way while the sums are formed
       double pc = 0.0, pd = 0.0, pw = 0.0, po = 0.0, pr = 0.0;
       auto fetch = [&](int u) {
@@ -644,61 +346,13 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
       };
       fetch(tid);
       __syncthreads();
-      const int Q = ss.Q;
-      for (int base = 0; base < G.nbase * Q; base += SLE_THREADS) {
-        const Share sh = base ? Share(G.nbase, 2, nphi, base + tid) : ss;
-        const int i = sh.o;
-        double ce = 0.0, se = 0.0, co = 0.0, so = 0.0;
-        if (base + tid < G.nbase * Q) {
-          int t = sh.t0;
-#pragma unroll 2
-          for (int m = 2 * sh.q; m < M; m += 2 * Q) {
-            const double2 w = S.tw[tw_at(t)], v = S.Gd[m];
-            ce = fma(v.x, w.x, ce);
-            se = fma(v.y, w.y, se);
-            if (m + 1 < M) {
-              int t1 = t + i;
-              if (t1 >= nphi) t1 -= nphi;
-              const double2 w1 = S.tw[tw_at(t1)], v1 = S.Gd[m + 1];
-              co = fma(v1.x, w1.x, co);
-              so = fma(v1.y, w1.y, so);
-            }
-            t += sh.step;
-            if (t >= nphi) t -= nphi;
-          }
-        }
-        if (Q == 1) {
-          if (base + tid < G.nbase) {
-            reinterpret_cast<double2*>(S.X)[2 * i] = make_double2(ce, se);
-            reinterpret_cast<double2*>(S.X)[2 * i + 1] = make_double2(co, so);
-          }
-        } else {
-          part[tid] = ce;
-          part[SLE_THREADS + tid] = se;
-          part[2 * SLE_THREADS + tid] = co;
-          part[3 * SLE_THREADS + tid] = so;
-        }
-      }
-      __syncthreads();
-      if (Q > 1) {
-        for (int u = tid; u < 4 * G.nbase; u += SLE_THREADS) {
-          const int s4 = u / G.nbase, i = u - s4 * G.nbase;
-          double v = 0.0;
-#pragma unroll 4
-          for (int c = 0; c < Q; ++c) v += part[s4 * SLE_THREADS + c * G.nbase + i];
-          S.X[4 * i + s4] = v;
-        }
-        __syncthreads();
-      }
+      S.row_synthesis();
       double acc = 0.0, dmx = -HUGE_VAL, dmn = -HUGE_VAL, smx = -HUGE_VAL, smn = -HUGE_VAL;  // minima negated
       for (int u = tid; u < 4 * G.nbase; u += SLE_THREADS) {
         if (u != tid) fetch(u);
         const int i = u >> 2, pt = u & 3;
         if (!G.has(i, pt)) continue;
-        const double2 e = reinterpret_cast<const double2*>(S.X)[2 * i], o = reinterpret_cast<const double2*>(S.X)[2 * i + 1];
-        const double ev = pt < 2 ? e.x - e.y : e.x + e.y, ov = pt < 2 ? o.x - o.y : o.x + o.y;
-        double v = (pt & 1) ? ev - ov : ev + ov;
-        v += pr;
+        const double v = S.value(i, pt) + pr;
         const size_t p = row + G.at(i, pt);
         A.Sraw[p] = v;
         S.L[G.at(i, pt)] = RHO_ICE * pd + RHO_WATER * (pc * v) + pw;
@@ -738,7 +392,7 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
         const int slot = k == 0 ? RP_CS : k == 1 ? RP_DMAX : k == 2 ? RP_DMIN : k == 3 ? RP_SMAX : RP_SMIN;
         if (lane == 0) __stcg(A.rowpart + slot * nlat + j, v);
       }
-      row_analysis(G, M, S, sa, part, F + j, nlat);
+      S.row_analysis(F + j, nlat);
     }
     if (!grid_barrier(A.bar, target, A.wait_ns)) return bar_fail(A);
   }
@@ -773,15 +427,7 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
   flips = __reduce_add_sync(0xffffffffu, flips);
   if (lane == 0 && flips) atomicAdd(&A.sc->flips, flips);
   // the CTA that finishes last adds the rows' mass and resets the barrier
-  __shared__ int s_last;
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    s_last = atomicAdd(A.bar + 1, 1u) == gridDim.x - 1;
-    __threadfence();
-  }
-  __syncthreads();
-  if (s_last && wid == 0) {
+  if (pass_last(A.bar) && wid == 0) {
     const double v = warp_rows(A.rowpart + RP_MASS * nlat, A.wts, nlat, A.dlon);
     if (lane == 0) {
       A.sc->mass_Cs = v - zeta_int;
@@ -804,81 +450,104 @@ __global__ void k_mass(SleScalars* sc, const double* __restrict__ rowpart, const
   if (threadIdx.x == 0) sc->mass_Cs = m - sc->zeta_int;
 }
 
-static const void* pass_kernel(int mode) {
-  return mode == 2 ? (const void*)k_sle_pass<2> : mode == 1 ? (const void*)k_sle_pass<1> : (const void*)k_sle_pass<0>;
+// the variant and grid of a handle's passes, by the sea-level pass (its adjoint
+// has less static shared memory and the same registers a CTA)
+void pass_plan(vg_handle* h, const void* const kernel[3]) {
+  if (h->sle_grid != 0) return;
+  const Grid& G = h->grid;
+  const size_t scr = sle_pass_scratch(G);
+  int dev = 0, nsm = 0, lim = 0;
+  VG_CUDA(cudaGetDevice(&dev));
+  VG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  VG_CUDA(cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  cudaFuncAttributes fa;
+  VG_CUDA(cudaFuncGetAttributes(&fa, kernel[0]));
+  const size_t room = (size_t)lim - fa.sharedSizeBytes, psz = (size_t)(p_pitch((G.nlat + 1) / 2) + 6) * (G.lmax + 1);
+  const int ctas = h->p.sle_ctas > 0 ? std::min(h->p.sle_ctas, nsm) : nsm;
+  h->sle_mode = scr * sizeof(double) > room ? 2 : G.M <= ctas && (scr + psz) * sizeof(double) <= room ? 1 : 0;
+  h->sle_shm = h->sle_mode == 2 ? 0 : (scr + (h->sle_mode == 1 ? psz : 0)) * sizeof(double);
+  int per_sm = 0;
+  const void* fn = kernel[h->sle_mode];
+  if (h->sle_shm) raise_smem_limit(fn, h->sle_shm);
+  VG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, SLE_THREADS, h->sle_shm));
+  if (per_sm < 1) throw Error("sle_solve: the fused inner loop does not fit on an SM");
+  const int grid = h->p.sle_ctas > 0 ? std::min(h->p.sle_ctas, nsm * per_sm) : nsm;
+  if (h->sle_mode == 2) h->d_sle_big.alloc(scr * (size_t)grid);
+  if (!h->d_gbar.p) h->d_gbar.alloc(4);
+  // from here on the last CTA of each launch resets the barrier
+  VG_CUDA(cudaMemsetAsync(h->d_gbar.p, 0, 4 * sizeof(unsigned int), h->stream));
+  h->sle_grid = grid;
 }
 
-static void launch_pass(vg_handle* h) {
+void pass_base(vg_handle* h, PassBase& A) {
   const Grid& G = h->grid;
-  cudaStream_t s = h->stream;
-  const size_t scr = sle_pass_scratch(G);
-  if (h->sle_grid == 0) {
-    int dev = 0, nsm = 0, per_sm = 0, lim = 0;
-    VG_CUDA(cudaGetDevice(&dev));
-    VG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    VG_CUDA(cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    cudaFuncAttributes fa;
-    VG_CUDA(cudaFuncGetAttributes(&fa, pass_kernel(0)));
-    const size_t room = (size_t)lim - fa.sharedSizeBytes, psz = (size_t)(p_pitch((G.nlat + 1) / 2) + 6) * (G.lmax + 1);
-    const int ctas = h->p.sle_ctas > 0 ? std::min(h->p.sle_ctas, nsm) : nsm;
-    h->sle_mode = scr * sizeof(double) > room ? 2 : G.M <= ctas && (scr + psz) * sizeof(double) <= room ? 1 : 0;
-    h->sle_shm = h->sle_mode == 2 ? 0 : (scr + (h->sle_mode == 1 ? psz : 0)) * sizeof(double);
-    const void* fn = pass_kernel(h->sle_mode);
-    if (h->sle_shm) raise_smem_limit(fn, h->sle_shm);
-    VG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, SLE_THREADS, h->sle_shm));
-    if (per_sm < 1) throw Error("sle_solve: the fused inner loop does not fit on an SM");
-    h->sle_grid = h->p.sle_ctas > 0 ? std::min(h->p.sle_ctas, nsm * per_sm) : nsm;
-    if (!h->d_gbar.p) h->d_gbar.alloc(4);
-    VG_CUDA(cudaMemsetAsync(h->d_gbar.p, 0, 4 * sizeof(unsigned int), s));  // later: by the last CTA of each launch
-    if (h->sle_mode == 2) h->d_sle_big.alloc(scr * (size_t)h->sle_grid);
-  }
-  PassArgs A;
   A.nphi = G.nphi;
   A.nlat = G.nlat;
   A.M = G.M;
-  A.nlm = G.nlm;
-  A.nk = h->nk;
   A.lmax = G.lmax;
+  A.dlon = 2.0 * PI / (double)G.nphi;
+  A.cs = G.d_cos.p;
+  A.sn = G.d_sin.p;
+  A.plm = G.d_plm.p;
+  A.wts = G.d_wts.p;
+  A.mbeg = G.d_mbeg.p;
+  A.F = h->d_F.p;
+  A.FC = h->d_F.p + (size_t)2 * G.M * G.nlat;
+  A.D = h->d_Gs.p;
+  A.cst = h->d_ulm.p;
+  A.rowpart = h->d_rowpart.p;
+  A.big = h->sle_mode == 2 ? h->d_sle_big.p : nullptr;
+  A.scr = sle_pass_scratch(G);
+  A.sc = h->d_sc_.p;
+  A.bar = h->d_gbar.p;
+  A.wait_ns = h->wait_ns;
+}
+
+void pass_launch(vg_handle* h, const void* const kernel[3], void* args) {
+  void* a[] = {args};
+  if (h->sle_shm) raise_smem_limit(kernel[h->sle_mode], h->sle_shm);
+  VG_CUDA(cudaLaunchCooperativeKernel(kernel[h->sle_mode], dim3(h->sle_grid), dim3(SLE_THREADS), a, h->sle_shm,
+                                      h->stream));
+  ++h->n_launch;
+}
+
+void check_pass_barrier(vg_handle* h) {
+  unsigned int b[4] = {0, 0, 0, 0};
+  if (h->d_gbar.p) VG_CUDA(cudaMemcpyAsync(b, h->d_gbar.p, sizeof(b), cudaMemcpyDeviceToHost, h->stream));
+  VG_CUDA(cudaStreamSynchronize(h->stream));
+  if (b[2] == 0) return;
+  h->sle_grid = 0;  // the barrier's counters are set up again before the next launch
+  throw Error("sle_solve: grid barrier of the fused inner loop timed out");
+}
+
+static void launch_pass(vg_handle* h) {
+  static const void* const kernel[3] = {(const void*)k_sle_pass<0>, (const void*)k_sle_pass<1>,
+                                        (const void*)k_sle_pass<2>};
+  pass_plan(h, kernel);
+  PassArgs A;
+  pass_base(h, A);
+  A.nk = h->nk;
   A.n_inner = h->p.sle_n_inner;
   A.subgrid = h->p.sle_subgrid;
   A.fixed = h->p.sle_fixed_ocean;
   A.tol = h->p.sle_tol;
-  A.dlon = 2.0 * PI / (double)G.nphi;
   A.g = h->g;
   A.ice = h->d_ice_now.p;
   A.topo0 = h->d_z_bed_eq.p;
   A.C0 = h->d_C0.p;
   A.dig = h->d_dig.p;
   A.C = h->d_C.p;
-  A.cs = G.d_cos.p;
-  A.sn = G.d_sin.p;
-  A.plm = G.d_plm.p;
-  A.wts = G.d_wts.p;
   A.gu = h->d_gu.p;
   A.gn = h->d_gn.p;
   A.drift = h->d_drift.p;
   A.srot = (h->rot_on || h->srot_ext) ? h->d_srot.p : nullptr;
   A.lm2k = h->d_lm2k.p;
-  A.mbeg = G.d_mbeg.p;
   A.wcorr = h->d_wcorr.p;
   A.rsl = h->d_rsl.p;
-  A.F = h->d_F.p;
-  A.FC = h->d_F.p + (size_t)2 * G.M * G.nlat;
   A.sigma = h->d_sigma.p;
-  A.cst = h->d_ulm.p;
-  A.D = h->d_Gs.p;
   A.Sraw = h->d_Sraw.p;
   A.Cn = h->d_C_next.p;
-  A.rowpart = h->d_rowpart.p;
-  A.sc = h->d_sc_.p;
-  A.big = h->sle_mode == 2 ? h->d_sle_big.p : nullptr;
-  A.scr = scr;
-  A.bar = h->d_gbar.p;
-  A.wait_ns = h->wait_ns;
-  void* args[] = {&A};
-  VG_CUDA(cudaLaunchCooperativeKernel(pass_kernel(h->sle_mode), dim3(h->sle_grid), dim3(SLE_THREADS), args,
-                                      h->sle_shm, s));
-  ++h->n_launch;
+  pass_launch(h, kernel, &A);
 }
 
 static void read_scalars(vg_handle* h) {

@@ -69,3 +69,41 @@ def test_result_does_not_depend_on_the_ctas():
     a, b = run(33, 40, 76, {}), run(33, 40, 76, {}, ctas=3)
     for x, y in zip(a.fields(), b.fields()):
         assert np.array_equal(x, y)
+
+
+def misfit(lmax, nlat, nphi, opts, ctas=0):
+    m = run(lmax, nlat, nphi, opts, ctas)
+    topo, ice = fields(nlat, nphi, True)
+    rng = np.random.default_rng(lmax)
+    sites = rng.choice(np.flatnonzero(topo > 100.0), 12).astype(np.int32)
+    ices = np.stack([0.8 * ice, 0.7 * ice])
+    return m, ices, sites, rng.standard_normal((2, 12))
+
+
+@pytest.mark.parametrize("lmax,nlat,nphi,opts", [
+    (7, 9, 15, {}),
+    (21, 24, 46, {"sle_n_inner": 1}),
+    (33, 40, 76, {"sle_fixed_ocean": 1}),
+    (4, 7000, 10, {}),
+])
+def test_pass_adjoint_matches_differences(lmax, nlat, nphi, opts):
+    """As test_gpu_adjoint_sle.py: quadratic in the ice, central differences to 1e-6 of the gradient's scale."""
+    m, ices, sites, obs = misfit(lmax, nlat, nphi, opts)
+    g = m.sle_misfit_grad(ices, 150.0, sites, obs)[1].reshape(2, -1)
+    rng = np.random.default_rng(5)
+    for _ in range(3):
+        d = rng.standard_normal(ices.shape) * ices
+        h = 1e-6
+        fd = (m.sle_misfit(ices + h * d, 150.0, sites, obs) - m.sle_misfit(ices - h * d, 150.0, sites, obs)) / (2 * h)
+        an = float(np.sum(g * d))
+        scale = max(abs(an), abs(fd), float(np.sqrt(np.sum((g * d) ** 2))))
+        assert abs(an - fd) <= 1e-6 * scale, (an, fd, scale)
+
+
+def test_pass_adjoint_does_not_depend_on_the_ctas():
+    out = []
+    for ctas in (0, 3):
+        m, ices, sites, obs = misfit(33, 40, 76, {}, ctas)
+        out.append(m.sle_misfit_grad(ices, 150.0, sites, obs))
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1])
