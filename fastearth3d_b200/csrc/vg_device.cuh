@@ -104,38 +104,6 @@ __device__ __forceinline__ void deg1_solve_cta(const double* __restrict__ ab, in
 // transforms (src/vilma_sht.f90:11-15): f_i = Re G_0 + 2 Re sum_{m>0} G_m e^{i m phi_i},
 // and F_m = (2 pi / nphi) sum_i f_i e^{-i m phi_i}.
 
-// row (smem, nphi) -> F[m] = (re, im) at F + 2*m*stride, m < M
-__device__ __forceinline__ void row_fourier_analysis(const double* row, int nphi, int M, const double* __restrict__ cs,
-                                                     const double* __restrict__ sn, double* F, size_t stride) {
-  const double sc = 2.0 * 3.14159265358979323846 / (double)nphi;
-  for (int m = threadIdx.x; m < M; m += blockDim.x) {
-    double re = 0.0, im = 0.0;
-    int t = 0;
-    for (int i = 0; i < nphi; ++i) {
-      double f = row[i];
-      re += f * __ldg(&cs[t]);
-      im -= f * __ldg(&sn[t]);
-      t += m;
-      if (t >= nphi) t -= nphi;
-    }
-    F[2 * (size_t)m * stride] = re * sc;
-    F[2 * (size_t)m * stride + 1] = im * sc;
-  }
-}
-
-// G (smem, M complex interleaved) -> f_i for i < nphi (called per thread for its i)
-__device__ __forceinline__ double row_fourier_synth_at(const double* G, int M, int i, int nphi,
-                                                       const double* __restrict__ cs, const double* __restrict__ sn) {
-  double acc = 0.0;
-  int t = i;
-  for (int m = 1; m < M; ++m) {
-    acc += G[2 * m] * __ldg(&cs[t]) - G[2 * m + 1] * __ldg(&sn[t]);
-    t += i;
-    if (t >= nphi) t -= nphi;
-  }
-  return G[0] + 2.0 * acc;
-}
-
 // CTA reductions (fixed order: deterministic for a fixed block size)
 __device__ __forceinline__ double block_sum(double v, double* red) {
   red[threadIdx.x] = v;

@@ -72,24 +72,24 @@ __global__ void k_pass_setup(int nphi, int nlat, int set_c0, int io1, int fixed,
 
 // the closing load of a solve whose last pass had no ocean: total surface load
 // (assemble_load, src/vilma_sle.f90:387-403), its longitude transform, row sums of C rsl
-__global__ void k_load_fourier(int nphi, int nlat, int M, const double* __restrict__ dig,
-                               const double* __restrict__ C, const double* __restrict__ rsl,
-                               const double* __restrict__ wcorr, const double* __restrict__ cs,
-                               const double* __restrict__ sn, double* __restrict__ F,
-                               double* __restrict__ rowpart) {
-  extern __shared__ double row[];
-  __shared__ double red[128];
+__global__ void __launch_bounds__(SLE_THREADS, 2)
+    k_load_fourier(int nphi, int nlat, int M, const double* __restrict__ dig, const double* __restrict__ C,
+                   const double* __restrict__ rsl, const double* __restrict__ wcorr, const double* __restrict__ cs,
+                   const double* __restrict__ sn, double* __restrict__ F, double* __restrict__ rowpart) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ __align__(16) double part[4 * SLE_THREADS];
+  __shared__ double red[32];
+  const Rows<SLE_THREADS> R(nphi, M, cs, sn, sm, part);
   int j = blockIdx.x;
   double s = 0.0;
   for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
     size_t p = (size_t)j * nphi + i;
-    row[i] = RHO_ICE * dig[p] + RHO_WATER * (C[p] * rsl[p]) + (wcorr ? wcorr[p] : 0.0);
+    R.L[i] = RHO_ICE * dig[p] + RHO_WATER * (C[p] * rsl[p]) + (wcorr ? wcorr[p] : 0.0);
     s += C[p] * rsl[p];
   }
   s = block_sum_w(s, red);
   if (threadIdx.x == 0) rowpart[RP_MASS * nlat + j] = s;
-  __syncthreads();
-  row_fourier_analysis(row, nphi, M, cs, sn, F + (size_t)j * 2, nlat);
+  R.row_analysis(reinterpret_cast<double2*>(F) + j, nlat);
 }
 
 // End of an interval, a block per row: with ice1 the ice becomes the interval's
@@ -438,9 +438,8 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
 
 // doubles of a CTA's work area: the twiddles, then the larger of the two phases
 static size_t sle_pass_scratch(const Grid& G) {
-  const size_t nbase = G.nphi % 2 ? (G.nphi + 1) / 2 : G.nphi / 4 + 1, nh = (G.nlat + 1) / 2;
-  const size_t rows = 2 * (size_t)G.M + 4 * nbase + G.nphi, orders = 2 * (4 * nh + G.lmax + 1);
-  return 2 * (size_t)(G.nphi + (G.nphi >> 3) + 1) + (std::max(rows, orders) + 1) / 2 * 2;
+  const size_t tw = 2 * (size_t)(G.nphi + (G.nphi >> 3) + 1), orders = 2 * (4 * (size_t)((G.nlat + 1) / 2) + G.lmax + 1);
+  return (std::max(rows_scratch(G.nphi, G.M), tw + orders) + 1) / 2 * 2;
 }
 
 // int C rsl - zeta of that load
@@ -612,9 +611,11 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
   // the closing load's spectrum (from the pass, unless that had no ocean) and the
   // memory advance (src/vilma_sle.f90:353-358)
   if (!closed) {
-    k_load_fourier<<<nlat, 128, nphi * sizeof(double), s>>>(nphi, nlat, M, h->d_dig.p, h->d_C.p, h->d_rsl.p,
-                                                            ocean_seen ? h->d_wcorr.p : nullptr, G.d_cos.p,
-                                                            G.d_sin.p, h->d_F.p, rp);
+    const size_t shm = rows_scratch(nphi, M) * sizeof(double);
+    raise_smem_limit((const void*)k_load_fourier, shm);
+    k_load_fourier<<<nlat, SLE_THREADS, shm, s>>>(nphi, nlat, M, h->d_dig.p, h->d_C.p, h->d_rsl.p,
+                                                  ocean_seen ? h->d_wcorr.p : nullptr, G.d_cos.p, G.d_sin.p, h->d_F.p,
+                                                  rp);
     ++h->n_launch;
     if (p.sle_n_outer < 1) {
       k_mass<<<1, 32, 0, s>>>(sc, rp, G.d_wts.p, nlat, dlon);

@@ -2,6 +2,7 @@
 // Device code shared by the fused sea-level pass (vg_sle.cu) and its adjoint
 // (vg_adjoint.cu): cooperative kernels whose CTAs own orders in one phase and
 // grid rows in the next, with a grid barrier between the two.
+#include <algorithm>
 #include <type_traits>
 
 #include "vg_device.cuh"
@@ -122,10 +123,11 @@ struct Lon {
 // This thread's share of a longitude sum over `n` outputs with Q parts each:
 // part q of output o, the twiddle index t0 of its first term and the step between
 // its terms (a term advances the index by o, `mul` terms of other parts between)
+template <int T>
 struct Share {
   int Q, q, o, t0, step;
   __device__ __forceinline__ Share(int n, int mul, int nphi, int u) {
-    Q = max(1, min(16, SLE_THREADS / n));
+    Q = max(1, min(16, T / n));
     q = u / n;
     o = u - q * n;
     t0 = (int)(((unsigned)(mul * q) * (unsigned)o) % (unsigned)nphi);
@@ -133,51 +135,33 @@ struct Share {
   }
 };
 
-// MODE of a pass. A CTA with one order keeps that order's Legendre functions (northern rows) in
-// shared memory (MODE 1), where they fit: the barriers invalidate L1, so read
-// through it (MODE 0) they come from L2 in each iteration (106 us a pass at lmax
-// 128 and 77 at lmax 85, against 100 and 76). MODE 2, a grid whose
-// work area does not fit in shared memory: the work area is A.scr doubles a CTA of
-// global memory.
-//
-// The work area: twiddles, then the rows' phase (a row's spectrum Gd, per base
-// longitude four values X, a row of the grid L) or, in the same space, the
-// orders' (northern rows Fe [4][nh], degrees dl); in mode 1 the order's Legendre
-// functions Ps and six numbers a degree Ks follow.
-template <int MODE>
-struct Pass {
+// Longitude transforms of one row by the T threads of a CTA, in both directions
+// split by the reflection and the half period: four sums over a quarter of the
+// longitudes. Shared memory: twiddles tw, the row's spectrum Gd or the row L (the
+// one is read before the other is written), per base longitude four values X;
+// part: 4 T doubles.
+template <int T>
+struct Rows {
   Lon G;
-  int nlat, M, nh, pp;
-  double2 *tw, *Gd, *Fe, *dl;
-  double *X, *L, *Ps, *Ks, *part;
-  Share ss, sa;
-  __device__ __forceinline__ Pass(const PassBase& A, double* sm, double* part_)
-      : G(A.nphi), nlat(A.nlat), M(A.M), nh((A.nlat + 1) / 2), pp(p_pitch((A.nlat + 1) / 2)), part(part_),
-        ss(G.nbase, 2, A.nphi, threadIdx.x), sa(A.M, 1, A.nphi, threadIdx.x) {
+  int M;
+  double2 *tw, *Gd;
+  double *X, *L, *part;
+  Share<T> ss, sa;
+  __device__ __forceinline__ Rows(int nphi, int M_, const double* cs, const double* sn, double* sm, double* part_)
+      : G(nphi), M(M_), part(part_), ss(G.nbase, 2, nphi, threadIdx.x), sa(M_, 1, nphi, threadIdx.x) {
     tw = reinterpret_cast<double2*>(sm);
-    Gd = tw + tw_at(A.nphi) + 1;
-    X = reinterpret_cast<double*>(Gd + M);
-    L = X + 4 * G.nbase;
-    Fe = Gd;
-    dl = Fe + 4 * nh;
-    Ps = sm + A.scr;
-    Ks = Ps + (size_t)(A.lmax + 1) * pp;
-    if (MODE == 1 && blockIdx.x < M) {
-      const int m = blockIdx.x;
-      for (int u = threadIdx.x; u < (A.lmax - m + 1) * nh; u += SLE_THREADS) {
-        const int x = u / nh, j = u - x * nh;
-        Ps[(size_t)x * pp + j] = A.plm[(size_t)(A.mbeg[m] + x) * nlat + j];
-      }
-    }
-    for (int t = threadIdx.x; t < A.nphi; t += SLE_THREADS) tw[tw_at(t)] = make_double2(A.cs[t], A.sn[t]);
+    Gd = tw + tw_at(nphi) + 1;
+    L = reinterpret_cast<double*>(Gd);
+    X = L + (max(2 * M, nphi) + 1) / 2 * 2;
+    for (int t = threadIdx.x; t < nphi; t += T) tw[tw_at(t)] = make_double2(cs[t], sn[t]);
   }
 
   // F(m) = 2 pi / nphi sum_i L_i e^{-i m phi_i} of the row in L, to out[m stride]
   __device__ __forceinline__ void row_analysis(double2* out, int stride) const {
     const int tid = threadIdx.x;
-    for (int i = tid; i < G.nbase; i += SLE_THREADS) {
+    for (int i = tid; i < G.nbase; i += T) {
       double v[4];
-  #pragma unroll
+#pragma unroll
       for (int pt = 0; pt < 4; ++pt) v[pt] = G.has(i, pt) ? L[G.at(i, pt)] : 0.0;
       double4 x;
       if (G.even) {
@@ -192,14 +176,14 @@ struct Pass {
     __syncthreads();
     const int Q = sa.Q;
     const double sc = 2.0 * PI / (double)G.nphi;
-    for (int base = 0; base < M * Q; base += SLE_THREADS) {
-      const Share sh = base ? Share(M, 1, G.nphi, base + tid) : sa;
+    for (int base = 0; base < M * Q; base += T) {
+      const Share<T> sh = base ? Share<T>(M, 1, G.nphi, base + tid) : sa;
       const int m = sh.o;
       double re = 0.0, im = 0.0;
       if (base + tid < M * Q) {
         const double2* x = reinterpret_cast<const double2*>(X) + (m & 1);
         int t = sh.t0;
-  #pragma unroll 4
+#pragma unroll 4
         for (int i = sh.q; i < G.nbase; i += Q) {
           const double2 w = tw[tw_at(t)], v = x[2 * i];
           re = fma(v.x, w.x, re);
@@ -226,17 +210,114 @@ struct Pass {
     __syncthreads();
   }
 
+  // the four sums of each base longitude of the row whose spectrum is in Gd, into X
+  __device__ __forceinline__ void row_synthesis() const {
+    const int tid = threadIdx.x, nphi = G.nphi;
+    const int Q = ss.Q;
+    for (int base = 0; base < G.nbase * Q; base += T) {
+      const Share<T> sh = base ? Share<T>(G.nbase, 2, nphi, base + tid) : ss;
+      const int i = sh.o;
+      double ce = 0.0, se = 0.0, co = 0.0, so = 0.0;
+      if (base + tid < G.nbase * Q) {
+        int t = sh.t0;
+#pragma unroll 2
+        for (int m = 2 * sh.q; m < M; m += 2 * Q) {
+          const double2 w = tw[tw_at(t)], v = Gd[m];
+          ce = fma(v.x, w.x, ce);
+          se = fma(v.y, w.y, se);
+          if (m + 1 < M) {
+            int t1 = t + i;
+            if (t1 >= nphi) t1 -= nphi;
+            const double2 w1 = tw[tw_at(t1)], v1 = Gd[m + 1];
+            co = fma(v1.x, w1.x, co);
+            so = fma(v1.y, w1.y, so);
+          }
+          t += sh.step;
+          if (t >= nphi) t -= nphi;
+        }
+      }
+      if (Q == 1) {
+        if (base + tid < G.nbase) {
+          reinterpret_cast<double2*>(X)[2 * i] = make_double2(ce, se);
+          reinterpret_cast<double2*>(X)[2 * i + 1] = make_double2(co, so);
+        }
+      } else {
+        part[tid] = ce;
+        part[T + tid] = se;
+        part[2 * T + tid] = co;
+        part[3 * T + tid] = so;
+      }
+    }
+    __syncthreads();
+    if (Q > 1) {
+      for (int u = tid; u < 4 * G.nbase; u += T) {
+        const int s4 = u / G.nbase, i = u - s4 * G.nbase;
+        double v = 0.0;
+#pragma unroll 4
+        for (int c = 0; c < Q; ++c) v += part[s4 * T + c * G.nbase + i];
+        X[4 * i + s4] = v;
+      }
+      __syncthreads();
+    }
+  }
+  // and the field at a base longitude's point from them
+  __device__ __forceinline__ double value(int i, int pt) const {
+    const double2 e = reinterpret_cast<const double2*>(X)[2 * i], o = reinterpret_cast<const double2*>(X)[2 * i + 1];
+    const double ev = pt < 2 ? e.x - e.y : e.x + e.y, ov = pt < 2 ? o.x - o.y : o.x + o.y;
+    return (pt & 1) ? ev - ov : ev + ov;
+  }
+};
+// doubles of its shared memory
+inline size_t rows_scratch(int nphi, int M) {
+  const size_t nbase = nphi % 2 ? (nphi + 1) / 2 : nphi / 4 + 1;
+  return 2 * (size_t)(nphi + (nphi >> 3) + 1) + ((size_t)std::max(2 * M, nphi) + 1) / 2 * 2 + 4 * nbase;
+}
+constexpr size_t SMEM_CTA = 227 * 1024;  // shared memory that a CTA can have
+
+// A CTA's part of a pass. MODE 1: a CTA with one order keeps that order's Legendre
+// functions (northern rows) in shared memory, where they fit: the barriers
+// invalidate L1, so read through it (MODE 0) they come from L2 in each iteration
+// (106 us a pass at lmax 128 and 77 at lmax 85, against 100 and 76). MODE 2, a grid
+// whose work area does not fit in shared memory: the work area is A.scr doubles a
+// CTA of global memory.
+//
+// The work area: that of Rows; after its twiddles, in the same space, the orders'
+// phase (northern rows Fe [4][nh], degrees dl); in mode 1 the order's Legendre
+// functions Ps and six numbers a degree Ks follow.
+template <int MODE>
+struct Pass : Rows<SLE_THREADS> {
+  int nlat, nh, pp;
+  double2 *Fe, *dl;
+  double *Ps, *Ks;
+  __device__ __forceinline__ Pass(const PassBase& A, double* sm, double* part_)
+      : Rows<SLE_THREADS>(A.nphi, A.M, A.cs, A.sn, sm, part_),
+        nlat(A.nlat),
+        nh((A.nlat + 1) / 2),
+        pp(p_pitch((A.nlat + 1) / 2)) {
+    Fe = Gd;
+    dl = Fe + 4 * nh;
+    Ps = sm + A.scr;
+    Ks = Ps + (size_t)(A.lmax + 1) * pp;
+    if (MODE == 1 && blockIdx.x < M) {
+      const int m = blockIdx.x;
+      for (int u = threadIdx.x; u < (A.lmax - m + 1) * nh; u += SLE_THREADS) {
+        const int x = u / nh, j = u - x * nh;
+        Ps[(size_t)x * pp + j] = A.plm[(size_t)(A.mbeg[m] + x) * nlat + j];
+      }
+    }
+  }
+
   // northern rows of order m, folded at the equator and times the quadrature
   // weights (1 with `unit`); with `both` the ocean's after the load's
   __device__ __forceinline__ void order_fold(const PassBase& A, int m, bool both, bool unit) const {
-  for (int u = threadIdx.x; u < (both ? 2 * nh : nh); u += SLE_THREADS) {
-    const int f = u >= nh, j = u - f * nh, jm = nlat - 1 - j;  // f: of rho_w C
-    const double2* src = reinterpret_cast<const double2*>(f ? A.FC : A.F) + (size_t)m * nlat;
-    const double2 a = __ldcg(src + j), b = jm != j ? __ldcg(src + jm) : make_double2(0.0, 0.0);
-    const double w = f || !unit ? A.wts[j] : 1.0;
-    Fe[(2 * f) * nh + j] = make_double2(w * (a.x + b.x), w * (a.y + b.y));
-    Fe[(2 * f + 1) * nh + j] = make_double2(w * (a.x - b.x), w * (a.y - b.y));
-  }
+    for (int u = threadIdx.x; u < (both ? 2 * nh : nh); u += SLE_THREADS) {
+      const int f = u >= nh, j = u - f * nh, jm = nlat - 1 - j;  // f: of rho_w C
+      const double2* src = reinterpret_cast<const double2*>(f ? A.FC : A.F) + (size_t)m * nlat;
+      const double2 a = __ldcg(src + j), b = jm != j ? __ldcg(src + jm) : make_double2(0.0, 0.0);
+      const double w = f || !unit ? A.wts[j] : 1.0;
+      Fe[(2 * f) * nh + j] = make_double2(w * (a.x + b.x), w * (a.y + b.y));
+      Fe[(2 * f + 1) * nh + j] = make_double2(w * (a.x - b.x), w * (a.y - b.y));
+    }
   }
 
   // Legendre analysis of order m, eight lanes a degree, up to three degrees a
@@ -352,63 +433,6 @@ struct Pass {
         if (jm != j) __stcg(D + (size_t)jm * M + m, make_double2(w * (er - orr), w * (ei - oi)));
       }
     }
-  }
-
-  // the four sums of each base longitude of the row whose spectrum is in Gd, into X
-  __device__ __forceinline__ void row_synthesis() const {
-    const int tid = threadIdx.x, nphi = G.nphi;
-    const int Q = ss.Q;
-    for (int base = 0; base < G.nbase * Q; base += SLE_THREADS) {
-      const Share sh = base ? Share(G.nbase, 2, nphi, base + tid) : ss;
-      const int i = sh.o;
-      double ce = 0.0, se = 0.0, co = 0.0, so = 0.0;
-      if (base + tid < G.nbase * Q) {
-        int t = sh.t0;
-#pragma unroll 2
-        for (int m = 2 * sh.q; m < M; m += 2 * Q) {
-          const double2 w = tw[tw_at(t)], v = Gd[m];
-          ce = fma(v.x, w.x, ce);
-          se = fma(v.y, w.y, se);
-          if (m + 1 < M) {
-            int t1 = t + i;
-            if (t1 >= nphi) t1 -= nphi;
-            const double2 w1 = tw[tw_at(t1)], v1 = Gd[m + 1];
-            co = fma(v1.x, w1.x, co);
-            so = fma(v1.y, w1.y, so);
-          }
-          t += sh.step;
-          if (t >= nphi) t -= nphi;
-        }
-      }
-      if (Q == 1) {
-        if (base + tid < G.nbase) {
-          reinterpret_cast<double2*>(X)[2 * i] = make_double2(ce, se);
-          reinterpret_cast<double2*>(X)[2 * i + 1] = make_double2(co, so);
-        }
-      } else {
-        part[tid] = ce;
-        part[SLE_THREADS + tid] = se;
-        part[2 * SLE_THREADS + tid] = co;
-        part[3 * SLE_THREADS + tid] = so;
-      }
-    }
-    __syncthreads();
-    if (Q > 1) {
-      for (int u = tid; u < 4 * G.nbase; u += SLE_THREADS) {
-        const int s4 = u / G.nbase, i = u - s4 * G.nbase;
-        double v = 0.0;
-#pragma unroll 4
-        for (int c = 0; c < Q; ++c) v += part[s4 * SLE_THREADS + c * G.nbase + i];
-        X[4 * i + s4] = v;
-      }
-      __syncthreads();
-    }
-  }
-  // and the field at a base longitude's point from them
-  __device__ __forceinline__ double value(int i, int pt) const {
-    const double2 e = reinterpret_cast<const double2*>(X)[2 * i], o = reinterpret_cast<const double2*>(X)[2 * i + 1];
-    const double ev = pt < 2 ? e.x - e.y : e.x + e.y, ov = pt < 2 ? o.x - o.y : o.x + o.y;
-    return (pt & 1) ? ev - ov : ev + ov;
   }
 };
 
