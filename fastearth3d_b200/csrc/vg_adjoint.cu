@@ -35,6 +35,7 @@
 #include "vg_device.cuh"
 #include "vg_internal.cuh"
 #include "vg_sle_pass.cuh"
+#include "vg_sweep.cuh"
 
 namespace vg {
 
@@ -205,294 +206,104 @@ __device__ __forceinline__ void rhs_T(const double* __restrict__ Kp, const doubl
     }
 }
 
-// ---- shared-memory staging of the transposed sweeps (cp.async, double-buffered) ----
-constexpr int TS_CH = 32;                     // band columns (sweep steps) per chunk
-constexpr int TS_BAND = 2 * TS_CH * VG_LDAB;  // two band chunks
-constexpr int TS_AUX = 2 * TS_CH * 32;        // two chunks of per-lane entering values
-constexpr int TS_WARP = TS_BAND + TS_AUX;     // doubles of shared memory per warp
-constexpr int TS_WARPS = 4;                   // warps (tasks) per block
-
-__device__ __forceinline__ void ts_cp8(double* s, const double* g) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(s);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(g) : "memory");
-}
-__device__ __forceinline__ void ts_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void ts_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
-// band records of columns [c0, c0 + TS_CH) of one degree; zero outside [0, nd)
-__device__ __forceinline__ void ts_stage_band(double* dst, const double* ab, int c0, int nd, int lane) {
-  for (int t = lane; t < TS_CH * VG_LDAB; t += 32) {
-    const int col = c0 + t / VG_LDAB;
-    if (col >= 0 && col < nd)
-      ts_cp8(dst + t, ab + (size_t)col * VG_LDAB + (t % VG_LDAB));
-    else
-      dst[t] = 0.0;
+// drift^T for degree 1 (slots 0, 1; four right-hand sides): the CM projection
+// transposed, then the transposed Green's block, D1T columns a warp
+constexpr int D1T = 4;
+__device__ __forceinline__ void drift_T_deg1(int task, int nr, int nk, int deg1_cm, const double* __restrict__ null1,
+                                             const double* __restrict__ G1T, const double* __restrict__ dUn_bar,
+                                             const double* __restrict__ dVn_bar, const double* __restrict__ surf_bar,
+                                             double* __restrict__ w, int lane) {
+  const int ncol = 2 * nr, nrow = 2 * nr + 1, fs = 4 * (nr - 1) + 2;
+  const double fa_n = null1[fs];
+  const bool proj = deg1_cm && fa_n != 0.0;
+  double cb[4] = {0.0, 0.0, 0.0, 0.0}, a[D1T][4] = {};
+  for (int r = lane; r < nrow; r += 32) {
+    const int node = r >> 1, dof = r < 2 * nr ? 4 * node + (r & 1) : fs;
+    const double nl = null1[dof];
+    double g[D1T];
+#pragma unroll
+    for (int i = 0; i < D1T; ++i) g[i] = __ldg(G1T + (size_t)min(task * D1T + i, ncol - 1) * nrow + r);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // (slot, re/im)
+      const int kk = q >> 1, ri = q & 1;
+      double v = 0.0;
+      if (r < 2 * nr) {
+        v = ((r & 1) ? dVn_bar : dUn_bar)[((size_t)ri * nr + node) * nk + kk];
+        if (node == nr - 1 && !(r & 1)) v += surf_bar[(size_t)ri * nk + kk];
+      } else if (deg1_cm) {
+        v = surf_bar[(size_t)(2 + ri) * nk + kk];
+      }
+      cb[q] = fma(v, nl, cb[q]);
+#pragma unroll
+      for (int i = 0; i < D1T; ++i) a[i][q] = fma(g[i], v, a[i][q]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    for (int o = 16; o > 0; o >>= 1) {
+      cb[q] += __shfl_xor_sync(0xffffffffu, cb[q], o);
+#pragma unroll
+      for (int i = 0; i < D1T; ++i) a[i][q] += __shfl_xor_sync(0xffffffffu, a[i][q], o);
+    }
+  if (lane != 0) return;
+#pragma unroll
+  for (int i = 0; i < D1T; ++i) {
+    const int c = task * D1T + i;
+    if (c >= ncol) break;
+    // forward: x += c null, c = -x[F] / fa_n  =>  c_bar = <x_bar, null>, x_bar[F] -= c_bar / fa_n
+    const double gF = G1T[(size_t)c * nrow + 2 * nr];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      w[((size_t)(q & 1) * ncol + c) * nk + (q >> 1)] = proj ? a[i][q] - gF * (cb[q] / fa_n) : a[i][q];
   }
 }
 
-// Transposed drift solves (degrees >= 2), one warp per task: up to 16 slots of
-// one degree x (re, im), the forward sweeps' task list. With A = P L U the
-// dgbtf2 factor (kl = 6, kv = 12) and the drift's right-hand side scaled by
-// the column equilibration dc:
-//   U^T sweep (ascending): x_j = (z_j - sum_{i<=12} U(j-i, j) x_{j-i}) / U(j, j),
-//     z_j = dc_j (U-bar, V-bar, F-bar at the dofs of node j/4; surface terms at
-//     the last node), the 12 previous values in registers;
-//   L^T sweep (descending, pivots undone): x_j -= sum_{i<=6} L(j+i, j) x_{j+i},
-//     then swap x_j and x_{j + jp_j}; a value leaves the 7-value window once
-//     no later swap can reach it.
-// The degree's band columns stream through shared memory in chunks of 32 so
-// that every load on the recurrences is a shared-memory load; the per-lane
-// entering values (U-bar / V-bar in the U^T sweep, its output in the L^T
-// sweep) are staged the same way one chunk ahead.
-__global__ void __launch_bounds__(32 * TS_WARPS) k_drift_T(int nr, int nd, int nk, const int4* __restrict__ tasks,
-                                                           int ntask, const double* __restrict__ ab_all,
-                                                           const double* __restrict__ dcv,
-                                                           const double* __restrict__ dUn_bar,
-                                                           const double* __restrict__ dVn_bar,
-                                                           const double* __restrict__ surf_bar,
-                                                           double* __restrict__ w) {
-  constexpr int KL = 6, KV = 12;
-  extern __shared__ double smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tix = blockIdx.x * TS_WARPS + warp;
-  if (tix >= ntask) return;  // whole warp
+// Transposed drift solves, a warp per task: up to 16 slots of one degree x (re,
+// im), the forward sweeps' task list and records; after them the degree-1 columns.
+// w[(2 node + uv) nk + k]: the adjoint of the equilibrated forcing. Bound like the
+// forward sweeps by the recurrence over the nodes: a column at a time, with the
+// interchanges undone step by step, it took 169 us at lmax 64 with 50 elements,
+// beside 34 us of one block for degree 1; 21 for both now.
+__global__ void __launch_bounds__(32) k_drift_T(int nr, int nk, int deg1_cm, const int4* __restrict__ tasks, int ntask,
+                                                const double* __restrict__ lrec, const double* __restrict__ urec,
+                                                const double* __restrict__ null1, const double* __restrict__ G1T,
+                                                const double* __restrict__ dUn_bar, const double* __restrict__ dVn_bar,
+                                                const double* __restrict__ surf_bar, double* __restrict__ ys,
+                                                double* __restrict__ w) {
+  extern __shared__ __align__(16) double smem[];
+  const int lane = threadIdx.x, tix = blockIdx.x;
+  if (tix >= ntask)
+    return drift_T_deg1(tix - ntask, nr, nk, deg1_cm, null1, G1T, dUn_bar, dVn_bar, surf_bar, w, lane);
   const int4 T = tasks[tix];
   const int l = T.x, k0 = T.y, nsl = T.z;
   const int sl = lane & 15, ri = lane >> 4;
   const bool valid = sl < nsl;
   const int k = k0 + (valid ? sl : 0);
-  double* sband = smem + (size_t)warp * TS_WARP;
-  double* saux = sband + TS_BAND;
-  const double* ab = ab_all + (size_t)(l - 2) * VG_LDAB * nd;
-  const double* dc = dcv + (size_t)(l - 2) * nd;
-  const double* ub = dUn_bar + (size_t)ri * nr * nk + k;
-  const double* vb = dVn_bar + (size_t)ri * nr * nk + k;
-  double* x = w + (size_t)ri * nd * nk + k;
-  const double sU = surf_bar[(size_t)(0 + ri) * nk + k], sF = surf_bar[(size_t)(2 + ri) * nk + k];
-  // ---- U^T sweep ----
-  // entering U-bar, V-bar of chunk c (columns 32c .. 32c+31 = nodes 8c .. 8c+7) at slot (2 node' + uv)
-  auto stage_z = [&](double* dst, int c) {
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const int node = 8 * c + (q >> 1);
-      if (node < nr)
-        ts_cp8(dst + q * 32 + lane, ((q & 1) ? vb : ub) + (size_t)node * nk);
-      else
-        dst[q * 32 + lane] = 0.0;
-    }
-  };
-  const int nch = (nd + TS_CH - 1) / TS_CH;
-  ts_stage_band(sband, ab, 0, nd, lane);
-  stage_z(saux, 0);
-  ts_commit();
-  double wv[KV];  // wv[i] = x_{j-1-i}
-#pragma unroll
-  for (int i = 0; i < KV; ++i) wv[i] = 0.0;
-  for (int c = 0; c < nch; ++c) {
-    const int cur = c & 1;
-    if (c + 1 < nch) {
-      ts_stage_band(sband + (cur ^ 1) * TS_CH * VG_LDAB, ab, TS_CH * (c + 1), nd, lane);
-      stage_z(saux + (cur ^ 1) * TS_CH * 32, c + 1);
-      ts_commit();
-      ts_wait<1>();
-    } else {
-      ts_wait<0>();
-    }
-    __syncwarp();
-    const double* bandc = sband + cur * TS_CH * VG_LDAB;
-    const double* zin = saux + cur * TS_CH * 32;
-#pragma unroll 4
-    for (int jj = 0; jj < TS_CH; ++jj) {
-      const int j = TS_CH * c + jj;
-      if (j >= nd) break;
-      const int node = j >> 2, typ = j & 3;
-      double raw = (typ == 0) ? zin[(2 * (jj >> 2)) * 32 + lane] : (typ == 1) ? zin[(2 * (jj >> 2) + 1) * 32 + lane] : 0.0;
-      if (node == nr - 1) {
-        if (typ == 0) raw += sU;
-        if (typ == 2) raw = sF;
-      }
-      const double* col = bandc + jj * VG_LDAB;
-      double t = __ldg(&dc[j]) * raw;
-#pragma unroll
-      for (int i = 1; i <= KV; ++i)
-        if (i <= j) t -= col[KV - i] * wv[i - 1];
-      t = t / col[KV];
-      if (valid) x[(size_t)j * nk] = t;
-#pragma unroll
-      for (int i = KV - 1; i > 0; --i) wv[i] = wv[i - 1];
-      wv[0] = t;
-    }
-    __syncwarp();  // the buffer just read is refilled by the next prefetch
-  }
-  __threadfence_block();  // x stores before this lane's own cp.async reads of them
-  // ---- L^T sweep: steps j = nd-2 .. 0; chunk c covers j = jhi-31 .. jhi, jhi = nd-2-32c ----
-  auto stage_x = [&](double* dst, int c) {
-    const int jlo = nd - 2 - TS_CH * c - (TS_CH - 1);
-#pragma unroll 4
-    for (int q = 0; q < TS_CH; ++q) {
-      const int j = jlo + q;
-      if (j >= 0 && valid)
-        ts_cp8(dst + q * 32 + lane, x + (size_t)j * nk);
-      else
-        dst[q * 32 + lane] = 0.0;
-    }
-  };
-  double v[KL + 1];  // v[i] = x_{j+i}, starting at j = nd - 1 (nothing beyond it)
-  v[0] = valid ? x[(size_t)(nd - 1) * nk] : 0.0;
-#pragma unroll
-  for (int i = 1; i <= KL; ++i) v[i] = 0.0;
-  const int nchl = (nd - 1 + TS_CH - 1) / TS_CH;
-  if (nchl > 0) {
-    ts_stage_band(sband, ab, nd - 2 - (TS_CH - 1), nd, lane);
-    stage_x(saux, 0);
-    ts_commit();
-  }
-  for (int c = 0; c < nchl; ++c) {
-    const int cur = c & 1, jlo = nd - 2 - TS_CH * c - (TS_CH - 1);
-    if (c + 1 < nchl) {
-      ts_stage_band(sband + (cur ^ 1) * TS_CH * VG_LDAB, ab, jlo - TS_CH, nd, lane);
-      stage_x(saux + (cur ^ 1) * TS_CH * 32, c + 1);
-      ts_commit();
-      ts_wait<1>();
-    } else {
-      ts_wait<0>();
-    }
-    __syncwarp();
-    const double* bandc = sband + cur * TS_CH * VG_LDAB;
-    const double* xin = saux + cur * TS_CH * 32;
-#pragma unroll 4
-    for (int jj = TS_CH - 1; jj >= 0; --jj) {
-      const int j = jlo + jj;
-      if (j < 0) break;
-      const double out = v[KL];  // x_{j+1+KL} is final
-      if (valid && j + 1 + KL <= nd - 1) x[(size_t)(j + 1 + KL) * nk] = out;
-#pragma unroll
-      for (int i = KL; i > 0; --i) v[i] = v[i - 1];
-      const double* col = bandc + jj * VG_LDAB;
-      double t = xin[jj * 32 + lane];
-#pragma unroll
-      for (int i = 1; i <= KL; ++i)
-        if (j + i <= nd - 1) t -= col[KV + i] * v[i];
-      v[0] = t;
-      const int d = (int)col[20];  // jp_j = ipiv_j - j, 0 .. KL
-      if (d != 0) {
-        double vd = v[0];
-#pragma unroll
-        for (int i = 1; i <= KL; ++i)
-          if (i == d) {
-            vd = v[i];
-            v[i] = v[0];
-          }
-        v[0] = vd;
-      }
-    }
-    __syncwarp();
-  }
-  if (valid) {
-#pragma unroll
-    for (int i = 0; i <= KL; ++i)
-      if (i <= nd - 1) x[(size_t)i * nk] = v[i];
-  }
+  double* x = w + (size_t)ri * 2 * nr * nk + k;
+  sw::band_sweeps_T(lrec + (l - 2) * sw::lrec_size(nr), urec + (l - 2) * sw::urec_size(nr), nr,
+                    dUn_bar + (size_t)ri * nr * nk + k, dVn_bar + (size_t)ri * nr * nk + k, nk,
+                    surf_bar[(size_t)ri * nk + k], surf_bar[(size_t)(2 + ri) * nk + k],
+                    ys + (size_t)tix * sw::scratch(nr), smem, lane, [&](int node, double U, double V) {
+                      if (!valid) return;
+                      x[(size_t)(2 * node) * nk] = U;
+                      x[(size_t)(2 * node + 1) * nk] = V;
+                    });
 }
 
-// K^T after the transposed solves (degrees >= 2): a thread per (slot,
-// element, re/im), f_bar = dr x at the element's four test dofs
-__global__ void __launch_bounds__(256) k_rhs_T(int ne, int nd, int nk, const int* __restrict__ kdeg,
-                                               const double* __restrict__ drv, const double* __restrict__ K,
-                                               const double* __restrict__ w, double* __restrict__ lam_new) {
+// K^T after the transposed solves: a thread per (slot, element, re/im), f_bar =
+// dr x at the element's four test dofs
+__global__ void __launch_bounds__(256) k_rhs_T(int ne, int nr, int nd, int nk, const int* __restrict__ kdeg,
+                                               const double* __restrict__ drv, const double* __restrict__ dr1,
+                                               const double* __restrict__ K, const double* __restrict__ w,
+                                               double* __restrict__ lam_new) {
   const int k = blockIdx.x * 32 + threadIdx.x, e = blockIdx.y * 8 + threadIdx.y, ri = blockIdx.z;
   if (k >= nk || e >= ne) return;
   const int l = kdeg[k];
-  if (l < 2) return;
-  const double* dr = drv + (size_t)(l - 2) * nd;
-  const double* x = w + (size_t)ri * nd * nk + k;
-  const double fb[4] = {dr[4 * e] * x[(size_t)(4 * e) * nk], dr[4 * (e + 1)] * x[(size_t)(4 * (e + 1)) * nk],
-                        dr[4 * e + 1] * x[(size_t)(4 * e + 1) * nk],
-                        dr[4 * (e + 1) + 1] * x[(size_t)(4 * (e + 1) + 1) * nk]};
+  const double* dr = l < 2 ? dr1 : drv + (size_t)(l - 2) * nd;
+  const double* x = w + ((size_t)ri * 2 * nr + 2 * e) * nk + k;
+  const double fb[4] = {dr[4 * e] * x[0], dr[4 * (e + 1)] * x[(size_t)2 * nk], dr[4 * e + 1] * x[nk],
+                        dr[4 * (e + 1) + 1] * x[(size_t)3 * nk]};
   rhs_T(K + ((size_t)l * ne + e) * 48, fb, lam_new, ri, e, k, ne, nk);
-}
-
-// drift^T for degree 1 (slots 0, 1; four right-hand sides): the CM projection
-// transposed, then the transposed Green's block
-__global__ void __launch_bounds__(512) k_drift_T_deg1(int ne, int nr, int nk, int deg1_cm,
-                                                      const double* __restrict__ dr1,
-                                                      const double* __restrict__ null1,
-                                                      const double* __restrict__ G1T, const double* __restrict__ K,
-                                                      const double* __restrict__ dUn_bar,
-                                                      const double* __restrict__ dVn_bar,
-                                                      const double* __restrict__ surf_bar,
-                                                      double* __restrict__ lam_new) {
-  extern __shared__ double sh[];
-  const int ncol = 2 * nr, nrow = 2 * nr + 1;
-  double* xb = sh;              // [4][nrow]
-  double* fb = sh + 4 * nrow;   // [4][ncol]
-  __shared__ double s_c[4];
-  for (int t = threadIdx.x; t < 4 * nrow; t += blockDim.x) {
-    const int q = t / nrow, r = t % nrow, kk = q >> 1, ri = q & 1;
-    double v = 0.0;
-    if (r < 2 * nr) {
-      const int node = r >> 1;
-      v = (r & 1) ? dVn_bar[((size_t)ri * nr + node) * nk + kk] : dUn_bar[((size_t)ri * nr + node) * nk + kk];
-      if (node == nr - 1 && !(r & 1)) v += surf_bar[(size_t)(0 + ri) * nk + kk];
-    } else if (deg1_cm) {
-      v = surf_bar[(size_t)(2 + ri) * nk + kk];
-    }
-    xb[t] = v;
-  }
-  __syncthreads();
-  const int fs = 4 * (nr - 1) + 2;
-  const double fa_n = null1[fs];
-  if (deg1_cm && fa_n != 0.0) {
-    // forward: x += c null, c = -x[F] / fa_n  =>  c_bar = <x_bar, null>, x_bar[F] -= c_bar / fa_n
-    if (threadIdx.x < 4) {
-      double c = 0.0;
-      for (int r = 0; r < nrow; ++r) {
-        const int dof = (r < 2 * nr) ? 4 * (r >> 1) + (r & 1) : fs;
-        c += xb[threadIdx.x * nrow + r] * null1[dof];
-      }
-      s_c[threadIdx.x] = c;
-    }
-    __syncthreads();
-    if (threadIdx.x < 4) xb[threadIdx.x * nrow + 2 * nr] -= s_c[threadIdx.x] / fa_n;
-    __syncthreads();
-  }
-  {  // f_bar = G1^T x_bar: a warp per column c (rows of G1T contiguous), lanes over r
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int c = wid; c < ncol; c += nw) {
-      const double* gc = G1T + (size_t)c * nrow;
-      double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-      for (int r = lane; r < nrow; r += 32) {
-        const double gv = gc[r];
-        a0 += gv * xb[r];
-        a1 += gv * xb[nrow + r];
-        a2 += gv * xb[2 * nrow + r];
-        a3 += gv * xb[3 * nrow + r];
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-        a2 += __shfl_xor_sync(0xffffffffu, a2, o);
-        a3 += __shfl_xor_sync(0xffffffffu, a3, o);
-      }
-      if (lane == 0) {
-        const double sc = dr1[4 * (c >> 1) + (c & 1)];  // bh row c = dr1 * f at (node, U or V)
-        fb[c] = sc * a0;
-        fb[ncol + c] = sc * a1;
-        fb[2 * ncol + c] = sc * a2;
-        fb[3 * ncol + c] = sc * a3;
-      }
-    }
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < 4 * ne; t += blockDim.x) {
-    const int q = t / ne, e = t % ne, kk = q >> 1, ri = q & 1;
-    const double* f = fb + q * ncol;
-    const double fe[4] = {f[2 * e], f[2 * (e + 1)], f[2 * e + 1], f[2 * (e + 1) + 1]};
-    rhs_T(K + ((size_t)1 * ne + e) * 48, fe, lam_new, ri, e, kk, ne, nk);
-  }
 }
 
 // G1T[c][r] = G1[r][c] (degree-1 Green's block, rows r < nrow, columns c < ncol)
@@ -920,9 +731,9 @@ struct StateGuard {
 };
 
 
-// buffers and one-time attributes of a reverse sweep
+// buffers of a reverse sweep
 void reverse_prepare(vg_handle* h, AdjWork& W) {
-  const int nk = h->nk, nr = h->nr, ne = h->ne, nd = h->ndof;
+  const int nk = h->nk, nr = h->nr, ne = h->ne;
   const size_t S = h->d_mem[0].n;
   ensure(W.lam, S);
   ensure(W.lam_new, S);
@@ -930,7 +741,7 @@ void reverse_prepare(vg_handle* h, AdjWork& W) {
   ensure(W.dVn_bar, (size_t)2 * nr * nk);
   ensure(W.surf_bar, (size_t)4 * nk);
   ensure(W.qbar, 2 * (size_t)h->grid.nlm);
-  ensure(W.w, (size_t)2 * nd * nk);
+  ensure(W.w, (size_t)2 * 2 * nr * nk);
   ensure(W.E, (size_t)5 * 2 * ne * nk);
   if (h->tor_on) {
     ensure(W.lam_t, h->d_tmem[0].n);
@@ -945,12 +756,6 @@ void reverse_prepare(vg_handle* h, AdjWork& W) {
     W.G1T.alloc((size_t)nrow * ncol);
     k_transpose<<<(nrow * ncol + 255) / 256, 256, 0, h->stream>>>(nrow, ncol, h->d_G1.p, W.G1T.p);
     VG_CUDA(cudaGetLastError());
-  }
-  static std::atomic<bool> ts_attr{false};  // set once; concurrent handles may race to it
-  if (!ts_attr) {
-    VG_CUDA(cudaFuncSetAttribute(k_drift_T, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(TS_WARPS * TS_WARP * sizeof(double))));
-    ts_attr = true;
   }
 }
 
@@ -980,14 +785,12 @@ void drift_T(vg_handle* h, AdjWork& W) {
   const int nk = h->nk, nr = h->nr, ne = h->ne, nd = h->ndof;
   const dim3 eg((nk + 31) / 32, (ne + 7) / 8, 2);
   cudaStream_t s = h->stream;
-  const size_t shm1 = (size_t)(4 * (2 * nr + 1) + 4 * 2 * nr) * sizeof(double);
-  const size_t ts_smem = (size_t)TS_WARPS * TS_WARP * sizeof(double);
-  k_drift_T<<<(h->ntask + TS_WARPS - 1) / TS_WARPS, 32 * TS_WARPS, ts_smem, s>>>(
-      nr, nd, nk, h->d_tasks.p, h->ntask, h->d_ab.p, h->d_dc.p, W.dUn_bar.p, W.dVn_bar.p, W.surf_bar.p, W.w.p);
-  k_rhs_T<<<eg, dim3(32, 8), 0, s>>>(ne, nd, nk, h->d_kdeg.p, h->d_dr.p, h->d_Krhs.p, W.w.p, W.lam_new.p);
-  k_drift_T_deg1<<<1, 512, shm1, s>>>(ne, nr, nk, h->p.deg1_cm, h->d_dr1.p, h->d_null1.p, W.G1T.p, h->d_Krhs.p,
-                                      W.dUn_bar.p, W.dVn_bar.p, W.surf_bar.p, W.lam_new.p);
-  h->n_launch += 3;
+  k_drift_T<<<h->ntask + (2 * nr + D1T - 1) / D1T, 32, sw::SMEM * sizeof(double), s>>>(
+      nr, nk, h->p.deg1_cm, h->d_tasks.p, h->ntask, h->d_lrec.p, h->d_urec.p, h->d_null1.p, W.G1T.p, W.dUn_bar.p,
+      W.dVn_bar.p, W.surf_bar.p, h->d_xs.p, W.w.p);
+  k_rhs_T<<<eg, dim3(32, 8), 0, s>>>(ne, nr, nd, nk, h->d_kdeg.p, h->d_dr.p, h->d_dr1.p, h->d_Krhs.p, W.w.p,
+                                     W.lam_new.p);
+  h->n_launch += 2;
   VG_CUDA(cudaGetLastError());
   if (h->tor_on) drift_tor_T(h, W.Et.p, W.Wb.p, W.gb.p, W.lam_t_new.p);
 }

@@ -232,5 +232,132 @@ __device__ __forceinline__ void band_sweeps(const double* __restrict__ lrec, con
   wait<0>();
 }
 
+// The transposed solve, from the same records: xU, xV (stride xst a node) the
+// adjoints of the solution at the nodes' U and V dofs, sU and sF what the last
+// node's U and F dofs add; out(node, U, V) receives the adjoint of the forcing,
+// nodes descending. U^T ascends: a node's values are final once the nodes below
+// have added theirs (p1, p2: what they add to the next node and the one after).
+// L^T descends through the transposed 7 x 5 maps. As many instructions and a
+// shorter chain than the solve itself.
+template <class Out>
+__device__ __forceinline__ void band_sweeps_T(const double* __restrict__ lrec, const double* __restrict__ urec, int nr,
+                                              const double* xU, const double* xV, size_t xst, double sU, double sF,
+                                              double* y, double* sm, int lane, Out out) {
+  const int nc = chunks(nr);
+  auto stage_u = [&](int c) {
+    if (c < nc) {
+      double* d = sm + (c & 1) * STAGE;
+      const double* r = urec + (size_t)c * NCH * UN;
+#pragma unroll
+      for (int t = 0; t < 3; ++t)
+        if (lane + 32 * t < NCH * UN / 2) cp16(d + 2 * (lane + 32 * t), r + 2 * (lane + 32 * t));
+      double* a = d + NCH * LN + lane;
+#pragma unroll
+      for (int q = 0; q < 2 * NCH; ++q) {
+        const int node = NCH * c + (q >> 1);
+        if (node < nr)
+          cp8(a + q * 32, ((q & 1) ? xV : xU) + (size_t)node * xst);
+        else
+          a[q * 32] = 0.0;
+      }
+    }
+    commit();
+  };
+  constexpr int off[4] = {24, 15, 7, 0};
+  stage_u(0);
+  double p1[4] = {0.0, 0.0, 0.0, 0.0}, p2[3] = {0.0, 0.0, 0.0};
+  for (int c = 0; c < nc; ++c) {
+    stage_u(c + 1);
+    wait<1>();
+    __syncwarp();
+    const double* rec = sm + (c & 1) * STAGE;
+    const double* a = rec + NCH * LN + lane;
+    double* yc = y + (size_t)c * NCH * 4 * 32 + lane;
+#pragma unroll
+    for (int n = 0; n < NCH; ++n) {
+      double u[UN];
+#pragma unroll
+      for (int i = 0; i < UN; i += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(rec + n * UN + i);
+        u[i] = v.x;
+        u[i + 1] = v.y;
+      }
+      const bool top = NCH * c + n == nr - 1;
+      double x[4] = {a[(2 * n) * 32] + (top ? sU : 0.0) + p1[0], a[(2 * n + 1) * 32] + p1[1],
+                     (top ? sF : 0.0) + p1[2], p1[3]};
+      double q1[4] = {p2[0], p2[1], p2[2], 0.0}, q2[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+#pragma unroll
+        for (int t = s + 1; t < 4; ++t) x[t] = fma(u[off[s] + t - s - 1], x[s], x[t]);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) q1[t] = fma(u[off[s] + 3 - s + t], x[s], q1[t]);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) q2[t] = fma(u[off[s] + 7 - s + t], x[s], q2[t]);
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        yc[(4 * n + t) * 32] = x[t];
+        p1[t] = q1[t];
+      }
+#pragma unroll
+      for (int t = 0; t < 3; ++t) p2[t] = q2[t];
+    }
+    __syncwarp();  // the stage is refilled next
+  }
+  __threadfence_block();  // the L sweep's copies read what the other lanes stored
+  __syncwarp();
+  auto stage_l = [&](int c) {
+    if (c >= 0) {
+      double* d = sm + (c & 1) * STAGE;
+      const double* r = lrec + (size_t)c * NCH * LN;
+#pragma unroll
+      for (int t = 0; t < 3; ++t)
+        if (lane + 32 * t < NCH * LN / 2) cp16(d + 2 * (lane + 32 * t), r + 2 * (lane + 32 * t));
+      const double* yc = y + (size_t)c * NCH * 4 * 32;
+#pragma unroll
+      for (int t = 0; t < NCH * 2; ++t) cp16(d + NCH * LN + 2 * (lane + 32 * t), yc + 2 * (lane + 32 * t));
+    }
+    commit();
+  };
+  stage_l(nc - 1);
+  double cb[3] = {0.0, 0.0, 0.0};  // the adjoint of the values carried to the node above
+  for (int c = nc - 1; c >= 0; --c) {
+    stage_l(c - 1);
+    wait<1>();
+    __syncwarp();
+    const double* rec = sm + (c & 1) * STAGE;
+    const double* a = rec + NCH * LN + lane;
+#pragma unroll
+    for (int n = NCH - 1; n >= 0; --n) {
+      double m[LN];
+#pragma unroll
+      for (int i = 0; i < LN; i += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(rec + n * LN + i);
+        m[i] = v.x;
+        m[i + 1] = v.y;
+      }
+      double o[5];
+#pragma unroll
+      for (int q = 0; q < 5; ++q) o[q] = m[q] * a[(4 * n) * 32];
+#pragma unroll
+      for (int i = 1; i < 4; ++i)
+#pragma unroll
+        for (int q = 0; q < 5; ++q) o[q] = fma(m[5 * i + q], a[(4 * n + i) * 32], o[q]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int q = 0; q < 5; ++q) o[q] = fma(m[5 * (4 + i) + q], cb[i], o[q]);
+      const int node = NCH * c + n;
+      if (node + 1 < nr) out(node + 1, o[3], o[4]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) cb[i] = o[i];
+    }
+    __syncwarp();
+  }
+  out(0, cb[0], cb[1]);
+  wait<0>();
+}
+
 }  // namespace sw
 }  // namespace vg

@@ -51,3 +51,32 @@ def test_rotation_channels_match_oracle_at_chunk_edges(n_elem):
     assert rel(g.fields()[0], o.fields()[0]) < TOL
     mg, mo = g.rotation()[0], o.rotation()[0]
     assert abs(mg - mo) <= TOL * abs(mo)
+
+
+@pytest.mark.parametrize("lmax,counts,cm", [(2, [1, 2, 2, 1], 1), (15, [1, 2, 3, 1], 0), (16, [2, 3, 2, 1], 1),
+                                            (17, [2, 3, 3, 1], 1)])
+def test_transposed_sweeps_match_differences(lmax, counts, cm):
+    """The gradient through the transposed solves: the misfit is quadratic in the load, so central differences are
+    exact up to rounding; 1e-6 of the gradient's scale along the direction, as in test_gpu_adjoint_sle.py."""
+    p = vlib.default_params()
+    p.lmax, p.nlat, p.nphi, p.deg1_cm = lmax, lmax + 1, 2 * lmax + 2, cm
+    for i, c in enumerate(counts):
+        p.ne_layer[i] = c
+    m = vlib.Model(p)
+    rng = np.random.default_rng(lmax)
+    sites = rng.choice(m.ng, size=9, replace=False)
+    dt = 100.0 * synth.SEC_PER_YEAR
+
+    def draw():
+        s = 1e3 * (rng.standard_normal((5, m.nlm)) + 1j * rng.standard_normal((5, m.nlm)))
+        s[:, : lmax + 1] = s[:, : lmax + 1].real
+        return s
+
+    sigma, obs = draw(), 0.01 * rng.standard_normal((5, 9))
+    _, g = m.misfit_grad(sigma, dt, sites, obs, ckpt_every=2)
+    for _ in range(3):
+        d = draw()
+        h = 1e-3
+        fd = (m.misfit(sigma + h * d, dt, sites, obs) - m.misfit(sigma - h * d, dt, sites, obs)) / (2 * h)
+        t = g.real * d.real + g.imag * d.imag
+        assert abs(fd - t.sum()) <= 1e-6 * max(abs(fd), np.sqrt((t**2).sum()))
