@@ -462,7 +462,11 @@ void pass_plan(vg_handle* h, const void* const kernel[3]) {
   cudaFuncAttributes fa;
   VG_CUDA(cudaFuncGetAttributes(&fa, kernel[0]));
   const size_t room = (size_t)lim - fa.sharedSizeBytes, psz = (size_t)(p_pitch((G.nlat + 1) / 2) + 6) * (G.lmax + 1);
-  const int ctas = h->p.sle_ctas > 0 ? std::min(h->p.sle_ctas, nsm) : nsm;
+  // a CTA per order and row: more would only lengthen the barrier (at lmax 85 73 us a
+  // pass against 76 with all SMs), and what is left holds another handle's pass (six
+  // handles of up to lmax 64: 2.47 ms an update against 3.26)
+  const int want = std::min(nsm, std::max(G.M, G.nlat));
+  const int ctas = h->p.sle_ctas > 0 ? std::min(h->p.sle_ctas, nsm) : want;
   h->sle_mode = scr * sizeof(double) > room ? 2 : G.M <= ctas && (scr + psz) * sizeof(double) <= room ? 1 : 0;
   h->sle_shm = h->sle_mode == 2 ? 0 : (scr + (h->sle_mode == 1 ? psz : 0)) * sizeof(double);
   int per_sm = 0;
@@ -470,7 +474,7 @@ void pass_plan(vg_handle* h, const void* const kernel[3]) {
   if (h->sle_shm) raise_smem_limit(fn, h->sle_shm);
   VG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, SLE_THREADS, h->sle_shm));
   if (per_sm < 1) throw Error("sle_solve: the fused inner loop does not fit on an SM");
-  const int grid = h->p.sle_ctas > 0 ? std::min(h->p.sle_ctas, nsm * per_sm) : nsm;
+  const int grid = h->p.sle_ctas > 0 ? std::min(h->p.sle_ctas, nsm * per_sm) : want;
   if (h->sle_mode == 2) h->d_sle_big.alloc(scr * (size_t)grid);
   if (!h->d_gbar.p) h->d_gbar.alloc(4);
   // from here on the last CTA of each launch resets the barrier
