@@ -376,7 +376,7 @@ __global__ void k_c_bytes(int ng, const double* __restrict__ C, unsigned char* _
 // ice_int_bar w_j dlon), ice_int_bar the sum of dphi_bar / <C>, into the adjoints
 // of this interval's end ice (frac) and of the previous interval's (1 - frac).
 // Bound by latency like the pass itself: nine kernels an iteration took 40 us and
-// their launches at lmax 64, this takes 11.
+// their launches at lmax 64, this takes 10.
 struct RevArgs : PassBase {
   int nk, K, fresh;  // fresh: digbar starts at zero
   double C_int, g, frac;
@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_rev(RevArgs A) {
     for (int j = blockIdx.x; j < nlat; j += gridDim.x) {
       const size_t row = (size_t)j * nphi;
       const double w = A.wts[j];
-      for (int m = tid; m < M; m += SLE_THREADS) S.Gd[m] = __ldcg(reinterpret_cast<const double2*>(A.D) + (size_t)j * M + m);
+      S.load_spectrum([&](int m) { return __ldcg(reinterpret_cast<const double2*>(A.D) + (size_t)j * M + m); });
       __syncthreads();
       S.row_synthesis();
       double acc = 0.0;
@@ -1061,8 +1061,8 @@ void sle_interval(vg_handle* h, AdjWork& W, int n, double dt_yr, int nsite) {
 // starting rsl, surf_bar and the ice adjoints accumulate
 void rev_pass(vg_handle* h, AdjWork& W, const unsigned char* C, const TapePass& P, bool fresh, double frac, double* gi1,
               double* gi0, double* rb) {
-  static const void* const kernel[3] = {(const void*)k_sle_rev<0>, (const void*)k_sle_rev<1>,
-                                        (const void*)k_sle_rev<2>};
+  static const void* const kernel[4] = {(const void*)k_sle_rev<0>, (const void*)k_sle_rev<1>,
+                                        (const void*)k_sle_rev<2>, (const void*)k_sle_rev<3>};
   RevArgs A;
   pass_base(h, A);  // (the forward has planned the passes)
   A.nk = h->nk;

@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(SHT_T, 2)
                        const double* __restrict__ sn, double* __restrict__ F) {
   extern __shared__ __align__(16) double sm[];
   __shared__ __align__(16) double part[4 * SHT_T];
-  const Rows<SHT_T> R(nphi, M, cs, sn, sm, part);
+  const Rows<SHT_T, false> R(nphi, M, cs, sn, sm, part);
   const int j = blockIdx.x, b = blockIdx.y;
   const double* src = f + ((size_t)b * nlat + j) * nphi;
   for (int i = threadIdx.x; i < nphi; i += SHT_T) R.L[i] = src[i];
@@ -126,13 +126,13 @@ __global__ void __launch_bounds__(SHT_T, 2)
                     const double* __restrict__ sn, double* __restrict__ f) {
   extern __shared__ __align__(16) double sm[];
   __shared__ __align__(16) double part[4 * SHT_T];
-  const Rows<SHT_T> R(nphi, M, cs, sn, sm, part);
+  const Rows<SHT_T, false> R(nphi, M, cs, sn, sm, part);
   const int j = blockIdx.x, b = blockIdx.y;
-  for (int m = threadIdx.x; m < M; m += SHT_T) {
+  R.load_spectrum([&](int m) {
     const double2 v = G[((size_t)b * M + m) * nlat + j];
     const double c = m == 0 ? 1.0 : 2.0;
-    R.Gd[m] = make_double2(c * v.x, c * v.y);
-  }
+    return make_double2(c * v.x, c * v.y);
+  });
   __syncthreads();
   R.row_synthesis();
   double* out = f + ((size_t)b * nlat + j) * nphi;
@@ -167,7 +167,7 @@ __global__ void k_fourier_synth_long(const double2* __restrict__ G, int nphi, in
 
 void fourier_analysis_dev(vg_handle* h, const double* d_f, int batch, double* d_F) {
   const Grid& G = h->grid;
-  const size_t shm = rows_scratch(G.nphi, G.M) * sizeof(double);
+  const size_t shm = rows_scratch(G.nphi, G.M, false) * sizeof(double);
   raise_smem_limit((const void*)k_fourier_analysis, shm);
   k_fourier_analysis<<<dim3(G.nlat, batch), SHT_T, shm, h->stream>>>(d_f, G.nphi, G.nlat, G.M, G.d_cos.p, G.d_sin.p,
                                                                      d_F);
@@ -192,7 +192,7 @@ void legendre_synth_dev(vg_handle* h, const double* d_q, int batch, double* d_G)
 }
 void fourier_synth_dev(vg_handle* h, const double* d_G, int batch, double* d_f) {
   const Grid& G = h->grid;
-  const size_t shm = rows_scratch(G.nphi, G.M) * sizeof(double);
+  const size_t shm = rows_scratch(G.nphi, G.M, false) * sizeof(double);
   const dim3 grid(G.nlat, batch);
   if (shm + 4 * SHT_T * sizeof(double) <= SMEM_CTA) {
     raise_smem_limit((const void*)k_fourier_synth, shm);

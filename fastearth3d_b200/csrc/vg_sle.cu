@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(SLE_THREADS, 2)
   extern __shared__ __align__(16) double sm[];
   __shared__ __align__(16) double part[4 * SLE_THREADS];
   __shared__ double red[32];
-  const Rows<SLE_THREADS> R(nphi, M, cs, sn, sm, part);
+  const Rows<SLE_THREADS, false> R(nphi, M, cs, sn, sm, part);
   int j = blockIdx.x;
   double s = 0.0;
   for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
@@ -165,8 +165,8 @@ __global__ void k_step_end(int nphi, int nlat, double dlon, const double* __rest
 // Five phases with four barriers, two syntheses and serial row integrals took 254
 // us a pass of eight iterations at lmax 128 (1004 at lmax 256), beside 70 us of
 // small kernels for the integrals, the coastline and the closing load that the
-// pass now holds; it takes 100 us (362). Of an iteration's cycles at lmax 128 the
-// barriers are 4700, O 9000 (order 0, which the others wait for), R 12000.
+// pass now holds; it takes 77 us (344). Of an iteration's cycles at lmax 128 the
+// barriers are 5000, O 8000 (order 0, which the others wait for), R 8000.
 struct PassArgs : PassBase {
   int nk, n_inner, subgrid, fixed;
   double tol, g;
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
     // ---- R: rows of this CTA
     for (int j = blockIdx.x; j < nlat; j += gridDim.x) {
       const size_t row = (size_t)j * nphi;
-      for (int m = tid; m < M; m += SLE_THREADS) S.Gd[m] = __ldcg(reinterpret_cast<const double2*>(A.D) + (size_t)j * M + m);
+      S.load_spectrum([&](int m) { return __ldcg(reinterpret_cast<const double2*>(A.D) + (size_t)j * M + m); });
       // this thread's first grid point, on its way while the sums are formed
       double pc = 0.0, pd = 0.0, pw = 0.0, po = 0.0, pr = 0.0;
       auto fetch = [&](int u) {
@@ -437,9 +437,9 @@ __global__ void __launch_bounds__(SLE_THREADS) k_sle_pass(PassArgs A) {
 }
 
 // doubles of a CTA's work area: the twiddles, then the larger of the two phases
-static size_t sle_pass_scratch(const Grid& G) {
-  const size_t tw = 2 * (size_t)(G.nphi + (G.nphi >> 3) + 1), orders = 2 * (4 * (size_t)((G.nlat + 1) / 2) + G.lmax + 1);
-  return (std::max(rows_scratch(G.nphi, G.M), tw + orders) + 1) / 2 * 2;
+static size_t sle_pass_scratch(const Grid& G, bool sq) {
+  const size_t orders = 2 * (4 * (size_t)((G.nlat + 1) / 2) + G.lmax + 1);
+  return (std::max(rows_scratch(G.nphi, G.M, sq), rows_table(G.nphi, sq) + orders) + 1) / 2 * 2;
 }
 
 // int C rsl - zeta of that load
@@ -451,10 +451,9 @@ __global__ void k_mass(SleScalars* sc, const double* __restrict__ rowpart, const
 
 // the variant and grid of a handle's passes, by the sea-level pass (its adjoint
 // has less static shared memory and the same registers a CTA)
-void pass_plan(vg_handle* h, const void* const kernel[3]) {
+void pass_plan(vg_handle* h, const void* const kernel[4]) {
   if (h->sle_grid != 0) return;
   const Grid& G = h->grid;
-  const size_t scr = sle_pass_scratch(G);
   int dev = 0, nsm = 0, lim = 0;
   VG_CUDA(cudaGetDevice(&dev));
   VG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -462,13 +461,16 @@ void pass_plan(vg_handle* h, const void* const kernel[3]) {
   cudaFuncAttributes fa;
   VG_CUDA(cudaFuncGetAttributes(&fa, kernel[0]));
   const size_t room = (size_t)lim - fa.sharedSizeBytes, psz = (size_t)(p_pitch((G.nlat + 1) / 2) + 6) * (G.lmax + 1);
-  // a CTA per order and row: more would only lengthen the barrier (at lmax 85 73 us a
-  // pass against 76 with all SMs), and what is left holds another handle's pass (six
+  // a CTA per order and row: more would only lengthen the barrier (at lmax 85 3 us of a
+  // pass), and what is left holds another handle's pass (six
   // handles of up to lmax 64: 2.47 ms an update against 3.26)
   const int want = std::min(nsm, std::max(G.M, G.nlat));
   const int ctas = h->p.sle_ctas > 0 ? std::min(h->p.sle_ctas, nsm) : want;
-  h->sle_mode = scr * sizeof(double) > room ? 2 : G.M <= ctas && (scr + psz) * sizeof(double) <= room ? 1 : 0;
-  h->sle_shm = h->sle_mode == 2 ? 0 : (scr + (h->sle_mode == 1 ? psz : 0)) * sizeof(double);
+  const size_t scr = sle_pass_scratch(G, false), ssq = sle_pass_scratch(G, true);
+  h->sle_mode = scr * sizeof(double) > room ? 2 : 0;
+  if (G.nphi % 2 == 0 && ssq * sizeof(double) <= room)
+    h->sle_mode = G.M <= ctas && (ssq + psz) * sizeof(double) <= room ? 1 : 3;
+  h->sle_shm = h->sle_mode == 2 ? 0 : (h->sle_mode == 0 ? scr : ssq + (h->sle_mode == 1 ? psz : 0)) * sizeof(double);
   int per_sm = 0;
   const void* fn = kernel[h->sle_mode];
   if (h->sle_shm) raise_smem_limit(fn, h->sle_shm);
@@ -500,13 +502,13 @@ void pass_base(vg_handle* h, PassBase& A) {
   A.cst = h->d_ulm.p;
   A.rowpart = h->d_rowpart.p;
   A.big = h->sle_mode == 2 ? h->d_sle_big.p : nullptr;
-  A.scr = sle_pass_scratch(G);
+  A.scr = sle_pass_scratch(G, (h->sle_mode & 1) != 0);
   A.sc = h->d_sc_.p;
   A.bar = h->d_gbar.p;
   A.wait_ns = h->wait_ns;
 }
 
-void pass_launch(vg_handle* h, const void* const kernel[3], void* args) {
+void pass_launch(vg_handle* h, const void* const kernel[4], void* args) {
   void* a[] = {args};
   if (h->sle_shm) raise_smem_limit(kernel[h->sle_mode], h->sle_shm);
   VG_CUDA(cudaLaunchCooperativeKernel(kernel[h->sle_mode], dim3(h->sle_grid), dim3(SLE_THREADS), a, h->sle_shm,
@@ -524,8 +526,8 @@ void check_pass_barrier(vg_handle* h) {
 }
 
 static void launch_pass(vg_handle* h) {
-  static const void* const kernel[3] = {(const void*)k_sle_pass<0>, (const void*)k_sle_pass<1>,
-                                        (const void*)k_sle_pass<2>};
+  static const void* const kernel[4] = {(const void*)k_sle_pass<0>, (const void*)k_sle_pass<1>,
+                                        (const void*)k_sle_pass<2>, (const void*)k_sle_pass<3>};
   pass_plan(h, kernel);
   PassArgs A;
   pass_base(h, A);
@@ -615,7 +617,7 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
   // the closing load's spectrum (from the pass, unless that had no ocean) and the
   // memory advance (src/vilma_sle.f90:353-358)
   if (!closed) {
-    const size_t shm = rows_scratch(nphi, M) * sizeof(double);
+    const size_t shm = rows_scratch(nphi, M, false) * sizeof(double);
     raise_smem_limit((const void*)k_load_fourier, shm);
     k_load_fourier<<<nlat, SLE_THREADS, shm, s>>>(nphi, nlat, M, h->d_dig.p, h->d_C.p, h->d_rsl.p,
                                                   ocean_seen ? h->d_wcorr.p : nullptr, G.d_cos.p, G.d_sin.p, h->d_F.p,

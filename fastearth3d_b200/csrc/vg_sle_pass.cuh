@@ -137,23 +137,52 @@ struct Share {
 
 // Longitude transforms of one row by the T threads of a CTA, in both directions
 // split by the reflection and the half period: four sums over a quarter of the
-// longitudes. Shared memory: twiddles tw, the row's spectrum Gd or the row L (the
-// one is read before the other is written), per base longitude four values X;
-// part: 4 T doubles.
-template <int T>
+// longitudes. Shared memory: twiddles, the row's spectrum Gd or the row L (the one is
+// read before the other is written), per base longitude four values X (twice that
+// with SQ); part: 4 T doubles.
+//
+// The sums are bound by their shared-memory reads of the twiddles. From the table tw
+// of the nphi angles a warp's reads have stride m (or i) modulo nphi: three lanes of
+// eight meet in a bank on average. With SQ, for even nphi, the square table W of
+// the angles m i, m and i up to nphi / 4, is read along its rows in both
+// directions, without conflicts, and half as often: orders m and half - m share
+// a twiddle up to signs. At lmax 128 a row's synthesis took 4900 cycles and its
+// analysis 4700, with SQ 2450 and 2600 (a pass 98 us and 79).
+template <int T, bool SQ>
 struct Rows {
   Lon G;
-  int M;
+  int M, nrep;  // nrep: orders m <= half / 2, each with half - m
   double2 *tw, *Gd;
   double *X, *L, *part;
   Share<T> ss, sa;
   __device__ __forceinline__ Rows(int nphi, int M_, const double* cs, const double* sn, double* sm, double* part_)
-      : G(nphi), M(M_), part(part_), ss(G.nbase, 2, nphi, threadIdx.x), sa(M_, 1, nphi, threadIdx.x) {
+      : G(nphi), M(M_), nrep(min(M_, G.nbase)), part(part_), ss(G.nbase, 2, nphi, threadIdx.x),
+        sa(SQ ? nrep : M_, 1, nphi, threadIdx.x) {
     tw = reinterpret_cast<double2*>(sm);
-    Gd = tw + tw_at(nphi) + 1;
+    Gd = tw + (SQ ? G.nbase * G.nbase : tw_at(nphi) + 1);
     L = reinterpret_cast<double*>(Gd);
-    X = L + (max(2 * M, nphi) + 1) / 2 * 2;
-    for (int t = threadIdx.x; t < nphi; t += T) tw[tw_at(t)] = make_double2(cs[t], sn[t]);
+    X = L + (max(SQ ? 4 * G.nbase : 2 * M, nphi) + 1) / 2 * 2;
+    if (SQ) {
+      for (int u = threadIdx.x; u < G.nbase * G.nbase; u += T) {
+        const int a = u / G.nbase, b = u - a * G.nbase, t = (a * b) % nphi;
+        tw[u] = make_double2(cs[t], sn[t]);
+      }
+    } else {
+      for (int t = threadIdx.x; t < nphi; t += T) tw[tw_at(t)] = make_double2(cs[t], sn[t]);
+    }
+  }
+
+  // the row's spectrum, get(m), into Gd
+  template <class Get>
+  __device__ __forceinline__ void load_spectrum(Get get) const {
+    if (SQ) {
+      for (int u = threadIdx.x; u < 2 * nrep; u += T) {
+        const int r = u >> 1, m = (u & 1) ? G.half - r : r;
+        Gd[u] = m < M && !((u & 1) && 2 * r == G.half) ? get(m) : make_double2(0.0, 0.0);
+      }
+    } else {
+      for (int m = threadIdx.x; m < M; m += T) Gd[m] = get(m);
+    }
   }
 
   // F(m) = 2 pi / nphi sum_i L_i e^{-i m phi_i} of the row in L, to out[m stride]
@@ -170,40 +199,78 @@ struct Rows {
       } else {
         x = make_double4(v[0] + v[2], v[0] - v[2], v[0] + v[2], v[0] - v[2]);
       }
-      reinterpret_cast<double2*>(X)[2 * i] = make_double2(x.x, x.y);
-      reinterpret_cast<double2*>(X)[2 * i + 1] = make_double2(x.z, x.w);
+      double2* o = reinterpret_cast<double2*>(X) + (SQ ? 4 : 2) * i;
+      o[0] = make_double2(x.x, x.y);
+      o[1] = make_double2(x.z, x.w);
+      if (SQ) {  // times (-1)^i, for the orders half - m
+        const double sg = (i & 1) ? -1.0 : 1.0;
+        o[2] = make_double2(sg * x.x, sg * x.y);
+        o[3] = make_double2(sg * x.z, sg * x.w);
+      }
     }
     __syncthreads();
-    const int Q = sa.Q;
-    const double sc = 2.0 * PI / (double)G.nphi;
-    for (int base = 0; base < M * Q; base += T) {
-      const Share<T> sh = base ? Share<T>(M, 1, G.nphi, base + tid) : sa;
-      const int m = sh.o;
-      double re = 0.0, im = 0.0;
-      if (base + tid < M * Q) {
-        const double2* x = reinterpret_cast<const double2*>(X) + (m & 1);
-        int t = sh.t0;
+    if (SQ) {
+      const int Q = sa.Q, m = sa.o, pm = m & 1, pp = (G.half - m) & 1;
+      const double2* x = reinterpret_cast<const double2*>(X);
+      double2 f = make_double2(0.0, 0.0), g = make_double2(0.0, 0.0);
+      if (tid < nrep * Q) {
 #pragma unroll 4
-        for (int i = sh.q; i < G.nbase; i += Q) {
-          const double2 w = tw[tw_at(t)], v = x[2 * i];
-          re = fma(v.x, w.x, re);
-          im = fma(-v.y, w.y, im);
-          t += sh.step;
-          if (t >= G.nphi) t -= G.nphi;
+        for (int i = sa.q; i < G.nbase; i += Q) {
+          const double2 w = tw[i * G.nbase + m], v = x[4 * i + pm], u = x[4 * i + 2 + pp];
+          f.x = fma(v.x, w.x, f.x);
+          f.y = fma(-v.y, w.y, f.y);
+          g.x = fma(u.x, w.x, g.x);
+          g.y = fma(u.y, w.y, g.y);
         }
       }
-      if (Q == 1) {
-        if (base + tid < M) __stcg(out + (size_t)m * stride, make_double2(re * sc, im * sc));
-      } else {
-        part[2 * tid] = re;
-        part[2 * tid + 1] = im;
-        __syncthreads();
-        if (tid < M) {
-          for (int c = 1; c < Q; ++c) {
-            re += part[2 * (tid + c * M)];
-            im += part[2 * (tid + c * M) + 1];
+      double2* p2 = reinterpret_cast<double2*>(part);
+      p2[tid] = f;
+      p2[T + tid] = g;
+      __syncthreads();
+      if (tid < 2 * nrep) {
+        const int b = tid >= nrep, r = tid - b * nrep, mo = b ? G.half - r : r;
+        double re = 0.0, im = 0.0;
+#pragma unroll 4
+        for (int c = 0; c < Q; ++c) {
+          const double2 v = p2[b * T + c * nrep + r];
+          re += v.x;
+          im += v.y;
+        }
+        const double sc = 2.0 * PI / (double)G.nphi;
+        if (mo < M && !(b && 2 * r == G.half)) __stcg(out + (size_t)mo * stride, make_double2(re * sc, im * sc));
+      }
+    } else {
+      const int Q = sa.Q;
+      const double sc = 2.0 * PI / (double)G.nphi;
+      for (int base = 0; base < M * Q; base += T) {
+        const Share<T> sh = base ? Share<T>(M, 1, G.nphi, base + tid) : sa;
+        const int m = sh.o;
+        double re = 0.0, im = 0.0;
+        if (base + tid < M * Q) {
+          const double2* x = reinterpret_cast<const double2*>(X) + (m & 1);
+          int t = sh.t0;
+#pragma unroll 4
+          for (int i = sh.q; i < G.nbase; i += Q) {
+            const double2 w = tw[tw_at(t)], v = x[2 * i];
+            re = fma(v.x, w.x, re);
+            im = fma(-v.y, w.y, im);
+            t += sh.step;
+            if (t >= G.nphi) t -= G.nphi;
           }
-          __stcg(out + (size_t)m * stride, make_double2(re * sc, im * sc));
+        }
+        if (Q == 1) {
+          if (base + tid < M) __stcg(out + (size_t)m * stride, make_double2(re * sc, im * sc));
+        } else {
+          part[2 * tid] = re;
+          part[2 * tid + 1] = im;
+          __syncthreads();
+          if (tid < M) {
+            for (int c = 1; c < Q; ++c) {
+              re += part[2 * (tid + c * M)];
+              im += part[2 * (tid + c * M) + 1];
+            }
+            __stcg(out + (size_t)m * stride, make_double2(re * sc, im * sc));
+          }
         }
       }
     }
@@ -214,42 +281,67 @@ struct Rows {
   __device__ __forceinline__ void row_synthesis() const {
     const int tid = threadIdx.x, nphi = G.nphi;
     const int Q = ss.Q;
-    for (int base = 0; base < G.nbase * Q; base += T) {
-      const Share<T> sh = base ? Share<T>(G.nbase, 2, nphi, base + tid) : ss;
-      const int i = sh.o;
-      double ce = 0.0, se = 0.0, co = 0.0, so = 0.0;
-      if (base + tid < G.nbase * Q) {
-        int t = sh.t0;
+    if (SQ) {
+      const int i = ss.o;
+      double c[2][2] = {}, v[2][2] = {};  // [order's parity][m or half - m], cosine and sine sums
+      if (tid < G.nbase * Q) {
 #pragma unroll 2
-        for (int m = 2 * sh.q; m < M; m += 2 * Q) {
-          const double2 w = tw[tw_at(t)], v = Gd[m];
-          ce = fma(v.x, w.x, ce);
-          se = fma(v.y, w.y, se);
-          if (m + 1 < M) {
-            int t1 = t + i;
-            if (t1 >= nphi) t1 -= nphi;
-            const double2 w1 = tw[tw_at(t1)], v1 = Gd[m + 1];
-            co = fma(v1.x, w1.x, co);
-            so = fma(v1.y, w1.y, so);
+        for (int r = 2 * ss.q; r < nrep; r += 2 * Q) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (r + h >= nrep) break;
+            const double2 w = tw[(r + h) * G.nbase + i], a = Gd[2 * (r + h)], b = Gd[2 * (r + h) + 1];
+            c[h][0] = fma(a.x, w.x, c[h][0]);
+            v[h][0] = fma(a.y, w.y, v[h][0]);
+            c[h][1] = fma(b.x, w.x, c[h][1]);
+            v[h][1] = fma(b.y, w.y, v[h][1]);
           }
-          t += sh.step;
-          if (t >= nphi) t -= nphi;
         }
       }
-      if (Q == 1) {
-        if (base + tid < G.nbase) {
-          reinterpret_cast<double2*>(X)[2 * i] = make_double2(ce, se);
-          reinterpret_cast<double2*>(X)[2 * i + 1] = make_double2(co, so);
+      const double sg = (i & 1) ? -1.0 : 1.0;
+      const bool odd = G.half & 1;  // half - m has the other parity
+      part[tid] = c[0][0] + sg * (odd ? c[1][1] : c[0][1]);
+      part[T + tid] = v[0][0] - sg * (odd ? v[1][1] : v[0][1]);
+      part[2 * T + tid] = c[1][0] + sg * (odd ? c[0][1] : c[1][1]);
+      part[3 * T + tid] = v[1][0] - sg * (odd ? v[0][1] : v[1][1]);
+    } else {
+      for (int base = 0; base < G.nbase * Q; base += T) {
+        const Share<T> sh = base ? Share<T>(G.nbase, 2, nphi, base + tid) : ss;
+        const int i = sh.o;
+        double ce = 0.0, se = 0.0, co = 0.0, so = 0.0;
+        if (base + tid < G.nbase * Q) {
+          int t = sh.t0;
+#pragma unroll 2
+          for (int m = 2 * sh.q; m < M; m += 2 * Q) {
+            const double2 w = tw[tw_at(t)], v = Gd[m];
+            ce = fma(v.x, w.x, ce);
+            se = fma(v.y, w.y, se);
+            if (m + 1 < M) {
+              int t1 = t + i;
+              if (t1 >= nphi) t1 -= nphi;
+              const double2 w1 = tw[tw_at(t1)], v1 = Gd[m + 1];
+              co = fma(v1.x, w1.x, co);
+              so = fma(v1.y, w1.y, so);
+            }
+            t += sh.step;
+            if (t >= nphi) t -= nphi;
+          }
         }
-      } else {
-        part[tid] = ce;
-        part[T + tid] = se;
-        part[2 * T + tid] = co;
-        part[3 * T + tid] = so;
+        if (Q == 1) {
+          if (base + tid < G.nbase) {
+            reinterpret_cast<double2*>(X)[2 * i] = make_double2(ce, se);
+            reinterpret_cast<double2*>(X)[2 * i + 1] = make_double2(co, so);
+          }
+        } else {
+          part[tid] = ce;
+          part[T + tid] = se;
+          part[2 * T + tid] = co;
+          part[3 * T + tid] = so;
+        }
       }
     }
     __syncthreads();
-    if (Q > 1) {
+    if (SQ || Q > 1) {
       for (int u = tid; u < 4 * G.nbase; u += T) {
         const int s4 = u / G.nbase, i = u - s4 * G.nbase;
         double v = 0.0;
@@ -267,30 +359,41 @@ struct Rows {
     return (pt & 1) ? ev - ov : ev + ov;
   }
 };
-// doubles of its shared memory
-inline size_t rows_scratch(int nphi, int M) {
+// doubles of its shared memory: the twiddles, and all of it
+inline size_t rows_table(int nphi, bool sq) {
+  const size_t nbase = nphi / 4 + 1;
+  return 2 * (sq ? nbase * nbase : (size_t)(nphi + (nphi >> 3) + 1));
+}
+inline size_t rows_scratch(int nphi, int M, bool sq) {
   const size_t nbase = nphi % 2 ? (nphi + 1) / 2 : nphi / 4 + 1;
-  return 2 * (size_t)(nphi + (nphi >> 3) + 1) + ((size_t)std::max(2 * M, nphi) + 1) / 2 * 2 + 4 * nbase;
+  return rows_table(nphi, sq) + (std::max(sq ? 4 * nbase : 2 * (size_t)M, (size_t)nphi) + 1) / 2 * 2 +
+         (sq ? 8 : 4) * nbase;
 }
 constexpr size_t SMEM_CTA = 227 * 1024;  // shared memory that a CTA can have
 
-// A CTA's part of a pass. MODE 1: a CTA with one order keeps that order's Legendre
-// functions (northern rows) in shared memory, where they fit: the barriers
-// invalidate L1, so read through it (MODE 0) they come from L2 in each iteration
-// (106 us a pass at lmax 128 and 77 at lmax 85, against 100 and 76). MODE 2, a grid
-// whose work area does not fit in shared memory: the work area is A.scr doubles a
-// CTA of global memory.
+// A CTA's part of a pass. MODE 1: the square twiddles, and a CTA with one order
+// keeps that order's Legendre functions (northern rows) in shared memory, where both
+// fit: the barriers invalidate L1, so read through it they come from L2 in each
+// iteration (84 us a pass at lmax 128 and 68 at lmax 85 in MODE 3, 77 and 63 here).
+// MODE 3: the square twiddles alone. MODE 0: neither fits, or nphi is odd. MODE 2, a
+// grid whose work area does not fit in shared memory: the work area is A.scr
+// doubles a CTA of global memory.
 //
 // The work area: that of Rows; after its twiddles, in the same space, the orders'
 // phase (northern rows Fe [4][nh], degrees dl); in mode 1 the order's Legendre
 // functions Ps and six numbers a degree Ks follow.
 template <int MODE>
-struct Pass : Rows<SLE_THREADS> {
+struct Pass : Rows<SLE_THREADS, (MODE & 1) != 0> {
+  using R = Rows<SLE_THREADS, (MODE & 1) != 0>;
+  using R::G;
+  using R::M;
+  using R::Gd;
+  using R::part;
   int nlat, nh, pp;
   double2 *Fe, *dl;
   double *Ps, *Ks;
   __device__ __forceinline__ Pass(const PassBase& A, double* sm, double* part_)
-      : Rows<SLE_THREADS>(A.nphi, A.M, A.cs, A.sn, sm, part_),
+      : R(A.nphi, A.M, A.cs, A.sn, sm, part_),
         nlat(A.nlat),
         nh((A.nlat + 1) / 2),
         pp(p_pitch((A.nlat + 1) / 2)) {
@@ -336,24 +439,22 @@ struct Pass : Rows<SLE_THREADS> {
       if (mine) open(xk, kc);
       double re[NV] = {}, im[NV] = {}, rc[NV] = {}, ic[NV] = {};
       const double* P[NV];
-      const double2* fe[NV];
+      const double2* fe = Fe + (xa & 1) * nh;  // NX is even: a thread's degrees have one parity
 #pragma unroll
       for (int v = 0; v < NV; ++v) {
         const int x = min(xa + v * NX, nl - 1);  // past the end: a valid row, result unused
         P[v] = MODE == 1 ? Ps + (size_t)x * pp : A.plm + (size_t)(lm0 + x) * nlat;
-        fe[v] = Fe + (x & 1) * nh;
       }
       auto sums = [&](auto NVc, auto FIRST) {
-#pragma unroll 3
+#pragma unroll 1  // the phases run through their code once: short code is fetched sooner
         for (int j = lw; j < nh; j += W) {
+          const double2 f = fe[j], c = FIRST.value ? fe[2 * nh + j] : f;
 #pragma unroll
           for (int v = 0; v < NVc.value; ++v) {
             const double p = MODE == 1 ? P[v][j] : __ldg(P[v] + j);
-            const double2 f = fe[v][j];
             re[v] = fma(p, f.x, re[v]);
             im[v] = fma(p, f.y, im[v]);
             if (FIRST.value) {
-              const double2 c = fe[v][2 * nh + j];
               rc[v] = fma(p, c.x, rc[v]);
               ic[v] = fma(p, c.y, ic[v]);
             }
@@ -399,7 +500,7 @@ struct Pass : Rows<SLE_THREADS> {
       if (u < nh * Q) {
         const double* P = MODE == 1 ? Ps + j : A.plm + (size_t)lm0 * nlat + j;
         const int pt = MODE == 1 ? pp : nlat;
-#pragma unroll 4
+#pragma unroll 2
         for (int x = 2 * q; x < nl; x += 2 * Q) {
           const double p = MODE == 1 ? P[(size_t)x * pt] : __ldg(P + (size_t)x * pt);
           const double2 d = dl[x];
@@ -451,9 +552,9 @@ __device__ __forceinline__ bool pass_last(unsigned int* bar) {
 
 // host side (vg_sle.cu): the variant, shared memory and grid of a handle's
 // passes, once, and what their arguments have in common
-void pass_plan(vg_handle* h, const void* const kernel[3]);
+void pass_plan(vg_handle* h, const void* const kernel[4]);
 void pass_base(vg_handle* h, PassBase& A);
-void pass_launch(vg_handle* h, const void* const kernel[3], void* args);
+void pass_launch(vg_handle* h, const void* const kernel[4], void* args);
 void check_pass_barrier(vg_handle* h);  // synchronises; throws if a wait of a pass gave up
 
 }  // namespace vg

@@ -1,7 +1,7 @@
 """The fused sea-level pass at the edges of its work split: grids with and
 without an equator row, even, twice-odd and odd longitude counts, one order and
-several a CTA (more orders than CTAs; three CTAs for everything), a work area
-larger than shared memory, a fixed coastline, the subgrid load, one inner
+several a CTA (more orders than CTAs; three CTAs for everything), rows too long
+for the square twiddle table, a work area larger than shared memory, a fixed coastline, the subgrid load, one inner
 iteration, a solve with no ocean; GPU = oracle with test_gpu_parity.py's
 tolerances, the same iteration counts, and the same result whatever the CTAs."""
 import numpy as np
@@ -52,6 +52,7 @@ def run(lmax, nlat, nphi, opts, ctas=0, gpu=True, ocean=True):
     (21, 24, 46, {"sle_n_inner": 1}),
     (33, 40, 76, {"sle_n_outer": 1}),
     (150, 151, 302, {}),
+    (16, 17, 800, {}),
     (4, 7000, 10, {}),
 ])
 def test_pass_matches_oracle(lmax, nlat, nphi, opts):
