@@ -288,6 +288,12 @@ __global__ void __launch_bounds__(256) k_advance_1d(const double* __restrict__ m
   double amax = 0.0;
   if (k < nk && e < ne) {
     if (active[e]) {
+      const size_t base = mem_idx(0, ri, e, 0, k, ne, nk), plane = mem_idx(1, 0, 0, 0, 0, ne, nk);
+      double old[3][4];  // on its way first
+#pragma unroll
+      for (int s3 = 0; s3 < 3; ++s3)
+#pragma unroll
+        for (int m = 0; m < 4; ++m) old[s3][m] = __ldcs(mem + base + s3 * plane + (size_t)m * nk);
       const int l = kdeg[k], lm = k2lm[k];
       const double s = sigma[2 * lm + ri];
       const double* xu = xUn + (size_t)l * nr;
@@ -310,14 +316,13 @@ __global__ void __launch_bounds__(256) k_advance_1d(const double* __restrict__ m
       }
 #pragma unroll
       for (int m = 0; m < 4; ++m) {
-        size_t iA = mem_idx(0, ri, e, m, k, ne, nk), iB = mem_idx(1, ri, e, m, k, ne, nk),
-               iC = mem_idx(2, ri, e, m, k, ne, nk);
-        double An = om * mem[iA] - two_muM * a[m];
-        double Bn = om * mem[iB] - two_muM * b[m];
-        double Cn = om * mem[iC] - two_muM * c[m];
-        nxt[iA] = An;
-        nxt[iB] = Bn;
-        nxt[iC] = Cn;
+        double An = om * old[0][m] - two_muM * a[m];
+        double Bn = om * old[1][m] - two_muM * b[m];
+        double Cn = om * old[2][m] - two_muM * c[m];
+        double* o = nxt + base + (size_t)m * nk;
+        o[0] = An;
+        o[plane] = Bn;
+        o[2 * plane] = Cn;
         amax = nanmax(amax, nanmax(fabs(An), nanmax(fabs(Bn), fabs(Cn))));
       }
     }

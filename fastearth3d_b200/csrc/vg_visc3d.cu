@@ -27,6 +27,7 @@
 // (the grid identities of src/vilma_tensor_sh.f90:244-266).
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <initializer_list>
 
 #include "vg_device.cuh"
@@ -105,7 +106,10 @@ struct V3Args {
 // Blocks of 32 slots x 8 3-D elements. The memory and drift are read along
 // the slot index (coalesced); the operand rows X[k][ch][f][ri] are written
 // through a shared tile [ch][f in block][slot] so that each (slot, channel)
-// row's 6 x 8 entries go out as one contiguous run.
+// row's 6 x 8 entries go out as one contiguous run. Neighbouring blocks share the
+// rows (the element blocks run fastest). Bound by HBM: the memory and drift in, X
+// out; at lmax 128 with 54 3-D elements of 100, 53 us with a division an entry and
+// the loads of one component at a time, 37 now (floor 27).
 constexpr int V3_TK = 32, V3_TE = 8, V3_TC = 6 * V3_TE, V3_TP = V3_TK + 1;  // tile: columns per row, padded slots
 
 template <class T, int NC>
@@ -113,26 +117,44 @@ __global__ void __launch_bounds__(256) k_v3_gather(V3Args A, T* __restrict__ X) 
   extern __shared__ unsigned char v3_sm[];
   T* tile = reinterpret_cast<T*>(v3_sm);  // [NC ch][V3_TC][V3_TP]
   const int kx = threadIdx.x, ey = threadIdx.y;
-  const int k0 = blockIdx.x * V3_TK, e0 = blockIdx.y * V3_TE;
+  const int k0 = blockIdx.y * V3_TK, e0 = blockIdx.x * V3_TE;
   const int k = k0 + kx, ei = e0 + ey;
   if (k < A.nk && ei < A.ne3d) {
     const int e = A.e3d[ei], l = A.kdeg[k], lm = A.k2lm[k];
+    const size_t nk = A.nk, plane = mem_idx(0, 1, 0, 0, 0, A.ne, A.nk);  // from re to im, from component to component
+    const double* mem = A.mem + mem_idx(0, 0, e, 0, k, A.ne, A.nk);
+    const double* dU = A.dUn + (size_t)e * nk + k;
+    const double* dV = A.dVn + (size_t)e * nk + k;
+    double old[2][3][4], du[2][4];  // all of this thread's operands on their way at once
+#pragma unroll
+    for (int ri = 0; ri < 2; ++ri) {
+      const size_t o = (size_t)ri * A.nr * nk;
+      du[ri][0] = dU[o];
+      du[ri][1] = dU[o + nk];
+      du[ri][2] = dV[o];
+      du[ri][3] = dV[o + nk];
+#pragma unroll
+      for (int s3 = 0; s3 < 3; ++s3)
+#pragma unroll
+        for (int lam = 0; lam < 4; ++lam) old[ri][s3][lam] = mem[(2 * s3 + ri) * plane + lam * nk];
+    }
     const double Jr = A.Jr[l], twoMu = 2.0 * A.mu[e];
     const double* xu = A.xUn + (size_t)l * A.nr;
     const double* xv = A.xVn + (size_t)l * A.nr;
+#pragma unroll
     for (int ri = 0; ri < 2; ++ri) {
       const double s = A.sigma[2 * lm + ri];
-      const double U0 = s * xu[e] + A.dUn[((size_t)ri * A.nr + e) * A.nk + k];
-      const double U1 = s * xu[e + 1] + A.dUn[((size_t)ri * A.nr + e + 1) * A.nk + k];
-      const double V0 = s * xv[e] + A.dVn[((size_t)ri * A.nr + e) * A.nk + k];
-      const double V1 = s * xv[e + 1] + A.dVn[((size_t)ri * A.nr + e + 1) * A.nk + k];
+      const double U0 = s * xu[e] + du[ri][0];
+      const double U1 = s * xu[e + 1] + du[ri][1];
+      const double V0 = s * xv[e] + du[ri][2];
+      const double V1 = s * xv[e + 1] + du[ri][3];
       double eps[3][4];
       strain_coeffs(U0, U1, V0, V1, Jr, eps[0], eps[1], eps[2]);
 #pragma unroll
       for (int s3 = 0; s3 < 3; ++s3)
 #pragma unroll
         for (int lam = 0; lam < 4; ++lam) {
-          double v = A.mem[mem_idx(s3, ri, e, lam, k, A.ne, A.nk)] + twoMu * eps[s3][lam];
+          double v = old[ri][s3][lam] + twoMu * eps[s3][lam];
           if (lam == 2) v = -Jr * v;  // trace channel enters the synthesis as -l(l+1) c
           tile[((size_t)lam * V3_TC + ey * 6 + s3 * 2 + ri) * V3_TP + kx] = (T)v;
         }
@@ -161,10 +183,19 @@ __global__ void __launch_bounds__(256) k_v3_gather(V3Args A, T* __restrict__ X) 
       atomic_max_bits(A.gmax + (size_t)lam * A.ncf + 6 * e0 + cc, mx);
     }
   }
-  for (int t = threadIdx.y * V3_TK + threadIdx.x; t < nkb * NC * w; t += V3_TK * V3_TE) {
-    const int kl = t / (NC * w), rem = t % (NC * w), lam = rem / w, c = rem % w;
+  // a warp per (slot, channel) run, two columns a lane
+  using V = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+  const int c = 2 * threadIdx.x;
+  if (c >= w) return;
+#pragma unroll 4
+  for (int u = threadIdx.y; u < nkb * NC; u += V3_TE) {
+    const int kl = u / NC, lam = u % NC;
     const size_t xr = A.lm_rows ? (size_t)A.k2lm[k0 + kl] : (size_t)(k0 + kl);
-    X[(xr * NC + lam) * A.ncf + 6 * e0 + c] = tile[((size_t)lam * V3_TC + c) * V3_TP + kl];
+    const T* t = tile + ((size_t)lam * V3_TC + c) * V3_TP + kl;
+    V v;
+    v.x = t[0];
+    v.y = t[V3_TP];
+    *reinterpret_cast<V*>(X + (xr * NC + lam) * A.ncf + 6 * e0 + c) = v;
   }
 }
 
@@ -1219,30 +1250,39 @@ static void lon_check(const vg_handle* h) {
 
 // Channel normalisations and the increment form c += Delta
 // (src/vilma_response.f90:1281-1318): one thread per (slot, 3-D element);
-// the block's maxima of |new memory| per slot go into A.mnext.
-template <class T, int NQ>
-__device__ __forceinline__ double v3_scatter_one(const V3Args& A, const T* __restrict__ R,
+// the block's maxima of |new memory| per slot go into A.mnext. Blocks of 32 slots x TE
+// elements: the products' rows R[k][quadrature][f][ri] run along the elements and
+// the memory along the slots, so the rows come in as contiguous runs through a
+// shared tile. Bound by HBM (the memory in and out and the rows once); read by
+// its own thread, each (re, im) pair took a sector of its own: 99 us at lmax 128
+// with 54 3-D elements of 100, 50 now (floor 46).
+template <class V, int NQ, int TE>
+__device__ __forceinline__ double v3_scatter_one(const V3Args& A, const V* tile, const double (&old)[3][2][4],
                                                  const double* __restrict__ n6, int k, int ei) {
   double amax = 0.0;
   const int e = A.e3d[ei], l = A.kdeg[k];
-  const double J = A.Jr[l], nn = n6[l];
-  const T* row = R + (size_t)k * NQ * A.ncf;
+  const double nn = n6[l], rJ = 1.0 / A.Jr[l], rn = nn != 0.0 ? 1.0 / nn : 0.0;
+  double* nxt = A.nxt + mem_idx(0, 0, e, 0, k, A.ne, A.nk);
+  const size_t step = mem_idx(0, 1, 0, 0, 0, A.ne, A.nk);  // from re to im, from component to component
+#pragma unroll
   for (int s3 = 0; s3 < 3; ++s3) {
-    const int f = 3 * ei + s3;
     double q[NQ][2];
 #pragma unroll
-    for (int p = 0; p < NQ; ++p)
-#pragma unroll
-      for (int ri = 0; ri < 2; ++ri) q[p][ri] = (double)row[(size_t)p * A.ncf + 2 * f + ri];
+    for (int p = 0; p < NQ; ++p) {
+      const V v = tile[p * 3 * TE + s3];
+      q[p][0] = (double)v.x;
+      q[p][1] = (double)v.y;
+    }
     if (NQ == 10) {  // lambda 3: (wD.RP + i wP.(m/sin RT)) / J; lambda 4: (wG.TP / 2 + i wH.(TT - PP)) / n4
-      const double n4 = 0.25 * nn;
       double t[2][2];
       const int d = A.tor_swap ? NQ - 4 : NQ - 3, p = A.tor_swap ? NQ - 3 : NQ - 4;  // wD.RP, wP.(m/sin RT)
-      t[0][0] = (q[d][0] - q[p][1]) / J;
-      t[0][1] = (q[d][1] + q[p][0]) / J;
-      t[1][0] = n4 != 0.0 ? (0.5 * q[NQ - 2][0] - q[NQ - 1][1]) / n4 : 0.0;
-      t[1][1] = n4 != 0.0 ? (0.5 * q[NQ - 2][1] + q[NQ - 1][0]) / n4 : 0.0;
+      t[0][0] = (q[d][0] - q[p][1]) * rJ;
+      t[0][1] = (q[d][1] + q[p][0]) * rJ;
+      t[1][0] = nn != 0.0 ? (0.5 * q[NQ - 2][0] - q[NQ - 1][1]) * (4.0 * rn) : 0.0;  // n4 = nn / 4
+      t[1][1] = nn != 0.0 ? (0.5 * q[NQ - 2][1] + q[NQ - 1][0]) * (4.0 * rn) : 0.0;
+#pragma unroll
       for (int ri = 0; ri < 2; ++ri)
+#pragma unroll
         for (int lam = 0; lam < 2; ++lam) {
           const size_t idx = tmem_idx(s3, ri, e, lam, k, A.ne, A.nk);
           A.tnxt[idx] = A.tmem[idx] + t[lam][ri];
@@ -1251,40 +1291,96 @@ __device__ __forceinline__ double v3_scatter_one(const V3Args& A, const T* __res
     double d[4][2];
     d[0][0] = q[0][0];
     d[0][1] = q[0][1];
-    d[1][0] = (q[1][0] + q[2][1]) / J;  // (wD.RT - i wP.(m/sin RP)) / J
-    d[1][1] = (q[1][1] - q[2][0]) / J;
-    d[2][0] = q[3][0] / (-2.0 * J);
-    d[2][1] = q[3][1] / (-2.0 * J);
-    d[3][0] = nn != 0.0 ? (q[4][0] + 2.0 * q[5][1]) / nn : 0.0;  // (wG.(TT-PP) - 2i wH.TP) / n6
-    d[3][1] = nn != 0.0 ? (q[4][1] - 2.0 * q[5][0]) / nn : 0.0;
+    d[1][0] = (q[1][0] + q[2][1]) * rJ;  // (wD.RT - i wP.(m/sin RP)) / J
+    d[1][1] = (q[1][1] - q[2][0]) * rJ;
+    d[2][0] = q[3][0] * (-0.5 * rJ);
+    d[2][1] = q[3][1] * (-0.5 * rJ);
+    d[3][0] = nn != 0.0 ? (q[4][0] + 2.0 * q[5][1]) * rn : 0.0;  // (wG.(TT-PP) - 2i wH.TP) / n6
+    d[3][1] = nn != 0.0 ? (q[4][1] - 2.0 * q[5][0]) * rn : 0.0;
+#pragma unroll
     for (int ri = 0; ri < 2; ++ri)
+#pragma unroll
       for (int lam = 0; lam < 4; ++lam) {
-        size_t idx = mem_idx(s3, ri, e, lam, k, A.ne, A.nk);
-        const double v = A.mem[idx] + d[lam][ri];
-        A.nxt[idx] = v;
+        const double v = old[s3][ri][lam] + d[lam][ri];
+        nxt[(2 * s3 + ri) * step + (size_t)lam * A.nk] = v;
         amax = nanmax(amax, fabs(v));
       }
   }
   return amax;
 }
 
-template <class T, int NQ = 6>
-__global__ void __launch_bounds__(256) k_v3_scatter(V3Args A, const T* __restrict__ R,
-                                                    const double* __restrict__ n6) {
-  __shared__ double red[8][33];
-  const int k = blockIdx.x * 32 + threadIdx.x, ei = blockIdx.y * 8 + threadIdx.y;
-  double amax = 0.0;
-  if (k < A.nk && ei < A.ne3d) amax = v3_scatter_one<T, NQ>(A, R, n6, k, ei);
-  if (A.mnext) {  // the same in every thread of the block
-    red[threadIdx.y][threadIdx.x] = amax;
-    __syncthreads();
-    if (threadIdx.y == 0 && k < A.nk) {
-      double v = red[0][threadIdx.x];
+// tile pitch in (re, im) pairs: odd, so that 16-byte reads along the slots miss no bank
+template <int NQ, int TE>
+constexpr int v3_scatter_pitch() {
+  return NQ * 3 * TE + 1 - NQ * 3 * TE % 2;
+}
+
+template <class V, int NQ, int TE>
+__global__ void __launch_bounds__(32 * TE) k_v3_scatter(V3Args A, const V* __restrict__ R,
+                                                        const double* __restrict__ n6) {
+  extern __shared__ __align__(16) unsigned char v3_sm[];
+  __shared__ double red[TE][33];
+  V* tile = reinterpret_cast<V*>(v3_sm);
+  constexpr int PITCH = v3_scatter_pitch<NQ, TE>();
+  const int kx = threadIdx.x, ey = threadIdx.y, k0 = blockIdx.y * 32, e0 = blockIdx.x * TE;
+  const int k = k0 + kx, ei = e0 + ey;
+  const bool on = k < A.nk && ei < A.ne3d;
+  const int nkb = min(32, A.nk - k0), nv = 3 * min(TE, A.ne3d - e0);
+  if (kx < nv) {
+    const V* src = R + ((size_t)(k0 + ey) * NQ) * A.nf + 3 * e0 + kx;
+    unsigned dst = (unsigned)__cvta_generic_to_shared(tile + ey * PITCH + kx);
+    for (int kl = ey; kl < nkb; kl += TE) {
 #pragma unroll
-      for (int t = 1; t < 8; ++t) v = nanmax(v, red[t][threadIdx.x]);
+      for (int p = 0; p < NQ; ++p)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(dst + p * 3 * TE * (unsigned)sizeof(V)),
+                     "l"(src + (size_t)p * A.nf), "n"(sizeof(V))
+                     : "memory");
+      src += (size_t)TE * NQ * A.nf;
+      dst += TE * PITCH * (unsigned)sizeof(V);
+    }
+  }
+  double old[3][2][4];  // the memory, on its way beside the rows
+  if (on) {
+    const double* mem = A.mem + mem_idx(0, 0, A.e3d[ei], 0, k, A.ne, A.nk);
+    const size_t step = mem_idx(0, 1, 0, 0, 0, A.ne, A.nk);
+#pragma unroll
+    for (int s3 = 0; s3 < 3; ++s3)
+#pragma unroll
+      for (int ri = 0; ri < 2; ++ri)
+#pragma unroll
+        for (int lam = 0; lam < 4; ++lam) old[s3][ri][lam] = __ldcs(mem + (2 * s3 + ri) * step + (size_t)lam * A.nk);
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();
+  double amax = 0.0;
+  if (on) amax = v3_scatter_one<V, NQ, TE>(A, tile + kx * PITCH + 3 * ey, old, n6, k, ei);
+  if (A.mnext) {  // the same in every thread of the block
+    red[ey][kx] = amax;
+    __syncthreads();
+    if (ey == 0 && k < A.nk) {
+      double v = red[0][kx];
+#pragma unroll
+      for (int t = 1; t < TE; ++t) v = nanmax(v, red[t][kx]);
       atomic_max_bits(reinterpret_cast<unsigned long long*>(A.mnext) + k, v);
     }
   }
+}
+
+template <class V, int NQ, int TE>
+static void launch_scatter(vg_handle* h, const V3Args& A, const V* R) {
+  constexpr size_t shm = 32 * v3_scatter_pitch<NQ, TE>() * sizeof(V);
+  raise_smem_limit((const void*)k_v3_scatter<V, NQ, TE>, shm);
+  k_v3_scatter<V, NQ, TE><<<dim3((h->ne3d + TE - 1) / TE, (h->nk + 31) / 32), dim3(32, TE), shm, h->stream>>>(
+      A, R, h->d_n6.p);
+  ++h->n_launch;
+  VG_CUDA(cudaGetLastError());
+}
+static void launch_scatter(vg_handle* h, const V3Args& A) {
+  const double2* R = reinterpret_cast<const double2*>(h->d_dy.p);
+  if (h->tor_on)
+    launch_scatter<double2, 10, 4>(h, A, R);
+  else
+    launch_scatter<double2, 6, 4>(h, A, R);
 }
 
 // the gather tile (the FP64 one is above the default 48 KB)
@@ -1422,7 +1518,7 @@ void visc3d_advance(vg_handle* h, const double* d_sigma, double dt, const double
   A.nf = nf;
   A.ncf = ncf;
   A.mnext = h->d_mnorm.p + (size_t)(1 - h->cur) * h->nk;
-  dim3 gg((h->nk + 31) / 32, (h->ne3d + 7) / 8);
+  const dim3 gg((h->ne3d + V3_TE - 1) / V3_TE, (h->nk + V3_TK - 1) / V3_TK);
   v3_tile_attributes();
   if (h->p.visc3d_precision == VG_VISC3D_SPLIT_TC) {
     float *X32 = nullptr, *dy32 = nullptr;
@@ -1435,9 +1531,7 @@ void visc3d_advance(vg_handle* h, const double* d_sigma, double dt, const double
     }
     visc3d_tc_run(h, dt, trap);
     PhaseScope pc(h, VG_PH_V3_SCATTER);
-    k_v3_scatter<float><<<gg, dim3(32, 8), 0, s>>>(A, dy32, h->d_n6.p);
-    ++h->n_launch;
-    VG_CUDA(cudaGetLastError());
+    launch_scatter<float2, 6, 4>(h, A, reinterpret_cast<const float2*>(dy32));
     return;
   }
   if (h->p.visc3d_precision == VG_VISC3D_EXACT_TC) {
@@ -1456,12 +1550,7 @@ void visc3d_advance(vg_handle* h, const double* d_sigma, double dt, const double
     }
     visc3d_oz_run(h, dt, trap);
     PhaseScope pc(h, VG_PH_V3_SCATTER);
-    if (h->tor_on)
-      k_v3_scatter<double, 10><<<gg, dim3(32, 8), 0, s>>>(A, h->d_dy.p, h->d_n6.p);
-    else
-      k_v3_scatter<double><<<gg, dim3(32, 8), 0, s>>>(A, h->d_dy.p, h->d_n6.p);
-    ++h->n_launch;
-    VG_CUDA(cudaGetLastError());
+    launch_scatter(h, A);
     return;
   }
   {
@@ -1519,12 +1608,7 @@ void visc3d_advance(vg_handle* h, const double* d_sigma, double dt, const double
     launch_gemm(h, S, 1);
   }
   PhaseScope pc(h, VG_PH_V3_SCATTER);
-  if (h->tor_on)
-    k_v3_scatter<double, 10><<<gg, dim3(32, 8), 0, s>>>(A, h->d_dy.p, h->d_n6.p);
-  else
-    k_v3_scatter<double><<<gg, dim3(32, 8), 0, s>>>(A, h->d_dy.p, h->d_n6.p);
-  ++h->n_launch;
-  VG_CUDA(cudaGetLastError());
+  launch_scatter(h, A);
 }
 
 // ------------------------------------------------------------------ adjoint
