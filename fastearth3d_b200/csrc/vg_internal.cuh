@@ -131,8 +131,7 @@ struct vg_handle {
   // into an error (vg_set_wait_limit)
   unsigned long long wait_ns = 2000000000ull;
   cudaStream_t stream = nullptr;
-  // second stream: the spectral memory advance beside the 3-D pass, and the
-  // drift beside the sea-level pass setup, joined before the fused loop reads it
+  // second stream: the spectral memory advance beside the 3-D pass
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // sizes

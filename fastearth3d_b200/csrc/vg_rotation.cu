@@ -45,9 +45,10 @@ struct RotArgs {
 // dissipative right-hand side of each (channel, re/im) in the reference's
 // element order (src/vilma_viscoelastic.f90:441-480), then the equilibrated
 // band solve (src/vilma_radial_fe.f90:578-605), in two kernels:
-//   k_rot_elem   one thread per (channel, re/im, element): the element's
-//                contributions to its four test dofs (two Gauss points, the
-//                FP64 divisions of the strain constants), into A.fl
+//   k_rot_elem   eight lanes per (channel, re/im, element), one for each Gauss
+//                point and test dof of the element's contributions, into A.fl
+//                (a lane for all eight ran 120 FP64 divisions in a row: 19 us at
+//                100 elements, 9 now)
 //   k_rot_begin  one block: the nodal forcing of the four right-hand sides
 //                (node n: element n-1's second test dof, then element n's
 //                first, as the serial loop adds them) times the row scales,
@@ -63,31 +64,26 @@ constexpr int ROT_ELEM_THREADS = 64;
 __global__ void __launch_bounds__(ROT_ELEM_THREADS) k_rot_elem(RotArgs A) {
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   const int ne = A.ne;
-  if (w >= 4 * ne) return;
   const double xg = 0.5773502691896257;
-  const int q = w / ne, e = w % ne, ch = q >> 1, ri = q & 1;
+  const int qe = min(w >> 3, 4 * ne - 1), ig = (w >> 2) & 1, tt = w & 3;
+  const int q = qe / ne, e = qe % ne, ch = q >> 1, ri = q & 1;
   const double* mem = A.mem + (size_t)ch * 6 * ne * 4;
   const double* Am = mem + (size_t)(0 * 2 + ri) * ne * 4;
   const double* Bm = mem + (size_t)(1 * 2 + ri) * ne * 4;
   const double* Cm = mem + (size_t)(2 * 2 + ri) * ne * 4;
   const double rk = A.r[e], rk1 = A.r[e + 1], h = rk1 - rk;
-  double floc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int ig = 0; ig < 2; ++ig) {
-    const double gp = ig == 0 ? -xg : xg;
-    const double ra = 0.5 * (h * gp + rk + rk1);
-    const double psik = (rk1 - ra) / h, psik1 = (ra - rk) / h;
-    double tauV[4];
-    for (int m = 0; m < 4; ++m) tauV[m] = Am[e * 4 + m] / h + Bm[e * 4 + m] * psik / ra + Cm[e * 4 + m] * psik1 / ra;
-    for (int tt = 0; tt < 4; ++tt) {
-      double D = 0.0;
-      for (int m = 0; m < 4; ++m) {
-        const double deps = A.sa[tt * 4 + m] / h + A.sb[tt * 4 + m] * psik / ra + A.sc[tt * 4 + m] * psik1 / ra;
-        D = D + A.nrm[m] * tauV[m] * deps;
-      }
-      floc[tt] = floc[tt] - D * ra * ra * h * 0.5;
-    }
+  const double gp = ig == 0 ? -xg : xg;
+  const double ra = 0.5 * (h * gp + rk + rk1);
+  const double psik = (rk1 - ra) / h, psik1 = (ra - rk) / h;
+  double D = 0.0;
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const double tauV = Am[e * 4 + m] / h + Bm[e * 4 + m] * psik / ra + Cm[e * 4 + m] * psik1 / ra;
+    const double deps = A.sa[tt * 4 + m] / h + A.sb[tt * 4 + m] * psik / ra + A.sc[tt * 4 + m] * psik1 / ra;
+    D = D + A.nrm[m] * tauV * deps;
   }
-  for (int tt = 0; tt < 4; ++tt) A.fl[((size_t)q * ne + e) * 4 + tt] = floc[tt];
+  const double v = D * ra * ra * h * 0.5, v1 = __shfl_xor_sync(0xffffffffu, v, 4);
+  if (ig == 0 && (w >> 3) < 4 * ne) A.fl[(size_t)qe * 4 + tt] = (0.0 - v) - v1;  // the Gauss points in order
 }
 
 __global__ void __launch_bounds__(ROT_THREADS) k_rot_begin(RotArgs A) {
@@ -162,17 +158,20 @@ struct SolveArgs {
 };
 
 // rotation_solve_m + rotation_commit (src/vilma_rotation.f90:170-190, 224-233):
-// the rigid inertia from the row sums (in row order), the algebraic Liouville
+// the rigid inertia from the row sums, the algebraic Liouville
 // solve for m, then the forward-Euler memory commit of both channels with
 // (cload, m): one thread per (channel, re/im, element).
 __global__ void k_rot_solve_commit(RotArgs A, SolveArgs S) {
   __shared__ double s_c[4];  // cload re, im, m re, im
+  __shared__ double red[32];
+  double i13 = 0.0, i23 = 0.0;
+  for (int j = threadIdx.x; j < S.nlat; j += blockDim.x) {
+    i13 += S.w[j] * S.rows[j] * S.dlon;
+    i23 += S.w[j] * S.rows[S.nlat + j] * S.dlon;
+  }
+  i13 = block_sum_w(i13, red);
+  i23 = block_sum_w(i23, red);
   if (threadIdx.x == 0) {
-    double i13 = 0.0, i23 = 0.0;
-    for (int j = 0; j < S.nlat; ++j) {
-      i13 += S.w[j] * S.rows[j] * S.dlon;
-      i23 += S.w[j] * S.rows[S.nlat + j] * S.dlon;
-    }
     const double Ir = -S.a4 * i13, Ii = -S.a4 * i23;
     const double clr = Ir * S.scl, cli = Ii * S.scl;
     const double Itr = -(S.Fe_load * clr + A.scal[RS_DF_LOAD]), Iti = -(S.Fe_load * cli + A.scal[RS_DF_LOAD + 1]);
@@ -337,7 +336,7 @@ void rotation_setup(vg_handle* h) {
 // the drift of both channels from the entering memory
 // (rotation_begin_step, src/vilma_rotation.f90:154-168)
 static void rot_begin_launch(vg_handle* h, const RotArgs& A, cudaStream_t s) {
-  k_rot_elem<<<(4 * A.ne + ROT_ELEM_THREADS - 1) / ROT_ELEM_THREADS, ROT_ELEM_THREADS, 0, s>>>(A);
+  k_rot_elem<<<(32 * A.ne + ROT_ELEM_THREADS - 1) / ROT_ELEM_THREADS, ROT_ELEM_THREADS, 0, s>>>(A);
   k_rot_begin<<<1, ROT_THREADS, 0, s>>>(A);
   h->n_launch += 2;
   VG_CUDA(cudaGetLastError());
@@ -381,7 +380,7 @@ void rotation_advance(vg_handle* h, const double* d_sigma, double dt) {
   S.rows = h->d_rot_rows.p;
   const RotArgs A = rot_args(h);
   for (int k = 0; k < n_sub; ++k) {
-    rot_begin_launch(h, A, s);
+    if (k > 0) rot_begin_launch(h, A, s);  // the first sub-step starts from the interval's own begin
     k_rot_solve_commit<<<1, 256, 0, s>>>(A, S);
     ++h->n_launch;
     VG_CUDA(cudaGetLastError());
