@@ -98,12 +98,6 @@ __device__ __forceinline__ void deg1_solve_cta(const double* __restrict__ ab, in
   }
 }
 
-// --------------------------------------------------------------------------
-// Longitude transforms of one latitude row, CTA-cooperative, twiddles from
-// tables cos/sin(2 pi t / nphi). The real-field convention of the Gauss-grid
-// transforms (src/vilma_sht.f90:11-15): f_i = Re G_0 + 2 Re sum_{m>0} G_m e^{i m phi_i},
-// and F_m = (2 pi / nphi) sum_i f_i e^{-i m phi_i}.
-
 // CTA reductions (fixed order: deterministic for a fixed block size)
 __device__ __forceinline__ double block_sum(double v, double* red) {
   red[threadIdx.x] = v;
@@ -116,8 +110,8 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   __syncthreads();
   return r;
 }
-// The same reductions through warp shuffles (two block barriers instead of
-// one per tree level); blockDim a multiple of 32, every thread gets the
+// The same through warp shuffles (two block barriers instead of one per tree
+// level); blockDim a multiple of 32, every thread gets the
 // result; the warp partials are added in warp order.
 __device__ __forceinline__ double block_sum_w(double v, double* red) {
 #pragma unroll
@@ -128,28 +122,6 @@ __device__ __forceinline__ double block_sum_w(double v, double* red) {
   __syncthreads();
   double r = red[0];
   for (int w = 1; w < nw; ++w) r += red[w];
-  return r;
-}
-__device__ __forceinline__ double block_max_w(double v, double* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int nw = blockDim.x >> 5;
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double r = red[0];
-  for (int w = 1; w < nw; ++w) r = nanmax(r, red[w]);
-  return r;
-}
-__device__ __forceinline__ double block_max(double v, double* red) {
-  red[threadIdx.x] = v;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) red[threadIdx.x] = nanmax(red[threadIdx.x], red[threadIdx.x + o]);
-    __syncthreads();
-  }
-  double r = red[0];
-  __syncthreads();
   return r;
 }
 

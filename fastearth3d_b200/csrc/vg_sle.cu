@@ -568,13 +568,12 @@ void sync_scalars(vg_handle* h) { read_scalars(h); }
 // into the other state buffer; the caller decides to keep or drop it.
 void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
   const Grid& G = h->grid;
-  const int ng = G.ng, nlat = G.nlat, nphi = G.nphi, M = G.M, nlm = G.nlm;
+  const int ng = G.ng, nlat = G.nlat, nphi = G.nphi, M = G.M;
   const double dlon = 2.0 * PI / (double)nphi;
   cudaStream_t s = h->stream;
   const vg_params& p = h->p;
   SleScalars* sc = h->d_sc_.p;
   double* rp = h->d_rowpart.p;
-  const int eb = 256, eg = (ng + eb - 1) / eb;
   if (!p.sle_warm_start) VG_CUDA(cudaMemsetAsync(h->d_rsl.p, 0, ng * sizeof(double), s));
   if (p.sle_n_outer < 1) VG_CUDA(cudaMemsetAsync(sc, 0, sizeof(SleScalars), s));  // (else by the first pass)
   const bool trap = p.scheme == VG_SCHEME_TRAP && !report_only;

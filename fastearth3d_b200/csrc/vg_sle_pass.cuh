@@ -135,7 +135,9 @@ struct Share {
   }
 };
 
-// Longitude transforms of one row by the T threads of a CTA, in both directions
+// Longitude transforms of one row by the T threads of a CTA (src/vilma_sht.f90:11-15:
+// f_i = Re G_0 + 2 Re sum_{m>0} G_m e^{i m phi_i}, F_m = (2 pi / nphi) sum_i f_i
+// e^{-i m phi_i}; Gd holds G_0 and 2 G_m), in both directions
 // split by the reflection and the half period: four sums over a quarter of the
 // longitudes. Shared memory: twiddles, the row's spectrum Gd or the row L (the one is
 // read before the other is written), per base longitude four values X (twice that
