@@ -273,8 +273,8 @@ def stage_work(w, info, precision):
            "v3_scatter": {"bytes": 2 * state3 + dy},
            "drift": {"bytes": algorithmic_bytes(info, "drift")},
            "advance_1d": {"bytes": algorithmic_bytes(info, "advance_1d")}}
-    if precision == "fp64":  # one kernel runs the whole longitude pass
-        out["v3_lon_inv"] = {"flop": inv + fwd, "bytes": 2 * S + rate}
+    if precision == "fp64":  # one kernel runs the whole longitude pass; the reflection halves its sums
+        out["v3_lon_inv"] = {"flop": (inv + fwd) / 2, "bytes": 2 * S + rate}
     return out
 
 
