@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(SHT_T, 2)
 constexpr int AN_L = 32, AN_J = 256;
 __global__ void __launch_bounds__(8 * AN_L)
     k_legendre_analysis(const double2* __restrict__ F, int lmax, int nlat, int M, int nlm, const int* __restrict__ mbeg,
-                        const double* __restrict__ plm, const double* __restrict__ wts, double2* __restrict__ q) {
+                        const double* __restrict__ plm, const double* __restrict__ wts, double* __restrict__ q) {
   __shared__ double2 fe[2][AN_J];
   const int m = blockIdx.x, x0 = blockIdx.y * AN_L, b = blockIdx.z, nl = lmax - m + 1;
   if (x0 >= nl) return;
@@ -73,7 +73,11 @@ __global__ void __launch_bounds__(8 * AN_L)
     re += __shfl_xor_sync(0xffffffffu, re, o);
     im += __shfl_xor_sync(0xffffffffu, im, o);
   }
-  if (lw == 0 && x < nl) q[(size_t)b * nlm + mbeg[m] + x] = make_double2(re, im);
+  if (lw == 0 && x < nl) {  // two stores: the caller's vector may start at any double
+    double* o = q + 2 * ((size_t)b * nlm + mbeg[m] + x);
+    o[0] = re;
+    o[1] = im;
+  }
 }
 
 // G = sum_l q_lm plm[lm][j]: a CTA per order and 32 northern rows, its eight warps
@@ -178,7 +182,7 @@ void legendre_analysis_dev(vg_handle* h, const double* d_F, int batch, double* d
   const Grid& G = h->grid;
   k_legendre_analysis<<<dim3(G.M, (G.lmax + AN_L) / AN_L, batch), 8 * AN_L, 0, h->stream>>>(
       reinterpret_cast<const double2*>(d_F), G.lmax, G.nlat, G.M, G.nlm, G.d_mbeg.p, G.d_plm.p, G.d_wts.p,
-      reinterpret_cast<double2*>(d_q));
+      d_q);
   ++h->n_launch;
   VG_CUDA(cudaGetLastError());
 }

@@ -33,3 +33,26 @@ def test_transforms_match_oracle(lmax, nlat, nphi):
     if nphi <= 6144:
         f = rng.standard_normal(nlat * nphi)
         assert rel(g.analysis(f), o.analysis(f)) < 1e-12
+
+
+def test_noalloc_analysis_into_any_double():
+    """The caller's device vectors may start at any double: shifted by one, the same spectrum to the bit."""
+    import ctypes as C
+
+    import torch
+
+    p = vlib.default_params()
+    p.lmax, p.nlat, p.nphi = 33, 34, 68
+    m = vlib.Model(p)
+    f = torch.from_numpy(np.random.default_rng(2).standard_normal(m.ng + 1)).cuda()
+    out = []
+    for shift in (0, 1):
+        q = torch.zeros(2 * m.nlm + 1, dtype=torch.float64, device="cuda")
+        g = torch.zeros(m.ng + 1, dtype=torch.float64, device="cuda")
+        g[shift:shift + m.ng] = f[:m.ng]
+        torch.cuda.synchronize()
+        rc = vlib.lib().vg_sht_analysis_noalloc(m.h, C.c_void_p(g[shift:].data_ptr()), C.c_void_p(q[shift:].data_ptr()), 1)
+        assert rc == 0
+        torch.cuda.synchronize()
+        out.append(q[shift:shift + 2 * m.nlm].cpu().numpy())
+    assert np.array_equal(*out)
