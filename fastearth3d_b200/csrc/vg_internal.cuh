@@ -26,11 +26,15 @@
 // rows 0..18 = dgbtf2 band (kl = ku = 6), 19 = 1/pivot, 20 = pivot offset
 #define VG_LDAB 21
 
+// The runtime also keeps the error for the thread's next cudaGetLastError, which
+// after a launch would read it as that launch's: it is taken out here.
 #define VG_CUDA(call)                                                                  \
   do {                                                                                   \
     cudaError_t _e = (call);                                                             \
-    if (_e != cudaSuccess)                                                               \
+    if (_e != cudaSuccess) {                                                             \
+      (void)cudaGetLastError();                                                          \
       throw vg::Error(std::string(#call) + ": " + cudaGetErrorString(_e));              \
+    }                                                                                    \
   } while (0)
 
 namespace vg {
