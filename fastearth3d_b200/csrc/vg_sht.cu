@@ -20,18 +20,26 @@ namespace vg {
 
 constexpr int SHT_T = 512;
 
-// a CTA per row
+// a CTA per row (LONG: a row whose tables do not fit in shared memory)
+template <bool LONG>
 __global__ void __launch_bounds__(SHT_T, 2)
     k_fourier_analysis(const double* __restrict__ f, int nphi, int nlat, int M, const double* __restrict__ cs,
                        const double* __restrict__ sn, double* __restrict__ F) {
   extern __shared__ __align__(16) double sm[];
-  __shared__ __align__(16) double part[4 * SHT_T];
-  const Rows<SHT_T, false> R(nphi, M, cs, sn, sm, part);
   const int j = blockIdx.x, b = blockIdx.y;
   const double* src = f + ((size_t)b * nlat + j) * nphi;
-  for (int i = threadIdx.x; i < nphi; i += SHT_T) R.L[i] = src[i];
-  __syncthreads();
-  R.row_analysis(reinterpret_cast<double2*>(F) + (size_t)b * M * nlat + j, nlat);
+  double2* out = reinterpret_cast<double2*>(F) + (size_t)b * M * nlat + j;
+  if constexpr (LONG) {
+    for (int i = threadIdx.x; i < nphi; i += SHT_T) sm[i] = src[i];
+    __syncthreads();
+    long_row_analysis<SHT_T>(sm, nphi, M, cs, sn, out, nlat);
+  } else {
+    __shared__ __align__(16) double part[4 * SHT_T];
+    const Rows<SHT_T, false> R(nphi, M, cs, sn, sm, part);
+    for (int i = threadIdx.x; i < nphi; i += SHT_T) R.L[i] = src[i];
+    __syncthreads();
+    R.row_analysis(out, nlat);
+  }
 }
 
 // q = sum_j w_j plm[lm][j] F[m][j]: a CTA per order and AN_L degrees, eight lanes a
@@ -147,8 +155,8 @@ __global__ void __launch_bounds__(SHT_T, 2)
   }
 }
 
-// the same for rows whose tables do not fit in shared memory (more than about
-// 8000 longitudes): a thread per longitude, all orders
+// the same for rows whose tables do not fit in shared memory: a thread per
+// longitude, all orders
 __global__ void k_fourier_synth_long(const double2* __restrict__ G, int nphi, int nlat, int M,
                                      const double* __restrict__ cs, const double* __restrict__ sn,
                                      double* __restrict__ f) {
@@ -171,10 +179,16 @@ __global__ void k_fourier_synth_long(const double2* __restrict__ G, int nphi, in
 
 void fourier_analysis_dev(vg_handle* h, const double* d_f, int batch, double* d_F) {
   const Grid& G = h->grid;
-  const size_t shm = rows_scratch(G.nphi, G.M, false) * sizeof(double);
-  raise_smem_limit((const void*)k_fourier_analysis, shm);
-  k_fourier_analysis<<<dim3(G.nlat, batch), SHT_T, shm, h->stream>>>(d_f, G.nphi, G.nlat, G.M, G.d_cos.p, G.d_sin.p,
-                                                                     d_F);
+  check_row(G);
+  const dim3 grid(G.nlat, batch);
+  if (rows_fit(G.nphi, G.M, SHT_T)) {
+    const size_t shm = rows_scratch(G.nphi, G.M, false) * sizeof(double);
+    raise_smem_limit((const void*)k_fourier_analysis<false>, shm);
+    k_fourier_analysis<false><<<grid, SHT_T, shm, h->stream>>>(d_f, G.nphi, G.nlat, G.M, G.d_cos.p, G.d_sin.p, d_F);
+  } else {
+    k_fourier_analysis<true><<<grid, SHT_T, G.nphi * sizeof(double), h->stream>>>(d_f, G.nphi, G.nlat, G.M, G.d_cos.p,
+                                                                                G.d_sin.p, d_F);
+  }
   ++h->n_launch;
   VG_CUDA(cudaGetLastError());
 }
@@ -196,9 +210,9 @@ void legendre_synth_dev(vg_handle* h, const double* d_q, int batch, double* d_G)
 }
 void fourier_synth_dev(vg_handle* h, const double* d_G, int batch, double* d_f) {
   const Grid& G = h->grid;
-  const size_t shm = rows_scratch(G.nphi, G.M, false) * sizeof(double);
   const dim3 grid(G.nlat, batch);
-  if (shm + 4 * SHT_T * sizeof(double) <= SMEM_CTA) {
+  if (rows_fit(G.nphi, G.M, SHT_T)) {
+    const size_t shm = rows_scratch(G.nphi, G.M, false) * sizeof(double);
     raise_smem_limit((const void*)k_fourier_synth, shm);
     k_fourier_synth<<<grid, SHT_T, shm, h->stream>>>(reinterpret_cast<const double2*>(d_G), G.nphi, G.nlat, G.M,
                                                      G.d_cos.p, G.d_sin.p, d_f);

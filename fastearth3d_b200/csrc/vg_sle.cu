@@ -72,24 +72,35 @@ __global__ void k_pass_setup(int nphi, int nlat, int set_c0, int io1, int fixed,
 
 // the closing load of a solve whose last pass had no ocean: total surface load
 // (assemble_load, src/vilma_sle.f90:387-403), its longitude transform, row sums of C rsl
+// (LONG: rows whose tables do not fit in shared memory)
+template <bool LONG>
 __global__ void __launch_bounds__(SLE_THREADS, 2)
     k_load_fourier(int nphi, int nlat, int M, const double* __restrict__ dig, const double* __restrict__ C,
                    const double* __restrict__ rsl, const double* __restrict__ wcorr, const double* __restrict__ cs,
                    const double* __restrict__ sn, double* __restrict__ F, double* __restrict__ rowpart) {
   extern __shared__ __align__(16) double sm[];
-  __shared__ __align__(16) double part[4 * SLE_THREADS];
   __shared__ double red[32];
-  const Rows<SLE_THREADS, false> R(nphi, M, cs, sn, sm, part);
-  int j = blockIdx.x;
-  double s = 0.0;
-  for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
-    size_t p = (size_t)j * nphi + i;
-    R.L[i] = RHO_ICE * dig[p] + RHO_WATER * (C[p] * rsl[p]) + (wcorr ? wcorr[p] : 0.0);
-    s += C[p] * rsl[p];
+  const int j = blockIdx.x;
+  double2* out = reinterpret_cast<double2*>(F) + j;
+  auto load = [&](double* row) {
+    double s = 0.0;
+    for (int i = threadIdx.x; i < nphi; i += blockDim.x) {
+      size_t p = (size_t)j * nphi + i;
+      row[i] = RHO_ICE * dig[p] + RHO_WATER * (C[p] * rsl[p]) + (wcorr ? wcorr[p] : 0.0);
+      s += C[p] * rsl[p];
+    }
+    s = block_sum_w(s, red);
+    if (threadIdx.x == 0) rowpart[RP_MASS * nlat + j] = s;
+  };
+  if constexpr (LONG) {
+    load(sm);
+    long_row_analysis<SLE_THREADS>(sm, nphi, M, cs, sn, out, nlat);
+  } else {
+    __shared__ __align__(16) double part[4 * SLE_THREADS];
+    const Rows<SLE_THREADS, false> R(nphi, M, cs, sn, sm, part);
+    load(R.L);
+    R.row_analysis(out, nlat);
   }
-  s = block_sum_w(s, red);
-  if (threadIdx.x == 0) rowpart[RP_MASS * nlat + j] = s;
-  R.row_analysis(reinterpret_cast<double2*>(F) + j, nlat);
 }
 
 // End of an interval, a block per row: with ice1 the ice becomes the interval's
@@ -616,11 +627,14 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
   // the closing load's spectrum (from the pass, unless that had no ocean) and the
   // memory advance (src/vilma_sle.f90:353-358)
   if (!closed) {
-    const size_t shm = rows_scratch(nphi, M, false) * sizeof(double);
-    raise_smem_limit((const void*)k_load_fourier, shm);
-    k_load_fourier<<<nlat, SLE_THREADS, shm, s>>>(nphi, nlat, M, h->d_dig.p, h->d_C.p, h->d_rsl.p,
-                                                  ocean_seen ? h->d_wcorr.p : nullptr, G.d_cos.p, G.d_sin.p, h->d_F.p,
-                                                  rp);
+    check_row(G);
+    const bool fit = rows_fit(nphi, M, SLE_THREADS);
+    const size_t shm = (fit ? rows_scratch(nphi, M, false) : (size_t)nphi) * sizeof(double);
+    const auto kernel = fit ? k_load_fourier<false> : k_load_fourier<true>;
+    raise_smem_limit((const void*)kernel, shm);
+    kernel<<<nlat, SLE_THREADS, shm, s>>>(
+        nphi, nlat, M, h->d_dig.p, h->d_C.p, h->d_rsl.p, ocean_seen ? h->d_wcorr.p : nullptr, G.d_cos.p, G.d_sin.p,
+        h->d_F.p, rp);
     ++h->n_launch;
     if (p.sle_n_outer < 1) {
       k_mass<<<1, 32, 0, s>>>(sc, rp, G.d_wts.p, nlat, dlon);

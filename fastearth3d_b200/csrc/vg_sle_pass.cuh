@@ -372,6 +372,34 @@ inline size_t rows_scratch(int nphi, int M, bool sq) {
          (sq ? 8 : 4) * nbase;
 }
 constexpr size_t SMEM_CTA = 227 * 1024;  // shared memory that a CTA can have
+// whether the work area of rows fits beside the partial sums of T threads and a block reduction's words:
+// up to 6346 longitudes (5137 of an odd count, whose base longitudes are twice as many)
+inline bool rows_fit(int nphi, int M, int T) {
+  return (rows_scratch(nphi, M, false) + 4 * (size_t)T + 32) * sizeof(double) <= SMEM_CTA;
+}
+
+// The analysis of a row that does not fit: the row alone in shared memory, all its longitudes by a thread per
+// order (longitudes up to LONG_ROW, 48 KB).
+constexpr int LONG_ROW = 6144;
+inline void check_row(const Grid& G) {
+  if (G.nphi > LONG_ROW) throw Error("longitude analysis: rows of more than 6144 longitudes are not supported");
+}
+template <int T>
+__device__ __forceinline__ void long_row_analysis(const double* row, int nphi, int M, const double* __restrict__ cs,
+                                                  const double* __restrict__ sn, double2* out, int stride) {
+  const double sc = 2.0 * PI / (double)nphi;
+  for (int m = threadIdx.x; m < M; m += T) {
+    double re = 0.0, im = 0.0;
+    int t = 0;
+    for (int i = 0; i < nphi; ++i) {
+      re = fma(row[i], __ldg(&cs[t]), re);
+      im = fma(-row[i], __ldg(&sn[t]), im);
+      t += m;
+      if (t >= nphi) t -= nphi;
+    }
+    out[(size_t)m * stride] = make_double2(re * sc, im * sc);
+  }
+}
 
 // A CTA's part of a pass. MODE 1: the square twiddles, and a CTA with one order
 // keeps that order's Legendre functions (northern rows) in shared memory, where both
