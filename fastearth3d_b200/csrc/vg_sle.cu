@@ -659,7 +659,8 @@ void update_dev(vg_handle* h, const double* d_ice1, double dt_yr) {
   cudaStream_t s = h->stream;
   const vg_params& p = h->p;
   const double dt = dt_yr * SEC_PER_YEAR;
-  const double t0 = h->time_yr * SEC_PER_YEAR, t1 = t0 + dt, span = t1 - t0;
+  // in seconds, the clock that a restart carries and that response steps move too
+  const double t0 = h->time_s, t1 = t0 + dt, span = t1 - t0;
   const int eb = 256, eg = (ng + eb - 1) / eb;
   h->worst_mass_resid = 0.0;
   // rotational feedback: drift frozen at the interval start, s_rot held across
@@ -789,7 +790,7 @@ void update_dev(vg_handle* h, const double* d_ice1, double dt_yr) {
   // polar motion to the interval end under the converged load (:411-421)
   if (h->rot_on) rotation_advance(h, h->d_sigma.p, span);
   h->time_yr += dt_yr;
-  h->time_s = h->time_yr * SEC_PER_YEAR;  // not the sub-steps' sum: a restart's clock (seconds) gives time_yr back
+  h->time_s = t1;  // the next interval's start, here and after a restart; not the sub-steps' sum
   finish_step(h, d_ice1);
 }
 
