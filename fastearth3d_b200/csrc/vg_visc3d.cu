@@ -769,8 +769,13 @@ __device__ __forceinline__ void stage_out(const double* __restrict__ X, double* 
 // coefficients in shared memory. Tables in shared memory (STAB) where they fit
 // beside the groups' 16-row buffers (three groups of four warps with TWIN, two
 // without: nphi up to 258), else their operand fragments from L2, stored in the
-// order the lanes read, eight warps on 32 rows (16 on the largest grids); there
-// TWIN gains nothing (2.98 against 2.86 ms at lmax 256).
+// order the lanes read, eight warps on 32 rows, CG = 4 column groups of them (16
+// rows past 16 column tiles, 514 columns; past 24, 770 columns, 8 rows and CG = 8,
+// up to lon_check's bound at about 1300 columns); there TWIN gains nothing (2.98
+// against 2.86 ms at lmax 256). The lines between the shapes are where the next
+// smaller one's accumulators or tables end; us at lmax 128 with 54 elements on
+// 258 | 260, 514 | 516 and 768 | 772 columns 434 | 622, 861 | 1261 and 1568 | 1721
+// (1024: 1978; the FMA kernel 1486 | 1483, 3422 | 3426, 4605 | 5495 and 6395).
 // Bound: at lmax 128, 54 elements 8.4 GFLOP, 230 us at the FP64 rate, and 518 MB,
 // 79 us. Measured 427 us, the products' pipe half busy: the copies, the
 // pointwise pass and the outputs of a group take as long as its products, and
@@ -783,7 +788,7 @@ struct LonPlan {
   int kss, ksa;         // four-term steps of the synthesis and the analysis
   int nts, nta;         // their 8-column tiles
   int PK, PT, TR;       // pitches of the buffer and of the tables, table rows
-  int G, MT, NW;        // shape (see above)
+  int G, CG, MT, NW;    // shape (see above)
   int twin, stab;
   size_t smem;
 };
@@ -804,6 +809,7 @@ static int lon_pitch(int n) {  // the next pitch of 4 or 12 mod 16 doubles: conf
 }
 
 constexpr size_t LON_SMEM_CTA = 226 * 1024;
+static int lon_rows(const LonPlan& P) { return 8 * P.MT * ((P.G == 1 ? 8 : 4) / P.CG); }  // of a group's tile
 
 static LonPlan lon_plan(const vg_handle* h) {
   const Grid& G = h->grid;
@@ -829,6 +835,7 @@ static LonPlan lon_plan(const vg_handle* h) {
     tab = (size_t)(twin ? 2 : 4) * P.TR * P.PT * sizeof(double);
     tile = 16 * (size_t)(4 * P.PK + 2) * sizeof(double) + 16;  // a group's 16-row buffer
   };
+  P.CG = 4;
   P.MT = 2;
   P.stab = 1;
   // TWIN where half is odd, the tables then fit and most of the half - m are orders carried
@@ -843,11 +850,12 @@ static LonPlan lon_plan(const vg_handle* h) {
       P.stab = 0;
       P.G = 1;
       P.MT = nt <= 16 ? 2 : 1;
+      P.CG = nt <= 24 ? 4 : 8;
     }
   }
   P.NW = P.stab ? (nt <= 4 ? 1 : 2) : nt <= 12 ? 3 : nt <= 16 ? 4 : 6;
-  P.smem = (P.stab ? tab : 0) + (P.G == 1 ? P.MT : P.G) * tile;
-  if (nt > 24 || P.smem > LON_SMEM_CTA) throw Error("visc3d: grid too large for the FP64 longitude pass");
+  P.smem = (P.stab ? tab : 0) + (P.G == 1 ? (lon_rows(P) + 15) / 16 : P.G) * tile;
+  if (nt > P.CG * P.NW || P.smem > LON_SMEM_CTA) throw Error("visc3d: grid too large for the FP64 longitude pass");
   return P;
 }
 
@@ -885,8 +893,8 @@ static void lon_plan_tables(vg_handle* h) {
 // the even and odd coefficients of a row fall in different banks
 __device__ __forceinline__ int lon_sum(int s4, int step) { return s4 * step + (s4 >> 1) * 2; }
 
-// the accumulator tiles of N column tiles t = ng + 4 i: C[mt][i][sum] += buf (rows) x table
-template <int MT, int NW, int N, bool STAB, bool TWIN, bool ANA>
+// the accumulator tiles of N column tiles t = ng + CG i: C[mt][i][sum] += buf (rows) x table
+template <int CG, int MT, int NW, int N, bool STAB, bool TWIN, bool ANA>
 __device__ __forceinline__ void lon_products(double2 (&C)[MT][NW][4], const double* a, int astep, int arow,
                                              const double* tab, int TS, int PT, const double* frag, int steps, int ng,
                                              int lane) {
@@ -895,7 +903,7 @@ __device__ __forceinline__ void lon_products(double2 (&C)[MT][NW][4], const doub
   auto load_b = [&](int ks, double (&b)[N][NS]) {
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      const int t = ng + 4 * i;
+      const int t = ng + CG * i;
 #pragma unroll
       for (int s4 = 0; s4 < NS; ++s4)
         b[i][s4] = STAB ? (ANA ? tab[s4 * TS + (8 * t + lr) * PT + 4 * ks + lk]
@@ -935,26 +943,26 @@ __device__ __forceinline__ void lon_products(double2 (&C)[MT][NW][4], const doub
 }
 
 // the same for a warp's n <= N column tiles (n differs between the warps)
-template <int MT, int NW, int N, bool STAB, bool TWIN, bool ANA>
+template <int CG, int MT, int NW, int N, bool STAB, bool TWIN, bool ANA>
 __device__ __forceinline__ void lon_products_n(int n, double2 (&C)[MT][NW][4], const double* a, int astep, int arow,
                                                const double* tab, int TS, int PT, const double* frag, int steps,
                                                int ng, int lane) {
   if constexpr (N > 0) {
     if (n == N)
-      lon_products<MT, NW, N, STAB, TWIN, ANA>(C, a, astep, arow, tab, TS, PT, frag, steps, ng, lane);
+      lon_products<CG, MT, NW, N, STAB, TWIN, ANA>(C, a, astep, arow, tab, TS, PT, frag, steps, ng, lane);
     else
-      lon_products_n<MT, NW, N - 1, STAB, TWIN, ANA>(n, C, a, astep, arow, tab, TS, PT, frag, steps, ng, lane);
+      lon_products_n<CG, MT, NW, N - 1, STAB, TWIN, ANA>(n, C, a, astep, arow, tab, TS, PT, frag, steps, ng, lane);
   }
 }
 
-template <int G, int MT, int NW, bool STAB, bool TWIN, bool TOR>
+template <int G, int CG, int MT, int NW, bool STAB, bool TWIN, bool TOR>
 __global__ void __launch_bounds__(G == 3 ? 384 : 256, 1) k_v3_lon(const __grid_constant__ LonArgs A) {
-  constexpr int GW = G == 1 ? 8 : 4, NMP = GW / 4, ROWS = 8 * MT * NMP, GT = 32 * GW, NQ = TOR ? 10 : 6;
+  constexpr int GW = G == 1 ? 8 : 4, NMP = GW / CG, ROWS = 8 * MT * NMP, GT = 32 * GW, NQ = TOR ? 10 : 6;
   constexpr int RG = ROWS / 4, MSTEP = GW / RG;  // staging: groups of four rows, warps on the same group
   extern __shared__ __align__(16) double lsm[];
   const LonPlan& P = A.P;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, lk = lane & 3;
-  const int g = warp / GW, wg = warp % GW, ng = wg & 3, mp = wg >> 2, tg = tid % GT;
+  const int g = warp / GW, wg = warp % GW, ng = wg % CG, mp = wg / CG, tg = tid % GT;
   const int PK = P.PK, PT = P.PT, TS = P.TR * P.PT, half = P.half, nphi = A.nphi, M = P.M;
   const double* tab = STAB ? lsm : A.TM;
   if (STAB) {
@@ -991,7 +999,7 @@ __global__ void __launch_bounds__(G == 3 ? 384 : 256, 1) k_v3_lon(const __grid_c
       const ptrdiff_t part = TOR ? (ptrdiff_t)2 * A.nf * (q == 5 ? 3 : 5) : 0;  // 1 -> 6, 2 -> 7, 4 -> 9, 5 -> 8
       const bool has = TOR && live && (q == 1 || q == 2 || q >= 4);
       double* d = buf + r * PK;
-      constexpr int NB = 9 * NW;  // loads in flight together: a whole tile's of the first shape
+      constexpr int NB = CG == 4 ? 9 * NW : 12;  // loads in flight together: a whole tile's of the first shape
       for (int m0 = wg / RG; m0 < nmb; m0 += NB * MSTEP) {
         double2 z[NB];
 #pragma unroll
@@ -1058,7 +1066,7 @@ __global__ void __launch_bounds__(G == 3 ? 384 : 256, 1) k_v3_lon(const __grid_c
         C[mt][i][1] = C[mt][i][2] = C[mt][i][3] = make_double2(0.0, 0.0);
       }
     }
-    lon_products_n<MT, NW, NW, STAB, TWIN, false>((P.nts - ng + 3) >> 2, C, afrag, BS, PK, tab, TS, PT, A.FS, P.kss, ng, lane);
+    lon_products_n<CG, MT, NW, NW, STAB, TWIN, false>((P.nts - ng + CG - 1) / CG, C, afrag, BS, PK, tab, TS, PT, A.FS, P.kss, ng, lane);
     auto row_of = [&](int r) {
       const int row = row0 + r, q = row / A.nf, f = row - q * A.nf;
       return Row{row < nrow, q, A.rate + ((size_t)(f / 3) * A.nlat + j) * nphi,
@@ -1117,13 +1125,13 @@ __global__ void __launch_bounds__(G == 3 ? 384 : 256, 1) k_v3_lon(const __grid_c
       double n[NW][2][4];
 #pragma unroll
       for (int i = 0; i < NW; ++i) {
-        const int lon = 8 * (ng + 4 * i) + 2 * lk + 1;
+        const int lon = 8 * (ng + CG * i) + 2 * lk + 1;
         rates(R, lon, n[i][0]);
         rates(R, lon + 1, n[i][1]);
       }
 #pragma unroll
       for (int i = 0; i < NW; ++i) {
-        const int t = ng + 4 * i, lon = 8 * t + 2 * lk + 1;
+        const int t = ng + CG * i, lon = 8 * t + 2 * lk + 1;
         if (t >= P.nts) continue;
         double o0[4], o1[4];
         // TWIN: (-1)^i on the odd cosine sums, -(-1)^i on the odd sine sums; lon is odd, lon + 1 even
@@ -1159,7 +1167,7 @@ __global__ void __launch_bounds__(G == 3 ? 384 : 256, 1) k_v3_lon(const __grid_c
         C[mt][i][1] = C[mt][i][3] = make_double2(0.0, 0.0);
       }
     }
-    lon_products_n<MT, NW, NW, STAB, TWIN, true>((P.nta - ng + 3) >> 2, C, afrag, BS, PK, tab, TS, PT, A.FA, P.ksa, ng, lane);
+    lon_products_n<CG, MT, NW, NW, STAB, TWIN, true>((P.nta - ng + CG - 1) / CG, C, afrag, BS, PK, tab, TS, PT, A.FA, P.ksa, ng, lane);
     x0 = xk == 0 && xq == 0 ? z0[xr] : 0.0;  // m = 0: the sum over the row
     {
       const double* ar = buf + xr * PK;
@@ -1186,7 +1194,7 @@ __global__ void __launch_bounds__(G == 3 ? 384 : 256, 1) k_v3_lon(const __grid_c
       double* o0 = Sj + 2 * (row0 + rw + 8 * mt);
 #pragma unroll
       for (int i = 0; i < NW; ++i) {
-        const int t = ng + 4 * i, m = 2 * (8 * t + 2 * lk);
+        const int t = ng + CG * i, m = 2 * (8 * t + 2 * lk);
         if (t >= P.nta) continue;
         emit(R, o0, TWIN ? half - m - 2 : m + 1, C[mt][i][2].x, C[mt][i][3].x);
         emit(R, o0, m + 2, C[mt][i][0].x, C[mt][i][1].x);
@@ -1201,21 +1209,22 @@ __global__ void __launch_bounds__(G == 3 ? 384 : 256, 1) k_v3_lon(const __grid_c
 static void launch_lon(vg_handle* h, LonArgs A) {
   const bool tor = h->tor_on;
   void (*k)(const LonArgs) = nullptr;
-#define VG_LON(G_, MT_, NW_, ST_, TW_)                                                                             \
-  if (A.P.G == G_ && A.P.MT == MT_ && A.P.NW == NW_ && A.P.stab == ST_ && A.P.twin == TW_)                           \
-  k = tor ? k_v3_lon<G_, MT_, NW_, ST_ != 0, TW_ != 0, true> : k_v3_lon<G_, MT_, NW_, ST_ != 0, TW_ != 0, false>
-  VG_LON(3, 2, 1, 1, 1);
-  VG_LON(3, 2, 2, 1, 1);
-  VG_LON(2, 2, 1, 1, 0);
-  VG_LON(2, 2, 2, 1, 0);
-  VG_LON(1, 2, 3, 0, 0);
-  VG_LON(1, 2, 4, 0, 0);
-  VG_LON(1, 1, 6, 0, 0);
+#define VG_LON(G_, CG_, MT_, NW_, ST_, TW_)                                                                       \
+  if (A.P.G == G_ && A.P.CG == CG_ && A.P.MT == MT_ && A.P.NW == NW_ && A.P.stab == ST_ && A.P.twin == TW_)          \
+  k = tor ? k_v3_lon<G_, CG_, MT_, NW_, ST_ != 0, TW_ != 0, true> : k_v3_lon<G_, CG_, MT_, NW_, ST_ != 0, TW_ != 0, false>
+  VG_LON(3, 4, 2, 1, 1, 1);
+  VG_LON(3, 4, 2, 2, 1, 1);
+  VG_LON(2, 4, 2, 1, 1, 0);
+  VG_LON(2, 4, 2, 2, 1, 0);
+  VG_LON(1, 4, 2, 3, 0, 0);
+  VG_LON(1, 4, 2, 4, 0, 0);
+  VG_LON(1, 4, 1, 6, 0, 0);
+  VG_LON(1, 8, 1, 6, 0, 0);
 #undef VG_LON
   raise_smem_limit((const void*)k, A.P.smem);
   int nsm = 0;
   VG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
-  const int rows = A.P.G == 1 ? 16 * A.P.MT : 16;
+  const int rows = lon_rows(A.P);
   const long long tiles = (long long)A.nlat * ((6 * A.nf + rows - 1) / rows);
   k<<<(unsigned)std::min((tiles + A.P.G - 1) / A.P.G, (long long)nsm), A.P.G == 3 ? 384 : 256, A.P.smem, h->stream>>>(A);
   ++h->n_launch;
