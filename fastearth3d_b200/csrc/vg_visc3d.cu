@@ -1250,8 +1250,8 @@ static int lon_threads(const vg_handle* h, int LF) {
 constexpr size_t LON_SMEM_MAX = 220 * 1024;
 static void lon_attributes();  // the longitude kernels' shared-memory limit (defined after the transpose)
 
-static void lon_check(const vg_handle* h) {
-  if (lon_smem(h, LON_LF, true) > LON_SMEM_MAX || (h->tor_on && lon_smem(h, LON_LF_TOR, false, 10) > LON_SMEM_MAX))
+static void lon_check(const vg_handle* h, bool tor) {
+  if (lon_smem(h, LON_LF, true) > LON_SMEM_MAX || (tor && lon_smem(h, LON_LF_TOR, false, 10) > LON_SMEM_MAX))
     throw Error("visc3d: grid too large for the FP64 longitude pass");
 }
 
@@ -1407,6 +1407,35 @@ static void v3_tile_attributes() {
 
 // ------------------------------------------------------------------ host
 
+// A lateral viscosity that is refused on the way (a grid too large, no memory) leaves
+// the handle's earth laterally uniform, as it was.
+struct EnableGuard {
+  vg_handle* h;
+  std::vector<double> MkPerDt;
+  std::vector<char> active1d;
+  double max_rate;
+  bool done = false;
+  explicit EnableGuard(vg_handle* hh)
+      : h(hh), MkPerDt(hh->MkPerDt), active1d(hh->active1d_h), max_rate(hh->max_rate) {}
+  ~EnableGuard() {  // never throws
+    if (done) return;
+    cudaStreamSynchronize(h->stream);
+    h->MkPerDt = MkPerDt;
+    h->active1d_h = active1d;
+    h->max_rate = max_rate;
+    h->e3d_h.clear();
+    h->pert_mean3d.clear();
+    h->ne3d = 0;
+    h->lat_visc = h->tor_on = false;
+    if (h->tc_plan_release) h->tc_plan_release(h->tc_plan);
+    h->tc_plan = nullptr;
+    h->tc_plan_release = nullptr;
+    cudaMemcpyAsync(h->d_MkPerDt.p, MkPerDt.data(), MkPerDt.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream);
+    cudaMemcpyAsync(h->d_active1d.p, active1d.data(), active1d.size(), cudaMemcpyHostToDevice, h->stream);
+    cudaStreamSynchronize(h->stream);
+  }
+};
+
 void visc3d_enable(vg_handle* h, const double* pert) {
   const Grid& G = h->grid;
   const int ne = h->ne, ng = G.ng;
@@ -1418,6 +1447,7 @@ void visc3d_enable(vg_handle* h, const double* pert) {
                 "(toroidal = 1 needs visc3d_precision = VG_VISC3D_FP64 or VG_VISC3D_EXACT_TC)");
   // Maxwell-CFL rate: the grid maximum of mu/eta_eff over every Maxwell element
   // (src/vilma_response.f90:1783-1793, MkPerDt3 covers all elements)
+  EnableGuard guard(h);
   double rate_max = 0.0;
   for (int e = 0; e < ne; ++e) {
     if (h->MkPerDt[e] == 0.0) continue;
@@ -1453,10 +1483,17 @@ void visc3d_enable(vg_handle* h, const double* pert) {
   h->ne3d = (int)h->e3d_h.size();
   h->max_rate = rate_max;
   for (double v : h->MkPerDt) h->max_rate = std::max(h->max_rate, v);
+  if (h->ne3d > 0 && h->p.visc3d_precision == VG_VISC3D_FP64) {  // the grid fits the longitude pass, or they throw
+    lon_plan(h);
+    lon_check(h, h->p.toroidal != 0);
+  }
   h->d_MkPerDt.upload(h->MkPerDt, s);
   h->d_active1d.upload(h->active1d_h, s);
   h->lat_visc = true;
-  if (h->ne3d == 0) return;
+  if (h->ne3d == 0) {
+    guard.done = true;
+    return;
+  }
   h->d_e3d.upload(h->e3d_h, s);
   h->d_MkPerDt3.upload(rate3, s);
   // tables
@@ -1478,10 +1515,12 @@ void visc3d_enable(vg_handle* h, const double* pert) {
   if (h->p.toroidal) toroidal_enable(h);
   if (h->p.visc3d_precision == VG_VISC3D_SPLIT_TC) {
     visc3d_tc_enable(h);
+    guard.done = true;
     return;
   }
   if (h->p.visc3d_precision == VG_VISC3D_EXACT_TC) {
     visc3d_oz_enable(h);
+    guard.done = true;
     return;
   }
   // work buffers and longitude tables of the FP64 path
@@ -1491,9 +1530,9 @@ void visc3d_enable(vg_handle* h, const double* pert) {
   h->d_dy.alloc((size_t)(h->nk + 1) * np * ncf);
   lon_tables_build(h);
   lon_plan_tables(h);
-  lon_check(h);  // the grid fits the longitude pass (throws otherwise)
   lon_attributes();
   VG_CUDA(cudaStreamSynchronize(s));
+  guard.done = true;
 }
 
 void visc3d_advance(vg_handle* h, const double* d_sigma, double dt, const double* dUn, const double* dVn,

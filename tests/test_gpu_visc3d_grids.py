@@ -1,7 +1,7 @@
 """The FP64 3-D step on grids with many more columns than the transform needs:
 column counts at the edges of the path's shapes and up to its limit, with and without the
 toroidal channels; GPU = oracle to 1e-10 (response) and 1e-8 (memory) as in
-test_gpu_parity.py."""
+test_gpu_parity.py. A grid past the limit is refused, and the handle is then as it was."""
 import numpy as np
 import pytest
 
@@ -93,3 +93,11 @@ def test_gradient_on_a_wide_grid():
         fd = (g.misfit(sigma + h * d, dt, sites, obs) - g.misfit(sigma - h * d, dt, sites, obs)) / (2 * h)
         t = gr.real * d.real + gr.imag * d.imag
         assert abs(fd - t.sum()) <= 1e-6 * max(abs(fd), np.sqrt((t**2).sum()))
+
+def test_refused_grid_leaves_the_handle_as_it_was():
+    g, o = pair(8, 9, 1400)
+    for _ in range(2):  # the second time for the same reason
+        with pytest.raises(vlib.VilmaError, match="grid too large"):
+            g.enable_visc3d(pert(g))
+    assert g.info().ne3d == 0
+    compare(g, o)  # the laterally uniform earth, as without the call
