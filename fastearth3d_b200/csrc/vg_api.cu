@@ -142,6 +142,7 @@ int vg_create(const vg_params* p, vg_handle** out) {
     int ndev = 0;
     VG_CUDA(cudaGetDevice(&h->device));
     VG_CUDA(cudaGetDeviceCount(&ndev));
+    VG_CUDA(cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->device));
     VG_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     VG_CUDA(cudaStreamCreateWithFlags(&h->aux, cudaStreamNonBlocking));
     VG_CUDA(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));

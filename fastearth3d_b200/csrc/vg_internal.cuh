@@ -128,7 +128,7 @@ struct Grid {
 struct vg_handle {
   vg_params p;
   std::string err;
-  int device = 0;
+  int device = 0, nsm = 0;  // and its SMs
   // bound on the device-side waits that hand work between CTAs or warps (grid
   // barriers of the fused sea-level loop, producer / consumer waits of the
   // tensor-core stages); a wait that runs out raises a status the host turns

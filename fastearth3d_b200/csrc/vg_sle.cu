@@ -465,10 +465,9 @@ __global__ void k_mass(SleScalars* sc, const double* __restrict__ rowpart, const
 void pass_plan(vg_handle* h, const void* const kernel[4]) {
   if (h->sle_grid != 0) return;
   const Grid& G = h->grid;
-  int dev = 0, nsm = 0, lim = 0;
-  VG_CUDA(cudaGetDevice(&dev));
-  VG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  VG_CUDA(cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  const int nsm = h->nsm;
+  int lim = 0;
+  VG_CUDA(cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
   cudaFuncAttributes fa;
   VG_CUDA(cudaFuncGetAttributes(&fa, kernel[0]));
   const size_t room = (size_t)lim - fa.sharedSizeBytes, psz = (size_t)(p_pitch((G.nlat + 1) / 2) + 6) * (G.lmax + 1);

@@ -141,10 +141,7 @@ void autotune(vg_handle* h, double dt_yr, int knobs, const char* cache_path, int
   apply(h, best);
   // the fused sea-level loop's CTA count (only when the model has an ocean to solve for)
   if (!h->p.sle_fixed_ocean && (knobs & VG_TUNE_SLE)) {
-    int dev = 0, nsm = 0;
-    VG_CUDA(cudaGetDevice(&dev));
-    VG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const int cands[3] = {0, h->grid.nlat, 2 * nsm};  // 0: one per SM; the launch caps at what fits
+    const int cands[3] = {0, h->grid.nlat, 2 * h->nsm};  // 0: one per SM; the launch caps at what fits
     double t_best = -1.0;
     int c_best = best.sle_ctas;
     for (int c : cands) {

@@ -502,12 +502,12 @@ static void launch_gemm(vg_handle* h, GemmArgs A, int mode) {
   const int rows = mode == 0 ? (G.nlat + 1) / 2 : (G.lmax + 2) / 2;
   const int rtiles = (rows + GB_RT - 1) / GB_RT;
   A.rt = ((rows + rtiles - 1) / rtiles + 7) / 8 * 8;
-  // a CTA keeps its pipeline running over as many products as leave enough
-  // CTAs to fill the chip twice
+  // a CTA keeps its pipeline running over as many products as leave more CTAs
+  // than the chip holds at once (three an SM)
   const int ct = (A.ncf + GB_N - 1) / GB_N, base = ct * rtiles * G.M;
   A.pg = 1;
   for (int d = A.np; d > 1; --d)
-    if (A.np % d == 0 && base * (A.np / d) >= 4 * 148) {
+    if (A.np % d == 0 && base * (A.np / d) >= 4 * h->nsm) {
       A.pg = d;
       break;
     }
@@ -1222,11 +1222,9 @@ static void launch_lon(vg_handle* h, LonArgs A) {
   VG_LON(1, 8, 1, 6, 0, 0);
 #undef VG_LON
   raise_smem_limit((const void*)k, A.P.smem);
-  int nsm = 0;
-  VG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
   const int rows = lon_rows(A.P);
   const long long tiles = (long long)A.nlat * ((6 * A.nf + rows - 1) / rows);
-  k<<<(unsigned)std::min((tiles + A.P.G - 1) / A.P.G, (long long)nsm), A.P.G == 3 ? 384 : 256, A.P.smem, h->stream>>>(A);
+  k<<<(unsigned)std::min((tiles + A.P.G - 1) / A.P.G, (long long)h->nsm), A.P.G == 3 ? 384 : 256, A.P.smem, h->stream>>>(A);
   ++h->n_launch;
   VG_CUDA(cudaGetLastError());
 }
