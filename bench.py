@@ -60,7 +60,7 @@ def parse():
     ap.add_argument("--tf32", default="on", choices=["on", "off"],
                     help="also time the two-term TF32 tensor-core arm beside the exact one (with its rsl error)")
     ap.add_argument("--ensemble-sle-ctas", default="rows", choices=["sm", "rows", "tuned"],
-                    help="c4_ensemble: the fused sea-level loop's CTAs per instance (one per SM, one per grid row, "
+                    help="c4_ensemble: the fused sea-level pass's CTAs per instance (one per SM, one per grid row, "
                          "or the autotuner's choice, which also picks the exact stages' warp splits)")
     ap.add_argument("--toroidal", default="on", choices=["on", "off", "only"],
                     help="also time the FP64 path carrying the toroidal channels (toroidal = 1); "
@@ -534,8 +534,10 @@ def run_ensemble(args):
     def make(mb, split):
         p = mb.params(vlib.default_params)
         p.visc3d_precision = PRECISION[args.precision] if (split and mb.visc3d) else 0
-        if args.ensemble_sle_ctas == "rows":  # the fused sea-level loop on one CTA per grid row at most
+        if args.ensemble_sle_ctas == "rows":  # the fused sea-level pass on one CTA per grid row at most
             p.sle_ctas = mb.nlat
+        elif args.ensemble_sle_ctas == "sm":
+            p.sle_ctas = torch.cuda.get_device_properties(0).multi_processor_count
         m = vlib.Model(p)
         zb, hi = mb.reference()
         m.set_reference(zb, hi)

@@ -220,7 +220,7 @@ struct vg_handle {
   vg::DArr<double> d_rowpart;  // per-row partial results (9 * nlat)
   vg::DArr<unsigned int> d_end_count;  // rows that k_step_end has finished
   vg::DArr<unsigned int> d_gbar;  // grid barrier of the fused pass: arrivals, finished CTAs, error
-  int sle_grid = 0;               // CTAs of the cooperative launch of the pass (one per SM)
+  int sle_grid = 0;               // CTAs of the cooperative launch of the pass (0: not planned)
   // counters
   long long n_accept = 0, n_reject = 0, n_solve = 0, n_drift_solved = 0;
   int n_sub_last = 0, n_outer_last = 0, n_inner_last = 0, n_flip_last = 0;
@@ -266,7 +266,6 @@ void build_grid(Grid& G, int lmax, int nlat, int nphi, cudaStream_t s);
 // drift of memory buffer buf (-1: the current one) into the nodal targets
 // (nullptr: the handle's dUn, dVn) and the surface drift
 void launch_drift(vg_handle* h, int buf = -1, double* dUn = nullptr, double* dVn = nullptr, double* dWn = nullptr);
-// the same without the toroidal drift, on stream s
 // memory advance of one step (3-D elements pseudo-spectrally, the others per
 // slot), current buffer -> the other one, with the strain of (sigma, dUn,
 // dVn) (nullptr: the handle's drift), and the next buffer's per-slot norms and

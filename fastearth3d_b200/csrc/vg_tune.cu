@@ -6,8 +6,8 @@
 //   * the exact tensor-core stages' split of their 16 worker warps between
 //     converters (FP64 rows to digit planes) and epilogue (level
 //     combination, scaling, stores): 8 : 8 or 4 : 12, per stage;
-//   * the CTA count of the fused sea-level loop's cooperative grid: one per
-//     SM, one per Gauss row, or two per SM where they fit.
+//   * the CTA count of the fused sea-level pass's cooperative grid: one per
+//     order or Gauss row (the default), or one per SM, which is all that fits.
 // Each candidate runs a few whole intervals of the handle's own model on the
 // ice it holds, timed per phase by the handle's phase timers, from the same
 // saved driver state (put back after every trial and at the end). The best
@@ -139,9 +139,9 @@ void autotune(vg_handle* h, double dt_yr, int knobs, const char* cache_path, int
     }
   }
   apply(h, best);
-  // the fused sea-level loop's CTA count (only when the model has an ocean to solve for)
+  // the fused sea-level pass's CTA count (only when the model has an ocean to solve for)
   if (!h->p.sle_fixed_ocean && (knobs & VG_TUNE_SLE)) {
-    const int cands[3] = {0, h->grid.nlat, 2 * h->nsm};  // 0: one per SM; the launch caps at what fits
+    const int cands[2] = {0, h->nsm};  // 0: as many as orders or rows, at most one per SM
     double t_best = -1.0;
     int c_best = best.sle_ctas;
     for (int c : cands) {
