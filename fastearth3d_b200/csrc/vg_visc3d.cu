@@ -540,8 +540,8 @@ static void gemm_tables(const vg_handle* h, GemmArgs& A, bool weighted) {
 
 // ------------------------------------------------------------------ longitude
 
-// The longitude transforms of the FP64 path as register-tiled real DFT
-// contractions over dense twiddle tables, split by the parity of m
+// The longitude transforms of the transposed pass (k_v3_lon_T) as register-tiled
+// real DFT contractions over dense twiddle tables, split by the parity of m
 // (phi_{i + half} = phi_i + pi flips the odd orders):
 //   synthesis  E(r, i) = sum_{m even} A(r, 2m) cos(m phi_i) - A(r, 2m+1) sin(m phi_i),
 //              O(r, i) the same over odd m; g(i) = E + O, g(i + half) = E - O
@@ -574,6 +574,7 @@ static LonTables lon_tables(const vg_handle* h) {
   return T;
 }
 
+// (at a handle's first transposed pass: a model that takes no gradient needs none)
 static void lon_tables_build(vg_handle* h) {
   const Grid& G = h->grid;
   const LonTables T = lon_tables(h);
@@ -595,9 +596,10 @@ static void lon_tables_build(vg_handle* h) {
     }
   h->d_lon_tw.upload(tw, h->stream);
   h->d_lon_twt.upload(twt, h->stream);
+  VG_CUDA(cudaStreamSynchronize(h->stream));
 }
 
-// synthesis tiles over A (shared, [6 nfl][2 M2], row 6 fl + c): for each
+// synthesis tiles of the transposed pass over A (shared, [6 nfl][2 M2], row 6 fl + c): for each
 // (field fl, longitude i < half) calls epi(fl, i, g(i), g(i + half)) with the
 // six components' values
 template <class Epi>
@@ -701,8 +703,8 @@ __host__ __device__ __forceinline__ size_t lon_areg(int LF, const LonTables& T) 
 }
 
 constexpr int LON_THREADS = 384;
-constexpr int LON_LF = 3;  // fields per CTA: one element's three shape coefficients (two CTAs per SM)
-constexpr int LON_LF_TOR = 3;  // with the toroidal channels: staged in two halves, two CTAs per SM
+constexpr int LON_LF = 3;  // fields per CTA: one element's three shape coefficients
+constexpr int LON_LF_TOR = 3;  // with the toroidal channels: staged in two halves
 
 // the CTA's slice of the products S[m, j][q][f][ri] (fields f0 .. f0 + nft - 1,
 // a contiguous run of 2 nft doubles per (m, q)) to and from shared [m][q][2 nft]
@@ -1229,9 +1231,10 @@ static void launch_lon(vg_handle* h, LonArgs A) {
   VG_CUDA(cudaGetLastError());
 }
 
-// shared memory of the longitude pass (forward: adj = 0) and its transpose;
-// nq analysis inputs (10 with the toroidal channels, staged through the
-// coefficient region, which then grows to hold them)
+// shared memory of the transposed pass (adj = 0: without its per-field sums, which
+// bounds the grids of the toroidal channels); nq analysis inputs (10 with the
+// toroidal channels, staged through the coefficient region, which then grows to
+// hold them)
 static size_t lon_smem(const vg_handle* h, int LF, bool adj, int nq = 6) {
   const LonTables T = lon_tables(h);
   const int nphi = h->grid.nphi;
@@ -1526,7 +1529,6 @@ void visc3d_enable(vg_handle* h, const double* pert) {
   h->d_X.alloc((size_t)(h->nk + 1) * nch * ncf);
   h->d_Y.alloc(s_rows(G.M, G.nlat) * np * ncf);
   h->d_dy.alloc((size_t)(h->nk + 1) * np * ncf);
-  lon_tables_build(h);
   lon_plan_tables(h);
   lon_attributes();
   VG_CUDA(cudaStreamSynchronize(s));
@@ -1924,6 +1926,7 @@ void visc3d_adjoint(vg_handle* h, const double* gstore, double dt, const double*
     h->d_v3a_Yb.alloc(ny);
     h->d_v3a_dyb.alloc(nr6);  // slot row nk (degree 0) stays zero
     h->d_v3a_Rb.alloc(nr6);
+    lon_tables_build(h);
   }
   V3Args A;
   A.mem = h->d_mem[h->cur].p;
