@@ -306,13 +306,13 @@ __global__ void __launch_bounds__(256) k_rhs_T(int ne, int nr, int nd, int nk, c
   rhs_T(K + ((size_t)l * ne + e) * 48, fb, lam_new, ri, e, k, ne, nk);
 }
 
-// G1T[c][r] = G1[r][c] (degree-1 Green's block, rows r < nrow, columns c < ncol)
 // d J / d pert = scale * rate * d J / d (M dt), in place (scale = -ln 10 dt)
 __global__ void k_grad_pert(size_t n, double scale, const double* __restrict__ rate, double* __restrict__ g) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n) g[t] *= scale * rate[t];
 }
 
+// AT[c][r] = A[r][c] (the degree-1 Green's block, rows r < nrow, columns c < ncol)
 __global__ void k_transpose(int nrow, int ncol, const double* __restrict__ A, double* __restrict__ AT) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nrow * ncol) return;

@@ -94,8 +94,8 @@ struct DArr {
 // read back as one small struct when the host needs a decision.
 struct SleScalars {
   double C_int, ice_int, zeta_int, Cs_int, dphi, dmax, smax, mass_Cs;
-  int flips, n_inner;  // coastline flips; inner iterations done by the fused loop
-  int bar_error;       // a grid barrier of the fused loop gave up
+  int flips, n_inner;  // coastline flips; inner iterations done by the fused pass
+  int bar_error;       // a grid barrier of the fused pass gave up
   unsigned long long mem_norm_bits;  // max |memory| of the state the last advance wrote
   unsigned long long stage_status;   // status bits of its tensor-core stages
   double bsl;                        // barystatic sea level at the end of the interval
@@ -130,7 +130,7 @@ struct vg_handle {
   std::string err;
   int device = 0, nsm = 0;  // and its SMs
   // bound on the device-side waits that hand work between CTAs or warps (grid
-  // barriers of the fused sea-level loop, producer / consumer waits of the
+  // barriers of the fused sea-level pass, producer / consumer waits of the
   // tensor-core stages); a wait that runs out raises a status the host turns
   // into an error (vg_set_wait_limit)
   unsigned long long wait_ns = 2000000000ull;

@@ -74,7 +74,7 @@ void apply(vg_handle* h, const Choice& c) {
   if (oz_get_ncw(h, cur)) oz_set_ncw(h, c.ncw);
   if (h->p.sle_ctas != c.sle_ctas) {
     h->p.sle_ctas = c.sle_ctas;
-    h->sle_grid = 0;  // the fused loop's grid is sized again at its next launch
+    h->sle_grid = 0;  // the fused pass's grid is sized again at its next launch
   }
 }
 

@@ -101,10 +101,10 @@ struct V3Args {
   int tor_swap = 0;
 };
 
-// one thread per (slot k, 3-D element): strain of both histories, 24 values,
-// written as X[k][ch][f][ri] (FP64, or FP32 for the tensor-core stages)
-// Blocks of 32 slots x 8 3-D elements. The memory and drift are read along
-// the slot index (coalesced); the operand rows X[k][ch][f][ri] are written
+// One thread per (slot k, 3-D element): memory plus 2 mu strain, 24 values, as
+// operand rows X[k][ch][f][ri] (FP64, or FP32 for the tensor-core stages), in
+// blocks of 32 slots x 8 3-D elements. The memory and drift are read along the
+// slot index (coalesced); the rows are written
 // through a shared tile [ch][f in block][slot] so that each (slot, channel)
 // row's 6 x 8 entries go out as one contiguous run. Neighbouring blocks share the
 // rows (the element blocks run fastest). Bound by HBM: the memory and drift in, X
@@ -1265,7 +1265,8 @@ static void lon_check(const vg_handle* h, bool tor) {
 // the memory along the slots, so the rows come in as contiguous runs through a
 // shared tile. Bound by HBM (the memory in and out and the rows once); read by
 // its own thread, each (re, im) pair took a sector of its own: 99 us at lmax 128
-// with 54 3-D elements of 100, 50 now (floor 46).
+// with 54 3-D elements of 100, 50 now (floor 46). The normalisations multiply by
+// 1 / J and 1 / n6, one rounding more than a division.
 template <class V, int NQ, int TE>
 __device__ __forceinline__ double v3_scatter_one(const V3Args& A, const V* tile, const double (&old)[3][2][4],
                                                  const double* __restrict__ n6, int k, int ei) {
