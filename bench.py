@@ -115,46 +115,51 @@ def peaks():
 
 
 class ClockSampler:
-    """nvidia-smi clocks/throttle reasons sampled every 200 ms during the timed region."""
+    """SM clock and throttle reasons during the timed region, read through NVML every 10 ms (a program of its own takes
+    longer to start than a short region lasts)."""
 
-    Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
-         "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
-         "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
+    REASONS = {"hw_slowdown": 0x8, "hw_thermal_slowdown": 0x40, "sw_thermal_slowdown": 0x20, "sw_power_cap": 0x4}
 
     def __init__(self, index):
-        self.index, self.rows, self.proc = index, [], None
-
-    def __enter__(self):
+        self.rows, self.max, self.stop = [], None, threading.Event()
         try:
-            self.proc = subprocess.Popen(
-                ["nvidia-smi", "-i", str(self.index), f"--query-gpu={self.Q}", "--format=csv,noheader,nounits",
-                 "-lms", "200"], stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
-            self.t = threading.Thread(target=self._read, daemon=True)
-            self.t.start()
+            import pynvml as nv
+
+            nv.nvmlInit()
+            self.nv, self.dev = nv, nv.nvmlDeviceGetHandleByIndex(index)
+            self.max = nv.nvmlDeviceGetMaxClockInfo(self.dev, nv.NVML_CLOCK_SM)
+            self._sample()  # whether these queries are answered here
+            self.rows.clear()
         except Exception:
-            self.proc = None
-        return self
+            self.nv = None
+
+    def _sample(self):
+        self.rows.append((self.nv.nvmlDeviceGetClockInfo(self.dev, self.nv.NVML_CLOCK_SM),
+                          self.nv.nvmlDeviceGetCurrentClocksEventReasons(self.dev)))
 
     def _read(self):
-        for line in self.proc.stdout:
-            self.rows.append([x.strip() for x in line.split(",")])
+        try:
+            while not self.stop.wait(0.01):
+                self._sample()
+        except Exception:
+            pass  # what was sampled stays
+
+    def __enter__(self):
+        if self.nv:
+            self.t = threading.Thread(target=self._read, daemon=True)
+            self.t.start()
+        return self
 
     def __exit__(self, *a):
-        if self.proc:
-            self.proc.terminate()
-            try:
-                self.proc.wait(timeout=5)
-            except Exception:
-                self.proc.kill()
+        if self.nv:
+            self.stop.set()
+            self.t.join()
 
     def summary(self):
         if not self.rows:
             return {"sm_mhz": None, "sm_max_mhz": None, "reasons": ["unsampled"]}
-        sm = [float(r[1]) for r in self.rows if r[1].replace(".", "").isdigit()]
-        mx = [float(r[2]) for r in self.rows if r[2].replace(".", "").isdigit()]
-        names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
-        reasons = sorted({names[i] for r in self.rows for i in range(4) if len(r) > 5 + i and r[5 + i] == "Active"})
-        return {"sm_mhz": float(np.median(sm)) if sm else None, "sm_max_mhz": max(mx) if mx else None,
+        reasons = sorted(n for n, bit in self.REASONS.items() if any(r & bit for _, r in self.rows))
+        return {"sm_mhz": float(np.median([c for c, _ in self.rows])), "sm_max_mhz": float(self.max),
                 "reasons": reasons, "samples": len(self.rows)}
 
 
