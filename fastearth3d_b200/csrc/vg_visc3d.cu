@@ -18,8 +18,8 @@
 // With the toroidal channels carried (lambda 3, 4 as channels 4, 5) the
 // gather adds two channels, the synthesis four products (P.X4, D.X4, G.X5,
 // H.X5: rt -= i (m/sin) P.X4, rp += D.X4, Z4 = G e_tp - H (e_tt - e_pp)), the
-// longitude pass four analysis inputs (RP, m/sin RT, TP, TT - PP) and the
-// analysis four quadratures (wD, wP, wG, wH), normalised by 1/J and 1/n4 with
+// longitude pass four analysis inputs (m/sin RT, RP, TP, TT - PP) and the
+// analysis four quadratures (wP, wD, wG, wH), normalised by 1/J and 1/n4 with
 // n4 = n6 / 4 (src/vilma_tensor_sh.f90:168-203, 231-242, 270-322, 360-387).
 // G and H are the spin-2 kernels of Z6 written through P and dP/dtheta:
 //   G = -2 cot dP - l(l+1) P + 2 m^2/sin^2 P,   H = (m/sin)(dP - cot P)
@@ -773,8 +773,8 @@ __device__ __forceinline__ void stage_out(const double* __restrict__ X, double* 
 // without: nphi up to 258), else their operand fragments from L2, stored in the
 // order the lanes read, eight warps on 32 rows, CG = 4 column groups of them (16
 // rows past 16 column tiles, 514 columns; past 24, 770 columns, 8 rows and CG = 8,
-// up to lon_check's bound at about 1300 columns); there TWIN gains nothing (2.98
-// against 2.86 ms at lmax 256). The lines between the shapes are where the next
+// up to lon_check's bound, 1118 columns at lmax 128); there TWIN gains nothing
+// (2.98 against 2.86 ms at lmax 256). The lines between the shapes are where the next
 // smaller one's accumulators or tables end; us at lmax 128 with 54 elements on
 // 258 | 260, 514 | 516 and 768 | 772 columns 434 | 622, 861 | 1261 and 1568 | 1721
 // (1024: 1978; the FMA kernel 1486 | 1483, 3422 | 3426, 4605 | 5495 and 6395).
