@@ -179,9 +179,10 @@ __global__ void k_fourier_synth_long(const double2* __restrict__ G, int nphi, in
 
 void fourier_analysis_dev(vg_handle* h, const double* d_f, int batch, double* d_F) {
   const Grid& G = h->grid;
-  check_row(G);
   const dim3 grid(G.nlat, batch);
-  if (rows_fit(G.nphi, G.M, SHT_T)) {
+  const bool fit = rows_fit(G.nphi, G.M, SHT_T);
+  check_row(G.nphi, fit);
+  if (fit) {
     const size_t shm = rows_scratch(G.nphi, G.M, false) * sizeof(double);
     raise_smem_limit((const void*)k_fourier_analysis<false>, shm);
     k_fourier_analysis<false><<<grid, SHT_T, shm, h->stream>>>(d_f, G.nphi, G.nlat, G.M, G.d_cos.p, G.d_sin.p, d_F);

@@ -626,8 +626,8 @@ void sle_solve_dev(vg_handle* h, double dt, bool report_only) {
   // the closing load's spectrum (from the pass, unless that had no ocean) and the
   // memory advance (src/vilma_sle.f90:353-358)
   if (!closed) {
-    check_row(G);
-    const bool fit = rows_fit(nphi, M, SLE_THREADS);
+    const bool fit = rows_fit(nphi, M, SLE_THREADS, 32);  // (the block reduction's words)
+    check_row(nphi, fit);
     const size_t shm = (fit ? rows_scratch(nphi, M, false) : (size_t)nphi) * sizeof(double);
     const auto kernel = fit ? k_load_fourier<false> : k_load_fourier<true>;
     raise_smem_limit((const void*)kernel, shm);

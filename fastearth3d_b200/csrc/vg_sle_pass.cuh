@@ -372,17 +372,17 @@ inline size_t rows_scratch(int nphi, int M, bool sq) {
          (sq ? 8 : 4) * nbase;
 }
 constexpr size_t SMEM_CTA = 227 * 1024;  // shared memory that a CTA can have
-// whether the work area of rows fits beside the partial sums of T threads and a block reduction's words:
-// up to 6346 longitudes (5137 of an odd count, whose base longitudes are twice as many)
-inline bool rows_fit(int nphi, int M, int T) {
-  return (rows_scratch(nphi, M, false) + 4 * (size_t)T + 32) * sizeof(double) <= SMEM_CTA;
+// whether the work area of rows fits beside the partial sums of T threads and `more` doubles: up to 6354 longitudes
+// (5143 of an odd count, whose base longitudes are twice as many)
+inline bool rows_fit(int nphi, int M, int T, int more = 0) {
+  return (rows_scratch(nphi, M, false) + 4 * (size_t)T + more) * sizeof(double) <= SMEM_CTA;
 }
 
 // The analysis of a row that does not fit: the row alone in shared memory, all its longitudes by a thread per
 // order (longitudes up to LONG_ROW, 48 KB).
 constexpr int LONG_ROW = 6144;
-inline void check_row(const Grid& G) {
-  if (G.nphi > LONG_ROW) throw Error("longitude analysis: rows of more than 6144 longitudes are not supported");
+inline void check_row(int nphi, bool fit) {
+  if (!fit && nphi > LONG_ROW) throw Error("longitude analysis: rows of more than 6144 longitudes are not supported");
 }
 template <int T>
 __device__ __forceinline__ void long_row_analysis(const double* row, int nphi, int M, const double* __restrict__ cs,

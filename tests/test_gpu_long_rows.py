@@ -1,7 +1,7 @@
 """Rows of thousands of longitudes, at the edges of what the row transforms hold
-in shared memory: the analysis with odd and even counts up to its limit of
-6144, the closing load of a solve without an ocean, and the refusal past the
-limit; GPU = oracle to 1e-12 (transforms) and with test_gpu_parity.py's
+in shared memory: the analysis with odd and even counts up to its limits (6144,
+even counts as long as their tables fit), the closing load of a solve without an
+ocean, and the refusal past the limits; GPU = oracle to 1e-12 (transforms) and with test_gpu_parity.py's
 tolerances (solve)."""
 import numpy as np
 import pytest
@@ -25,14 +25,14 @@ def pair(*size):
     return model(vlib, vlib.Model, *size), model(orc, orc.Oracle, *size)
 
 
-@pytest.mark.parametrize("nphi", [5141, 5143, 6143, 6144])
+@pytest.mark.parametrize("nphi", [5141, 5143, 5145, 6143, 6144, 6146, 6354])
 def test_analysis_of_long_rows(nphi):
     g, o = pair(5, 6, nphi)
     f = np.random.default_rng(nphi).standard_normal(6 * nphi)
     assert rel(g.analysis(f), o.analysis(f)) < 1e-12
 
 
-@pytest.mark.parametrize("nphi", [5143, 6143])
+@pytest.mark.parametrize("nphi", [5143, 6143, 6346])
 def test_solve_without_an_ocean_on_long_rows(nphi):
     ms = pair(4, 5, nphi)
     lat = np.linspace(0.2, 2.9, 5)[:, None]
@@ -45,7 +45,7 @@ def test_solve_without_an_ocean_on_long_rows(nphi):
     check_models(*ms)
 
 
-@pytest.mark.parametrize("nphi", [6145, 6146, 9000])
+@pytest.mark.parametrize("nphi", [6145, 6356, 9000])
 def test_analysis_past_the_limit_is_refused(nphi):
     g = model(vlib, vlib.Model, 3, 4, nphi)
     with pytest.raises(vlib.VilmaError):
